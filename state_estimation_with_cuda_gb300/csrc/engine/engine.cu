@@ -366,8 +366,6 @@ void Engine::build_schedule(bool targets_ready) {
     n_pot_pairs_ = 0;
     sch_upd_.clear();
     sch_pot_ptr_.assign(1, 0);
-    sch_pan_ptr_.assign(1, 0);
-    sch_pan_.clear();
     sch_upd_ptr_.assign(1, 0);
     sch_tt_.clear();
     sch_tt_ptr_.assign(nl + 1, 0);
@@ -485,7 +483,7 @@ void Engine::build_schedule(bool targets_ready) {
         depth[s] = p >= 0 ? depth[p] + 1 : 0;
         if (flow_phase_[s] == 0) dmax = std::max(dmax, depth[s]);
     }
-    const int32_t per_panel = mixed_ ? 2 : 3;  // launches per panel step
+    const int32_t per_panel = 2;  // launches per panel step
     auto sync_cost = [&](bool by_depth) {
         std::vector<int32_t> pan(nl, 0);
         std::vector<char> has_small(nl, 0), has_big(nl, 0);
@@ -559,28 +557,22 @@ void Engine::build_schedule(bool targets_ready) {
             for (int32_t s : bigs) {
                 const int32_t f = P.sn_f[s], nc = P.sn_c0[s + 1] - P.sn_c0[s];
                 if (nc <= p * kTile) continue;
-                const int32_t tiles = (f + kTile - 1) / kTile;
                 const int32_t pb = std::min(kTile, nc - p * kTile);
                 const int32_t q0 = p * kTile + pb;
-                if (mixed_) {
-                    // one CTA per kPanelRows rows below the diagonal block
-                    const int32_t nch = std::max(1, (f - q0 + kPanelRows - 1) / kPanelRows);
-                    for (int32_t k = 0; k < nch; ++k) sch_pot_.push_back(make_int4(s, k, nch, n_pot_pairs_));
-                    pair_of[(static_cast<int64_t>(s) << 20) | p] = n_pot_pairs_;
-                    ++n_pot_pairs_;
-                } else {
-                    sch_pot_.push_back(make_int4(s, p, 0, 0));
-                }
-                if (!mixed_)  // FP64: the panel's row tiles below go to the multi-CTA solve
-                    for (int32_t ti = p + 1; ti < tiles; ++ti) sch_pan_.push_back(make_int4(s, ti, 0, 0));
+                // one CTA per chunk of rows below the diagonal block
+                const int32_t rows = mixed_ ? kPanelRows : kPanelRows64;
+                const int32_t nch = std::max(1, (f - q0 + rows - 1) / rows);
+                for (int32_t k = 0; k < nch; ++k) sch_pot_.push_back(make_int4(s, k, nch, n_pot_pairs_));
+                pair_of[(static_cast<int64_t>(s) << 20) | p] = n_pot_pairs_;
+                ++n_pot_pairs_;
                 if (q0 < f) {
-                    const int32_t ut = (f + kUpdTile - 1) / kUpdTile;
-                    for (int32_t tj = q0 / kUpdTile; tj < ut; ++tj)
+                    const int32_t edge = mixed_ ? kUpdTile : kUpdTile64;
+                    const int32_t ut = (f + edge - 1) / edge;
+                    for (int32_t tj = q0 / edge; tj < ut; ++tj)
                         for (int32_t ti = tj; ti < ut; ++ti) sch_upd_.push_back(make_int4(s, ti, tj, 0));
                 }
             }
             sch_pot_ptr_.push_back(static_cast<int32_t>(sch_pot_.size()));
-            sch_pan_ptr_.push_back(static_cast<int32_t>(sch_pan_.size()));
             sch_upd_ptr_.push_back(static_cast<int32_t>(sch_upd_.size()));
         }
         if (mixed_ && cfg.tile_flow && !bigs.empty()) build_tile_tasks(bigs, pair_of);
@@ -801,7 +793,6 @@ int32_t Engine::upload() {
         d_asm_child_ = c.take<AsmChild>(sch_asm_child_.size());
         d_pot_ = c.take<int4>(sch_pot_.size());
         d_pot_cnt_ = c.take<int32_t>(std::max(1, n_pot_pairs_));
-        d_pan_ = c.take<int4>(sch_pan_.size());
         d_upd_ = c.take<int4>(sch_upd_.size());
         d_tt_ = c.take<TileTask>(sch_tt_.size());
         d_tt_done_ = c.take<int32_t>(sch_tt_.size() + static_cast<size_t>(P.n_levels));
@@ -1001,7 +992,6 @@ int32_t Engine::upload() {
     chk(put(d_asm_, sch_asm_, st_));
     chk(put(d_asm_child_, sch_asm_child_, st_));
     chk(put(d_pot_, sch_pot_, st_));
-    chk(put(d_pan_, sch_pan_, st_));
     chk(put(d_upd_, sch_upd_, st_));
     chk(put(d_tt_, sch_tt_, st_));
     chk(put(d_flow_a_, sch_flow_a_, st_));
@@ -1057,8 +1047,6 @@ int32_t Engine::upload() {
     sched_.d_pot = d_pot_;
     sched_.d_pot_cnt = d_pot_cnt_;
     sched_.n_pot_pairs = n_pot_pairs_;
-    sched_.h_pan_ptr = sch_pan_ptr_.data();
-    sched_.d_pan = d_pan_;
     sched_.h_upd_ptr = sch_upd_ptr_.data();
     sched_.d_upd = d_upd_;
     sched_.h_all_ptr = sch_all_ptr_.data();

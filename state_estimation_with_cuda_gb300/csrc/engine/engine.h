@@ -268,8 +268,8 @@ private:
     LevelSchedule sched_{};
     // level schedule (host copies) and in-place storage layout
     std::vector<int32_t> sch_small_ptr_, sch_small_, sch_small_maxf_, sch_asm_ptr_, sch_panels_, sch_step_ptr_,
-        sch_pot_ptr_, sch_pan_ptr_, sch_upd_ptr_, sch_all_ptr_, sch_all_, sch_maxf_;
-    std::vector<int4> sch_pot_, sch_pan_, sch_upd_;
+        sch_pot_ptr_, sch_upd_ptr_, sch_all_ptr_, sch_all_, sch_maxf_;
+    std::vector<int4> sch_pot_, sch_upd_;
     std::vector<AsmItem> sch_asm_;
     std::vector<int2> ev_unit_, ev_grp_;  // evaluation units (DevNet::ev_unit / ev_grp)
     void build_eval_units();
@@ -303,7 +303,7 @@ private:
     int32_t* d_phase_nchild_ = nullptr;
     int32_t* d_nchild_ = nullptr;
     int32_t* d_ready_n_ = nullptr;               // [4] claim-list lengths
-    int32_t* d_pot_cnt_ = nullptr;               // FP32 tiled fronts: per (front, step) tile readers
+    int32_t* d_pot_cnt_ = nullptr;               // tiled fronts: per (front, step) tile readers
     TileTask* d_tt_ = nullptr;
     int32_t* d_tt_done_ = nullptr;
     int32_t n_pot_pairs_ = 0;
@@ -334,7 +334,6 @@ private:
     AsmItem* d_asm_ = nullptr;
     AsmChild* d_asm_child_ = nullptr;
     int4* d_pot_ = nullptr;
-    int4* d_pan_ = nullptr;
     int4* d_upd_ = nullptr;
     // targets_ready = false leaves the assembly items' target ranges to
     // fill_asm_targets(), for a schedule built before the gain targets exist.

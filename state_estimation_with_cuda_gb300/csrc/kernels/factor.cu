@@ -15,8 +15,8 @@
 // columns, update matrix = trailing block, both column-major with ld = f) and
 // are processed for a whole level at once by tile work lists: an assembly
 // kernel (one CTA per 32-column tile column, so every entry has one writer), a
-// panel kernel (each CTA factors the 32 x 32 diagonal tile and solves one row
-// tile against it) and a trailing-update kernel (one CTA per 32 x 32 tile).
+// panel kernel (each CTA factors the 32 x 32 diagonal tile and solves a chunk
+// of rows against it) and a trailing-update kernel (one CTA per tile).
 // The factor type T is double for the FP64 pipeline and float for the
 // mixed-precision one; the mixed pipeline forms the gain entries' sums in
 // float (gain_acc32, the default) or in double.
@@ -65,25 +65,47 @@ __device__ __forceinline__ bool front_frozen(const DevFactor& F, const DevWork& 
     return W.grid_flags && (W.grid_flags[F.sn_grid[s]] & FLAG_FROZEN);
 }
 
+// Positive and finite?  FP64 by the bit pattern: an FP64 comparison or
+// conversion occupies the FP64 pipe for 64 cycles, as any FP64 instruction.
+__device__ __forceinline__ bool pivot_ok(float d) { return d > 0.f && isfinite(d); }
+__device__ __forceinline__ bool pivot_ok(double d) {
+    const int hi = __double2hiint(d);
+    return hi < 0x7ff00000 && (hi > 0 || (hi == 0 && __double2loint(d) != 0));
+}
+
+// FP32 value of the leading bits of a positive d within the FP32 range (test
+// first), and the FP64 value of a positive FP32 one, by their bits.
+__device__ __forceinline__ bool in_fp32_range(double d) {
+    return static_cast<unsigned>((__double2hiint(d) >> 20) - (1023 - 100)) < 200u;
+}
+__device__ __forceinline__ float leading_fp32(double d) {
+    return __uint_as_float((static_cast<unsigned>(__double2hiint(d) - ((1023 - 127) << 20)) << 3) |
+                           (static_cast<unsigned>(__double2loint(d)) >> 29));
+}
+__device__ __forceinline__ double widen_fp32(float y) {
+    const unsigned b = __float_as_uint(y);
+    return __hiloint2double(static_cast<int>((b >> 3) + ((1023u - 127u) << 20)), static_cast<int>(b << 29));
+}
+
 // Pivot: L_kk = sqrt(d) and 1 / L_kk for a positive finite d (the callers
 // flag a non-positive or non-finite d as a matrix that is not positive
-// definite and go on with 1).  FP64: a reciprocal square root seeded in FP32
-// and refined by two Newton-Raphson steps y <- y (3 - d y^2) / 2 (each step
-// doubles the correct bits: ~24 -> 48 -> 96), which keeps serial FP64 work
-// short on a GPU with few FP64 units; the library routines are used outside
-// the FP32 range.
+// definite and go on with 1).  FP64: an FP32 reciprocal square root refined by
+// one third-order Newton (Householder) step, y (1 + e / 2 + 3 e^2 / 8) with
+// e = 1 - d y^2 (2^-22 -> 2^-66, then rounding): five FP64 instructions on
+// the chain where two second-order steps take eight; the library routines are
+// used outside the FP32 range.
 __device__ __forceinline__ void pivot_value(float d, float* sq, float* inv) {
     const float y = rsqrtf(d);  // the FP32 factor is a preconditioner of FP64 steps
     *sq = d * y;
     *inv = y;
 }
 __device__ __forceinline__ void pivot_value(double d, double* sq, double* inv) {
-    if (d > 1e-30 && d < 1e30) {
-        double y = static_cast<double>(rsqrtf(static_cast<float>(d)));
-        y = y * (1.5 - 0.5 * d * y * y);
-        y = y * (1.5 - 0.5 * d * y * y);
-        *sq = d * y;
-        *inv = y;
+    if (in_fp32_range(d)) {
+        const double y = widen_fp32(rsqrtf(leading_fp32(d)));
+        const double e = fma(-(d * y), y, 1.0);
+        const double z = fma(y * e, fma(0.375, e, 0.5), y);
+        *sq = d * z;
+        *inv = z;
     } else {
         *sq = sqrt(d);
         *inv = 1.0 / *sq;
@@ -235,8 +257,9 @@ __device__ __forceinline__ bool warp_potrf_bcast(float (&a)[KP], int kb, int lan
     for (int k = 0; k < KP; ++k) {
         if (k < kb) {
             float d = __shfl_sync(0xffffffffu, a[k], k);
-            bad |= !(d > 0.f) || !isfinite(d);
-            d = (d > 0.f && isfinite(d)) ? d : 1.f;
+            const bool ok = pivot_ok(d);
+            bad |= !ok;
+            d = ok ? d : 1.f;
             float sq, inv;
             pivot_value(d, &sq, &inv);
             const float lk = (lane == k) ? sq : (lane > k ? a[k] * inv : a[k]);
@@ -301,8 +324,9 @@ __device__ __forceinline__ bool warp_potrf_bcast(double (&a)[KP], int kb, int la
     for (int k = 0; k < KP; ++k) {
         if (k < kb) {
             double d = __shfl_sync(0xffffffffu, a[k], k);
-            bad |= !(d > 0.0) || !isfinite(d);
-            d = (d > 0.0 && isfinite(d)) ? d : 1.0;
+            const bool ok = pivot_ok(d);
+            bad |= !ok;
+            d = ok ? d : 1.0;
             double sq, inv;
             pivot_value(d, &sq, &inv);
             const double lk = (lane == k) ? sq : (lane > k ? a[k] * inv : a[k]);
@@ -421,7 +445,7 @@ __device__ void warp_front_factor(const DevFactor& F, const DevWork& W, const T*
     bool bad = false;
     for (int k = 0; k < nc; ++k) {
         T d = t.a[k * kWtLd + k];
-        const bool badk = !(d > T(0)) || !isfinite(d);
+        const bool badk = !pivot_ok(d);
         bad |= badk;
         d = badk ? T(1) : d;
         T sq, inv;
@@ -788,69 +812,193 @@ __global__ void __launch_bounds__(kThreads) k_big_assemble(DevFactor F, DevWork 
     }
 }
 
-// FP64 panel step p, part 1 (one CTA per front): warp 0 factors the diagonal
-// tile with a row per lane in registers (warp_potrf_bcast) and writes L_dd
-// back; the other warps solve the rows of tile p below the block (only a last
-// block narrower than a tile has any: x = a L_dd^-T by forward substitution in
-// registers; volatile reads keep the compiler from hoisting the factor into
-// registers across rows).  k_big_trsm takes the row tiles below on many CTAs;
-// then the trailing update.
-template <typename T>
-__global__ void __launch_bounds__(kThreads) k_big_potrf(DevFactor F, DevWork W, T* lx, const int4* work, int p) {
-    static_assert(sizeof(T) == 8, "FP32 panels use k_big_panel32");
-    constexpr int ld = kTile + 1;
-    __shared__ T D[kTile * ld];
-    __shared__ T rdiag[kTile];
-    __shared__ __align__(16) T colbuf[kTile];
-    const int s = work[blockIdx.x].x;
-    if (front_frozen(F, W, s)) return;  // the whole CTA, before any barrier
-    const int f = F.sn_f[s];
-    const int nc = F.sn_c0[s + 1] - F.sn_c0[s];
-    T* B = lx + F.sn_lx_off[s];
-    const int p0 = p * kTile;
-    const int pb = min(kTile, nc - p0);
-    if (threadIdx.x < 32) {
-        // warp 0: the diagonal block, row i in lane i's registers
-        const int i = threadIdx.x;
-        T a[kTile];
-#pragma unroll
-        for (int j = 0; j < kTile; ++j) a[j] = (i < pb && j <= i) ? B[(p0 + i) + (int64_t)(p0 + j) * f] : T(0);
-        T inv;
-        const bool bad = warp_potrf_bcast<kTile>(a, pb, i, &inv, colbuf);
-        if (bad && i == 0) atomicOr(singular_flags(F, W, s), FLAG_SINGULAR);
-#pragma unroll
-        for (int j = 0; j < kTile; ++j)
-            if (i < pb && j <= i) {
-                D[i + j * ld] = a[j];
-                B[(p0 + i) + (int64_t)(p0 + j) * f] = a[j];
-            }
-        if (i < pb) {
-            rdiag[i] = inv;
-            reinterpret_cast<T*>(W.rdiag)[F.sn_c0[s] + p0 + i] = inv;
+// 1 / d of a pivot, by the same means (y (1 + e + e^2), e = 1 - d y); a d
+// that is not positive and finite is replaced by 1 and reported.
+__device__ __forceinline__ double pivot_recip(double& d, bool& bad) {
+    if (in_fp32_range(d)) {
+        float yf;
+        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(yf) : "f"(leading_fp32(d)));
+        const double y = widen_fp32(yf);
+        const double e = fma(-d, y, 1.0);
+        return fma(y, fma(e, e, e), y);
+    }
+    if (!pivot_ok(d)) {
+        bad = true;
+        d = 1.0;
+    }
+    return 1.0 / d;
+}
+
+// Column counters of an elimination within one CTA: a column's owner raises
+// the counter after writing the column to shared memory, the other warps wait
+// for it (the CTA's warps are all resident, so the owner always runs; the wait
+// is bounded all the same).
+__device__ __forceinline__ void wait_column(int* ready, int k, uint32_t* status) {
+    const unsigned at = static_cast<unsigned>(__cvta_generic_to_shared(ready));
+    for (int spins = 0;; ++spins) {
+        int v;
+        asm volatile("ld.acquire.cta.shared.b32 %0, [%1];" : "=r"(v) : "r"(at) : "memory");
+        if (v >= k) break;
+        if (spins > (1 << 22)) {
+            atomicOr(status, FLAG_TIMEOUT);
+            break;
         }
     }
+    __syncwarp();
+}
+__device__ __forceinline__ void post_column(int* ready, int k) {
+    __syncwarp();
+    if ((threadIdx.x & 31) == 0) {
+        const unsigned at = static_cast<unsigned>(__cvta_generic_to_shared(ready));
+        asm volatile("st.release.cta.shared.b32 [%0], %1;" ::"r"(at), "r"(k) : "memory");
+    }
+}
+
+// Hand-over of one column between two warps on the chain, by a named barrier
+// of 64 threads (about 35 cycles; the counter above takes about 140).
+__device__ __forceinline__ void hand_over(int k) {
+    asm volatile("bar.arrive %0, 64;" ::"r"(1 + (k & 7)) : "memory");
+}
+__device__ __forceinline__ void take_over(int k) { asm volatile("bar.sync %0, 64;" ::"r"(1 + (k & 7)) : "memory"); }
+
+// FP64 panel step p of the tiled fronts: the diagonal block's factorisation
+// and the rows below it, one CTA per kPanelRows64 rows (each factors the
+// block itself; the CTA that reads the block last writes it back, so no CTA
+// reads an overwritten block and none waits for another).
+//
+// Bound: an FP64 warp instruction takes 64 cycles of its scheduler however
+// many lanes are active, so what counts is FP64 instructions per scheduler and
+// the serial chain of a pivot.  Hence: eight warps, two per scheduler (one
+// waits while the other issues; four warps took 45k cycles, eight 34k), each
+// owning the columns c = warp (mod 8) of the block (a lane per row) and of the
+// chunk (two columns of 16 rows per instruction); the elimination is
+// a_ij -= u_i (u_j / d) with the unscaled column u, so the chain holds a
+// reciprocal (3 FP64 instructions) instead of a square root (10), and the
+// square roots of all pivots are taken together, a lane each, at the end.
+// The owner of column k + 1 updates and publishes that column before its
+// others, and warps wait for columns, not for each other.  The chunk follows
+// one column behind the block, off the chain of the pivots.  Measured: a full
+// step in about 37k cycles (18 us), where one warp's factorisation of the block
+// and a launch of one-warp row solves took 47 + 22 us; the linear solve of a
+// 30k-bus grid went from 5.04 to 3.08 ms with this and k_big_update64.
+__global__ void __launch_bounds__(kPanelThreads64) k_big_panel64(DevFactor F, DevWork W, double* lx, const int4* work,
+                                                                 int p, int* step_cnt) {
+    static_assert(kPanelThreads64 == 256 && kPanelRows64 == 16 && kTile == 32, "thread tiling below");
+    constexpr int kW = kPanelThreads64 / 32, kQ = kTile / kW;  // columns per warp
+    __shared__ double us[kTile][kTile + kPanelRows64];  // column k: block rows, then chunk rows
+    __shared__ double ms[kTile][kTile];                 // u / d
+    __shared__ double dk[kTile];                        // pivots, then 1 / sqrt
+    __shared__ int ready, ready_x, last;            // columns published: block, chunk
+    const int4 wk = work[blockIdx.x];
+    const int s = wk.x, chunk = wk.y;
+    if (front_frozen(F, W, s)) return;  // the whole CTA, before any barrier
+    const int f = F.sn_f[s];
+    const int c0 = F.sn_c0[s];
+    const int nc = F.sn_c0[s + 1] - c0;
+    double* B = lx + F.sn_lx_off[s];
+    const int p0 = p * kTile;
+    const int pb = min(kTile, nc - p0);
+    const int r0 = p0 + pb + chunk * kPanelRows64;
+    const int nr = min(kPanelRows64, f - r0);  // <= 0: no rows below the block
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int xr = lane & (kPanelRows64 - 1), xh = lane >> 4;
+    if (threadIdx.x == 0) ready = ready_x = -1;
+    double a[kQ], x[kQ / 2];  // columns w + kW q; chunk columns w + kW (2 h + xh)
+#pragma unroll
+    for (int q = 0; q < kQ; ++q) {
+        const int c = w + kW * q;
+        a[q] = (c < pb && lane >= c && lane < pb) ? B[(p0 + lane) + (int64_t)(p0 + c) * f] : 0.0;
+    }
+#pragma unroll
+    for (int h = 0; h < kQ / 2; ++h) {
+        const int c = w + kW * (2 * h + xh);
+        x[h] = (c < pb && xr < nr) ? B[(r0 + xr) + (int64_t)(p0 + c) * f] : 0.0;
+    }
     __syncthreads();
-    if (threadIdx.x >= 32) {
-        // the rows of tile p below the block (a last block narrower than a
-        // tile): x = a L_dd^-T by forward substitution in registers
-        const volatile T* Dv = D;
-        const int r_end = min(p0 + kTile, f);
+    bool bad = false;
+    uint32_t* status = &W.status->flags;
+    // column k of this warp's block rows is final: its pivot, u and u / d
+    auto publish = [&](double& aq, int k) {
+        double d = __shfl_sync(0xffffffffu, aq, k);
+        us[k][lane] = aq;
+        ms[k][lane] = aq * pivot_recip(d, bad);
+        if (k + 1 < pb) hand_over(k);
+        if (lane == k) aq = d;
+        if (lane == 0) dk[k] = d;
+        post_column(&ready, k);
+    };
+    if (w == 0) publish(a[0], 0);
+#pragma unroll
+    for (int qq = 0; qq < kQ; ++qq) {
 #pragma unroll 1
-        for (int r = p0 + pb + threadIdx.x - 32; r < r_end; r += blockDim.x - 32) {
-            T x[kTile];
-#pragma unroll
-            for (int c = 0; c < kTile; ++c) x[c] = (c < pb) ? B[r + (int64_t)(p0 + c) * f] : T(0);
-#pragma unroll
-            for (int c = 0; c < kTile; ++c) {
-                if (c < pb) {
-                    x[c] *= rdiag[c];
-#pragma unroll
-                    for (int c2 = c + 1; c2 < kTile; ++c2) x[c2] -= x[c] * Dv[c2 + c * ld];
+        for (int kk = 0; kk < kW; ++kk) {
+            const int k = kW * qq + kk;
+            if (k >= pb) break;
+            const bool next = w == ((kk + 1) & (kW - 1)) && k + 1 < pb;
+            if (next) take_over(k);
+            else wait_column(&ready, k, status);
+            const double ub = us[k][lane];
+            int done = k;  // block columns up to here are final or updated
+            if (next) {
+                // the owner of column k + 1: q = qq, or qq + 1 past the group's end
+                const double m = ms[k][k + 1];
+                if (kk + 1 < kW) {
+                    a[qq] = fma(-ub, m, a[qq]);
+                    publish(a[qq], k + 1);
+                } else if (qq + 1 < kQ) {
+                    const int qn = qq + 1 < kQ ? qq + 1 : kQ - 1;
+                    a[qn] = fma(-ub, m, a[qn]);
+                    publish(a[qn], k + 1);
                 }
+                done = k + 1;
             }
 #pragma unroll
-            for (int c = 0; c < kTile; ++c)
-                if (c < pb) B[r + (int64_t)(p0 + c) * f] = x[c];
+            for (int q = qq; q < kQ; ++q) {
+                const int c = w + kW * q;
+                if (c > done && c < pb) a[q] = fma(-ub, ms[k][c], a[q]);
+            }
+            // the chunk's columns behind k - 1 by column k - 1; column k is then final
+            if (k > 0) {
+                wait_column(&ready_x, k - 1, status);
+                const double uc = us[k - 1][kTile + xr];
+#pragma unroll
+                for (int h = qq / 2; h < kQ / 2; ++h) {
+                    const int c = w + kW * (2 * h + xh);
+                    if (w + kW * (2 * h + 1) >= k) {
+                        const double xn = fma(-uc, ms[k - 1][c], x[h]);
+                        if (c >= k) x[h] = xn;
+                    }
+                    if (h == qq / 2 && w == kk) {
+                        if (xh == (qq & 1)) us[k][kTile + xr] = x[h];
+                        post_column(&ready_x, k);
+                    }
+                }
+            } else if (w == 0) {
+                if (xh == 0) us[0][kTile + xr] = x[0];
+                post_column(&ready_x, 0);
+            }
+        }
+    }
+    __syncthreads();  // every pivot is in dk; this CTA's reads of the block are long done
+    if (threadIdx.x == 0) last = atomicAdd(step_cnt + wk.w, 1) == wk.z - 1;
+    if (bad && lane == 0 && chunk == 0) atomicOr(singular_flags(F, W, s), FLAG_SINGULAR);
+    if (w == 0 && lane < pb) {
+        double sq, rs;
+        pivot_value(dk[lane], &sq, &rs);
+        dk[lane] = rs;
+        if (chunk == 0) reinterpret_cast<double*>(W.rdiag)[c0 + p0 + lane] = rs;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int h = 0; h < kQ / 2; ++h) {
+        const int c = w + kW * (2 * h + xh);
+        if (c < pb && xr < nr) B[(r0 + xr) + (int64_t)(p0 + c) * f] = x[h] * dk[c];
+    }
+    if (last) {
+#pragma unroll
+        for (int q = 0; q < kQ; ++q) {
+            const int c = w + kW * q;
+            if (c < pb && lane >= c && lane < pb) B[(p0 + lane) + (int64_t)(p0 + c) * f] = a[q] * dk[c];
         }
     }
 }
@@ -987,62 +1135,17 @@ __global__ void __launch_bounds__(kThreads) k_big_panel32(DevFactor F, DevWork W
     big_panel32_item<false>(F, W, lx, wk.x, p, wk.y, wk.z, wk.w, step_cnt);
 }
 
-// FP64 panel step p, part 2: X = A L_dd^-T for the row tiles ti > p, spread
-// over CTAs (one SM's FP64 rate cannot carry a whole panel).  One warp per
-// row tile and one lane per row, forward substitution in registers against
-// the diagonal tile staged in shared memory.
-template <typename T>
-constexpr int kTrsmWarps = sizeof(T) == 4 ? 8 : 4;
-
-template <typename T>
-__global__ void __launch_bounds__(32 * kTrsmWarps<T>) k_big_trsm(DevFactor F, DevWork W, T* lx, const int4* work,
-                                                                 int n_work, int p) {
-    __shared__ T lt[kTrsmWarps<T>][kTile][kTile + 1];  // lt[w][c][r] = L_dd[r][c]
-    __shared__ T rinv[kTrsmWarps<T>][kTile];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int item = blockIdx.x * kTrsmWarps<T> + warp;
-    if (item >= n_work) return;  // the whole warp; no block barrier follows
-    const int4 wk = work[item];
-    const int s = wk.x, ti = wk.y;
-    if (front_frozen(F, W, s)) return;  // the whole warp
-    const int f = F.sn_f[s];
-    const int nc = F.sn_c0[s + 1] - F.sn_c0[s];
-    T* B = lx + F.sn_lx_off[s];
-    const int p0 = p * kTile;
-    const int pb = min(kTile, nc - p0);
-    for (int c = 0; c < pb; ++c)
-        lt[warp][c][lane] = (lane < pb && lane > c) ? B[(p0 + lane) + (int64_t)(p0 + c) * f] : T(0);
-    if (lane < pb) rinv[warp][lane] = reinterpret_cast<const T*>(W.rdiag)[F.sn_c0[s] + p0 + lane];
-    __syncwarp();
-    const int r = ti * kTile + lane;
-    if (r < f) {
-        T x[kTile];
-#pragma unroll
-        for (int c = 0; c < kTile; ++c) x[c] = (c < pb) ? B[r + (int64_t)(p0 + c) * f] : T(0);
-#pragma unroll
-        for (int c = 0; c < kTile; ++c) {
-            if (c < pb) {
-                x[c] *= rinv[warp][c];
-#pragma unroll
-                for (int c2 = c + 1; c2 < kTile; ++c2) x[c2] -= x[c] * lt[warp][c][c2];
-            }
-        }
-#pragma unroll
-        for (int c = 0; c < kTile; ++c)
-            if (c < pb) B[r + (int64_t)(p0 + c) * f] = x[c];
-    }
-}
-
-// Trailing update of step p: the kUpdTile x kUpdTile tile (ti, tj) -= A_i A_j^T
+// FP32 trailing update of step p: the kUpdTile x kUpdTile tile (ti, tj) -= A_i A_j^T
 // over the panel's columns, restricted to rows >= cols >= p0 + pb.  The two
 // row blocks of the panel are staged k-major in shared memory; thread
 // (tr, tc) accumulates rows tr + 16u and columns tc + 16v (u, v < 2) in
 // registers, four shared loads per four FMAs (a thread per output needed
 // two per FMA), and its read-modify-writes of a column touch 16 consecutive
 // rows per half warp.
-template <typename T, bool kL2>
-__device__ __forceinline__ void big_update_item(const DevFactor& F, const DevWork& W, T* lx, int s, int p, int ti,
+template <bool kL2>
+__device__ __forceinline__ void big_update_item(const DevFactor& F, const DevWork& W, float* lx, int s, int p, int ti,
                                                 int tj) {
+    using T = float;
     static_assert(kThreads == 256 && kUpdTile == 32, "thread tiling below");
     constexpr int ld = kUpdTile + 1;
     __shared__ T Ai[kTile * ld];  // Ai[k * ld + r] = A(R0 + r, p0 + k)
@@ -1083,52 +1186,85 @@ __device__ __forceinline__ void big_update_item(const DevFactor& F, const DevWor
             if (gr >= gc && gr < f) dst[gr] = ld_entry<kL2>(dst + gr) - acc[u][v];
         }
     }
-    if constexpr (sizeof(T) == 4) {
-        // Look-ahead (FP32 tiled fronts): the tile that is the next step's
-        // diagonal block comes first in the step's work list; after its own
-        // update its CTA factors the block (L_dd) and inverts it in warp 0
-        // while the step's other tiles are still updating, and leaves L_dd^-1
-        // in the block's slot, the pivots' reciprocals in rdiag and the pivot
-        // check done, so that the next panel step only applies L_dd^-1.  The
-        // arithmetic is that of the panel kernel's own factorisation.
-        if (ti == tj && R0 == q0 && q0 < nc) {
-            constexpr int dld = kTile + 4, lt_ld = kTile + 4;  // 16-byte aligned rows
-            __shared__ __align__(16) float D[kTile * dld];
-            __shared__ float rdiag[kTile];
-            __shared__ float Lt[kTile * lt_ld];
-            __shared__ __align__(16) float colbuf[kTile];
-            __syncthreads();  // every update of this tile is written
-            const int pb2 = min(kTile, nc - q0);
-            if (threadIdx.x < 32) {
-                const int i = threadIdx.x;
-                float a[kTile];
+    // Look-ahead (FP32 tiled fronts): the tile that is the next step's
+    // diagonal block comes first in the step's work list; after its own
+    // update its CTA factors the block (L_dd) and inverts it in warp 0
+    // while the step's other tiles are still updating, and leaves L_dd^-1
+    // in the block's slot, the pivots' reciprocals in rdiag and the pivot
+    // check done, so that the next panel step only applies L_dd^-1.  The
+    // arithmetic is that of the panel kernel's own factorisation.
+    if (ti == tj && R0 == q0 && q0 < nc) {
+        constexpr int dld = kTile + 4, lt_ld = kTile + 4;  // 16-byte aligned rows
+        __shared__ __align__(16) float D[kTile * dld];
+        __shared__ float rdiag[kTile];
+        __shared__ float Lt[kTile * lt_ld];
+        __shared__ __align__(16) float colbuf[kTile];
+        __syncthreads();  // every update of this tile is written
+        const int pb2 = min(kTile, nc - q0);
+        if (threadIdx.x < 32) {
+            const int i = threadIdx.x;
+            float a[kTile];
 #pragma unroll
-                for (int j = 0; j < kTile; ++j)
-                    a[j] = (i < pb2 && j <= i) ? ld_entry<kL2>(B + (q0 + i) + (int64_t)(q0 + j) * f) : 0.f;
-                float inv;
-                const bool bad = warp_potrf_bcast<kTile>(a, pb2, i, &inv, colbuf);
-                if (bad && i == 0) atomicOr(singular_flags(F, W, s), FLAG_SINGULAR);
+            for (int j = 0; j < kTile; ++j)
+                a[j] = (i < pb2 && j <= i) ? ld_entry<kL2>(B + (q0 + i) + (int64_t)(q0 + j) * f) : 0.f;
+            float inv;
+            const bool bad = warp_potrf_bcast<kTile>(a, pb2, i, &inv, colbuf);
+            if (bad && i == 0) atomicOr(singular_flags(F, W, s), FLAG_SINGULAR);
 #pragma unroll
-                for (int j = 0; j < kTile; ++j) D[i + j * dld] = (i < pb2 && j <= i) ? a[j] : 0.f;
-                if (i < pb2) {
-                    rdiag[i] = inv;
-                    reinterpret_cast<float*>(W.rdiag)[F.sn_c0[s] + q0 + i] = inv;
-                }
-                __syncwarp();
-                warp_trinv_v4<kTile, dld>(reinterpret_cast<const float (*)[dld]>(D), rdiag, pb2, i, Lt, lt_ld);
-                __syncwarp();
-                for (int c = 0; c < pb2; ++c)
-                    if (i >= c && i < pb2) B[(q0 + i) + (int64_t)(q0 + c) * f] = Lt[c * lt_ld + i];
+            for (int j = 0; j < kTile; ++j) D[i + j * dld] = (i < pb2 && j <= i) ? a[j] : 0.f;
+            if (i < pb2) {
+                rdiag[i] = inv;
+                reinterpret_cast<float*>(W.rdiag)[F.sn_c0[s] + q0 + i] = inv;
             }
+            __syncwarp();
+            warp_trinv_v4<kTile, dld>(reinterpret_cast<const float (*)[dld]>(D), rdiag, pb2, i, Lt, lt_ld);
+            __syncwarp();
+            for (int c = 0; c < pb2; ++c)
+                if (i >= c && i < pb2) B[(q0 + i) + (int64_t)(q0 + c) * f] = Lt[c * lt_ld + i];
         }
     }
 }
 
-template <typename T>
-__global__ void __launch_bounds__(kThreads) k_big_update(DevFactor F, DevWork W, T* lx, const int4* work, int p) {
+__global__ void __launch_bounds__(kThreads) k_big_update32(DevFactor F, DevWork W, float* lx, const int4* work, int p) {
     const int4 wk = work[blockIdx.x];
     if (front_frozen(F, W, wk.x)) return;  // the whole CTA, before any barrier
-    big_update_item<T, false>(F, W, lx, wk.x, p, wk.y, wk.z);
+    big_update_item<false>(F, W, lx, wk.x, p, wk.y, wk.z);
+}
+
+// FP64 trailing update of step p, one CTA per kUpdTile64 x kUpdTile64 tile
+// and one entry per thread.  Bound: FP64 issue (two FMAs a cycle per SM), so
+// the tile is small: a 32 x 32 tile kept its SM for 16k cycles while a step
+// of a single grid has fewer such tiles than the GPU has SMs (30k-bus grid:
+// 12.5 us a step with 32 x 32 tiles, 5.8 us with 16 x 16).
+__global__ void __launch_bounds__(kUpdTile64 * kUpdTile64) k_big_update64(DevFactor F, DevWork W, double* lx,
+                                                                          const int4* work, int p) {
+    constexpr int kN = kUpdTile64, kAll = kN * kN;
+    __shared__ double Ai[kTile][kN + 1], Aj[kTile][kN + 1];  // [k][row]
+    const int4 wk = work[blockIdx.x];
+    const int s = wk.x;
+    if (front_frozen(F, W, s)) return;  // the whole CTA, before any barrier
+    const int f = F.sn_f[s];
+    const int nc = F.sn_c0[s + 1] - F.sn_c0[s];
+    double* B = lx + F.sn_lx_off[s];
+    const int p0 = p * kTile;
+    const int pb = min(kTile, nc - p0);
+    const int q0 = p0 + pb;
+    const int R0 = wk.y * kN, C0 = wk.z * kN;
+    const int tr = threadIdx.x % kN, tc = threadIdx.x / kN;
+    const int gr = R0 + tr, gc = C0 + tc;
+    const bool mine = gc >= q0 && gc < f && gr >= gc && gr < f;
+    double* dst = B + gr + (int64_t)gc * f;
+    double acc = mine ? *dst : 0.0;
+#pragma unroll
+    for (int k = tc; k < kTile; k += kAll / kN) {
+        const double* col = B + (int64_t)(p0 + k) * f;
+        Ai[k][tr] = (k < pb && R0 + tr < f) ? col[R0 + tr] : 0.0;
+        Aj[k][tr] = (k < pb && C0 + tr < f) ? col[C0 + tr] : 0.0;
+    }
+    __syncthreads();
+#pragma unroll 8
+    for (int k = 0; k < pb; ++k) acc = fma(-Ai[k][tr], Aj[k][tc], acc);
+    if (mine) *dst = acc;
 }
 
 // Bounded wait of the tiled-front dataflow (one lane per dependency): true
@@ -1208,7 +1344,7 @@ __global__ void __launch_bounds__(kThreads, kTileFlowBlocks)
             if (t.kind == 0)
                 big_panel32_item<true>(F, W, lx, t.s, t.p, t.a, t.b, t.aux, step_cnt);
             else
-                big_update_item<float, true>(F, W, lx, t.s, t.p, t.a, t.b);
+                big_update_item<true>(F, W, lx, t.s, t.p, t.a, t.b);
         }
         __syncthreads();
         if (tid == 0) publish_done(done + item);
@@ -1810,7 +1946,7 @@ cudaError_t factor_impl(const DevNet& net, const DevFactor& F, const DevWork& W,
             count_launches(1);
         }
     }
-    if (sizeof(T) == 4 && ls.n_pot_pairs > 0) {
+    if (ls.n_pot_pairs > 0) {
         cudaError_t e = cudaMemsetAsync(ls.d_pot_cnt, 0, sizeof(int) * (size_t)ls.n_pot_pairs, st);
         if (e != cudaSuccess) return e;
     }
@@ -1845,23 +1981,19 @@ cudaError_t factor_impl(const DevNet& net, const DevFactor& F, const DevWork& W,
                 const int npot = ls.h_pot_ptr[slot + 1] - ls.h_pot_ptr[slot];
                 const int nupd = ls.h_upd_ptr[slot + 1] - ls.h_upd_ptr[slot];
                 if (npot > 0) {
+                    const int4* work = ls.d_pot + ls.h_pot_ptr[slot];
                     if constexpr (sizeof(T) == 4)
-                        k_big_panel32<<<npot, kThreads, 0, st>>>(F, W, lx, ls.d_pot + ls.h_pot_ptr[slot], p,
-                                                                 ls.d_pot_cnt);
+                        k_big_panel32<<<npot, kThreads, 0, st>>>(F, W, lx, work, p, ls.d_pot_cnt);
                     else
-                        k_big_potrf<T><<<npot, kThreads, 0, st>>>(F, W, lx, ls.d_pot + ls.h_pot_ptr[slot], p);
+                        k_big_panel64<<<npot, kPanelThreads64, 0, st>>>(F, W, lx, work, p, ls.d_pot_cnt);
                     count_launches(1);
                 }
-                if constexpr (sizeof(T) == 8) {
-                    const int npan = ls.h_pan_ptr[slot + 1] - ls.h_pan_ptr[slot];
-                    if (npan > 0) {
-                        k_big_trsm<T><<<(npan + kTrsmWarps<T> - 1) / kTrsmWarps<T>, 32 * kTrsmWarps<T>, 0, st>>>(
-                            F, W, lx, ls.d_pan + ls.h_pan_ptr[slot], npan, p);
-                        count_launches(1);
-                    }
-                }
                 if (nupd > 0) {
-                    k_big_update<T><<<nupd, kThreads, 0, st>>>(F, W, lx, ls.d_upd + ls.h_upd_ptr[slot], p);
+                    const int4* work = ls.d_upd + ls.h_upd_ptr[slot];
+                    if constexpr (sizeof(T) == 4)
+                        k_big_update32<<<nupd, kThreads, 0, st>>>(F, W, lx, work, p);
+                    else
+                        k_big_update64<<<nupd, kUpdTile64 * kUpdTile64, 0, st>>>(F, W, lx, work, p);
                     count_launches(1);
                 }
             }

@@ -288,11 +288,9 @@ struct LevelSchedule {
     const int32_t* h_lvl_panels = nullptr;  // [n_levels] panel steps of the level
     const int32_t* h_step_ptr = nullptr;    // [n_levels+1] first step slot of a level
     const int32_t* h_pot_ptr = nullptr;     // [n_slots+1] offsets into d_pot
-    const int4* d_pot = nullptr;            // FP64: (big front); FP32: (big front, chunk, chunks, step pair)
-    int32_t* d_pot_cnt = nullptr;           // FP32: [n_pot_pairs] CTAs of a (front, step) done reading its tile
+    const int4* d_pot = nullptr;            // (big front, chunk, chunks, step pair)
+    int32_t* d_pot_cnt = nullptr;           // [n_pot_pairs] CTAs of a (front, step) done reading its diagonal tile
     int32_t n_pot_pairs = 0;
-    const int32_t* h_pan_ptr = nullptr;     // [n_slots+1] offsets into d_pan (FP64 only)
-    const int4* d_pan = nullptr;            // (big front, row tile below the panel)
     const int32_t* h_upd_ptr = nullptr;     // [n_slots+1] offsets into d_upd
     const int4* d_upd = nullptr;            // (big front, row tile, column tile)
     // FP32 tiled fronts as dataflow items, one persistent launch per level
@@ -429,11 +427,14 @@ cudaError_t launch_factor_solve_noalloc(const DevNet& net, const DevFactor& F, c
 constexpr int kTile = 32;
 // Rows per CTA of the FP32 panel solve of a tiled front.
 constexpr int kPanelRows = 128;
+// Rows and threads per CTA of the FP64 panel step (k_big_panel64).
+constexpr int kPanelRows64 = 16;
+constexpr int kPanelThreads64 = 256;
 // Rows per CTA of a tiled front's assembly (one CTA per tile column and row block).
 constexpr int kAsmRows = 128;
-// Edge of the trailing-update tiles of a tiled front (one CTA each; 64 left a
-// single grid's step on too few SMs: grid200k FP64 179 -> 203 ms).
+// Edge of the trailing-update tiles of a tiled front, FP32 and FP64 (one CTA each).
 constexpr int kUpdTile = 32;
+constexpr int kUpdTile64 = 16;
 
 // Sets the kernel attributes (dynamic shared memory limits) on the current
 // device; call before launching or capturing the factorisation.
