@@ -188,7 +188,8 @@ __device__ __forceinline__ void extend_add_children(const DevFactor& F, const T*
 //
 // Layout: column-major with a leading dimension padded to 16 bytes
 // (front_ld), so four consecutive rows of a column are one or two aligned
-// vector loads.  The partial factorisation runs over 32-column panels:
+// vector loads.  The FP32 partial factorisation runs over panels (FP64: see
+// front_factor):
 //   (1) warp 0 factors the diagonal block in registers (lane i holds row i,
 //       columns broadcast by shuffles) and leaves L11^T and 1/diag in shared
 //       memory;
@@ -232,13 +233,13 @@ __device__ __forceinline__ void store4<double>(double* p, const double (&v)[4]) 
 template <typename T>
 constexpr bool kInvDiag = sizeof(T) == 4;
 
-// Diagonal blocks in one warp's registers.  warp_potrf_bcast eliminates the
+// FP32 diagonal blocks in one warp's registers.  warp_potrf_bcast eliminates the
 // first kb columns of the rows the warp holds: lane i owns row i in a[]
 // (entries j <= i; zeros elsewhere); the remaining columns receive the Schur
 // complement update.  Per pivot k the pivot comes by shuffle, lanes below
 // scale their entry by 1 / L_kk, and every entry a_ij, k < j <= i, gets
 // a_ij -= l_ik l_jk, the column l_jk broadcast through the 16-byte-aligned
-// shared buffer col[] (four FP32 or two FP64 entries per load).  Entries
+// shared buffer col[] (four entries per load).  Entries
 // above the diagonal are left unmasked: a lane reads col[j] only for j > k,
 // written by lane j, whose value there is an entry of L, and the entries
 // above the diagonal are never written out.  Fully unrolled and branch-free
@@ -312,43 +313,6 @@ __device__ __forceinline__ void warp_trinv_v4(const float (*lt)[LTLD], const flo
         for (int i = 0; i < KP; ++i)
             if (i >= lane && i < kb) dst[i + lane * ld] = x[i];
     }
-}
-
-// FP64 form of warp_potrf_bcast (two entries per 16-byte load).
-template <int KP>
-__device__ __forceinline__ bool warp_potrf_bcast(double (&a)[KP], int kb, int lane, double* inv_out, double* col) {
-    static_assert(KP % 2 == 0, "whole double2 groups");
-    bool bad = false;
-    double my_inv = 0.0;
-#pragma unroll
-    for (int k = 0; k < KP; ++k) {
-        if (k < kb) {
-            double d = __shfl_sync(0xffffffffu, a[k], k);
-            const bool ok = pivot_ok(d);
-            bad |= !ok;
-            d = ok ? d : 1.0;
-            double sq, inv;
-            pivot_value(d, &sq, &inv);
-            const double lk = (lane == k) ? sq : (lane > k ? a[k] * inv : a[k]);
-            a[k] = lk;
-            my_inv = (lane == k) ? inv : my_inv;
-            if (k + 1 < KP) {
-                col[lane] = lk;
-                __syncwarp();
-#pragma unroll
-                for (int g = (k + 1) / 2; g < KP / 2; ++g) {
-                    const double2 v = reinterpret_cast<const double2*>(col)[g];
-                    const double w[2] = {v.x, v.y};
-#pragma unroll
-                    for (int q = 0; q < 2; ++q)
-                        if (2 * g + q > k) a[2 * g + q] = a[2 * g + q] - lk * w[q];
-                }
-                __syncwarp();
-            }
-        }
-    }
-    *inv_out = my_inv;
-    return bad;
 }
 
 constexpr int kWarpsPerCta = kThreads / 32;
@@ -496,25 +460,78 @@ __device__ void warp_front_factor(const DevFactor& F, const DevWork& W, const T*
     }
 }
 
+// 1 / d of a pivot, by the same means (y (1 + e + e^2), e = 1 - d y); a d
+// that is not positive and finite is replaced by 1 and reported.
+__device__ __forceinline__ double pivot_recip(double& d, bool& bad) {
+    if (in_fp32_range(d)) {
+        float yf;
+        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(yf) : "f"(leading_fp32(d)));
+        const double y = widen_fp32(yf);
+        const double e = fma(-d, y, 1.0);
+        return fma(y, fma(e, e, e), y);
+    }
+    if (!pivot_ok(d)) {
+        bad = true;
+        d = 1.0;
+    }
+    return 1.0 / d;
+}
+
+// Column counters of an elimination within one CTA: a column's owner raises
+// the counter after writing the column to shared memory, the other warps wait
+// for it (the CTA's warps are all resident, so the owner always runs; the wait
+// is bounded all the same).
+__device__ __forceinline__ void wait_column(int* ready, int k, uint32_t* status) {
+    const unsigned at = static_cast<unsigned>(__cvta_generic_to_shared(ready));
+    for (int spins = 0;; ++spins) {
+        int v;
+        asm volatile("ld.acquire.cta.shared.b32 %0, [%1];" : "=r"(v) : "r"(at) : "memory");
+        if (v >= k) break;
+        if (spins > (1 << 22)) {
+            atomicOr(status, FLAG_TIMEOUT);
+            break;
+        }
+    }
+    __syncwarp();
+}
+__device__ __forceinline__ void post_column(int* ready, int k) {
+    __syncwarp();
+    if ((threadIdx.x & 31) == 0) {
+        const unsigned at = static_cast<unsigned>(__cvta_generic_to_shared(ready));
+        asm volatile("st.release.cta.shared.b32 [%0], %1;" ::"r"(at), "r"(k) : "memory");
+    }
+}
+
+// Hand-over of one column between two warps on the chain, by a named barrier
+// of 64 threads (about 35 cycles; the counter above takes about 140).
+__device__ __forceinline__ void hand_over(int k) {
+    asm volatile("bar.arrive %0, 64;" ::"r"(1 + (k & 7)) : "memory");
+}
+__device__ __forceinline__ void take_over(int k) { asm volatile("bar.sync %0, 64;" ::"r"(1 + (k & 7)) : "memory"); }
+
 // Shared-memory scratch of one front besides the front itself.
 template <typename T>
-struct FrontSmem {
-    __align__(16) T lt[kPanel][kPanel + 4];  // lt[c][r] = L11[r][c] of the current panel (16-byte aligned rows)
-    __align__(16) T col[kPanel];             // pivot column broadcast of warp_potrf_bcast
-    T rinv[kPanel];                          // 1 / L11[c][c]
+struct FrontSmem;
+template <>
+struct FrontSmem<float> {
+    __align__(16) float lt[kPanel][kPanel + 4];  // lt[c][r] = L11[r][c] of the current panel (16-byte aligned rows)
+    __align__(16) float col[kPanel];             // pivot column broadcast of warp_potrf_bcast
+    float rinv[kPanel];                          // 1 / L11[c][c]
+};
+template <>
+struct FrontSmem<double> {
+    double ms[kPanel][kPanel];  // column k of the current panel's block, unscaled, over its pivot
+    double dk[kPanel];          // pivots, then 1 / sqrt
+    int ready, ready_x;         // columns published: first 32 rows, rows below
 };
 
-// Assembles and partially factorises front s in shared memory (Fm holds
-// front_ld(f) x f values) with panels of KP <= kPanel columns.
-template <typename T, int KP>
-__device__ void front_factor(const DevFactor& F, const DevWork& W, const T* gv, T* lx, T* ub, int s, T* Fm,
-                             FrontSmem<T>& sm) {
-    static_assert(KP <= kPanel && KP <= 32, "panel wider than a warp");
-    const int f = F.sn_f[s];
+// Front s with its gain entries and its children's update matrices, in shared
+// memory (Fm holds front_ld(f) x f values).
+template <typename T>
+__device__ __forceinline__ void front_assemble(const DevFactor& F, const T* gv, const T* lx, const T* ub, int s, int f,
+                                               T* Fm) {
     const int ldf = front_ld<T>(f);
-    const int nc = F.sn_c0[s + 1] - F.sn_c0[s];
     const int tid = threadIdx.x, nth = blockDim.x;
-    const int lane = tid & 31, warp = tid >> 5;
     for (int x = tid; x < ldf * f; x += nth) Fm[x] = T(0);
     __syncthreads();
     if (ldf == f) {
@@ -529,6 +546,183 @@ __device__ void front_factor(const DevFactor& F, const DevWork& W, const T* gv, 
     __syncthreads();
     extend_add_children<T>(F, lx, ub, s, Fm, ldf);
     __syncthreads();
+}
+
+// The finished front's L panel and update matrix to the factor arrays.
+template <typename T>
+__device__ __forceinline__ void front_store(const DevFactor& F, T* lx, T* ub, int s, int f, int nc, const T* Fm) {
+    const int ldf = front_ld<T>(f);
+    const int tid = threadIdx.x, nth = blockDim.x, lane = tid & 31, warp = tid >> 5;
+    T* L = lx + F.sn_lx_off[s];
+    for (int x = tid; x < f * nc; x += nth) {
+        const int c = x / f;
+        L[x] = Fm[(x - c * f) + c * ldf];
+    }
+    const int m = f - nc;
+    T* U = ub + F.sn_u_off[s];
+    const int nwarp = nth >> 5;
+    for (int j = warp; j < m; j += nwarp)
+        for (int i = lane; i < m; i += 32) U[i + (int64_t)j * m] = Fm[(nc + i) + (nc + j) * ldf];
+}
+
+// Assembles and partially factorises front s in shared memory, FP64, with
+// panels of KP columns.  Bound: FP64 issue (a warp instruction takes 64 cycles
+// of its scheduler) and the pivots' chain, as in k_big_panel64, whose scheme
+// the panels use: warp w owns the panel's columns w (mod 8), a lane per row,
+// in registers; a column's unscaled rows are published in its place in Fm and
+// its block's rows over the pivot in ms; the rows past the first 32 follow one
+// column behind.  The trailing update takes one entry per thread, the lower
+// triangle folded (column p with column m - 1 - p) into rows of m + 1 entries,
+// so that no lane idles.  Measured on a 30k-bus grid, against one warp's
+// factorisation of the block, a thread per row below it and 4 x 4 tiles in the
+// update: phase B 337 -> 202 us, phase A 261 -> 159, synchronous levels 82 -> 50.
+template <int KP>
+__device__ void front_factor(const DevFactor& F, const DevWork& W, const double* gv, double* lx, double* ub, int s,
+                             double* Fm, FrontSmem<double>& sm) {
+    static_assert(KP <= kPanel && kThreads == 256, "columns over eight warps");
+    constexpr int kW = kThreads / 32, kQ = KP / kW;
+    constexpr int kG = KP == kPanel ? (kSmallFrontMax + 31) / 32 : (kFlowSmallFMax + 31) / 32;  // row groups of 32
+    const int f = F.sn_f[s];
+    const int ldf = front_ld<double>(f);
+    const int nc = F.sn_c0[s + 1] - F.sn_c0[s];
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    front_assemble<double>(F, gv, lx, ub, s, f, Fm);
+    double* rdg = reinterpret_cast<double*>(W.rdiag) + F.sn_c0[s];
+    uint32_t* status = &W.status->flags;
+#pragma unroll 1
+    for (int k0 = 0; k0 < nc; k0 += KP) {
+        const int kb = min(KP, nc - k0);
+        const int nrow = f - k0;
+        const int ng = (nrow + 31) >> 5;  // <= kG
+        double* P = Fm + k0 + (int64_t)k0 * ldf;  // P[r + c * ldf]: row k0 + r, column k0 + c
+        if (tid == 0) sm.ready = sm.ready_x = -1;
+        double a[kQ][kG];
+#pragma unroll
+        for (int q = 0; q < kQ; ++q)
+#pragma unroll
+            for (int g = 0; g < kG; ++g) {
+                const int c = w + kW * q, r = 32 * g + lane;
+                a[q][g] = (c < kb && r < nrow) ? P[r + c * ldf] : 0.0;
+            }
+        __syncthreads();
+        bool bad = false;
+        auto publish = [&](double& aq, int k) {
+            double d = __shfl_sync(0xffffffffu, aq, k);
+            if (lane < nrow) P[lane + k * ldf] = aq;
+            sm.ms[k][lane] = aq * pivot_recip(d, bad);
+            if (k + 1 < kb) hand_over(k);
+            if (lane == k) aq = d;
+            if (lane == 0) sm.dk[k] = d;
+            post_column(&sm.ready, k);
+        };
+        if (w == 0) publish(a[0][0], 0);
+#pragma unroll
+        for (int qq = 0; qq < kQ; ++qq) {
+#pragma unroll 1
+            for (int kk = 0; kk < kW; ++kk) {
+                const int k = kW * qq + kk;
+                if (k >= kb) break;
+                const bool next = w == ((kk + 1) & (kW - 1)) && k + 1 < kb;
+                if (next) take_over(k);
+                else wait_column(&sm.ready, k, status);
+                const double ub0 = lane < nrow ? P[lane + k * ldf] : 0.0;
+                int done = k;
+                if (next) {
+                    const double m = sm.ms[k][k + 1];
+                    if (kk + 1 < kW) {
+                        a[qq][0] = fma(-ub0, m, a[qq][0]);
+                        publish(a[qq][0], k + 1);
+                    } else if (qq + 1 < kQ) {
+                        const int qn = qq + 1 < kQ ? qq + 1 : kQ - 1;
+                        a[qn][0] = fma(-ub0, m, a[qn][0]);
+                        publish(a[qn][0], k + 1);
+                    }
+                    done = k + 1;
+                }
+#pragma unroll
+                for (int q = qq; q < kQ; ++q) {
+                    const int c = w + kW * q;
+                    if (c > done && c < kb) a[q][0] = fma(-ub0, sm.ms[k][c], a[q][0]);
+                }
+                if (ng > 1) {
+                    // the rows past the first 32: columns behind k - 1 by column k - 1, then column k is final
+                    if (k > 0) {
+                        wait_column(&sm.ready_x, k - 1, status);
+                        double u[kG];
+#pragma unroll
+                        for (int g = 1; g < kG; ++g) u[g] = (32 * g + lane < nrow) ? P[32 * g + lane + (k - 1) * ldf] : 0.0;
+#pragma unroll
+                        for (int q = qq; q < kQ; ++q) {
+                            const int c = w + kW * q;
+                            if (c >= k && c < kb) {
+                                const double m = sm.ms[k - 1][c];
+#pragma unroll
+                                for (int g = 1; g < kG; ++g)
+                                    if (g < ng) a[q][g] = fma(-u[g], m, a[q][g]);
+                            }
+                            if (q == qq && w == kk) {
+#pragma unroll
+                                for (int g = 1; g < kG; ++g)
+                                    if (32 * g + lane < nrow) P[32 * g + lane + k * ldf] = a[q][g];
+                                post_column(&sm.ready_x, k);
+                            }
+                        }
+                    } else if (w == 0) {
+                        post_column(&sm.ready_x, 0);  // column 0 is in place
+                    }
+                }
+            }
+        }
+        if (bad && lane == 0) atomicOr(singular_flags(F, W, s), FLAG_SINGULAR);
+        __syncthreads();
+        if (w == 0 && lane < kb) {
+            double sq, rs;
+            pivot_value(sm.dk[lane], &sq, &rs);
+            sm.dk[lane] = rs;
+            rdg[k0 + lane] = rs;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < kQ; ++q) {
+            const int c = w + kW * q;
+            if (c < kb) {
+                const double rs = sm.dk[c];
+#pragma unroll
+                for (int g = 0; g < kG; ++g)
+                    if (g < ng && 32 * g + lane < nrow) P[32 * g + lane + c * ldf] = a[q][g] * rs;
+            }
+        }
+        __syncthreads();
+        const int q0 = k0 + kb, m = f - q0;
+        const int total = m * (m + 1) / 2;
+        const double* X = Fm + k0 * ldf;
+        for (int t = tid; t < total; t += kThreads) {
+            const int pr = t / (m + 1), pos = t - pr * (m + 1);
+            const bool first = pos < m - pr;
+            const int j = q0 + (first ? pr : m - 1 - pr);
+            const int i = j + (first ? pos : pos - (m - pr));
+            double acc = Fm[i + j * ldf];
+#pragma unroll 8
+            for (int k = 0; k < kb; ++k) acc = fma(-X[i + k * ldf], X[j + k * ldf], acc);
+            Fm[i + j * ldf] = acc;
+        }
+        __syncthreads();
+    }
+    front_store<double>(F, lx, ub, s, f, nc, Fm);
+}
+
+// FP32, with panels of KP <= kPanel columns.
+template <int KP>
+__device__ void front_factor(const DevFactor& F, const DevWork& W, const float* gv, float* lx, float* ub, int s,
+                             float* Fm, FrontSmem<float>& sm) {
+    using T = float;
+    static_assert(KP <= kPanel && KP <= 32, "panel wider than a warp");
+    const int f = F.sn_f[s];
+    const int ldf = front_ld<T>(f);
+    const int nc = F.sn_c0[s + 1] - F.sn_c0[s];
+    const int tid = threadIdx.x, nth = blockDim.x;
+    const int lane = tid & 31, warp = tid >> 5;
+    front_assemble<T>(F, gv, lx, ub, s, f, Fm);
     T* rdg = reinterpret_cast<T*>(W.rdiag) + F.sn_c0[s];
 #pragma unroll 1
     for (int k0 = 0; k0 < nc; k0 += KP) {
@@ -556,16 +750,14 @@ __device__ void front_factor(const DevFactor& F, const DevWork& W, const T* gv, 
                 }
         }
         __syncthreads();
-        // (2) FP32: warp 0 writes the inverse of the diagonal block into its
-        // slot.  The other threads (FP64: all): rows below the block,
-        // x = a L11^-T, one row per thread (f - q0 < kThreads - 32)
+        // (2) warp 0 writes the inverse of the diagonal block into its slot;
+        // the other threads: rows below the block, x = a L11^-T, one row per
+        // thread (f - q0 < kThreads - 32)
         const int q0 = k0 + kb;
-        constexpr int kInvThreads = kInvDiag<T> ? 32 : 0;
-        if (kInvDiag<T> && warp == 0) {
-            if constexpr (sizeof(T) == 4)
-                warp_trinv_v4<KP, kPanel + 4>(sm.lt, sm.rinv, kb, lane, Fm + k0 + k0 * ldf, ldf);
+        if (warp == 0) {
+            warp_trinv_v4<KP, kPanel + 4>(sm.lt, sm.rinv, kb, lane, Fm + k0 + k0 * ldf, ldf);
         } else {
-            const int r = q0 + tid - kInvThreads;
+            const int r = q0 + tid - 32;
             if (r < f) {
                 T x[KP];
 #pragma unroll
@@ -633,16 +825,7 @@ __device__ void front_factor(const DevFactor& F, const DevWork& W, const T* gv, 
         }
         __syncthreads();
     }
-    T* L = lx + F.sn_lx_off[s];
-    for (int x = tid; x < f * nc; x += nth) {
-        const int c = x / f;
-        L[x] = Fm[(x - c * f) + c * ldf];
-    }
-    const int m = f - nc;
-    T* U = ub + F.sn_u_off[s];
-    const int nwarp = nth >> 5;
-    for (int j = warp; j < m; j += nwarp)
-        for (int i = lane; i < m; i += 32) U[i + (int64_t)j * m] = Fm[(nc + i) + (nc + j) * ldf];
+    front_store<T>(F, lx, ub, s, f, nc, Fm);
 }
 
 // Panel widths: fronts of the high-occupancy dataflow phase (f <= 64) use
@@ -659,7 +842,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_front_small(DevFactor F, DevWor
     __shared__ FrontSmem<T> sm;
     const int s = fronts[blockIdx.x];
     if (front_frozen(F, W, s)) return;
-    front_factor<T, kPanel>(F, W, gv, lx, ub, s, reinterpret_cast<T*>(smem_raw), sm);
+    front_factor<kPanel>(F, W, gv, lx, ub, s, reinterpret_cast<T*>(smem_raw), sm);
 }
 
 // ---------------------------------------------------------------------------
@@ -736,7 +919,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) k_front_flow(DevFactor F
         int s = ready[item];
         while (s >= 0) {
             if (!front_frozen(F, W, s))
-                front_factor<T, KP>(F, W, gv, lx, ub, s, reinterpret_cast<T*>(smem_raw), sm);
+                front_factor<KP>(F, W, gv, lx, ub, s, reinterpret_cast<T*>(smem_raw), sm);
             __syncthreads();
             s = continue_up(F, phase, ph, nchild, cnt, s, &slot);
         }
@@ -811,55 +994,6 @@ __global__ void __launch_bounds__(kThreads) k_big_assemble(DevFactor F, DevWork 
         __syncthreads();
     }
 }
-
-// 1 / d of a pivot, by the same means (y (1 + e + e^2), e = 1 - d y); a d
-// that is not positive and finite is replaced by 1 and reported.
-__device__ __forceinline__ double pivot_recip(double& d, bool& bad) {
-    if (in_fp32_range(d)) {
-        float yf;
-        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(yf) : "f"(leading_fp32(d)));
-        const double y = widen_fp32(yf);
-        const double e = fma(-d, y, 1.0);
-        return fma(y, fma(e, e, e), y);
-    }
-    if (!pivot_ok(d)) {
-        bad = true;
-        d = 1.0;
-    }
-    return 1.0 / d;
-}
-
-// Column counters of an elimination within one CTA: a column's owner raises
-// the counter after writing the column to shared memory, the other warps wait
-// for it (the CTA's warps are all resident, so the owner always runs; the wait
-// is bounded all the same).
-__device__ __forceinline__ void wait_column(int* ready, int k, uint32_t* status) {
-    const unsigned at = static_cast<unsigned>(__cvta_generic_to_shared(ready));
-    for (int spins = 0;; ++spins) {
-        int v;
-        asm volatile("ld.acquire.cta.shared.b32 %0, [%1];" : "=r"(v) : "r"(at) : "memory");
-        if (v >= k) break;
-        if (spins > (1 << 22)) {
-            atomicOr(status, FLAG_TIMEOUT);
-            break;
-        }
-    }
-    __syncwarp();
-}
-__device__ __forceinline__ void post_column(int* ready, int k) {
-    __syncwarp();
-    if ((threadIdx.x & 31) == 0) {
-        const unsigned at = static_cast<unsigned>(__cvta_generic_to_shared(ready));
-        asm volatile("st.release.cta.shared.b32 [%0], %1;" ::"r"(at), "r"(k) : "memory");
-    }
-}
-
-// Hand-over of one column between two warps on the chain, by a named barrier
-// of 64 threads (about 35 cycles; the counter above takes about 140).
-__device__ __forceinline__ void hand_over(int k) {
-    asm volatile("bar.arrive %0, 64;" ::"r"(1 + (k & 7)) : "memory");
-}
-__device__ __forceinline__ void take_over(int k) { asm volatile("bar.sync %0, 64;" ::"r"(1 + (k & 7)) : "memory"); }
 
 // FP64 panel step p of the tiled fronts: the diagonal block's factorisation
 // and the rows below it, one CTA per kPanelRows64 rows (each factors the
