@@ -247,6 +247,7 @@ void Engine::build_tile_tasks(const std::vector<int32_t>& bigs,
                 for (int32_t k = (r0 - q0) / kPanelRows; r0 < r1 && k <= (r1 - 1 - q0) / kPanelRows; ++k)
                     push_dep(b.pid0[p] + k);
             }
+            if (ti == tj) push_dep(b.pid0[p]);  // the first chunk's item solves for y
             if (p > 0) push_dep(uid(b, p - 1, ti, tj));
             TileTask t{};
             t.kind = 1, t.s = b.s, t.p = p, t.a = ti, t.b = tj;
@@ -560,8 +561,8 @@ void Engine::build_schedule(bool targets_ready) {
                 const int32_t pb = std::min(kTile, nc - p * kTile);
                 const int32_t q0 = p * kTile + pb;
                 // one CTA per chunk of rows below the diagonal block
-                const int32_t rows = mixed_ ? kPanelRows : kPanelRows64;
-                const int32_t nch = std::max(1, (f - q0 + rows - 1) / rows);
+                const int32_t nch = mixed_ ? std::max(1, (f - q0 + kPanelRows - 1) / kPanelRows)
+                                           : (f - q0) / kPanelRows64 + 1;  // with the right-hand side as row f
                 for (int32_t k = 0; k < nch; ++k) sch_pot_.push_back(make_int4(s, k, nch, n_pot_pairs_));
                 pair_of[(static_cast<int64_t>(s) << 20) | p] = n_pot_pairs_;
                 ++n_pot_pairs_;
@@ -1234,21 +1235,21 @@ int32_t Engine::enqueue_iteration(const SolveParams& sp, bool refactor, int64_t*
     };
     if (sched_.compact) stage(ST_OTHER, [&] { return launch_ready_compact(fac_, work_, sched_, st_); });
     stage(ST_EVALUATE, [&] { return launch_evaluate(net_, work_, sp, st_); });
+    // a refactorisation takes the right-hand side along (launch_factor)
+    stage(ST_RHS, [&] { return launch_rhs(net_, fac_, work_, st_); });
     if (!mixed_) {
         if (refactor) stage(ST_FACTOR, [&] { return launch_factor(net_, fac_, work_, sched_, st_); });
-        stage(ST_RHS, [&] { return launch_rhs(net_, fac_, work_, st_); });
-        stage(ST_SOLVE, [&] { return launch_solve(fac_, work_, sched_, st_); });
+        stage(ST_SOLVE, [&] { return launch_solve(fac_, work_, sched_, !refactor, st_); });
         stage(ST_UPDATE, [&] { return update(work_.sol); });
     } else {
+        stage(ST_SOLVE, [&] { return launch_to_fp32(fac_, work_, st_); });
         if (refactor) stage(ST_FACTOR, [&] { return launch_factor32(net_, fac_, work_, sched_, st_); });
-        stage(ST_RHS, [&] { return launch_rhs(net_, fac_, work_, st_); });
         stage(ST_SOLVE, [&] {
-            cudaError_t ee = launch_to_fp32(fac_, work_, st_);
-            if (ee == cudaSuccess) ee = launch_solve32(fac_, work_, sched_, st_);
+            cudaError_t ee = launch_solve32(fac_, work_, sched_, !refactor, st_);
             if (ee == cudaSuccess) ee = launch_refine_begin(fac_, work_, st_);
             for (int32_t k = 0; k < cfg.refine_steps && ee == cudaSuccess; ++k) {
                 ee = launch_refine_residual(net_, fac_, work_, st_);
-                if (ee == cudaSuccess) ee = launch_solve32(fac_, work_, sched_, st_);
+                if (ee == cudaSuccess) ee = launch_solve32(fac_, work_, sched_, true, st_);
                 if (ee == cudaSuccess) ee = launch_refine_accumulate(fac_, work_, st_);
             }
             return ee;
@@ -1693,9 +1694,9 @@ int32_t Engine::factor_and_solve(const double* rhs_orig, double* x_orig) {
     std::vector<double> b(P.n_state);
     for (int32_t p = 0; p < P.n_state; ++p) b[p] = rhs_orig[P.state_of_ps[p]];
     cudaError_t e = cudaMemsetAsync(&work_.status->flags, 0, sizeof(uint32_t), st_);
-    if (e == cudaSuccess) e = launch_factor(net_, fac_, work_, sched_, st_);
     if (e == cudaSuccess) e = cudaMemcpyAsync(work_.rhs, b.data(), sizeof(double) * P.n_state, cudaMemcpyHostToDevice, st_);
-    if (e == cudaSuccess) e = launch_solve(fac_, work_, sched_, st_);
+    if (e == cudaSuccess) e = launch_factor(net_, fac_, work_, sched_, st_);
+    if (e == cudaSuccess) e = launch_solve(fac_, work_, sched_, false, st_);
     std::vector<double> x(P.n_state);
     if (e == cudaSuccess) e = cudaMemcpyAsync(x.data(), work_.sol, sizeof(double) * P.n_state, cudaMemcpyDeviceToHost, st_);
     if (e == cudaSuccess) e = cudaMemcpyAsync(h_status_, work_.status, sizeof(DevStatus), cudaMemcpyDeviceToHost, st_);

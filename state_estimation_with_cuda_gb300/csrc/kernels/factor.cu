@@ -30,6 +30,18 @@ namespace {
 
 constexpr int kThreads = 256;
 
+struct SolveVecs {
+    const void* rhs;  // [n_state] right-hand side, permuted (V)
+    void* sol;        // [n_state] solution, permuted (V)
+    void* su;         // solve update vectors (V)
+};
+// Entry r of front s's right-hand-side row: a pivot's in sol (y once it is
+// eliminated), a row's below them in the front's solve update vector.
+template <typename V>
+__device__ __forceinline__ V* rhs_entry(const SolveVecs& sv, int c0, int nc, int64_t su_off, int r) {
+    return r < nc ? static_cast<V*>(sv.sol) + c0 + r : static_cast<V*>(sv.su) + su_off + (r - nc);
+}
+
 // G entry = sum over its pairs (a, b) of (w h_a) h_b, the weighted entry
 // hw[a] written by the evaluation (FP64: the same product, so the same sum),
 // accumulated in ACC.
@@ -124,21 +136,25 @@ __device__ __forceinline__ const T* update_of(const DevFactor& F, const T* lx, c
 // the same entry and each entry's additions keep the children's order.  Per
 // child, the warp selects its columns 32 at a time (ballot over the relative
 // map), then loads up to four of them (four rows per lane each) before it
-// scatters them.  The caller follows with a block barrier.
+// scatters them.  The child's solve update vector is added to the front's
+// right-hand side (entry t at rhs[t * rhs_ld]) the same way.  The caller
+// follows with a block barrier.
 template <typename T>
-__device__ __forceinline__ void extend_add_children(const DevFactor& F, const T* lx, const T* ubase, int s, T* dst,
-                                                    int ldd) {
+__device__ __forceinline__ void extend_add_children(const DevFactor& F, const SolveVecs& sv, const T* lx,
+                                                    const T* ubase, int s, T* dst, int ldd, T* rhs, int rhs_ld) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
     for (int ci = F.sn_child_ptr[s]; ci < F.sn_child_ptr[s + 1]; ++ci) {
         const int c = F.sn_child[ci];
         const int m = F.sn_f[c] - (F.sn_c0[c + 1] - F.sn_c0[c]);
         const T* U = update_of<T>(F, lx, ubase, c);
         const int uld = F.sn_u_ld[c];
-        const int* rel = F.sn_relmap + F.sn_su_off[c];
+        const int64_t so = F.sn_su_off[c];
+        const int* rel = F.sn_relmap + so;
         for (int j0 = 0; j0 < m; j0 += 32) {
             const int jl = j0 + lane;
             const int tj = (jl < m) ? rel[jl] : -1;
             unsigned own = __ballot_sync(0xffffffffu, tj >= 0 && (tj % nwarp) == warp);
+            if ((own >> lane) & 1u) rhs[tj * rhs_ld] += __ldcg(static_cast<const T*>(sv.su) + so + jl);
             while (own) {
                 int js[4];
                 int cnt = 0;
@@ -322,6 +338,7 @@ template <typename T>
 struct WarpTile {
     T a[kWarpFrontMax * kWtLd];  // a[c * kWtLd + r] = front entry (r, c)
     T rinv[kWarpFrontMax];
+    T v[kWarpFrontMax];          // right-hand side of the front's rows
 };
 
 __device__ __forceinline__ int warp_claim(int* counter) {
@@ -352,13 +369,14 @@ __device__ __forceinline__ int warp_continue_up(const DevFactor& F, const int8_t
 }
 
 template <typename T>
-__device__ void warp_front_factor(const DevFactor& F, const DevWork& W, const T* gv, T* lx, T* ub, int s,
-                                  WarpTile<T>& t) {
+__device__ void warp_front_factor(const DevFactor& F, const DevWork& W, const SolveVecs& sv, const T* gv, T* lx, T* ub,
+                                  int s, WarpTile<T>& t) {
     const int lane = threadIdx.x & 31;
     const int f = F.sn_f[s];
     const int c0 = F.sn_c0[s];
     const int nc = F.sn_c0[s + 1] - c0;
     for (int c = 0; c < f; ++c) t.a[c * kWtLd + lane] = T(0);
+    t.v[lane] = lane < nc ? static_cast<const T*>(sv.rhs)[c0 + lane] : T(0);
     __syncwarp();
     {
         // original entries, four per lane in flight
@@ -386,7 +404,9 @@ __device__ void warp_front_factor(const DevFactor& F, const DevWork& W, const T*
         const int m = F.sn_f[ch] - (F.sn_c0[ch + 1] - F.sn_c0[ch]);  // < kWarpFrontMax: the parent holds m rows
         const T* U = update_of<T>(F, lx, ub, ch);
         const int uld = F.sn_u_ld[ch];
-        const int ri = lane < m ? F.sn_relmap[F.sn_su_off[ch] + lane] : 0;
+        const int64_t so = F.sn_su_off[ch];
+        const int ri = lane < m ? F.sn_relmap[so + lane] : 0;
+        if (lane < m) t.v[ri] += __ldcg(static_cast<const T*>(sv.su) + so + lane);
         for (int j = 0; j < m; j += 4) {
             T u[4];
 #pragma unroll
@@ -406,6 +426,9 @@ __device__ void warp_front_factor(const DevFactor& F, const DevWork& W, const T*
     // median 16 rows, 4 columns), which keeps the kernel small enough for the
     // instruction cache.
     T my_inv = T(0);
+    // FP64: the forward substitution rides along, row i's right-hand side in
+    // lane i.  FP32 applies L11^-1 below, as the forward sweep does.
+    T vi = t.v[lane];
     bool bad = false;
     for (int k = 0; k < nc; ++k) {
         T d = t.a[k * kWtLd + k];
@@ -416,6 +439,10 @@ __device__ void warp_front_factor(const DevFactor& F, const DevWork& W, const T*
         pivot_value(d, &sq, &inv);
         const bool below = lane > k && lane < f;
         const T lik = below ? t.a[k * kWtLd + lane] * inv : T(0);
+        if constexpr (!kInvDiag<T>) {
+            const T yk = __shfl_sync(0xffffffffu, vi, k) * inv;
+            vi = lane == k ? yk : (below ? vi - lik * yk : vi);
+        }
         __syncwarp();  // column k read by every lane before it is overwritten
         if (lane == k) {
             t.a[k * kWtLd + k] = sq;
@@ -453,11 +480,24 @@ __device__ void warp_front_factor(const DevFactor& F, const DevWork& W, const T*
             }
         }
         __syncwarp();
-        // L11^-1 into the diagonal block: lane i writes row i
+        // L11^-1 into the diagonal block: lane i writes row i; y = L11^-1 v1
+        T y = T(0);
         if (lane < nc)
-            for (int j = 0; j <= lane; ++j)
-                L[lane + j * f] = (j == lane) ? my_inv : t.a[lane * kWtLd + j];
+            for (int j = 0; j <= lane; ++j) {
+                const T l = (j == lane) ? my_inv : t.a[lane * kWtLd + j];
+                L[lane + j * f] = l;
+                y += l * t.v[j];
+            }
+        __syncwarp();
+        if (lane < nc) {
+            t.v[lane] = y;
+            vi = y;
+        }
+        __syncwarp();
+        if (lane >= nc)
+            for (int k = 0; k < nc; ++k) vi -= t.a[k * kWtLd + lane] * t.v[k];
     }
+    if (lane < f) *rhs_entry<T>(sv, c0, nc, F.sn_su_off[s], lane) = vi;
 }
 
 // 1 / d of a pivot, by the same means (y (1 + e + e^2), e = 1 - d y); a d
@@ -517,6 +557,7 @@ struct FrontSmem<float> {
     __align__(16) float lt[kPanel][kPanel + 4];  // lt[c][r] = L11[r][c] of the current panel (16-byte aligned rows)
     __align__(16) float col[kPanel];             // pivot column broadcast of warp_potrf_bcast
     float rinv[kPanel];                          // 1 / L11[c][c]
+    float v[kSmallFrontMax32];                   // right-hand side of the front's rows
 };
 template <>
 struct FrontSmem<double> {
@@ -526,10 +567,16 @@ struct FrontSmem<double> {
 };
 
 // Front s with its gain entries and its children's update matrices, in shared
-// memory (Fm holds front_ld(f) x f values).
+// memory (Fm holds front_ld(f) x f values), and its right-hand side (entry r at
+// rhs[r * rhs_ld]): the factorisation carries the forward substitution along.
+// The forward sweep of its own follows the same chain of the elimination tree
+// as the factorisation, reading every L panel back: 1.04 ms of a 4.4 ms step at
+// 200k buses (mixed), 0.56 of 7.1 at 60k (FP64); carried along, y costs each
+// front a few hundred cycles.  FP32 keeps the sweep's order of operations
+// (y = L11^-1 v per panel, then the rows below column by column): same bits.
 template <typename T>
-__device__ __forceinline__ void front_assemble(const DevFactor& F, const T* gv, const T* lx, const T* ub, int s, int f,
-                                               T* Fm) {
+__device__ __forceinline__ void front_assemble(const DevFactor& F, const SolveVecs& sv, const T* gv, const T* lx,
+                                               const T* ub, int s, int f, int c0, int nc, T* Fm, T* rhs, int rhs_ld) {
     const int ldf = front_ld<T>(f);
     const int tid = threadIdx.x, nth = blockDim.x;
     for (int x = tid; x < ldf * f; x += nth) Fm[x] = T(0);
@@ -543,16 +590,20 @@ __device__ __forceinline__ void front_assemble(const DevFactor& F, const T* gv, 
             Fm[(l - c * f) + c * ldf] = gv[tg];
         }
     }
+    for (int r = tid; r < f; r += nth) rhs[r * rhs_ld] = r < nc ? static_cast<const T*>(sv.rhs)[c0 + r] : T(0);
     __syncthreads();
-    extend_add_children<T>(F, lx, ub, s, Fm, ldf);
+    extend_add_children<T>(F, sv, lx, ub, s, Fm, ldf, rhs, rhs_ld);
     __syncthreads();
 }
 
-// The finished front's L panel and update matrix to the factor arrays.
+// The finished front's L panel, update matrix and right-hand side to the factor
+// and solve arrays.
 template <typename T>
-__device__ __forceinline__ void front_store(const DevFactor& F, T* lx, T* ub, int s, int f, int nc, const T* Fm) {
+__device__ __forceinline__ void front_store(const DevFactor& F, const SolveVecs& sv, T* lx, T* ub, int s, int f,
+                                            int c0, int nc, const T* Fm, const T* rhs, int rhs_ld) {
     const int ldf = front_ld<T>(f);
     const int tid = threadIdx.x, nth = blockDim.x, lane = tid & 31, warp = tid >> 5;
+    for (int r = tid; r < f; r += nth) *rhs_entry<T>(sv, c0, nc, F.sn_su_off[s], r) = rhs[r * rhs_ld];
     T* L = lx + F.sn_lx_off[s];
     for (int x = tid; x < f * nc; x += nth) {
         const int c = x / f;
@@ -572,27 +623,29 @@ __device__ __forceinline__ void front_store(const DevFactor& F, T* lx, T* ub, in
 // in registers; a column's unscaled rows are published in its place in Fm and
 // its block's rows over the pivot in ms; the rows past the first 32 follow one
 // column behind.  The trailing update takes one entry per thread, the lower
-// triangle folded (column p with column m - 1 - p) into rows of m + 1 entries,
+// triangle folded (column p with column m - 1 - p) into rows of m + 1 entries
+// (then the right-hand side, which is row f of the front),
 // so that no lane idles.  Measured on a 30k-bus grid, against one warp's
 // factorisation of the block, a thread per row below it and 4 x 4 tiles in the
 // update: phase B 337 -> 202 us, phase A 261 -> 159, synchronous levels 82 -> 50.
 template <int KP>
-__device__ void front_factor(const DevFactor& F, const DevWork& W, const double* gv, double* lx, double* ub, int s,
-                             double* Fm, FrontSmem<double>& sm) {
+__device__ void front_factor(const DevFactor& F, const DevWork& W, const SolveVecs& sv, const double* gv, double* lx,
+                             double* ub, int s, double* Fm, FrontSmem<double>& sm) {
     static_assert(KP <= kPanel && kThreads == 256, "columns over eight warps");
     constexpr int kW = kThreads / 32, kQ = KP / kW;
-    constexpr int kG = KP == kPanel ? (kSmallFrontMax + 31) / 32 : (kFlowSmallFMax + 31) / 32;  // row groups of 32
+    constexpr int kG = ((KP == kPanel ? kSmallFrontMax : kFlowSmallFMax) + 1 + 31) / 32;  // row groups of 32
     const int f = F.sn_f[s];
     const int ldf = front_ld<double>(f);
-    const int nc = F.sn_c0[s + 1] - F.sn_c0[s];
+    const int c0 = F.sn_c0[s];
+    const int nc = F.sn_c0[s + 1] - c0;
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-    front_assemble<double>(F, gv, lx, ub, s, f, Fm);
-    double* rdg = reinterpret_cast<double*>(W.rdiag) + F.sn_c0[s];
+    front_assemble<double>(F, sv, gv, lx, ub, s, f, c0, nc, Fm, Fm + f, ldf);
+    double* rdg = reinterpret_cast<double*>(W.rdiag) + c0;
     uint32_t* status = &W.status->flags;
 #pragma unroll 1
     for (int k0 = 0; k0 < nc; k0 += KP) {
         const int kb = min(KP, nc - k0);
-        const int nrow = f - k0;
+        const int nrow = f + 1 - k0;  // with the right-hand-side row
         const int ng = (nrow + 31) >> 5;  // <= kG
         double* P = Fm + k0 + (int64_t)k0 * ldf;  // P[r + c * ldf]: row k0 + r, column k0 + c
         if (tid == 0) sm.ready = sm.ready_x = -1;
@@ -694,13 +747,13 @@ __device__ void front_factor(const DevFactor& F, const DevWork& W, const double*
         }
         __syncthreads();
         const int q0 = k0 + kb, m = f - q0;
-        const int total = m * (m + 1) / 2;
+        const int tri = m * (m + 1) / 2;
         const double* X = Fm + k0 * ldf;
-        for (int t = tid; t < total; t += kThreads) {
+        for (int t = tid; t < tri + m; t += kThreads) {  // the last m: the right-hand-side row
             const int pr = t / (m + 1), pos = t - pr * (m + 1);
             const bool first = pos < m - pr;
-            const int j = q0 + (first ? pr : m - 1 - pr);
-            const int i = j + (first ? pos : pos - (m - pr));
+            const int j = q0 + (t >= tri ? t - tri : first ? pr : m - 1 - pr);
+            const int i = t >= tri ? f : j + (first ? pos : pos - (m - pr));
             double acc = Fm[i + j * ldf];
 #pragma unroll 8
             for (int k = 0; k < kb; ++k) acc = fma(-X[i + k * ldf], X[j + k * ldf], acc);
@@ -708,22 +761,31 @@ __device__ void front_factor(const DevFactor& F, const DevWork& W, const double*
         }
         __syncthreads();
     }
-    front_store<double>(F, lx, ub, s, f, nc, Fm);
+    front_store<double>(F, sv, lx, ub, s, f, c0, nc, Fm, Fm + f, ldf);
 }
 
 // FP32, with panels of KP <= kPanel columns.
 template <int KP>
-__device__ void front_factor(const DevFactor& F, const DevWork& W, const float* gv, float* lx, float* ub, int s,
-                             float* Fm, FrontSmem<float>& sm) {
+__device__ void front_factor(const DevFactor& F, const DevWork& W, const SolveVecs& sv, const float* gv, float* lx,
+                             float* ub, int s, float* Fm, FrontSmem<float>& sm) {
     using T = float;
     static_assert(KP <= kPanel && KP <= 32, "panel wider than a warp");
     const int f = F.sn_f[s];
     const int ldf = front_ld<T>(f);
-    const int nc = F.sn_c0[s + 1] - F.sn_c0[s];
+    const int c0 = F.sn_c0[s];
+    const int nc = F.sn_c0[s + 1] - c0;
     const int tid = threadIdx.x, nth = blockDim.x;
     const int lane = tid & 31, warp = tid >> 5;
-    front_assemble<T>(F, gv, lx, ub, s, f, Fm);
-    T* rdg = reinterpret_cast<T*>(W.rdiag) + F.sn_c0[s];
+    front_assemble<T>(F, sv, gv, lx, ub, s, f, c0, nc, Fm, sm.v, 1);
+    // v_i -= L_i,k0.. y of a finished panel, by threads [t0, t0 + nt)
+    auto rhs_below = [&](int k0, int kb, int t0, int nt) {
+        for (int i = k0 + kb + tid - t0; tid >= t0 && i < f; i += nt) {
+            float acc = sm.v[i];
+            for (int k = 0; k < kb; ++k) acc -= Fm[i + (k0 + k) * ldf] * sm.v[k0 + k];
+            sm.v[i] = acc;
+        }
+    };
+    T* rdg = reinterpret_cast<T*>(W.rdiag) + c0;
 #pragma unroll 1
     for (int k0 = 0; k0 < nc; k0 += KP) {
         const int kb = min(KP, nc - k0);
@@ -748,6 +810,8 @@ __device__ void front_factor(const DevFactor& F, const DevWork& W, const float* 
                     Fm[i + (k0 + j) * ldf] = a[j];
                     sm.lt[j][lane] = a[j];
                 }
+        } else if (k0 > 0) {
+            rhs_below(k0 - KP, KP, 32, nth - 32);  // the other warps meanwhile: the previous panel's y
         }
         __syncthreads();
         // (2) warp 0 writes the inverse of the diagonal block into its slot;
@@ -776,6 +840,14 @@ __device__ void front_factor(const DevFactor& F, const DevWork& W, const float* 
             }
         }
         __syncthreads();
+        // y = L11^-1 v of the panel's rows, a lane per row (as in the forward sweep)
+        if (warp == 0) {
+            float y = 0.f;
+            if (lane < kb)
+                for (int j = 0; j <= lane; ++j) y += Fm[k0 + lane + (k0 + j) * ldf] * sm.v[k0 + j];
+            __syncwarp();
+            if (lane < kb) sm.v[k0 + lane] = y;
+        }
         // (3) trailing update of the lower triangle, 4x4 tiles on 4-aligned
         // rows; tiles are numbered down each tile column so that neighbouring
         // threads touch neighbouring rows (conflict-free vector accesses)
@@ -825,7 +897,10 @@ __device__ void front_factor(const DevFactor& F, const DevWork& W, const float* 
         }
         __syncthreads();
     }
-    front_store<T>(F, lx, ub, s, f, nc, Fm);
+    const int kl = (nc - 1) / KP * KP;  // the last panel (nc > 0)
+    rhs_below(kl, nc - kl, 0, nth);
+    __syncthreads();
+    front_store<T>(F, sv, lx, ub, s, f, c0, nc, Fm, sm.v, 1);
 }
 
 // Panel widths: fronts of the high-occupancy dataflow phase (f <= 64) use
@@ -836,13 +911,13 @@ template <typename T>
 constexpr int kMinBlocksA = sizeof(T) == 4 ? 3 : 2;
 
 template <typename T>
-__global__ void __launch_bounds__(kThreads, 1) k_front_small(DevFactor F, DevWork W, const T* gv, T* lx, T* ub,
-                                                             const int* fronts) {
+__global__ void __launch_bounds__(kThreads, 1) k_front_small(DevFactor F, DevWork W, SolveVecs sv, const T* gv, T* lx,
+                                                             T* ub, const int* fronts) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ FrontSmem<T> sm;
     const int s = fronts[blockIdx.x];
     if (front_frozen(F, W, s)) return;
-    front_factor<kPanel>(F, W, gv, lx, ub, s, reinterpret_cast<T*>(smem_raw), sm);
+    front_factor<kPanel>(F, W, sv, gv, lx, ub, s, reinterpret_cast<T*>(smem_raw), sm);
 }
 
 // ---------------------------------------------------------------------------
@@ -905,8 +980,8 @@ __device__ __forceinline__ int continue_up(const DevFactor& F, const int8_t* pha
 }
 
 template <typename T, int KP, int kMinBlocks>
-__global__ void __launch_bounds__(kThreads, kMinBlocks) k_front_flow(DevFactor F, DevWork W, const T* gv, T* lx,
-                                                                     T* ub, const int* ready, const int* n_ready,
+__global__ void __launch_bounds__(kThreads, kMinBlocks) k_front_flow(DevFactor F, DevWork W, SolveVecs sv, const T* gv,
+                                                                     T* lx, T* ub, const int* ready, const int* n_ready,
                                                                      const int8_t* phase, int ph,
                                                                      const int32_t* nchild, int* counter, int* cnt) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -919,7 +994,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) k_front_flow(DevFactor F
         int s = ready[item];
         while (s >= 0) {
             if (!front_frozen(F, W, s))
-                front_factor<KP>(F, W, gv, lx, ub, s, reinterpret_cast<T*>(smem_raw), sm);
+                front_factor<KP>(F, W, sv, gv, lx, ub, s, reinterpret_cast<T*>(smem_raw), sm);
             __syncthreads();
             s = continue_up(F, phase, ph, nchild, cnt, s, &slot);
         }
@@ -946,8 +1021,8 @@ __device__ __forceinline__ int lower_bound_i32(const int* a, int lo, int hi, int
 // block's target range and its contributing children with their column and
 // row ranges come from the host schedule (AsmItem / AsmChild).
 template <typename T>
-__global__ void __launch_bounds__(kThreads) k_big_assemble(DevFactor F, DevWork W, const T* gv, T* lx, T* ub,
-                                                           const AsmItem* work, const AsmChild* kids) {
+__global__ void __launch_bounds__(kThreads) k_big_assemble(DevFactor F, DevWork W, SolveVecs sv, const T* gv, T* lx,
+                                                           T* ub, const AsmItem* work, const AsmChild* kids) {
     const AsmItem wk = work[blockIdx.x];
     const int s = wk.s, tj = wk.tj, rb = wk.rb;
     if (front_frozen(F, W, s)) return;  // the whole CTA, before any barrier
@@ -956,6 +1031,12 @@ __global__ void __launch_bounds__(kThreads) k_big_assemble(DevFactor F, DevWork 
     const int c0 = tj * kTile, c1 = min(c0 + kTile, f);
     const int R0 = c0 + rb * kAsmRows, R1 = min(R0 + kAsmRows, f);
     const int tid = threadIdx.x, nth = blockDim.x;
+    // Row block 0 also assembles the tile column's right-hand-side entries (b of
+    // its pivots, the children's solve update vectors): it holds the diagonal,
+    // so its list has every child with a column here.
+    __shared__ T vv[kTile];
+    const int p0 = F.sn_c0[s], nc = F.sn_c0[s + 1] - p0;
+    if (rb == 0 && tid < kTile) vv[tid] = c0 + tid < nc ? static_cast<const T*>(sv.rhs)[p0 + c0 + tid] : T(0);
     for (int x = tid; x < (c1 - c0) * (R1 - R0); x += nth) {
         const int c = c0 + x / (R1 - R0), r = R0 + x % (R1 - R0);
         if (r >= c) B[r + (int64_t)c * f] = T(0);
@@ -974,6 +1055,8 @@ __global__ void __launch_bounds__(kThreads) k_big_assemble(DevFactor F, DevWork 
         const T* U = update_of<T>(F, lx, ub, c);
         const int uld = F.sn_u_ld[c];
         const int lane = tid & 31, warp = tid >> 5, nwarp = nth >> 5;
+        if (rb == 0 && warp == nwarp - 1 && ch.j0 + lane < ch.j1)
+            vv[rel[ch.j0 + lane] - c0] += static_cast<const T*>(sv.su)[F.sn_su_off[c] + ch.j0 + lane];
         for (int j = ch.j0 + warp; j < ch.j1; j += nwarp) {
             const int64_t pj = (int64_t)rel[j] * f;
             const T* Uj = U + (int64_t)j * uld;
@@ -993,6 +1076,7 @@ __global__ void __launch_bounds__(kThreads) k_big_assemble(DevFactor F, DevWork 
         }
         __syncthreads();
     }
+    if (rb == 0 && tid < c1 - c0) *rhs_entry<T>(sv, p0, nc, F.sn_su_off[s], c0 + tid) = vv[tid];
 }
 
 // FP64 panel step p of the tiled fronts: the diagonal block's factorisation
@@ -1015,8 +1099,8 @@ __global__ void __launch_bounds__(kThreads) k_big_assemble(DevFactor F, DevWork 
 // step in about 37k cycles (18 us), where one warp's factorisation of the block
 // and a launch of one-warp row solves took 47 + 22 us; the linear solve of a
 // 30k-bus grid went from 5.04 to 3.08 ms with this and k_big_update64.
-__global__ void __launch_bounds__(kPanelThreads64) k_big_panel64(DevFactor F, DevWork W, double* lx, const int4* work,
-                                                                 int p, int* step_cnt) {
+__global__ void __launch_bounds__(kPanelThreads64) k_big_panel64(DevFactor F, DevWork W, SolveVecs sv, double* lx,
+                                                                 const int4* work, int p, int* step_cnt) {
     static_assert(kPanelThreads64 == 256 && kPanelRows64 == 16 && kTile == 32, "thread tiling below");
     constexpr int kW = kPanelThreads64 / 32, kQ = kTile / kW;  // columns per warp
     __shared__ double us[kTile][kTile + kPanelRows64];  // column k: block rows, then chunk rows
@@ -1033,9 +1117,12 @@ __global__ void __launch_bounds__(kPanelThreads64) k_big_panel64(DevFactor F, De
     const int p0 = p * kTile;
     const int pb = min(kTile, nc - p0);
     const int r0 = p0 + pb + chunk * kPanelRows64;
-    const int nr = min(kPanelRows64, f - r0);  // <= 0: no rows below the block
+    const int nr = min(kPanelRows64, f + 1 - r0);  // row f: the right-hand side
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int xr = lane & (kPanelRows64 - 1), xh = lane >> 4;
+    // entry (r0 + xr, p0 + c) of the chunk: column stride 1 in the right-hand-side row
+    double* const xb = r0 + xr == f ? static_cast<double*>(sv.sol) + c0 + p0 : B + (r0 + xr) + (int64_t)p0 * f;
+    const int64_t xld = r0 + xr == f ? 1 : f;
     if (threadIdx.x == 0) ready = ready_x = -1;
     double a[kQ], x[kQ / 2];  // columns w + kW q; chunk columns w + kW (2 h + xh)
 #pragma unroll
@@ -1046,7 +1133,7 @@ __global__ void __launch_bounds__(kPanelThreads64) k_big_panel64(DevFactor F, De
 #pragma unroll
     for (int h = 0; h < kQ / 2; ++h) {
         const int c = w + kW * (2 * h + xh);
-        x[h] = (c < pb && xr < nr) ? B[(r0 + xr) + (int64_t)(p0 + c) * f] : 0.0;
+        x[h] = (c < pb && xr < nr) ? xb[c * xld] : 0.0;
     }
     __syncthreads();
     bool bad = false;
@@ -1126,7 +1213,7 @@ __global__ void __launch_bounds__(kPanelThreads64) k_big_panel64(DevFactor F, De
 #pragma unroll
     for (int h = 0; h < kQ / 2; ++h) {
         const int c = w + kW * (2 * h + xh);
-        if (c < pb && xr < nr) B[(r0 + xr) + (int64_t)(p0 + c) * f] = x[h] * dk[c];
+        if (c < pb && xr < nr) xb[c * xld] = x[h] * dk[c];
     }
     if (last) {
 #pragma unroll
@@ -1155,8 +1242,8 @@ __device__ __forceinline__ T ld_entry(const T* p) {
 // tile last (a counter per front and step) writes L_dd^-1 into it for the
 // solves: no CTA reads an overwritten tile, and none waits for another.
 template <bool kL2>
-__device__ __forceinline__ void big_panel32_item(const DevFactor& F, const DevWork& W, float* lx, int s, int p,
-                                                 int chunk, int nchunk, int pair, int* step_cnt) {
+__device__ __forceinline__ void big_panel32_item(const DevFactor& F, const DevWork& W, const SolveVecs& sv, float* lx,
+                                                 int s, int p, int chunk, int nchunk, int pair, int* step_cnt) {
     static_assert(kThreads == 256 && kPanelRows == 128 && kTile == 32, "thread tiling below");
     constexpr int ld = kTile + 4;          // 16-byte aligned rows
     constexpr int lt_ld = kTile + 4;       // 16-byte aligned rows
@@ -1172,7 +1259,7 @@ __device__ __forceinline__ void big_panel32_item(const DevFactor& F, const DevWo
     float* B = lx + F.sn_lx_off[s];
     const int p0 = p * kTile;
     const int pb = min(kTile, nc - p0);
-    const int r0 = p0 + pb + chunk * kPanelRows;    // first row of the chunk
+    const int r0 = p0 + pb + chunk * kPanelRows;     // first row of the chunk
     const int nr = max(0, min(kPanelRows, f - r0));  // its rows
     const int tid = threadIdx.x;
     // From the second step on, the previous step's trailing update has already
@@ -1225,6 +1312,18 @@ __device__ __forceinline__ void big_panel32_item(const DevFactor& F, const DevWo
         warp_trinv_v4<kTile, ld>(reinterpret_cast<const float (*)[ld]>(D), rdiag, pb, i, Lt, lt_ld);
     }
     __syncthreads();
+    if (chunk == 0 && tid < 32) {
+        // y = L_dd^-1 v of the block's right-hand-side entries, a lane per row
+        float* yv = static_cast<float*>(sv.sol) + F.sn_c0[s] + p0;
+        const float v = tid < pb ? ld_entry<kL2>(yv + tid) : 0.f;
+        float y = 0.f;
+#pragma unroll
+        for (int j = 0; j < kTile; ++j) {
+            const float vj = __shfl_sync(0xffffffffu, v, j);
+            if (j <= tid && j < pb) y += Lt[j * lt_ld + tid] * vj;
+        }
+        if (tid < pb) yv[tid] = y;
+    }
     {
         // thread (rg, cg): rows 4rg..4rg+3, columns 4cg..4cg+3 of the chunk
         const int cg = tid & 7, rg = tid >> 3;
@@ -1262,11 +1361,11 @@ __device__ __forceinline__ void big_panel32_item(const DevFactor& F, const DevWo
     }
 }
 
-__global__ void __launch_bounds__(kThreads) k_big_panel32(DevFactor F, DevWork W, float* lx, const int4* work, int p,
-                                                          int* step_cnt) {
+__global__ void __launch_bounds__(kThreads) k_big_panel32(DevFactor F, DevWork W, SolveVecs sv, float* lx,
+                                                          const int4* work, int p, int* step_cnt) {
     const int4 wk = work[blockIdx.x];
     if (front_frozen(F, W, wk.x)) return;  // the whole CTA, before any barrier
-    big_panel32_item<false>(F, W, lx, wk.x, p, wk.y, wk.z, wk.w, step_cnt);
+    big_panel32_item<false>(F, W, sv, lx, wk.x, p, wk.y, wk.z, wk.w, step_cnt);
 }
 
 // FP32 trailing update of step p: the kUpdTile x kUpdTile tile (ti, tj) -= A_i A_j^T
@@ -1277,8 +1376,8 @@ __global__ void __launch_bounds__(kThreads) k_big_panel32(DevFactor F, DevWork W
 // two per FMA), and its read-modify-writes of a column touch 16 consecutive
 // rows per half warp.
 template <bool kL2>
-__device__ __forceinline__ void big_update_item(const DevFactor& F, const DevWork& W, float* lx, int s, int p, int ti,
-                                                int tj) {
+__device__ __forceinline__ void big_update_item(const DevFactor& F, const DevWork& W, const SolveVecs& sv, float* lx,
+                                                int s, int p, int ti, int tj) {
     using T = float;
     static_assert(kThreads == 256 && kUpdTile == 32, "thread tiling below");
     constexpr int ld = kUpdTile + 1;
@@ -1298,6 +1397,19 @@ __device__ __forceinline__ void big_update_item(const DevFactor& F, const DevWor
         Aj[k * ld + r] = (k < pb && C0 + r < f) ? ld_entry<kL2>(col + C0 + r) : T(0);
     }
     __syncthreads();
+    if (ti == tj && threadIdx.x >= kThreads - 32) {
+        // the last warp of a diagonal tile: the tile's right-hand-side entries,
+        // a lane per column
+        const int c = threadIdx.x & 31, gc = C0 + c;
+        if (gc >= q0 && gc < f) {
+            const T* y = static_cast<const T*>(sv.sol) + F.sn_c0[s] + p0;
+            T* v = rhs_entry<T>(sv, F.sn_c0[s], nc, F.sn_su_off[s], gc);
+            T acc = ld_entry<kL2>(v);
+#pragma unroll 8
+            for (int k = 0; k < pb; ++k) acc -= Aj[k * ld + c] * ld_entry<kL2>(y + k);
+            *v = acc;
+        }
+    }
     const int tr = threadIdx.x & 15, tc = threadIdx.x >> 4;
     T acc[2][2] = {{T(0), T(0)}, {T(0), T(0)}};
 #pragma unroll 4
@@ -1359,10 +1471,11 @@ __device__ __forceinline__ void big_update_item(const DevFactor& F, const DevWor
     }
 }
 
-__global__ void __launch_bounds__(kThreads) k_big_update32(DevFactor F, DevWork W, float* lx, const int4* work, int p) {
+__global__ void __launch_bounds__(kThreads) k_big_update32(DevFactor F, DevWork W, SolveVecs sv, float* lx,
+                                                           const int4* work, int p) {
     const int4 wk = work[blockIdx.x];
     if (front_frozen(F, W, wk.x)) return;  // the whole CTA, before any barrier
-    big_update_item<false>(F, W, lx, wk.x, p, wk.y, wk.z);
+    big_update_item<false>(F, W, sv, lx, wk.x, p, wk.y, wk.z);
 }
 
 // FP64 trailing update of step p, one CTA per kUpdTile64 x kUpdTile64 tile
@@ -1370,10 +1483,10 @@ __global__ void __launch_bounds__(kThreads) k_big_update32(DevFactor F, DevWork 
 // the tile is small: a 32 x 32 tile kept its SM for 16k cycles while a step
 // of a single grid has fewer such tiles than the GPU has SMs (30k-bus grid:
 // 12.5 us a step with 32 x 32 tiles, 5.8 us with 16 x 16).
-__global__ void __launch_bounds__(kUpdTile64 * kUpdTile64) k_big_update64(DevFactor F, DevWork W, double* lx,
-                                                                          const int4* work, int p) {
+__global__ void __launch_bounds__(kUpdTile64 * kUpdTile64) k_big_update64(DevFactor F, DevWork W, SolveVecs sv,
+                                                                          double* lx, const int4* work, int p) {
     constexpr int kN = kUpdTile64, kAll = kN * kN;
-    __shared__ double Ai[kTile][kN + 1], Aj[kTile][kN + 1];  // [k][row]
+    __shared__ double Ai[kTile][kN + 1], Aj[kTile][kN + 1];  // [k][row]; Ai's last column: y
     const int4 wk = work[blockIdx.x];
     const int s = wk.x;
     if (front_frozen(F, W, s)) return;  // the whole CTA, before any barrier
@@ -1386,18 +1499,30 @@ __global__ void __launch_bounds__(kUpdTile64 * kUpdTile64) k_big_update64(DevFac
     const int R0 = wk.y * kN, C0 = wk.z * kN;
     const int tr = threadIdx.x % kN, tc = threadIdx.x / kN;
     const int gr = R0 + tr, gc = C0 + tc;
-    const bool mine = gc >= q0 && gc < f && gr >= gc && gr < f;
+    // A diagonal tile's right-hand-side entries v_j -= sum y_k X_jk fall to
+    // threads above the diagonal: (j, j + 1), and (0, last) for the last column.
+    const bool diag = wk.y == wk.z;
+    const bool rhs = diag && (tc == tr + 1 || (tr == 0 && tc == kN - 1));
+    const int jv = (tc == tr + 1) ? tr : kN - 1;
+    bool mine = gc >= q0 && gc < f && gr >= gc && gr < f;
     double* dst = B + gr + (int64_t)gc * f;
+    if (rhs) {
+        mine = C0 + jv >= q0 && C0 + jv < f;
+        if (mine) dst = rhs_entry<double>(sv, F.sn_c0[s], nc, F.sn_su_off[s], C0 + jv);
+    }
     double acc = mine ? *dst : 0.0;
 #pragma unroll
     for (int k = tc; k < kTile; k += kAll / kN) {
         const double* col = B + (int64_t)(p0 + k) * f;
         Ai[k][tr] = (k < pb && R0 + tr < f) ? col[R0 + tr] : 0.0;
         Aj[k][tr] = (k < pb && C0 + tr < f) ? col[C0 + tr] : 0.0;
+        if (diag && tr == 0) Ai[k][kN] = k < pb ? static_cast<const double*>(sv.sol)[F.sn_c0[s] + p0 + k] : 0.0;
     }
     __syncthreads();
+    const double* ai = &Ai[0][rhs ? kN : tr];
+    const double* aj = &Aj[0][rhs ? jv : tc];
 #pragma unroll 8
-    for (int k = 0; k < pb; ++k) acc = fma(-Ai[k][tr], Aj[k][tc], acc);
+    for (int k = 0; k < pb; ++k) acc = fma(-ai[k * (kN + 1)], aj[k * (kN + 1)], acc);
     if (mine) *dst = acc;
 }
 
@@ -1434,7 +1559,7 @@ __device__ __forceinline__ bool wait_tile(const int* flag, uint32_t* status, lon
 // timed out, publish without computing.
 constexpr int kTileFlowBlocks = 3;
 __global__ void __launch_bounds__(kThreads, kTileFlowBlocks)
-    k_big_flow32(DevFactor F, DevWork W, float* lx, const TileTask* tasks, int n, int* done, int* counter,
+    k_big_flow32(DevFactor F, DevWork W, SolveVecs sv, float* lx, const TileTask* tasks, int n, int* done, int* counter,
                  int* step_cnt) {
     constexpr int kWords = sizeof(TileTask) / sizeof(int);
     static_assert(kWords <= 32, "one lane per task word");
@@ -1476,9 +1601,9 @@ __global__ void __launch_bounds__(kThreads, kTileFlowBlocks)
         __syncthreads();
         if (!skip) {
             if (t.kind == 0)
-                big_panel32_item<true>(F, W, lx, t.s, t.p, t.a, t.b, t.aux, step_cnt);
+                big_panel32_item<true>(F, W, sv, lx, t.s, t.p, t.a, t.b, t.aux, step_cnt);
             else
-                big_update_item<true>(F, W, lx, t.s, t.p, t.a, t.b);
+                big_update_item<true>(F, W, sv, lx, t.s, t.p, t.a, t.b);
         }
         __syncthreads();
         if (tid == 0) publish_done(done + item);
@@ -1497,12 +1622,6 @@ __global__ void __launch_bounds__(kThreads, kTileFlowBlocks)
 // dot products against the solved rows (backward) use every thread with
 // coalesced reads of the column-major panel.
 // ---------------------------------------------------------------------------
-struct SolveVecs {
-    const void* rhs;  // [n_state] right-hand side, permuted (V)
-    void* sol;        // [n_state] solution, permuted (V)
-    void* su;         // solve update vectors (V)
-};
-
 // Forward step of a warp front: v = [b of own columns; 0] + children's update
 // vectors (in child order), y = L11^-1 v1, update vector v2 - L21 y.
 template <typename T, typename V>
@@ -1863,8 +1982,8 @@ template <typename T>
 constexpr int kMinBlocksW = sizeof(T) == 4 ? 4 : 2;
 
 template <typename T>
-__global__ void __launch_bounds__(kThreads, kMinBlocksW<T>) k_front_warp(DevFactor F, DevWork W, const T* gv, T* lx,
-                                                                         T* ub, const int* ready, const int* n_ready,
+__global__ void __launch_bounds__(kThreads, kMinBlocksW<T>) k_front_warp(DevFactor F, DevWork W, SolveVecs sv, const T* gv,
+                                                                         T* lx, T* ub, const int* ready, const int* n_ready,
                                                                          const int8_t* phase, int ph,
                                                                          const int32_t* nchild, int* counter,
                                                                          int* cnt) {
@@ -1876,7 +1995,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocksW<T>) k_front_warp(DevFact
         if (item >= nr) break;
         int s = ready[item];
         while (s >= 0) {
-            if (!front_frozen(F, W, s)) warp_front_factor<T>(F, W, gv, lx, ub, s, t);
+            if (!front_frozen(F, W, s)) warp_front_factor<T>(F, W, sv, gv, lx, ub, s, t);
             s = warp_continue_up(F, phase, ph, nchild, cnt, s);
         }
     }
@@ -2048,7 +2167,7 @@ cudaError_t prepare_impl() {
 template <typename T, typename HV>
 cudaError_t factor_impl(const DevNet& net, const DevFactor& F, const DevWork& W, const LevelSchedule& ls, const HV* hval,
                         const HV* hw,
-                        T* lx, T* ub, cudaStream_t st) {
+                        T* lx, T* ub, SolveVecs sv, cudaStream_t st) {
     T* gv = reinterpret_cast<T*>(W.gvals);
     if (ls.n_tgt > 0) {
         if (sizeof(T) == 4 && ls.gain_acc32)
@@ -2057,26 +2176,29 @@ cudaError_t factor_impl(const DevNet& net, const DevFactor& F, const DevWork& W,
             k_gain_values<T, HV, double><<<grid_for(ls.n_tgt, 256), 256, 0, st>>>(F, W, hval, hw, gv, ls.n_tgt);
         count_launches(1);
     }
-    if (ls.flow_a_n + ls.flow_b_n + ls.flow_w_n > 0) {
-        cudaError_t e = cudaMemsetAsync(W.flow, 0, sizeof(int) * (size_t)(F.n_super + 8), st);
+    {
+        // the flags and counters of the factorisation and of the backward sweep after it
+        cudaError_t e = cudaMemsetAsync(W.flow, 0, sizeof(int) * (3 * (size_t)F.n_super + 16), st);
         if (e != cudaSuccess) return e;
+    }
+    if (ls.flow_a_n + ls.flow_b_n + ls.flow_w_n > 0) {
         int* counters = W.flow + F.n_super;
         if (ls.flow_w_n > 0) {
             k_front_warp<T><<<ls.flow_w_grid, kThreads, sizeof(WarpTile<T>) * kWarpsPerCta, st>>>(
-                F, W, gv, lx, ub, ls.d_flow_w, ls.d_ready_n + 4, ls.d_phase, 3, ls.d_phase_nchild, counters + 2,
+                F, W, sv, gv, lx, ub, ls.d_flow_w, ls.d_ready_n + 4, ls.d_phase, 3, ls.d_phase_nchild, counters + 2,
                 W.flow);
             count_launches(1);
         }
         if (ls.flow_a_n > 0) {
             const int mf = ls.flow_a_maxf;
             k_front_flow<T, kPanelSmall, kMinBlocksA<T>><<<ls.flow_a_grid, kThreads, front_smem<T>(mf), st>>>(
-                F, W, gv, lx, ub, ls.d_flow_a, ls.d_ready_n + 0, ls.d_phase, 1, ls.d_phase_nchild, counters + 0, W.flow);
+                F, W, sv, gv, lx, ub, ls.d_flow_a, ls.d_ready_n + 0, ls.d_phase, 1, ls.d_phase_nchild, counters + 0, W.flow);
             count_launches(1);
         }
         if (ls.flow_b_n > 0) {
             const int mf = ls.flow_b_maxf;
             k_front_flow<T, kPanel, 1><<<ls.flow_b_grid, kThreads, front_smem<T>(mf), st>>>(
-                F, W, gv, lx, ub, ls.d_flow_b, ls.d_ready_n + 1, ls.d_phase, 2, ls.d_phase_nchild, counters + 1, W.flow);
+                F, W, sv, gv, lx, ub, ls.d_flow_b, ls.d_ready_n + 1, ls.d_phase, 2, ls.d_phase_nchild, counters + 1, W.flow);
             count_launches(1);
         }
     }
@@ -2093,19 +2215,20 @@ cudaError_t factor_impl(const DevNet& net, const DevFactor& F, const DevWork& W,
         const int ns = ls.h_small_ptr[l + 1] - ls.h_small_ptr[l];
         if (ns > 0) {
             const int mf = ls.h_small_maxf[l];
-            k_front_small<T><<<ns, kThreads, front_smem<T>(mf), st>>>(F, W, gv, lx, ub,
-                                                                                  ls.d_small + ls.h_small_ptr[l]);
+            k_front_small<T><<<ns, kThreads, front_smem<T>(mf), st>>>(F, W, sv, gv, lx, ub,
+                                                                      ls.d_small + ls.h_small_ptr[l]);
             count_launches(1);
         }
         const int na = ls.h_asm_ptr[l + 1] - ls.h_asm_ptr[l];
         if (na > 0) {
-            k_big_assemble<T><<<na, kThreads, 0, st>>>(F, W, gv, lx, ub, ls.d_asm + ls.h_asm_ptr[l], ls.d_asm_child);
+            k_big_assemble<T><<<na, kThreads, 0, st>>>(F, W, sv, gv, lx, ub, ls.d_asm + ls.h_asm_ptr[l],
+                                                   ls.d_asm_child);
             count_launches(1);
             const int nt = tile_flow ? ls.h_tt_ptr[l + 1] - ls.h_tt_ptr[l] : 0;
             if constexpr (sizeof(T) == 4) {
                 if (nt > 0) {
                     k_big_flow32<<<std::min(nt, ls.tt_grid), kThreads, 0, st>>>(
-                        F, W, lx, ls.d_tt + ls.h_tt_ptr[l], nt, ls.d_tt_done + ls.h_tt_ptr[l],
+                        F, W, sv, lx, ls.d_tt + ls.h_tt_ptr[l], nt, ls.d_tt_done + ls.h_tt_ptr[l],
                         ls.d_tt_done + ls.n_tt + l, ls.d_pot_cnt);
                     count_launches(1);
                 }
@@ -2117,17 +2240,17 @@ cudaError_t factor_impl(const DevNet& net, const DevFactor& F, const DevWork& W,
                 if (npot > 0) {
                     const int4* work = ls.d_pot + ls.h_pot_ptr[slot];
                     if constexpr (sizeof(T) == 4)
-                        k_big_panel32<<<npot, kThreads, 0, st>>>(F, W, lx, work, p, ls.d_pot_cnt);
+                        k_big_panel32<<<npot, kThreads, 0, st>>>(F, W, sv, lx, work, p, ls.d_pot_cnt);
                     else
-                        k_big_panel64<<<npot, kPanelThreads64, 0, st>>>(F, W, lx, work, p, ls.d_pot_cnt);
+                        k_big_panel64<<<npot, kPanelThreads64, 0, st>>>(F, W, sv, lx, work, p, ls.d_pot_cnt);
                     count_launches(1);
                 }
                 if (nupd > 0) {
                     const int4* work = ls.d_upd + ls.h_upd_ptr[slot];
                     if constexpr (sizeof(T) == 4)
-                        k_big_update32<<<nupd, kThreads, 0, st>>>(F, W, lx, work, p);
+                        k_big_update32<<<nupd, kThreads, 0, st>>>(F, W, sv, lx, work, p);
                     else
-                        k_big_update64<<<nupd, kUpdTile64 * kUpdTile64, 0, st>>>(F, W, lx, work, p);
+                        k_big_update64<<<nupd, kUpdTile64 * kUpdTile64, 0, st>>>(F, W, sv, lx, work, p);
                     count_launches(1);
                 }
             }
@@ -2136,31 +2259,39 @@ cudaError_t factor_impl(const DevNet& net, const DevFactor& F, const DevWork& W,
     return cudaGetLastError();
 }
 
+// Forward and backward sweeps (forward), or the backward sweep alone after a
+// factorisation that carried the right-hand side along (factor_impl, which
+// also cleared the flags).
 template <typename T>
 cudaError_t solve_impl(const DevFactor& F, const DevWork& W, const LevelSchedule& ls, const T* lx, const T* rdiag,
-                       SolveVecs sv, cudaStream_t st) {
+                       SolveVecs sv, bool forward, cudaStream_t st) {
     if (ls.solve_flow) {
         // flags: [0, n_super) forward, [n_super, 2 n_super) backward, then counters
         const int ns = F.n_super;
         int* fwd_done = W.flow + ns + 8;
         int* bwd_done = fwd_done + ns;
         int* counters = bwd_done + ns;
-        cudaError_t e = cudaMemsetAsync(fwd_done, 0, sizeof(int) * (size_t)(2 * ns + 8), st);
-        if (e != cudaSuccess) return e;
         const size_t smem = solve_smem<T>(ls.solve_maxf);
         // warp fronts first going up, last coming down
-        if (ls.flow_w_n > 0) {
-            k_fwd_warp<T, T><<<ls.solve_w_grid, kThreads, 0, st>>>(F, W, lx, rdiag, sv, ls.d_flow_w, ls.d_ready_n + 4,
-                                                                   ls.d_phase, 3, ls.d_phase_nchild, counters + 2,
-                                                                   fwd_done);
-            count_launches(1);
+        if (forward) {
+            cudaError_t e = cudaMemsetAsync(fwd_done, 0, sizeof(int) * (size_t)(2 * ns + 8), st);
+            if (e != cudaSuccess) return e;
+            if (ls.flow_w_n > 0) {
+                k_fwd_warp<T, T><<<ls.solve_w_grid, kThreads, 0, st>>>(F, W, lx, rdiag, sv, ls.d_flow_w,
+                                                                       ls.d_ready_n + 4, ls.d_phase, 3,
+                                                                       ls.d_phase_nchild, counters + 2, fwd_done);
+                count_launches(1);
+            }
+            if (ls.up_n > 0) {
+                k_fwd_flow<T, T><<<ls.up_grid, kThreads, smem, st>>>(F, W, lx, rdiag, sv, ls.d_up, ls.d_ready_n + 2,
+                                                                     ls.d_nchild, counters + 0, fwd_done);
+                count_launches(1);
+            }
         }
         if (ls.up_n > 0) {
-            k_fwd_flow<T, T><<<ls.up_grid, kThreads, smem, st>>>(F, W, lx, rdiag, sv, ls.d_up, ls.d_ready_n + 2,
-                                                                 ls.d_nchild, counters + 0, fwd_done);
             k_bwd_flow<T, T><<<ls.solve_grid, kThreads, smem, st>>>(F, W, lx, rdiag, sv, ls.d_down, ls.d_ready_n + 3,
                                                                     counters + 1, bwd_done);
-            count_launches(2);
+            count_launches(1);
         }
         if (ls.down_w_n > 0) {
             k_bwd_warp<T, T><<<ls.solve_w_grid, kThreads, 0, st>>>(F, W, lx, rdiag, sv, ls.d_down_w, ls.d_ready_n + 5,
@@ -2169,7 +2300,7 @@ cudaError_t solve_impl(const DevFactor& F, const DevWork& W, const LevelSchedule
         }
         return cudaGetLastError();
     }
-    for (int l = 0; l < ls.n_levels; ++l) {
+    for (int l = 0; forward && l < ls.n_levels; ++l) {
         const int n = ls.h_all_ptr[l + 1] - ls.h_all_ptr[l];
         if (n > 0) {
             k_fwd<T, T><<<n, kThreads, solve_smem<T>(ls.h_lvl_maxf[l]), st>>>(F, lx, rdiag, sv,
@@ -2239,24 +2370,29 @@ cudaError_t prepare_factor_kernels() {
     return e;
 }
 
+namespace {
+SolveVecs vecs32(const DevWork& W) { return SolveVecs{W.rhs32, W.sol32, W.su32}; }
+SolveVecs vecs64(const DevWork& W) { return SolveVecs{W.rhs, W.sol, W.su}; }
+}  // namespace
+
 cudaError_t launch_factor32(const DevNet& net, const DevFactor& F, const DevWork& W, const LevelSchedule& ls,
                             cudaStream_t st) {
-    return factor_impl<float, float>(net, F, W, ls, W.hval32, W.hw32, W.lx32, W.u32, st);
+    return factor_impl<float, float>(net, F, W, ls, W.hval32, W.hw32, W.lx32, W.u32, vecs32(W), st);
 }
 
-cudaError_t launch_solve32(const DevFactor& F, const DevWork& W, const LevelSchedule& ls, cudaStream_t st) {
-    return solve_impl<float>(F, W, ls, W.lx32, reinterpret_cast<const float*>(W.rdiag),
-                             SolveVecs{W.rhs32, W.sol32, W.su32}, st);
+cudaError_t launch_solve32(const DevFactor& F, const DevWork& W, const LevelSchedule& ls, bool forward,
+                           cudaStream_t st) {
+    return solve_impl<float>(F, W, ls, W.lx32, reinterpret_cast<const float*>(W.rdiag), vecs32(W), forward, st);
 }
 
 cudaError_t launch_factor(const DevNet& net, const DevFactor& F, const DevWork& W, const LevelSchedule& ls,
                           cudaStream_t st) {
-    return factor_impl<double, double>(net, F, W, ls, W.hval, W.hw, W.lx, W.u, st);
+    return factor_impl<double, double>(net, F, W, ls, W.hval, W.hw, W.lx, W.u, vecs64(W), st);
 }
 
-cudaError_t launch_solve(const DevFactor& F, const DevWork& W, const LevelSchedule& ls, cudaStream_t st) {
-    return solve_impl<double>(F, W, ls, W.lx, reinterpret_cast<const double*>(W.rdiag),
-                              SolveVecs{W.rhs, W.sol, W.su}, st);
+cudaError_t launch_solve(const DevFactor& F, const DevWork& W, const LevelSchedule& ls, bool forward,
+                         cudaStream_t st) {
+    return solve_impl<double>(F, W, ls, W.lx, reinterpret_cast<const double*>(W.rdiag), vecs64(W), forward, st);
 }
 
 cudaError_t launch_gain_export(const DevNet& net, const DevFactor& F, const DevWork& W, int32_t n_tgt, double* out,
@@ -2365,10 +2501,8 @@ cudaError_t launch_factor_solve_noalloc(const DevNet& net, const DevFactor& F, c
         k_state_to_ps<<<grid_for(n, 256), 256, 0, st>>>(net, F, d_rhs, W2.rhs);
         count_launches(1);
     }
-    e = factor_impl<double, double>(net, F, W2, ls, W2.hval, W2.hw, W2.lx, W2.u, st);
-    if (e == cudaSuccess)
-        e = solve_impl<double>(F, W2, ls, W2.lx, reinterpret_cast<const double*>(W2.rdiag),
-                               SolveVecs{W2.rhs, W2.sol, W2.su}, st);
+    e = launch_factor(net, F, W2, ls, st);
+    if (e == cudaSuccess) e = launch_solve(F, W2, ls, false, st);
     if (e != cudaSuccess) return e;
     if (n > 0) {
         k_ps_to_state<<<grid_for(n, 256), 256, 0, st>>>(net, F, W2.sol, d_x);

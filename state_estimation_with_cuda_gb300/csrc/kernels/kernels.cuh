@@ -439,13 +439,19 @@ constexpr int kUpdTile64 = 16;
 // Sets the kernel attributes (dynamic shared memory limits) on the current
 // device; call before launching or capturing the factorisation.
 cudaError_t prepare_factor_kernels();
+// The factorisation carries the right-hand side (DevWork::rhs, FP32: rhs32)
+// along and leaves y = L^-1 b in sol (sol32); launch_solve with forward =
+// false then runs the backward sweep.  With forward = true it solves for a new
+// right-hand side with the factor at hand.
 cudaError_t launch_factor(const DevNet& net, const DevFactor& f, const DevWork& w, const LevelSchedule& ls,
                           cudaStream_t st);
-cudaError_t launch_solve(const DevFactor& f, const DevWork& w, const LevelSchedule& ls, cudaStream_t st);
+cudaError_t launch_solve(const DevFactor& f, const DevWork& w, const LevelSchedule& ls, bool forward,
+                         cudaStream_t st);
 // FP32 gain / factor and mixed solves (FP32 L, FP64 vectors).
 cudaError_t launch_factor32(const DevNet& net, const DevFactor& f, const DevWork& w, const LevelSchedule& ls,
                             cudaStream_t st);
-cudaError_t launch_solve32(const DevFactor& f, const DevWork& w, const LevelSchedule& ls, cudaStream_t st);
+cudaError_t launch_solve32(const DevFactor& f, const DevWork& w, const LevelSchedule& ls, bool forward,
+                           cudaStream_t st);
 
 // Kernels launched by this library since load (all engines of the process).
 extern std::atomic<int64_t> g_kernel_launches;
@@ -463,12 +469,12 @@ constexpr int32_t kSmallFrontMax = 160;
 constexpr int32_t kSmallFrontMax32 = 224;
 template <typename T>
 __host__ __device__ constexpr int32_t small_front_max() { return sizeof(T) == 4 ? kSmallFrontMax32 : kSmallFrontMax; }
-// Leading dimension of a front held in shared memory: f rounded up to a
-// multiple of 4 elements (16-byte aligned columns; 4-row tiles stay inside
-// their column).
+// Leading dimension of a front held in shared memory: its f rows, in FP64 also
+// the right-hand side as row f, rounded up to a multiple of 4 elements (16-byte
+// aligned columns; 4-row tiles stay inside their column).
 template <typename T>
 __host__ __device__ constexpr int32_t front_ld(int32_t f) {
-    return (f + 3) / 4 * 4;
+    return (f + (sizeof(T) == 8 ? 1 : 0) + 3) / 4 * 4;
 }
 template <typename T>
 __host__ __device__ constexpr size_t front_smem(int32_t f) {
