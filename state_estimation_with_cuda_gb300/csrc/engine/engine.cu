@@ -436,6 +436,39 @@ void Engine::build_schedule(bool targets_ready) {
             flow_phase_[s] = (warp_phase[front_grid[s]] && sub_maxf[s] <= kWarpFrontMax)
                                  ? 3
                                  : (sub_maxf[s] <= flow_small_f ? 1 : 2);
+    // assembly lists of the single-CTA fronts, by front and warp
+    asm_slot_.assign(ns, 0);
+    asm_ptr_.assign(1, 0);
+    asm_ent_.clear();
+    {
+        int32_t slots = 0;
+        int64_t total = 0;
+        for (int32_t s = 0; s < ns; ++s)
+            if (!big[s] && flow_phase_[s] != 3) {
+                asm_slot_[s] = slots++;
+                for (int32_t ci = P.sn_child_ptr[s]; ci < P.sn_child_ptr[s + 1]; ++ci) {
+                    const int32_t c = P.sn_child[ci];
+                    total += P.sn_f[c] - (P.sn_c0[c + 1] - P.sn_c0[c]);
+                }
+            }
+        asm_ptr_.reserve(static_cast<size_t>(kAsmWarps) * slots + 1);
+        asm_ent_.reserve(total);
+        std::vector<int2> list[kAsmWarps];
+        for (int32_t s = 0; s < ns; ++s) {
+            if (big[s] || flow_phase_[s] == 3) continue;
+            for (auto& l : list) l.clear();
+            for (int32_t ci = P.sn_child_ptr[s]; ci < P.sn_child_ptr[s + 1]; ++ci) {
+                const int32_t c = P.sn_child[ci];
+                const int32_t m = P.sn_f[c] - (P.sn_c0[c + 1] - P.sn_c0[c]);
+                const int32_t* rel = P.sn_relmap.data() + P.sn_su_off[c];
+                for (int32_t j = 0; j < m; ++j) list[rel[j] % kAsmWarps].push_back(make_int2(ci, j | rel[j] << 16));
+            }
+            for (const auto& l : list) {
+                asm_ent_.insert(asm_ent_.end(), l.begin(), l.end());
+                asm_ptr_.push_back(static_cast<int32_t>(asm_ent_.size()));
+            }
+        }
+    }
     int64_t lx = 0, uu = 0;
     for (int32_t s = 0; s < ns; ++s) {
         const int64_t f = P.sn_f[s], nc = P.sn_c0[s + 1] - P.sn_c0[s];
@@ -741,6 +774,10 @@ int32_t Engine::upload() {
         fac_.sn_u_ld = c.take<int32_t>(ns);
         fac_.sn_u_big = c.take<uint8_t>(ns);
         fac_.sn_pw = c.take<int8_t>(ns);
+        fac_.rec = c.take<FrontRec>(ns);
+        fac_.child_rec = c.take<ChildRec>(P.sn_child.size());
+        fac_.asm_ptr = c.take<int32_t>(asm_ptr_.size());
+        fac_.asm_ent = c.take<int2>(asm_ent_.size());
         fac_.sn_grid = batch_mode() ? c.take<int32_t>(ns) : nullptr;
         fac_.tgt_grid = batch_mode() ? c.take<int32_t>(P.tgt_local.size()) : nullptr;
         fac_.ps_grid = batch_mode() ? c.take<int32_t>(P.n_state) : nullptr;
@@ -942,6 +979,44 @@ int32_t Engine::upload() {
     chk(put(const_cast<int32_t*>(fac_.bus_ps_v), P.bus_ps_v, st_));
     chk(put(const_cast<int32_t*>(fac_.sn_u_ld), lay_u_ld_, st_));
     chk(put(const_cast<uint8_t*>(fac_.sn_u_big), lay_u_big_, st_));
+    chk(put(const_cast<int32_t*>(fac_.asm_ptr), asm_ptr_, st_));
+    chk(put(const_cast<int2*>(fac_.asm_ent), asm_ent_, st_));
+    std::vector<FrontRec> recs(ns);
+    std::vector<ChildRec> child_recs(P.sn_child.size());
+    {
+        std::vector<int32_t> grid_of(ns, 0);
+        if (batch_mode()) {
+            int32_t x = 0;
+            for (size_t g = 0; g < grid_plans_.size(); ++g)
+                for (int32_t k = 0; k < grid_plans_[g].n_super; ++k) grid_of[x++] = static_cast<int32_t>(g);
+        }
+        for (int32_t s = 0; s < ns; ++s) {
+            FrontRec& r = recs[s];
+            r = FrontRec{};
+            r.c0 = P.sn_c0[s];
+            r.nc = P.sn_c0[s + 1] - P.sn_c0[s];
+            r.f = P.sn_f[s];
+            r.parent = P.sn_parent[s];
+            r.tgt0 = P.sn_tgt_ptr[s];
+            r.tgt1 = P.sn_tgt_ptr[s + 1];
+            r.ch0 = P.sn_child_ptr[s];
+            r.ch1 = P.sn_child_ptr[s + 1];
+            r.lx_off = lay_lx_off_[s];
+            r.u_off = lay_u_off_[s];
+            r.su_off = P.sn_su_off[s];
+            const bool up = r.parent >= 0 && flow_phase_[s] != 0 && flow_phase_[r.parent] == flow_phase_[s];
+            r.up_n = up ? phase_nchild_[r.parent] : 0;
+            r.grid = grid_of[s];
+            r.asm_slot = asm_slot_[s];
+        }
+        for (size_t x = 0; x < P.sn_child.size(); ++x) {
+            const int32_t c = P.sn_child[x];
+            child_recs[x] = ChildRec{lay_u_off_[c], P.sn_su_off[c], P.sn_f[c] - (P.sn_c0[c + 1] - P.sn_c0[c]),
+                                     lay_u_ld_[c], lay_u_big_[c], 0};
+        }
+    }
+    chk(put(const_cast<FrontRec*>(fac_.rec), recs, st_));
+    chk(put(const_cast<ChildRec*>(fac_.child_rec), child_recs, st_));
     if (batch_mode()) {
         const int32_t G = static_cast<int32_t>(grids_.size());
         std::vector<int32_t> sg, boff(G + 1, 0), moff(G + 1, 0);

@@ -274,6 +274,9 @@ private:
     std::vector<int2> ev_unit_, ev_grp_;  // evaluation units (DevNet::ev_unit / ev_grp)
     void build_eval_units();
     std::vector<AsmChild> sch_asm_child_;
+    // assembly lists of the single-CTA fronts (DevFactor::asm_ptr / asm_ent)
+    std::vector<int32_t> asm_slot_, asm_ptr_;
+    std::vector<int2> asm_ent_;
     // FP32 tiled fronts as dataflow items (TileTask), per level
     std::vector<TileTask> sch_tt_;
     std::vector<int32_t> sch_tt_ptr_;

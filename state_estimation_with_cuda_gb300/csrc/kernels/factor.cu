@@ -76,6 +76,9 @@ __device__ __forceinline__ uint32_t* singular_flags(const DevFactor& F, const De
 __device__ __forceinline__ bool front_frozen(const DevFactor& F, const DevWork& W, int s) {
     return W.grid_flags && (W.grid_flags[F.sn_grid[s]] & FLAG_FROZEN);
 }
+__device__ __forceinline__ bool front_frozen(const DevWork& W, const FrontRec& R) {
+    return W.grid_flags && (W.grid_flags[R.grid] & FLAG_FROZEN);
+}
 
 // Positive and finite?  FP64 by the bit pattern: an FP64 comparison or
 // conversion occupies the FP64 pipe for 64 cycles, as any FP64 instruction.
@@ -130,70 +133,122 @@ __device__ __forceinline__ const T* update_of(const DevFactor& F, const T* lx, c
     return (F.sn_u_big[c] ? lx : ub) + F.sn_u_off[c];
 }
 
-// Extend-add of every child of front s with no barrier between children:
-// warp w owns the front's target columns t with t % nwarp == w and walks the
-// children in order, adding only into its own columns, so no two warps touch
-// the same entry and each entry's additions keep the children's order.  Per
-// child, the warp selects its columns 32 at a time (ballot over the relative
-// map), then loads up to four of them (four rows per lane each) before it
-// scatters them.  The child's solve update vector is added to the front's
+// Extend-add of every child of a single-CTA front with no barrier between
+// children: warp w owns the front's columns t with t % kAsmWarps == w and
+// walks its list of the children's columns (DevFactor::asm_ent, in child
+// order), so no two warps touch the same entry and each entry's additions keep
+// the children's order.  Bound: load latency.  The 32 list entries and child
+// records of a round are fetched a lane each; columns go eight at a time, 32
+// rows a step, the next step's loads in flight while this one is added (as a
+// walk over the children, each warp selecting its columns, the chain of
+// dependent loads per child made the assembly half of a front's time).  Columns
+// of a step with the same target (from different children) are added one after
+// the other; if any is longer than a step, the eight are cut before the second
+// of the two.  The children's solve update vectors are added to the front's
 // right-hand side (entry t at rhs[t * rhs_ld]) the same way.  The caller
-// follows with a block barrier.
+// follows with a block barrier.  Measured on the longest chain of a 10k-bus
+// grid (mixed): 19k -> 7.6k cycles for 4 children of a 73-row front, 97k -> 65k
+// for the 40 children of the 217-row root (one SM's L2 bandwidth).
 template <typename T>
 __device__ __forceinline__ void extend_add_children(const DevFactor& F, const SolveVecs& sv, const T* lx,
-                                                    const T* ubase, int s, T* dst, int ldd, T* rhs, int rhs_ld) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
-    for (int ci = F.sn_child_ptr[s]; ci < F.sn_child_ptr[s + 1]; ++ci) {
-        const int c = F.sn_child[ci];
-        const int m = F.sn_f[c] - (F.sn_c0[c + 1] - F.sn_c0[c]);
-        const T* U = update_of<T>(F, lx, ubase, c);
-        const int uld = F.sn_u_ld[c];
-        const int64_t so = F.sn_su_off[c];
-        const int* rel = F.sn_relmap + so;
-        for (int j0 = 0; j0 < m; j0 += 32) {
-            const int jl = j0 + lane;
-            const int tj = (jl < m) ? rel[jl] : -1;
-            unsigned own = __ballot_sync(0xffffffffu, tj >= 0 && (tj % nwarp) == warp);
-            if ((own >> lane) & 1u) rhs[tj * rhs_ld] += __ldcg(static_cast<const T*>(sv.su) + so + jl);
-            while (own) {
-                int js[4];
-                int cnt = 0;
+                                                    const T* ubase, const FrontRec& R, T* dst, int ldd, T* rhs,
+                                                    int rhs_ld) {
+    constexpr unsigned kAll = 0xffffffffu;
+    constexpr int kB = 8;  // columns per step
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int e1 = F.asm_ptr[R.asm_slot * kAsmWarps + warp + 1];
+    for (int eb = F.asm_ptr[R.asm_slot * kAsmWarps + warp]; eb < e1; eb += 32) {
+        const int n = min(32, e1 - eb);
+        const T* up = nullptr;
+        const int* rel = nullptr;
+        int len = 0, t = 0;  // rows from the diagonal down, target column
+        T bv = T(0);
+        if (lane < n) {
+            const int2 en = F.asm_ent[eb + lane];
+            const ChildRec c = F.child_rec[en.x];
+            const int j = en.y & 0xffff;
+            t = en.y >> 16;
+            len = c.m - j;
+            up = (c.big ? lx : ubase) + c.u_off + (int64_t)j * c.ld + j;
+            rel = F.sn_relmap + c.su_off + j;
+            bv = __ldcg(static_cast<const T*>(sv.su) + c.su_off + j);
+        }
+        // the entry before with the same target (-1: none of this round)
+        const unsigned before = __match_any_sync(kAll, lane < n ? t : -1 - lane) & ((1u << lane) - 1u);
+        const int prev = 31 - __clz(before);
+        // the batch from column q0: its columns, its longest one, shared targets
+        struct Batch {
+            int q0, cnt, longest;
+            bool dup;
+        };
+        auto batch = [&](int q0) {
+            Batch z;
+            z.q0 = q0;
+            z.cnt = min(kB, n - q0);
+            const bool in = lane >= q0 && lane < q0 + z.cnt;
+            z.longest = __reduce_max_sync(kAll, in ? len : 0);
+            const unsigned cut = __ballot_sync(kAll, in && prev >= q0);
+            z.dup = cut != 0u;
+            if (z.dup && z.longest > 32) {
+                z.cnt = __ffs(cut) - 1 - q0;
+                z.dup = false;
+            }
+            return z;
+        };
+        T u[kB], un[kB];
+        int ri[kB], rn[kB];
+        auto load = [&](const Batch& z, int ib, T (&x)[kB], int (&r)[kB]) {
 #pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    js[q] = -1;
-                    if (own) {
-                        const int b = __ffs(own) - 1;
-                        own &= own - 1;
-                        js[q] = j0 + b;
-                        ++cnt;
-                    }
+            for (int k = 0; k < kB; ++k) {
+                const int q = z.q0 + k, row = ib + lane;
+                const T* p = reinterpret_cast<const T*>(__shfl_sync(kAll, reinterpret_cast<unsigned long long>(up), q));
+                const int* rp =
+                    reinterpret_cast<const int*>(__shfl_sync(kAll, reinterpret_cast<unsigned long long>(rel), q));
+                const bool ok = row < __shfl_sync(kAll, len, q) && k < z.cnt;
+                x[k] = ok ? __ldcg(p + row) : T(0);
+                r[k] = ok ? rp[row] : -1;
+            }
+        };
+        Batch z = batch(0);
+        load(z, 0, u, ri);
+        int ib = 0;
+        for (;;) {
+            Batch zn = z;
+            int nib = ib + 32;
+            bool more = true;
+            if (nib >= z.longest) {
+                nib = 0;
+                more = z.q0 + z.cnt < n;
+                if (more) zn = batch(z.q0 + z.cnt);
+            }
+            if (more) load(zn, nib, un, rn);
+            int to[kB];
+#pragma unroll
+            for (int k = 0; k < kB; ++k) to[k] = ri[k] + __shfl_sync(kAll, t, z.q0 + k) * ldd;
+            if (!z.dup) {
+                if (ib == 0 && lane >= z.q0 && lane < z.q0 + z.cnt) rhs[t * rhs_ld] += bv;
+                T cur[kB];
+#pragma unroll
+                for (int k = 0; k < kB; ++k) cur[k] = ri[k] >= 0 ? dst[to[k]] : T(0);
+#pragma unroll
+                for (int k = 0; k < kB; ++k)
+                    if (ri[k] >= 0) dst[to[k]] = cur[k] + u[k];
+            } else {
+#pragma unroll
+                for (int k = 0; k < kB; ++k) {
+                    if (lane == z.q0 + k && k < z.cnt) rhs[t * rhs_ld] += bv;  // a batch of one step
+                    if (ri[k] >= 0) dst[to[k]] += u[k];
+                    __syncwarp();
                 }
-                const int jmin = js[0];  // the smallest column has the most rows
-                for (int ib = 0;; ib += 128) {
-                    T u[4][4];
-                    int ri[4][4];
+            }
+            __syncwarp();
+            if (!more) break;
+            z = zn;
+            ib = nib;
 #pragma unroll
-                    for (int q = 0; q < 4; ++q)
-#pragma unroll
-                        for (int t = 0; t < 4; ++t) {
-                            const int j = js[q];
-                            const int i = j + ib + lane + 32 * t;
-                            const bool ok = j >= 0 && i < m;
-                            u[q][t] = ok ? __ldcg(U + (int64_t)j * uld + i) : T(0);
-                            ri[q][t] = ok ? rel[i] : -1;
-                        }
-#pragma unroll
-                    for (int q = 0; q < 4; ++q) {
-                        const int j = js[q];
-                        if (j < 0) continue;
-                        const int pj = __shfl_sync(0xffffffffu, tj, j - j0) * ldd;
-#pragma unroll
-                        for (int t = 0; t < 4; ++t)
-                            if (ri[q][t] >= 0) dst[ri[q][t] + pj] += u[q][t];
-                    }
-                    if (jmin + ib + 128 >= m) break;
-                }
-                (void)cnt;
+            for (int k = 0; k < kB; ++k) {
+                u[k] = un[k];
+                ri[k] = rn[k];
             }
         }
     }
@@ -347,8 +402,27 @@ __device__ __forceinline__ int warp_claim(int* counter) {
     return __shfl_sync(0xffffffffu, item, 0);
 }
 
-// Lane 0 counts finished front s into its parent when the parent belongs to
-// the same phase; returns the parent when this completed its last child.
+// Counts a finished front into its parent when the parent belongs to the same
+// phase (R.up_n > 0); returns the parent when this completed its last child.
+// One thread, after the barrier that ends the front.
+__device__ __forceinline__ int count_up(const FrontRec& R, int* cnt) {
+    if (R.up_n <= 0) return -1;
+    int seen;
+    asm volatile("fence.acq_rel.gpu;" ::: "memory");
+    asm volatile("atom.add.relaxed.gpu.global.s32 %0, [%1], 1;" : "=r"(seen) : "l"(cnt + R.parent) : "memory");
+    if (seen + 1 != R.up_n) return -1;
+    asm volatile("fence.acq_rel.gpu;" ::: "memory");
+    return R.parent;
+}
+__device__ __forceinline__ int warp_continue_up(const FrontRec& R, int* cnt) {
+    __syncwarp();
+    int nxt = -1;
+    if ((threadIdx.x & 31) == 0) nxt = count_up(R, cnt);
+    nxt = __shfl_sync(0xffffffffu, nxt, 0);
+    __syncwarp();
+    return nxt;
+}
+// The forward sweep's counts go by its own children numbers.
 __device__ __forceinline__ int warp_continue_up(const DevFactor& F, const int8_t* phase, int ph, const int32_t* nchild,
                                                 int* cnt, int s) {
     __syncwarp();
@@ -368,104 +442,161 @@ __device__ __forceinline__ int warp_continue_up(const DevFactor& F, const int8_t
     return nxt;
 }
 
+// One warp: assembly in its tile, then the partial factorisation column by
+// column (left-looking): a pivot column takes the updates of the columns
+// before it in one accumulator a lane, and the trailing columns take theirs at
+// the end, four at a time, straight into the update matrix.  Every entry gets
+// the operations of the right-looking order in the same order, without its
+// read-modify-write of the tile per pivot (one shared-memory round trip per
+// entry and pivot was three quarters of a front's time).  FP64 packs the
+// trailing triangle into whole warps: an FP64 instruction costs 64 cycles
+// whatever its lanes do.  Measured on a 301-bus grid's chain of six warp fronts:
+// 73 -> 46 us (mixed), on a 30k-bus grid's 172 -> 108 us (FP64).
 template <typename T>
 __device__ void warp_front_factor(const DevFactor& F, const DevWork& W, const SolveVecs& sv, const T* gv, T* lx, T* ub,
-                                  int s, WarpTile<T>& t) {
+                                  const FrontRec& R, int s, WarpTile<T>& t) {
+    constexpr unsigned kAll = 0xffffffffu;
+    constexpr int kB = 8;  // a child's columns per step
     const int lane = threadIdx.x & 31;
-    const int f = F.sn_f[s];
-    const int c0 = F.sn_c0[s];
-    const int nc = F.sn_c0[s + 1] - c0;
-    for (int c = 0; c < f; ++c) t.a[c * kWtLd + lane] = T(0);
-    t.v[lane] = lane < nc ? static_cast<const T*>(sv.rhs)[c0 + lane] : T(0);
-    __syncwarp();
-    {
-        // original entries, four per lane in flight
-        const int tg0 = F.sn_tgt_ptr[s], tg1 = F.sn_tgt_ptr[s + 1];
-        for (int tb = tg0; tb < tg1; tb += 128) {
-            T g[4];
-            int l[4];
+    const int f = R.f, c0 = R.c0, nc = R.nc;
+    // original entries, four per lane in flight while the tile is cleared
+    const T b0 = lane < nc ? static_cast<const T*>(sv.rhs)[c0 + lane] : T(0);
+    for (int tb = R.tgt0; tb < R.tgt1 || tb == R.tgt0; tb += 128) {
+        T g[4];
+        int l[4];
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const int tg = tb + lane + 32 * q;
-                l[q] = tg < tg1 ? F.tgt_local[tg] : -1;  // row + col * f
-                g[q] = tg < tg1 ? gv[tg] : T(0);
-            }
-#pragma unroll
-            for (int q = 0; q < 4; ++q)
-                if (l[q] >= 0) {
-                    const int c = l[q] / f;
-                    t.a[c * kWtLd + (l[q] - c * f)] = g[q];
-                }
+        for (int q = 0; q < 4; ++q) {
+            const int tg = tb + lane + 32 * q;
+            l[q] = tg < R.tgt1 ? F.tgt_local[tg] : -1;  // row + col * f
+            g[q] = tg < R.tgt1 ? gv[tg] : T(0);
         }
+        if (tb == R.tgt0) {
+            for (int c = 0; c < f; ++c) t.a[c * kWtLd + lane] = T(0);
+            t.v[lane] = b0;
+            __syncwarp();
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+            if (l[q] >= 0) {
+                const int c = l[q] / f;
+                t.a[c * kWtLd + (l[q] - c * f)] = g[q];
+            }
     }
     __syncwarp();
-    for (int ci = F.sn_child_ptr[s]; ci < F.sn_child_ptr[s + 1]; ++ci) {
-        const int ch = F.sn_child[ci];
-        const int m = F.sn_f[ch] - (F.sn_c0[ch + 1] - F.sn_c0[ch]);  // < kWarpFrontMax: the parent holds m rows
-        const T* U = update_of<T>(F, lx, ub, ch);
-        const int uld = F.sn_u_ld[ch];
-        const int64_t so = F.sn_su_off[ch];
-        const int ri = lane < m ? F.sn_relmap[so + lane] : 0;
-        if (lane < m) t.v[ri] += __ldcg(static_cast<const T*>(sv.su) + so + lane);
-        for (int j = 0; j < m; j += 4) {
-            T u[4];
-#pragma unroll
-            for (int q = 0; q < 4; ++q)
-                u[q] = (j + q < m && lane >= j + q && lane < m) ? __ldcg(U + lane + (int64_t)(j + q) * uld) : T(0);
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const int rj = __shfl_sync(0xffffffffu, ri, (j + q) & 31);
-                if (j + q < m && lane >= j + q && lane < m) t.a[rj * kWtLd + ri] += u[q];
-            }
+    for (int cb = R.ch0; cb < R.ch1; cb += 32) {
+        const int n = min(32, R.ch1 - cb);
+        const T* up = nullptr;
+        long long so = 0;
+        int m = 0, ld = 0;
+        if (lane < n) {
+            const ChildRec c = F.child_rec[cb + lane];
+            up = (c.big ? lx : ub) + c.u_off;
+            so = c.su_off;
+            m = c.m;
+            ld = c.ld;
         }
-        __syncwarp();
+        // steps of kB columns of a child, the next step's loads in flight
+        T u[kB], un[kB], bv, bn;
+        int ri, rn;
+        auto load = [&](int ch, int j0, T (&x)[kB], int& r, T& b) {
+            const T* p = reinterpret_cast<const T*>(__shfl_sync(kAll, reinterpret_cast<unsigned long long>(up), ch));
+            const long long o = __shfl_sync(kAll, so, ch);
+            const int mm = __shfl_sync(kAll, m, ch), ll = __shfl_sync(kAll, ld, ch);
+            r = lane < mm ? F.sn_relmap[o + lane] : 0;
+            b = lane < mm && j0 == 0 ? __ldcg(static_cast<const T*>(sv.su) + o + lane) : T(0);
+#pragma unroll
+            for (int k = 0; k < kB; ++k)
+                x[k] = (j0 + k < mm && lane >= j0 + k && lane < mm) ? __ldcg(p + lane + (int64_t)(j0 + k) * ll) : T(0);
+        };
+        load(0, 0, u, ri, bv);
+        int ch = 0, j0 = 0;
+        for (;;) {
+            const int mm = __shfl_sync(kAll, m, ch);
+            int nch = ch, nj = j0 + kB;
+            if (nj >= mm) {
+                nch = ch + 1;
+                nj = 0;
+            }
+            const bool more = nch < n;
+            if (more) load(nch, nj, un, rn, bn);
+            if (j0 == 0 && lane < mm) t.v[ri] += bv;
+            T cur[kB];
+            int to[kB];
+#pragma unroll
+            for (int k = 0; k < kB; ++k) {
+                to[k] = __shfl_sync(kAll, ri, (j0 + k) & 31) * kWtLd + ri;
+                if (!(j0 + k < mm && lane >= j0 + k && lane < mm)) to[k] = -1;
+                cur[k] = to[k] >= 0 ? t.a[to[k]] : T(0);
+            }
+#pragma unroll
+            for (int k = 0; k < kB; ++k)
+                if (to[k] >= 0) t.a[to[k]] = cur[k] + u[k];
+            __syncwarp();
+            if (!more) break;
+            ch = nch;
+            j0 = nj;
+            ri = rn;
+            bv = bn;
+#pragma unroll
+            for (int k = 0; k < kB; ++k) u[k] = un[k];
+        }
     }
-    // Right-looking elimination of the first nc columns in the tile, lane i
-    // owning row i; the trailing columns receive the Schur complement.  The
-    // loops are bounded by the front's own size (warp fronts are narrow:
-    // median 16 rows, 4 columns), which keeps the kernel small enough for the
-    // instruction cache.
     T my_inv = T(0);
     // FP64: the forward substitution rides along, row i's right-hand side in
     // lane i.  FP32 applies L11^-1 below, as the forward sweep does.
     T vi = t.v[lane];
     bool bad = false;
     for (int k = 0; k < nc; ++k) {
-        T d = t.a[k * kWtLd + k];
+        T a = t.a[k * kWtLd + lane];
+#pragma unroll 4
+        for (int p = 0; p < k; ++p) a -= t.a[p * kWtLd + lane] * t.a[p * kWtLd + k];
+        T d = __shfl_sync(kAll, a, k);
         const bool badk = !pivot_ok(d);
         bad |= badk;
         d = badk ? T(1) : d;
         T sq, inv;
         pivot_value(d, &sq, &inv);
         const bool below = lane > k && lane < f;
-        const T lik = below ? t.a[k * kWtLd + lane] * inv : T(0);
+        const T lik = a * inv;
         if constexpr (!kInvDiag<T>) {
-            const T yk = __shfl_sync(0xffffffffu, vi, k) * inv;
+            const T yk = __shfl_sync(kAll, vi, k) * inv;
             vi = lane == k ? yk : (below ? vi - lik * yk : vi);
         }
-        __syncwarp();  // column k read by every lane before it is overwritten
         if (lane == k) {
             t.a[k * kWtLd + k] = sq;
             my_inv = inv;
         }
         if (below) t.a[k * kWtLd + lane] = lik;
         __syncwarp();
-        if (below)
-            for (int j = k + 1; j <= lane; ++j) t.a[j * kWtLd + lane] -= lik * t.a[k * kWtLd + j];
-        __syncwarp();
     }
     if (bad && lane == 0) atomicOr(singular_flags(F, W, s), FLAG_SINGULAR);
     if (lane < nc) reinterpret_cast<T*>(W.rdiag)[c0 + lane] = my_inv;
-    T* L = lx + F.sn_lx_off[s];
+    T* L = lx + R.lx_off;
     const int row0 = kInvDiag<T> ? nc : 0;  // FP32 writes its diagonal block as L11^-1 below
     if (lane < f)
         for (int c = 0; c < nc; ++c)
             if (lane >= c && lane >= row0) L[lane + c * f] = t.a[c * kWtLd + lane];
     const int m = f - nc;
-    T* Uo = ub + F.sn_u_off[s];
-    for (int j = nc; j < f; ++j)
-        if (lane >= j && lane < f) Uo[(lane - nc) + (j - nc) * m] = t.a[j * kWtLd + lane];
+    T* Uo = ub + R.u_off;
     if constexpr (kInvDiag<T>) {
+        for (int j = nc; j < f; j += 4) {
+            T a[4];
+            int jq[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                jq[q] = min(j + q, f - 1);
+                a[q] = t.a[jq[q] * kWtLd + lane];
+            }
+#pragma unroll 2
+            for (int p = 0; p < nc; ++p) {
+                const T li = t.a[p * kWtLd + lane];
+#pragma unroll
+                for (int q = 0; q < 4; ++q) a[q] -= li * t.a[p * kWtLd + jq[q]];
+            }
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                if (j + q < f && lane >= j + q && lane < f) Uo[(lane - nc) + (j + q - nc) * m] = a[q];
+        }
         // column j of L11^-1 by forward substitution, lane j; its entries
         // x_i (i > j) are kept transposed in the tile's free upper triangle,
         // at (row j, column i)
@@ -475,6 +606,7 @@ __device__ void warp_front_factor(const DevFactor& F, const DevWork& W, const So
             const int j = lane;
             for (int i = j + 1; i < nc; ++i) {
                 T acc = -t.a[j * kWtLd + i] * my_inv;  // L_ij x_j with x_j = 1 / L_jj
+#pragma unroll 4
                 for (int k = j + 1; k < i; ++k) acc -= t.a[k * kWtLd + i] * t.a[k * kWtLd + j];
                 t.a[i * kWtLd + j] = acc * t.rinv[i];
             }
@@ -482,22 +614,39 @@ __device__ void warp_front_factor(const DevFactor& F, const DevWork& W, const So
         __syncwarp();
         // L11^-1 into the diagonal block: lane i writes row i; y = L11^-1 v1
         T y = T(0);
-        if (lane < nc)
+        if (lane < nc) {
+#pragma unroll 4
             for (int j = 0; j <= lane; ++j) {
                 const T l = (j == lane) ? my_inv : t.a[lane * kWtLd + j];
                 L[lane + j * f] = l;
                 y += l * t.v[j];
             }
+        }
         __syncwarp();
         if (lane < nc) {
             t.v[lane] = y;
             vi = y;
         }
         __syncwarp();
-        if (lane >= nc)
+        if (lane >= nc) {
+#pragma unroll 4
             for (int k = 0; k < nc; ++k) vi -= t.a[k * kWtLd + lane] * t.v[k];
+        }
+    } else {
+        // the lower triangle folded (column p with column m - 1 - p) into rows of m + 1 entries
+        const int total = m * (m + 1) / 2;
+        for (int e = lane; e < total; e += 32) {
+            const int pr = e / (m + 1), pos = e - pr * (m + 1);
+            const bool first = pos < m - pr;
+            const int j = nc + (first ? pr : m - 1 - pr);
+            const int i = j + (first ? pos : pos - (m - pr));
+            T a = t.a[j * kWtLd + i];
+#pragma unroll 4
+            for (int p = 0; p < nc; ++p) a -= t.a[p * kWtLd + i] * t.a[p * kWtLd + j];
+            Uo[(i - nc) + (j - nc) * m] = a;
+        }
     }
-    if (lane < f) *rhs_entry<T>(sv, c0, nc, F.sn_su_off[s], lane) = vi;
+    if (lane < f) *rhs_entry<T>(sv, c0, nc, R.su_off, lane) = vi;
 }
 
 // 1 / d of a pivot, by the same means (y (1 + e + e^2), e = 1 - d y); a d
@@ -576,41 +725,48 @@ struct FrontSmem<double> {
 // (y = L11^-1 v per panel, then the rows below column by column): same bits.
 template <typename T>
 __device__ __forceinline__ void front_assemble(const DevFactor& F, const SolveVecs& sv, const T* gv, const T* lx,
-                                               const T* ub, int s, int f, int c0, int nc, T* Fm, T* rhs, int rhs_ld) {
+                                               const T* ub, const FrontRec& R, T* Fm, T* rhs, int rhs_ld) {
+    const int f = R.f, c0 = R.c0, nc = R.nc;
     const int ldf = front_ld<T>(f);
     const int tid = threadIdx.x, nth = blockDim.x;
-    for (int x = tid; x < ldf * f; x += nth) Fm[x] = T(0);
-    __syncthreads();
-    if (ldf == f) {
-        for (int tg = F.sn_tgt_ptr[s] + tid; tg < F.sn_tgt_ptr[s + 1]; tg += nth) Fm[F.tgt_local[tg]] = gv[tg];
+    // the first targets in flight while the front is cleared
+    const bool has = R.tgt0 + tid < R.tgt1;
+    const int l0 = has ? F.tgt_local[R.tgt0 + tid] : 0;  // row + col * f
+    const T g0 = has ? gv[R.tgt0 + tid] : T(0);
+    if constexpr (sizeof(T) == 4) {
+        for (int x = 4 * tid; x < ldf * f; x += 4 * nth) *reinterpret_cast<float4*>(Fm + x) = make_float4(0.f, 0.f, 0.f, 0.f);
     } else {
-        for (int tg = F.sn_tgt_ptr[s] + tid; tg < F.sn_tgt_ptr[s + 1]; tg += nth) {
-            const int l = F.tgt_local[tg];  // row + col * f
-            const int c = l / f;
-            Fm[(l - c * f) + c * ldf] = gv[tg];
-        }
+        for (int x = 2 * tid; x < ldf * f; x += 2 * nth) *reinterpret_cast<double2*>(Fm + x) = make_double2(0.0, 0.0);
     }
+    __syncthreads();
+    auto at = [&](int l) {
+        const int c = l / f;
+        return (l - c * f) + c * ldf;
+    };
+    if (has) Fm[at(l0)] = g0;
+    for (int tg = R.tgt0 + tid + nth; tg < R.tgt1; tg += nth) Fm[at(F.tgt_local[tg])] = gv[tg];
     for (int r = tid; r < f; r += nth) rhs[r * rhs_ld] = r < nc ? static_cast<const T*>(sv.rhs)[c0 + r] : T(0);
     __syncthreads();
-    extend_add_children<T>(F, sv, lx, ub, s, Fm, ldf, rhs, rhs_ld);
+    extend_add_children<T>(F, sv, lx, ub, R, Fm, ldf, rhs, rhs_ld);
     __syncthreads();
 }
 
 // The finished front's L panel, update matrix and right-hand side to the factor
 // and solve arrays.
 template <typename T>
-__device__ __forceinline__ void front_store(const DevFactor& F, const SolveVecs& sv, T* lx, T* ub, int s, int f,
-                                            int c0, int nc, const T* Fm, const T* rhs, int rhs_ld) {
+__device__ __forceinline__ void front_store(const SolveVecs& sv, T* lx, T* ub, const FrontRec& R, const T* Fm,
+                                            const T* rhs, int rhs_ld) {
+    const int f = R.f, c0 = R.c0, nc = R.nc;
     const int ldf = front_ld<T>(f);
     const int tid = threadIdx.x, nth = blockDim.x, lane = tid & 31, warp = tid >> 5;
-    for (int r = tid; r < f; r += nth) *rhs_entry<T>(sv, c0, nc, F.sn_su_off[s], r) = rhs[r * rhs_ld];
-    T* L = lx + F.sn_lx_off[s];
+    for (int r = tid; r < f; r += nth) *rhs_entry<T>(sv, c0, nc, R.su_off, r) = rhs[r * rhs_ld];
+    T* L = lx + R.lx_off;
     for (int x = tid; x < f * nc; x += nth) {
         const int c = x / f;
         L[x] = Fm[(x - c * f) + c * ldf];
     }
     const int m = f - nc;
-    T* U = ub + F.sn_u_off[s];
+    T* U = ub + R.u_off;
     const int nwarp = nth >> 5;
     for (int j = warp; j < m; j += nwarp)
         for (int i = lane; i < m; i += 32) U[i + (int64_t)j * m] = Fm[(nc + i) + (nc + j) * ldf];
@@ -630,16 +786,14 @@ __device__ __forceinline__ void front_store(const DevFactor& F, const SolveVecs&
 // update: phase B 337 -> 202 us, phase A 261 -> 159, synchronous levels 82 -> 50.
 template <int KP>
 __device__ void front_factor(const DevFactor& F, const DevWork& W, const SolveVecs& sv, const double* gv, double* lx,
-                             double* ub, int s, double* Fm, FrontSmem<double>& sm) {
+                             double* ub, const FrontRec& R, int s, double* Fm, FrontSmem<double>& sm) {
     static_assert(KP <= kPanel && kThreads == 256, "columns over eight warps");
     constexpr int kW = kThreads / 32, kQ = KP / kW;
     constexpr int kG = ((KP == kPanel ? kSmallFrontMax : kFlowSmallFMax) + 1 + 31) / 32;  // row groups of 32
-    const int f = F.sn_f[s];
+    const int f = R.f, c0 = R.c0, nc = R.nc;
     const int ldf = front_ld<double>(f);
-    const int c0 = F.sn_c0[s];
-    const int nc = F.sn_c0[s + 1] - c0;
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-    front_assemble<double>(F, sv, gv, lx, ub, s, f, c0, nc, Fm, Fm + f, ldf);
+    front_assemble<double>(F, sv, gv, lx, ub, R, Fm, Fm + f, ldf);
     double* rdg = reinterpret_cast<double*>(W.rdiag) + c0;
     uint32_t* status = &W.status->flags;
 #pragma unroll 1
@@ -761,22 +915,20 @@ __device__ void front_factor(const DevFactor& F, const DevWork& W, const SolveVe
         }
         __syncthreads();
     }
-    front_store<double>(F, sv, lx, ub, s, f, c0, nc, Fm, Fm + f, ldf);
+    front_store<double>(sv, lx, ub, R, Fm, Fm + f, ldf);
 }
 
 // FP32, with panels of KP <= kPanel columns.
 template <int KP>
 __device__ void front_factor(const DevFactor& F, const DevWork& W, const SolveVecs& sv, const float* gv, float* lx,
-                             float* ub, int s, float* Fm, FrontSmem<float>& sm) {
+                             float* ub, const FrontRec& R, int s, float* Fm, FrontSmem<float>& sm) {
     using T = float;
     static_assert(KP <= kPanel && KP <= 32, "panel wider than a warp");
-    const int f = F.sn_f[s];
+    const int f = R.f, c0 = R.c0, nc = R.nc;
     const int ldf = front_ld<T>(f);
-    const int c0 = F.sn_c0[s];
-    const int nc = F.sn_c0[s + 1] - c0;
     const int tid = threadIdx.x, nth = blockDim.x;
     const int lane = tid & 31, warp = tid >> 5;
-    front_assemble<T>(F, sv, gv, lx, ub, s, f, c0, nc, Fm, sm.v, 1);
+    front_assemble<T>(F, sv, gv, lx, ub, R, Fm, sm.v, 1);
     // v_i -= L_i,k0.. y of a finished panel, by threads [t0, t0 + nt)
     auto rhs_below = [&](int k0, int kb, int t0, int nt) {
         for (int i = k0 + kb + tid - t0; tid >= t0 && i < f; i += nt) {
@@ -900,7 +1052,7 @@ __device__ void front_factor(const DevFactor& F, const DevWork& W, const SolveVe
     const int kl = (nc - 1) / KP * KP;  // the last panel (nc > 0)
     rhs_below(kl, nc - kl, 0, nth);
     __syncthreads();
-    front_store<T>(F, sv, lx, ub, s, f, c0, nc, Fm, sm.v, 1);
+    front_store<T>(sv, lx, ub, R, Fm, sm.v, 1);
 }
 
 // Panel widths: fronts of the high-occupancy dataflow phase (f <= 64) use
@@ -916,8 +1068,9 @@ __global__ void __launch_bounds__(kThreads, 1) k_front_small(DevFactor F, DevWor
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ FrontSmem<T> sm;
     const int s = fronts[blockIdx.x];
-    if (front_frozen(F, W, s)) return;
-    front_factor<kPanel>(F, W, sv, gv, lx, ub, s, reinterpret_cast<T*>(smem_raw), sm);
+    const FrontRec R = F.rec[s];
+    if (front_frozen(W, R)) return;
+    front_factor<kPanel>(F, W, sv, gv, lx, ub, R, s, reinterpret_cast<T*>(smem_raw), sm);
 }
 
 // ---------------------------------------------------------------------------
@@ -982,8 +1135,7 @@ __device__ __forceinline__ int continue_up(const DevFactor& F, const int8_t* pha
 template <typename T, int KP, int kMinBlocks>
 __global__ void __launch_bounds__(kThreads, kMinBlocks) k_front_flow(DevFactor F, DevWork W, SolveVecs sv, const T* gv,
                                                                      T* lx, T* ub, const int* ready, const int* n_ready,
-                                                                     const int8_t* phase, int ph,
-                                                                     const int32_t* nchild, int* counter, int* cnt) {
+                                                                     int* counter, int* cnt) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ FrontSmem<T> sm;
     __shared__ int slot;
@@ -993,10 +1145,13 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) k_front_flow(DevFactor F
         if (item >= nr) break;
         int s = ready[item];
         while (s >= 0) {
-            if (!front_frozen(F, W, s))
-                front_factor<KP>(F, W, sv, gv, lx, ub, s, reinterpret_cast<T*>(smem_raw), sm);
+            const FrontRec R = F.rec[s];
+            if (!front_frozen(W, R)) front_factor<KP>(F, W, sv, gv, lx, ub, R, s, reinterpret_cast<T*>(smem_raw), sm);
             __syncthreads();
-            s = continue_up(F, phase, ph, nchild, cnt, s, &slot);
+            if (threadIdx.x == 0) slot = count_up(R, cnt);
+            __syncwarp();
+            __syncthreads();
+            s = slot;
         }
     }
 }
@@ -1984,9 +2139,7 @@ constexpr int kMinBlocksW = sizeof(T) == 4 ? 4 : 2;
 template <typename T>
 __global__ void __launch_bounds__(kThreads, kMinBlocksW<T>) k_front_warp(DevFactor F, DevWork W, SolveVecs sv, const T* gv,
                                                                          T* lx, T* ub, const int* ready, const int* n_ready,
-                                                                         const int8_t* phase, int ph,
-                                                                         const int32_t* nchild, int* counter,
-                                                                         int* cnt) {
+                                                                         int* counter, int* cnt) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     WarpTile<T>& t = reinterpret_cast<WarpTile<T>*>(smem_raw)[threadIdx.x >> 5];
     const int nr = *n_ready;
@@ -1995,8 +2148,9 @@ __global__ void __launch_bounds__(kThreads, kMinBlocksW<T>) k_front_warp(DevFact
         if (item >= nr) break;
         int s = ready[item];
         while (s >= 0) {
-            if (!front_frozen(F, W, s)) warp_front_factor<T>(F, W, sv, gv, lx, ub, s, t);
-            s = warp_continue_up(F, phase, ph, nchild, cnt, s);
+            const FrontRec R = F.rec[s];
+            if (!front_frozen(W, R)) warp_front_factor<T>(F, W, sv, gv, lx, ub, R, s, t);
+            s = warp_continue_up(R, cnt);
         }
     }
 }
@@ -2185,20 +2339,19 @@ cudaError_t factor_impl(const DevNet& net, const DevFactor& F, const DevWork& W,
         int* counters = W.flow + F.n_super;
         if (ls.flow_w_n > 0) {
             k_front_warp<T><<<ls.flow_w_grid, kThreads, sizeof(WarpTile<T>) * kWarpsPerCta, st>>>(
-                F, W, sv, gv, lx, ub, ls.d_flow_w, ls.d_ready_n + 4, ls.d_phase, 3, ls.d_phase_nchild, counters + 2,
-                W.flow);
+                F, W, sv, gv, lx, ub, ls.d_flow_w, ls.d_ready_n + 4, counters + 2, W.flow);
             count_launches(1);
         }
         if (ls.flow_a_n > 0) {
             const int mf = ls.flow_a_maxf;
             k_front_flow<T, kPanelSmall, kMinBlocksA<T>><<<ls.flow_a_grid, kThreads, front_smem<T>(mf), st>>>(
-                F, W, sv, gv, lx, ub, ls.d_flow_a, ls.d_ready_n + 0, ls.d_phase, 1, ls.d_phase_nchild, counters + 0, W.flow);
+                F, W, sv, gv, lx, ub, ls.d_flow_a, ls.d_ready_n + 0, counters + 0, W.flow);
             count_launches(1);
         }
         if (ls.flow_b_n > 0) {
             const int mf = ls.flow_b_maxf;
             k_front_flow<T, kPanel, 1><<<ls.flow_b_grid, kThreads, front_smem<T>(mf), st>>>(
-                F, W, sv, gv, lx, ub, ls.d_flow_b, ls.d_ready_n + 1, ls.d_phase, 2, ls.d_phase_nchild, counters + 1, W.flow);
+                F, W, sv, gv, lx, ub, ls.d_flow_b, ls.d_ready_n + 1, counters + 1, W.flow);
             count_launches(1);
         }
     }

@@ -84,6 +84,26 @@ struct DevNet {
     int32_t n_units;
 };
 
+// A front as its kernels read it, in one load: its sizes and places, its gain
+// targets and children, and its parent.  (Read array by array these were
+// chains of dependent loads, about 300 cycles each, at the head of every front.)
+struct __align__(16) FrontRec {
+    int32_t c0, nc, f, parent;
+    int32_t tgt0, tgt1, ch0, ch1;  // gain targets, children (ChildRec)
+    int64_t lx_off, u_off;
+    int64_t su_off;
+    int32_t up_n;  // children of the parent in this front's dataflow phase (0: the parent is not in it)
+    int32_t grid;
+    int32_t asm_slot;  // single-CTA fronts: its lists in asm_ptr
+    int32_t pad0, pad1, pad2;
+};
+// A child as its parent's assembly reads it.
+struct __align__(16) ChildRec {
+    int64_t u_off, su_off;
+    int32_t m, ld, big, pad;  // update matrix: m x m, leading dimension, in the factor array (big) or u
+};
+constexpr int kAsmWarps = 8;  // warps of a single-CTA front's assembly
+
 // Factorisation plan (device).
 struct DevFactor {
     int32_t n_super, n_state;
@@ -118,6 +138,13 @@ struct DevFactor {
     // columns per panel of each front's factorisation (16 or 32); the
     // diagonal block of every panel is stored inverted (L11^-1) in L
     const int8_t* sn_pw;
+    const FrontRec* rec;         // [n_super]
+    const ChildRec* child_rec;   // [children], as sn_child
+    // Assembly of the single-CTA fronts: per front (FrontRec::asm_slot) and warp
+    // w, the children's columns whose front column t has t % kAsmWarps == w, in
+    // child order: (child position, child column | t << 16)
+    const int32_t* asm_ptr;      // [kAsmWarps * slots + 1]
+    const int2* asm_ent;
 };
 
 // Mutable per-iteration state (device).
