@@ -374,7 +374,6 @@ void Engine::build_schedule(bool targets_ready) {
     sch_flow_a_.clear();
     sch_flow_w_.clear();
     sch_flow_b_.clear();
-    sch_down_.clear();
     sch_up_.clear();
     flow_a_maxf_ = flow_b_maxf_ = 0;
     lay_lx_off_.assign(ns + 1, 0);
@@ -614,12 +613,21 @@ void Engine::build_schedule(bool targets_ready) {
         sch_small_ptr_[l + 1] = static_cast<int32_t>(sch_small_.size());
         sch_asm_ptr_[l + 1] = static_cast<int32_t>(sch_asm_.size());
     }
-    // every front, top-down, for the backward dataflow sweep
-    // every front top-down for the backward sweeps: warp fronts apart
+    // every front top-down for the backward sweeps: warp fronts apart, the
+    // wide fronts with their ancestors first
     sch_down_.clear();
+    sch_down_top_.clear();
     sch_down_w_.clear();
-    for (auto it = sch_all_.rbegin(); it != sch_all_.rend(); ++it)
-        (flow_phase_[*it] == 3 ? sch_down_w_ : sch_down_).push_back(*it);
+    down_maxf_ = 0;
+    std::vector<char> top(ns, 0);
+    for (int32_t s = 0; s < ns; ++s) {  // children before their parents
+        if (P.sn_f[s] > kDownTopF) top[s] = 1;
+        if (top[s] && P.sn_parent[s] >= 0) top[P.sn_parent[s]] = 1;
+    }
+    for (auto it = sch_all_.rbegin(); it != sch_all_.rend(); ++it) {
+        if (!top[*it] && flow_phase_[*it] != 3) down_maxf_ = std::max(down_maxf_, P.sn_f[*it]);
+        (flow_phase_[*it] == 3 ? sch_down_w_ : top[*it] ? sch_down_top_ : sch_down_).push_back(*it);
+    }
     // continuation sweeps: children counts and initially ready fronts, the
     // ones with the most factor work on their path to the root first
     phase_nchild_.assign(ns, 0);
@@ -674,7 +682,7 @@ int32_t Engine::schedule_info(ScheduleInfo& out) {
     out.a_ready = static_cast<int32_t>(sch_flow_a_.size());
     out.b_ready = static_cast<int32_t>(sch_flow_b_.size());
     out.up_ready = static_cast<int32_t>(sch_up_.size());
-    out.down_n = static_cast<int32_t>(sch_down_.size());
+    out.down_n = static_cast<int32_t>(sch_down_.size() + sch_down_top_.size());
     out.down_warp_n = static_cast<int32_t>(sch_down_w_.size());
     for (size_t l = 0; l + 1 < sch_small_ptr_.size(); ++l)
         out.sync_levels += (sch_small_ptr_[l + 1] > sch_small_ptr_[l] || sch_asm_ptr_[l + 1] > sch_asm_ptr_[l]) ? 1 : 0;
@@ -837,6 +845,7 @@ int32_t Engine::upload() {
         d_flow_a_ = c.take<int32_t>(sch_flow_a_.size());
         d_flow_b_ = c.take<int32_t>(sch_flow_b_.size());
         d_down_ = c.take<int32_t>(sch_down_.size());
+        d_down_top_ = c.take<int32_t>(sch_down_top_.size());
         d_up_ = c.take<int32_t>(sch_up_.size());
         d_flow_w_ = c.take<int32_t>(sch_flow_w_.size());
         d_down_w_ = c.take<int32_t>(sch_down_w_.size());
@@ -1008,6 +1017,8 @@ int32_t Engine::upload() {
             r.up_n = up ? phase_nchild_[r.parent] : 0;
             r.grid = grid_of[s];
             r.asm_slot = asm_slot_[s];
+            r.pw = flow_phase_[s] == 1 ? kPanelFlowA : kTile;  // as sn_pw
+            r.rows_off = P.sn_rows_off[s];
         }
         for (size_t x = 0; x < P.sn_child.size(); ++x) {
             const int32_t c = P.sn_child[x];
@@ -1073,6 +1084,7 @@ int32_t Engine::upload() {
     chk(put(d_flow_a_, sch_flow_a_, st_));
     chk(put(d_flow_b_, sch_flow_b_, st_));
     chk(put(d_down_, sch_down_, st_));
+    chk(put(d_down_top_, sch_down_top_, st_));
     chk(put(d_up_, sch_up_, st_));
     chk(put(d_flow_w_, sch_flow_w_, st_));
     chk(put(d_down_w_, sch_down_w_, st_));
@@ -1131,7 +1143,7 @@ int32_t Engine::upload() {
     sched_.h_lvl_maxpanel = sch_maxpanel_.data();
     {
         const int32_t ms = max_solve_front();
-        FlowGrids g = flow_grids(mixed_, flow_a_maxf_, flow_b_maxf_, ms);
+        FlowGrids g = flow_grids(mixed_, flow_a_maxf_, flow_b_maxf_, ms, down_maxf_);
         const bool tt = mixed_ && !sch_tt_.empty() && !tile_tasks_bad_ && g.tile > 0;
         sched_.h_tt_ptr = sch_tt_ptr_.data();
         sched_.d_tt = d_tt_;
@@ -1143,7 +1155,7 @@ int32_t Engine::upload() {
         sched_.flow_w_grid = std::max(1, std::min(g.w, sched_.flow_w_n));
         sched_.d_down_w = d_down_w_;
         sched_.down_w_n = static_cast<int32_t>(sch_down_w_.size());
-        sched_.solve_w_grid = std::max(1, std::min(g.wsolve, std::max(sched_.flow_w_n, sched_.down_w_n)));
+        sched_.solve_w_grid = std::max(1, std::min(g.wsolve, sched_.flow_w_n));
         sched_.d_flow_a = d_flow_a_;
         sched_.flow_a_n = static_cast<int32_t>(sch_flow_a_.size());
         sched_.flow_a_maxf = flow_a_maxf_;
@@ -1154,13 +1166,19 @@ int32_t Engine::upload() {
         sched_.flow_b_grid = std::max(1, std::min(g.b, sched_.flow_b_n));
         sched_.d_phase = d_phase_;
         sched_.d_phase_nchild = d_phase_nchild_;
-        sched_.solve_flow = (cfg.dataflow && g.solve > 0) ? 1 : 0;
+        sched_.solve_flow = (cfg.dataflow && g.solve > 0 && g.down > 0 && g.down_top > 0 && g.down_w > 0) ? 1 : 0;
         sched_.d_up = d_up_;
         sched_.up_n = static_cast<int32_t>(sch_up_.size());
         sched_.d_nchild = d_nchild_;
         sched_.d_down = d_down_;
         sched_.solve_maxf = ms;
-        sched_.solve_grid = std::max(1, std::min(g.solve, ns));
+        sched_.d_down_top = d_down_top_;
+        sched_.down_n = static_cast<int32_t>(sch_down_.size());
+        sched_.down_top_n = static_cast<int32_t>(sch_down_top_.size());
+        sched_.down_maxf = down_maxf_;
+        sched_.down_grid = std::max(1, std::min(g.down, sched_.down_n));
+        sched_.down_top_grid = std::max(1, std::min(g.down_top, sched_.down_top_n));
+        sched_.down_w_grid = std::max(1, std::min(g.down_w, sched_.down_w_n));
         sched_.up_grid = std::max(1, std::min(g.solve, sched_.up_n));
         // claim-list lengths on the device; a batch claims from compacted copies
         sched_.d_ready_n = d_ready_n_;
@@ -1178,6 +1196,7 @@ int32_t Engine::upload() {
             sched_.d_down = d_cmp_[3];
             sched_.d_flow_w = d_cmp_[4];
             sched_.d_down_w = d_cmp_[5];
+            sched_.d_down_top = d_cmp_[6];
         }
     }
 

@@ -281,25 +281,26 @@ private:
     std::vector<TileTask> sch_tt_;
     std::vector<int32_t> sch_tt_ptr_;
     std::vector<int64_t> sch_maxpanel_;
-    std::vector<int32_t> sch_flow_a_, sch_flow_b_, sch_down_, sch_up_, sch_flow_w_, sch_down_w_, phase_nchild_, nchild_;
+    std::vector<int32_t> sch_flow_a_, sch_flow_b_, sch_down_, sch_down_top_, sch_up_, sch_flow_w_, sch_down_w_, phase_nchild_, nchild_;
     std::vector<char> flow_phase_;
     int32_t sync_by_depth_ = 0;
     int64_t sync_cost_height_ = 0, sync_cost_depth_ = 0;
-    int32_t flow_a_maxf_ = 0, flow_b_maxf_ = 0;
+    int32_t flow_a_maxf_ = 0, flow_b_maxf_ = 0, down_maxf_ = 0;
     int32_t* d_flow_a_ = nullptr;
     int32_t* d_flow_b_ = nullptr;
     int32_t* d_down_ = nullptr;
+    int32_t* d_down_top_ = nullptr;
     int32_t* d_up_ = nullptr;
     int32_t* d_flow_w_ = nullptr;
     int32_t* d_down_w_ = nullptr;
-    // the claim lists in LevelSchedule::src_lists order (A, B, up, down, warp, warp down)
+    // the claim lists in LevelSchedule::src_lists order (A, B, up, down, warp, warp down, top down)
     const std::vector<int32_t>& claim_list(int l) const {
         const std::vector<int32_t>* v[kReadyLists] = {&sch_flow_a_, &sch_flow_b_, &sch_up_, &sch_down_, &sch_flow_w_,
-                                                      &sch_down_w_};
+                                                      &sch_down_w_, &sch_down_top_};
         return *v[l];
     }
     int32_t* claim_dev(int l) const {
-        int32_t* v[kReadyLists] = {d_flow_a_, d_flow_b_, d_up_, d_down_, d_flow_w_, d_down_w_};
+        int32_t* v[kReadyLists] = {d_flow_a_, d_flow_b_, d_up_, d_down_, d_flow_w_, d_down_w_, d_down_top_};
         return v[l];
     }
     int8_t* d_phase_ = nullptr;

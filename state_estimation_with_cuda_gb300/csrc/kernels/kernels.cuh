@@ -95,7 +95,8 @@ struct __align__(16) FrontRec {
     int32_t up_n;  // children of the parent in this front's dataflow phase (0: the parent is not in it)
     int32_t grid;
     int32_t asm_slot;  // single-CTA fronts: its lists in asm_ptr
-    int32_t pad0, pad1, pad2;
+    int32_t pw;        // columns per panel of the factorisation
+    int64_t rows_off;  // rows below the pivots in sn_rows
 };
 // A child as its parent's assembly reads it.
 struct __align__(16) ChildRec {
@@ -342,20 +343,23 @@ struct LevelSchedule {
     const int8_t* d_phase = nullptr;         // [n_super] 1 = A, 2 = B, 0 = level-synchronous
     const int32_t* d_phase_nchild = nullptr; // [n_super] children in the same phase
     // dataflow solves over every front: forward by continuation from the
-    // leaves (d_up, up_n), backward in top-down order (d_down) waiting on parents
+    // leaves (d_up, up_n), backward in top-down order waiting on parents: the
+    // wide fronts and their ancestors (d_down_top), then the rest (d_down)
     int32_t solve_flow = 0;
     const int32_t* d_up = nullptr;
     int32_t up_n = 0;
     const int32_t* d_nchild = nullptr;       // [n_super] children
     const int32_t* d_down = nullptr;
-    int32_t solve_maxf = 0, solve_grid = 0, up_grid = 0;
+    const int32_t* d_down_top = nullptr;
+    int32_t down_n = 0, down_top_n = 0, down_maxf = 0, down_grid = 0, down_top_grid = 0;
+    int32_t solve_maxf = 0, up_grid = 0;
     // warp phase: initially ready warp fronts (factor and forward sweep) and
     // every warp front top-down (backward sweep)
     const int32_t* d_flow_w = nullptr;
     int32_t flow_w_n = 0, flow_w_grid = 0;
     const int32_t* d_down_w = nullptr;
-    int32_t down_w_n = 0, solve_w_grid = 0;
-    // Lengths of the claim lists (A, B, up, down, warp, warp down) as the
+    int32_t down_w_n = 0, solve_w_grid = 0, down_w_grid = 0;
+    // Lengths of the claim lists (A, B, up, down, warp, warp down, top down) as the
     // kernels read them, on the device.  In a batch the lists above are
     // compacted copies: before every iteration launch_ready_compact keeps, in
     // order, the entries of src_lists whose grid takes the step, so that
@@ -364,14 +368,14 @@ struct LevelSchedule {
     // lengths fixed.
     int32_t* d_ready_n = nullptr;
     int32_t compact = 0;
-    const int32_t* src_lists[6] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
-    int32_t* cmp_lists[6] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
-    int32_t src_n[6] = {0, 0, 0, 0, 0, 0};
+    const int32_t* src_lists[7] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
+    int32_t* cmp_lists[7] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
+    int32_t src_n[7] = {0, 0, 0, 0, 0, 0, 0};
     int32_t* d_chunk_cnt = nullptr;  // [ready_chunks(src_n)] scratch
 };
 
 // Claim lists and entries per CTA of their compaction.
-constexpr int kReadyLists = 6;
+constexpr int kReadyLists = 7;
 constexpr int kCompactChunk = 2048;
 inline int32_t ready_chunks(const int32_t* n) {
     int32_t c = 0;
@@ -431,9 +435,12 @@ constexpr int32_t kWarpPhaseMinFronts = 1;
 
 // Resident-CTA grid sizes of the persistent dataflow kernels (0 = cannot run).
 struct FlowGrids {
-    int32_t a, b, solve, w, wsolve, tile;
+    int32_t a, b, solve, w, wsolve, tile, down, down_top, down_w;
 };
-FlowGrids flow_grids(bool mixed, int32_t maxf_a, int32_t maxf_b, int32_t solve_maxf);
+FlowGrids flow_grids(bool mixed, int32_t maxf_a, int32_t maxf_b, int32_t solve_maxf, int32_t down_maxf);
+// Backward sweep: fronts wider than this, and their ancestors, run first in a
+// launch whose CTAs stage whole column blocks of their panels (k_bwd_flow).
+constexpr int32_t kDownTopF = 96;
 
 // Allocation-free FP64 factor/solve (scratch in a static device array).
 constexpr size_t kNoAllocScratchBytes = size_t(16) << 20;
