@@ -366,6 +366,7 @@ void Engine::build_schedule(bool targets_ready) {
     sch_pot_.clear();
     n_pot_pairs_ = 0;
     sch_upd_.clear();
+    sch_step_items_.clear();
     sch_pot_ptr_.assign(1, 0);
     sch_upd_ptr_.assign(1, 0);
     sch_tt_.clear();
@@ -516,7 +517,7 @@ void Engine::build_schedule(bool targets_ready) {
         depth[s] = p >= 0 ? depth[p] + 1 : 0;
         if (flow_phase_[s] == 0) dmax = std::max(dmax, depth[s]);
     }
-    const int32_t per_panel = 2;  // launches per panel step
+    const int32_t per_panel = mixed_ ? 1 : 2;  // launches per panel step
     auto sync_cost = [&](bool by_depth) {
         std::vector<int32_t> pan(nl, 0);
         std::vector<char> has_small(nl, 0), has_big(nl, 0);
@@ -586,27 +587,48 @@ void Engine::build_schedule(bool targets_ready) {
         }
         sch_panels_[l] = panels;
         sch_step_ptr_[l + 1] = sch_step_ptr_[l] + panels;
+        // FP64: a panel launch and an update launch per step.  FP32: one panel
+        // launch, then per step one launch that updates the trailing matrix and
+        // solves the next panel (or, as dataflow items, per level).
         for (int32_t p = 0; p < panels; ++p) {
             for (int32_t s : bigs) {
                 const int32_t f = P.sn_f[s], nc = P.sn_c0[s + 1] - P.sn_c0[s];
                 if (nc <= p * kTile) continue;
-                const int32_t pb = std::min(kTile, nc - p * kTile);
-                const int32_t q0 = p * kTile + pb;
-                // one CTA per chunk of rows below the diagonal block
-                const int32_t nch = mixed_ ? std::max(1, (f - q0 + kPanelRows - 1) / kPanelRows)
-                                           : (f - q0) / kPanelRows64 + 1;  // with the right-hand side as row f
-                for (int32_t k = 0; k < nch; ++k) sch_pot_.push_back(make_int4(s, k, nch, n_pot_pairs_));
-                pair_of[(static_cast<int64_t>(s) << 20) | p] = n_pot_pairs_;
-                ++n_pot_pairs_;
-                if (q0 < f) {
-                    const int32_t edge = mixed_ ? kUpdTile : kUpdTile64;
-                    const int32_t ut = (f + edge - 1) / edge;
-                    for (int32_t tj = q0 / edge; tj < ut; ++tj)
-                        for (int32_t ti = tj; ti < ut; ++ti) sch_upd_.push_back(make_int4(s, ti, tj, 0));
+                const int32_t q0 = p * kTile + std::min(kTile, nc - p * kTile);
+                auto panel_rows = [&](int32_t step) { return f - std::min(nc, (step + 1) * kTile); };
+                // one CTA per chunk of rows below the diagonal block (FP64: with the right-hand side as row f)
+                const int32_t nch = mixed_ ? std::max(1, (panel_rows(p) + kPanelRows - 1) / kPanelRows)
+                                           : panel_rows(p) / kPanelRows64 + 1;
+                if (!mixed_ || p == 0) {
+                    for (int32_t k = 0; k < nch; ++k) sch_pot_.push_back(make_int4(s, k, nch, n_pot_pairs_));
+                    pair_of[(static_cast<int64_t>(s) << 20) | p] = n_pot_pairs_;
+                    ++n_pot_pairs_;
                 }
+                if (q0 >= f) continue;
+                if (!mixed_) {
+                    const int32_t ut = (f + kUpdTile64 - 1) / kUpdTile64;
+                    for (int32_t tj = q0 / kUpdTile64; tj < ut; ++tj)
+                        for (int32_t ti = tj; ti < ut; ++ti) sch_upd_.push_back(make_int4(s, ti, tj, 0));
+                    continue;
+                }
+                StepItem it{s, 0, 0, -1, f, P.sn_c0[s], nc, 0, lay_lx_off_[s], P.sn_su_off[s]};
+                const bool next = q0 < nc;
+                if (next) {
+                    it.b = std::max(1, (panel_rows(p + 1) + kPanelRows - 1) / kPanelRows);
+                    it.pair = n_pot_pairs_++;
+                    for (it.a = 0; it.a < it.b; ++it.a) sch_step_items_.push_back(it);
+                }
+                it.pair = -1;
+                const int32_t ut = (f + kUpdTile - 1) / kUpdTile;
+                for (it.b = q0 / kUpdTile + (next ? 1 : 0); it.b < ut; ++it.b)
+                    for (it.a = it.b; it.a < ut; ++it.a) sch_step_items_.push_back(it);
             }
+            // the next panels first: the step after waits for them
+            if (mixed_)
+                std::stable_partition(sch_step_items_.begin() + sch_upd_ptr_.back(), sch_step_items_.end(),
+                                      [](const StepItem& it) { return it.pair >= 0; });
             sch_pot_ptr_.push_back(static_cast<int32_t>(sch_pot_.size()));
-            sch_upd_ptr_.push_back(static_cast<int32_t>(sch_upd_.size()));
+            sch_upd_ptr_.push_back(static_cast<int32_t>(mixed_ ? sch_step_items_.size() : sch_upd_.size()));
         }
         if (mixed_ && cfg.tile_flow && !bigs.empty()) build_tile_tasks(bigs, pair_of);
         sch_tt_ptr_[l + 1] = static_cast<int32_t>(sch_tt_.size());
@@ -840,6 +862,7 @@ int32_t Engine::upload() {
         d_pot_ = c.take<int4>(sch_pot_.size());
         d_pot_cnt_ = c.take<int32_t>(std::max(1, n_pot_pairs_));
         d_upd_ = c.take<int4>(sch_upd_.size());
+        d_step_ = c.take<StepItem>(sch_step_items_.size());
         d_tt_ = c.take<TileTask>(sch_tt_.size());
         d_tt_done_ = c.take<int32_t>(sch_tt_.size() + static_cast<size_t>(P.n_levels));
         d_flow_a_ = c.take<int32_t>(sch_flow_a_.size());
@@ -1080,6 +1103,7 @@ int32_t Engine::upload() {
     chk(put(d_asm_child_, sch_asm_child_, st_));
     chk(put(d_pot_, sch_pot_, st_));
     chk(put(d_upd_, sch_upd_, st_));
+    chk(put(d_step_, sch_step_items_, st_));
     chk(put(d_tt_, sch_tt_, st_));
     chk(put(d_flow_a_, sch_flow_a_, st_));
     chk(put(d_flow_b_, sch_flow_b_, st_));
@@ -1137,6 +1161,7 @@ int32_t Engine::upload() {
     sched_.n_pot_pairs = n_pot_pairs_;
     sched_.h_upd_ptr = sch_upd_ptr_.data();
     sched_.d_upd = d_upd_;
+    sched_.d_step = d_step_;
     sched_.h_all_ptr = sch_all_ptr_.data();
     sched_.d_all = d_all_;
     sched_.h_lvl_maxf = sch_maxf_.data();

@@ -270,6 +270,7 @@ private:
     std::vector<int32_t> sch_small_ptr_, sch_small_, sch_small_maxf_, sch_asm_ptr_, sch_panels_, sch_step_ptr_,
         sch_pot_ptr_, sch_upd_ptr_, sch_all_ptr_, sch_all_, sch_maxf_;
     std::vector<int4> sch_pot_, sch_upd_;
+    std::vector<StepItem> sch_step_items_;
     std::vector<AsmItem> sch_asm_;
     std::vector<int2> ev_unit_, ev_grp_;  // evaluation units (DevNet::ev_unit / ev_grp)
     void build_eval_units();
@@ -339,6 +340,7 @@ private:
     AsmChild* d_asm_child_ = nullptr;
     int4* d_pot_ = nullptr;
     int4* d_upd_ = nullptr;
+    StepItem* d_step_ = nullptr;
     // targets_ready = false leaves the assembly items' target ranges to
     // fill_asm_targets(), for a schedule built before the gain targets exist.
     void build_schedule(bool targets_ready = true);

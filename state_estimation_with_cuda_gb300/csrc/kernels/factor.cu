@@ -1524,17 +1524,17 @@ __global__ void __launch_bounds__(kThreads) k_big_panel32(DevFactor F, DevWork W
     big_panel32_item<false>(F, W, sv, lx, wk.x, p, wk.y, wk.z, wk.w, step_cnt);
 }
 
-// FP32 trailing update of step p: the kUpdTile x kUpdTile tile (ti, tj) -= A_i A_j^T
+// FP32 trailing update of step p as a dataflow item: tile (ti, tj) -= A_i A_j^T
 // over the panel's columns, restricted to rows >= cols >= p0 + pb.  The two
 // row blocks of the panel are staged k-major in shared memory; thread
 // (tr, tc) accumulates rows tr + 16u and columns tc + 16v (u, v < 2) in
 // registers, four shared loads per four FMAs (a thread per output needed
 // two per FMA), and its read-modify-writes of a column touch 16 consecutive
 // rows per half warp.
-template <bool kL2>
 __device__ __forceinline__ void big_update_item(const DevFactor& F, const DevWork& W, const SolveVecs& sv, float* lx,
                                                 int s, int p, int ti, int tj) {
     using T = float;
+    constexpr bool kL2 = true;
     static_assert(kThreads == 256 && kUpdTile == 32, "thread tiling below");
     constexpr int ld = kUpdTile + 1;
     __shared__ T Ai[kTile * ld];  // Ai[k * ld + r] = A(R0 + r, p0 + k)
@@ -1627,11 +1627,274 @@ __device__ __forceinline__ void big_update_item(const DevFactor& F, const DevWor
     }
 }
 
-__global__ void __launch_bounds__(kThreads) k_big_update32(DevFactor F, DevWork W, SolveVecs sv, float* lx,
-                                                           const int4* work, int p) {
-    const int4 wk = work[blockIdx.x];
-    if (front_frozen(F, W, wk.x)) return;  // the whole CTA, before any barrier
-    big_update_item<false>(F, W, sv, lx, wk.x, p, wk.y, wk.z);
+// FP32 step p of the tiled fronts in one launch: the trailing update of step p
+// and the panel of step p + 1.  A chunk's CTA of the next panel updates its own
+// rows of the panel's columns and, for itself, the diagonal block, which warp 0
+// then factors and inverts while the other warps update the chunk; then the
+// chunk is solved against the inverse.  No CTA waits for another: the diagonal
+// block is updated and factored by every chunk's CTA, and the one that has read
+// it last (a counter per front and step) writes L_dd^-1 into its slot.  The
+// other tiles are plain updates.  Bound: the chain of load latency, the block's
+// 32 pivots and its inverse.  Measured at 200k buses: 10.2 us a step, where the
+// update and the next panel as two launches took 11.0 + 5.1 us and two gaps.
+constexpr int kStepLd = kTile + 4, kStepRows = kPanelRows + 4;  // 16-byte aligned rows
+struct StepPanelSmem {
+    float xd[kTile * kStepLd];    // [k][r]: panel p, rows of the next diagonal block
+    float d[kTile * kStepLd];     // [j][i]: the diagonal block, then L_dd
+    float lt[kTile * kStepLd];    // [k][c] = L_dd^-1[c][k]
+    float xc[kTile * kStepRows];  // [k][r]: panel p, the chunk's rows
+    float as[kTile * kStepRows];  // [j][r]: the chunk, then X
+    float col[kTile], rdiag[kTile], v[kTile];
+    int last;
+};
+struct StepTileSmem {
+    float ai[kTile * (kUpdTile + 1)], aj[kTile * (kUpdTile + 1)];
+};
+__device__ __forceinline__ void step_panel(const DevFactor& F, const DevWork& W, const SolveVecs& sv, float* lx,
+                                           const StepItem& it, int p, int* step_cnt, StepPanelSmem& sm) {
+    static_assert(kThreads == 256 && kPanelRows == 128 && kTile == 32, "thread tiling below");
+    constexpr int kQ = kTile / (kThreads / 32), kU = kPanelRows / 32;
+    const int f = it.f, nc = it.nc, chunk = it.a;
+    float* B = lx + it.lx_off;
+    const int p0 = p * kTile, q0 = p0 + kTile;  // panel p is whole: there is a next one
+    const int pb = min(kTile, nc - q0);         // columns of the next panel
+    const int r0 = q0 + pb + chunk * kPanelRows, nr = max(0, min(kPanelRows, f - r0));
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    float* const y = static_cast<float*>(sv.sol) + it.c0;
+    {
+        // thread (i, j0): columns j0 + 8 q; rows i of the block, i + 32 u of the chunk
+        const int i = lane, j0 = warp;
+        float xd[kQ], dv[kQ], xc[kQ][kU], av[kQ][kU];
+#pragma unroll
+        for (int q = 0; q < kQ; ++q) {
+            const int j = j0 + q * (kThreads / 32);
+            const float* xcol = B + (int64_t)(p0 + j) * f;
+            const float* acol = B + (int64_t)(q0 + j) * f;
+            const bool in = q0 + j < f;
+            xd[q] = q0 + i < f ? xcol[q0 + i] : 0.f;
+            dv[q] = (j < pb && i < pb && i >= j) ? acol[q0 + i] : 0.f;
+#pragma unroll
+            for (int u = 0; u < kU; ++u) {
+                const int r = i + 32 * u;
+                xc[q][u] = r < nr ? xcol[r0 + r] : 0.f;
+                av[q][u] = (in && r < nr && r0 + r >= q0 + j) ? acol[r0 + r] : 0.f;
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < kQ; ++q) {
+            const int j = j0 + q * (kThreads / 32);
+            sm.xd[j * kStepLd + i] = xd[q];
+            sm.d[j * kStepLd + i] = dv[q];
+#pragma unroll
+            for (int u = 0; u < kU; ++u) {
+                sm.xc[j * kStepRows + i + 32 * u] = xc[q][u];
+                sm.as[j * kStepRows + i + 32 * u] = av[q][u];
+            }
+        }
+    }
+    __syncthreads();
+    if (tid == 0) sm.last = atomicAdd(step_cnt + it.pair, 1) == it.b - 1;  // this CTA's block reads are done
+    {
+        // the diagonal block's update: rows tr + 16 u, columns tc + 16 v
+        const int tr = tid & 15, tc = tid >> 4;
+        float acc[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
+#pragma unroll 8
+        for (int k = 0; k < kTile; ++k) {
+            const float a0 = sm.xd[k * kStepLd + tr], a1 = sm.xd[k * kStepLd + tr + 16];
+            const float b0 = sm.xd[k * kStepLd + tc], b1 = sm.xd[k * kStepLd + tc + 16];
+            acc[0][0] += a0 * b0;
+            acc[0][1] += a0 * b1;
+            acc[1][0] += a1 * b0;
+            acc[1][1] += a1 * b1;
+        }
+#pragma unroll
+        for (int u = 0; u < 2; ++u)
+#pragma unroll
+            for (int v = 0; v < 2; ++v) {
+                float* e = &sm.d[(tc + 16 * v) * kStepLd + tr + 16 * u];
+                *e = *e - acc[u][v];
+            }
+    }
+    __syncthreads();
+    if (warp == 0) {
+        const int i = lane;
+        float a[kTile];
+#pragma unroll
+        for (int j = 0; j < kTile; ++j) a[j] = (i < pb && j <= i) ? sm.d[i + j * kStepLd] : 0.f;
+        float inv;
+        const bool bad = warp_potrf_bcast<kTile>(a, pb, i, &inv, sm.col);
+        if (bad && i == 0 && chunk == 0) atomicOr(singular_flags(F, W, it.s), FLAG_SINGULAR);
+#pragma unroll
+        for (int j = 0; j < kTile; ++j) {
+            sm.d[i + j * kStepLd] = (i < pb && j <= i) ? a[j] : 0.f;
+            sm.lt[j * kStepLd + i] = 0.f;
+        }
+        if (i < pb) sm.rdiag[i] = inv;
+        if (chunk == 0 && i < pb) reinterpret_cast<float*>(W.rdiag)[it.c0 + q0 + i] = inv;
+        __syncwarp();
+        warp_trinv_v4<kTile, kStepLd>(reinterpret_cast<const float (*)[kStepLd]>(sm.d), sm.rdiag, pb, i, sm.lt, kStepLd);
+    } else {
+        // the chunk's update, 4 x 4 entries a turn
+        for (int t = tid - 32; t < kThreads; t += kThreads - 32) {
+            const int cg = t & 7, rg = t >> 3;
+            float acc[4][4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+#pragma unroll
+                for (int v = 0; v < 4; ++v) acc[u][v] = 0.f;
+#pragma unroll 8
+            for (int k = 0; k < kTile; ++k) {
+                float av[4], bv[4];
+                load4<float>(&sm.xc[k * kStepRows + 4 * rg], av);
+                load4<float>(&sm.xd[k * kStepLd + 4 * cg], bv);
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+#pragma unroll
+                    for (int v = 0; v < 4; ++v) acc[u][v] += av[u] * bv[v];
+            }
+#pragma unroll
+            for (int v = 0; v < 4; ++v) {
+                float cur[4];
+                load4<float>(&sm.as[(4 * cg + v) * kStepRows + 4 * rg], cur);
+#pragma unroll
+                for (int u = 0; u < 4; ++u) cur[u] = cur[u] - acc[u][v];
+                store4<float>(&sm.as[(4 * cg + v) * kStepRows + 4 * rg], cur);
+            }
+        }
+        if (chunk == 0 && warp == 1) {
+            // the right-hand side of the panel's tile column (entries past pb belong to rows below)
+            const int gc = q0 + lane;
+            float acc = 0.f;
+            if (gc < f) {
+                float* v = rhs_entry<float>(sv, it.c0, nc, it.su_off, gc);
+                acc = *v;
+#pragma unroll 8
+                for (int k = 0; k < kTile; ++k) acc -= sm.xd[k * kStepLd + lane] * y[p0 + k];
+                if (lane >= pb) *v = acc;
+            }
+            sm.v[lane] = acc;
+        }
+    }
+    __syncthreads();
+    if (chunk == 0 && warp == 0) {
+        // y = L_dd^-1 v, a lane per row
+        float yv = 0.f;
+        for (int j = 0; j < pb; ++j)
+            if (j <= lane) yv += sm.lt[j * kStepLd + lane] * sm.v[j];
+        if (lane < pb) y[q0 + lane] = yv;
+    }
+    {
+        // X = A (L_dd^-1)^T: rows 4 rg.., columns 4 cg..; columns past pb stay updated entries
+        const int cg = tid & 7, rg = tid >> 3;
+        float acc[4][4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+#pragma unroll
+            for (int v = 0; v < 4; ++v) acc[u][v] = 0.f;
+#pragma unroll 8
+        for (int k = 0; k < kTile; ++k) {
+            float av[4], lv[4];
+            load4<float>(&sm.as[k * kStepRows + 4 * rg], av);
+            load4<float>(&sm.lt[k * kStepLd + 4 * cg], lv);
+            if (k >= pb) {
+#pragma unroll
+                for (int u = 0; u < 4; ++u) av[u] = 0.f;
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+#pragma unroll
+                for (int v = 0; v < 4; ++v) acc[u][v] += av[u] * lv[v];
+        }
+        __syncthreads();  // every read of A is done
+#pragma unroll
+        for (int v = 0; v < 4; ++v)
+            if (4 * cg + v < pb)
+                *reinterpret_cast<float4*>(&sm.as[(4 * cg + v) * kStepRows + 4 * rg]) =
+                    make_float4(acc[0][v], acc[1][v], acc[2][v], acc[3][v]);
+    }
+    __syncthreads();
+    for (int x = tid; x < kTile * kPanelRows; x += kThreads) {
+        const int r = x % kPanelRows, k = x / kPanelRows;
+        if (r < nr && q0 + k < f && r0 + r >= q0 + k) B[(r0 + r) + (int64_t)(q0 + k) * f] = sm.as[k * kStepRows + r];
+    }
+    if (sm.last) {
+        for (int x = tid; x < kTile * kTile; x += kThreads) {
+            const int i = x % kTile, j = x / kTile;
+            if (i < pb && j <= i) B[(q0 + i) + (int64_t)(q0 + j) * f] = sm.lt[j * kStepLd + i];
+        }
+    }
+}
+
+__global__ void __launch_bounds__(kThreads) k_big_step32(DevFactor F, DevWork W, SolveVecs sv, float* lx,
+                                                         const StepItem* work, int p, int* step_cnt) {
+    __shared__ __align__(16) union {
+        StepPanelSmem panel;
+        StepTileSmem tile;
+    } sm;
+    const StepItem it = work[blockIdx.x];
+    if (W.grid_flags && front_frozen(F, W, it.s)) return;  // the whole CTA, before any barrier
+    if (it.pair >= 0) {
+        step_panel(F, W, sv, lx, it, p, step_cnt, sm.panel);
+        return;
+    }
+    constexpr int ld = kUpdTile + 1;
+    float* B = lx + it.lx_off;
+    const int f = it.f, nc = it.nc, ti = it.a, tj = it.b;
+    const int p0 = p * kTile, pb = min(kTile, nc - p0), q0 = p0 + pb;
+    const int R0 = ti * kUpdTile, C0 = tj * kUpdTile;
+    const int tid = threadIdx.x, tr = tid & 15, tc = tid >> 4;
+    // every load of the CTA in flight at once
+    float cur[2][2], xi[4], xj[4];
+#pragma unroll
+    for (int v = 0; v < 2; ++v)
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            const int gc = C0 + tc + 16 * v, gr = R0 + tr + 16 * u;
+            cur[u][v] = (gc >= q0 && gc < f && gr >= gc && gr < f) ? B[(int64_t)gc * f + gr] : 0.f;
+        }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const int r = tid & 31, k = (tid >> 5) + 8 * q;
+        const float* col = B + (int64_t)(p0 + k) * f;
+        xi[q] = (k < pb && R0 + r < f) ? col[R0 + r] : 0.f;
+        xj[q] = (k < pb && C0 + r < f) ? col[C0 + r] : 0.f;
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const int r = tid & 31, k = (tid >> 5) + 8 * q;
+        sm.tile.ai[k * ld + r] = xi[q];
+        sm.tile.aj[k * ld + r] = xj[q];
+    }
+    __syncthreads();
+    if (ti == tj && tid >= kThreads - 32) {
+        // the last warp of a diagonal tile: the tile's right-hand-side entries, a lane per column
+        const int c = tid & 31, gc = C0 + c;
+        if (gc >= q0 && gc < f) {
+            const float* y = static_cast<const float*>(sv.sol) + it.c0 + p0;
+            float* v = rhs_entry<float>(sv, it.c0, nc, it.su_off, gc);
+            float acc = *v;
+#pragma unroll 8
+            for (int k = 0; k < pb; ++k) acc -= sm.tile.aj[k * ld + c] * y[k];
+            *v = acc;
+        }
+    }
+    float acc[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
+#pragma unroll 4
+    for (int k = 0; k < pb; ++k) {
+        const float a0 = sm.tile.ai[k * ld + tr], a1 = sm.tile.ai[k * ld + tr + 16];
+        const float b0 = sm.tile.aj[k * ld + tc], b1 = sm.tile.aj[k * ld + tc + 16];
+        acc[0][0] += a0 * b0;
+        acc[0][1] += a0 * b1;
+        acc[1][0] += a1 * b0;
+        acc[1][1] += a1 * b1;
+    }
+#pragma unroll
+    for (int v = 0; v < 2; ++v)
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            const int gc = C0 + tc + 16 * v, gr = R0 + tr + 16 * u;
+            if (gc >= q0 && gc < f && gr >= gc && gr < f) B[(int64_t)gc * f + gr] = cur[u][v] - acc[u][v];
+        }
 }
 
 // FP64 trailing update of step p, one CTA per kUpdTile64 x kUpdTile64 tile
@@ -1759,7 +2022,7 @@ __global__ void __launch_bounds__(kThreads, kTileFlowBlocks)
             if (t.kind == 0)
                 big_panel32_item<true>(F, W, sv, lx, t.s, t.p, t.a, t.b, t.aux, step_cnt);
             else
-                big_update_item<true>(F, W, sv, lx, t.s, t.p, t.a, t.b);
+                big_update_item(F, W, sv, lx, t.s, t.p, t.a, t.b);
         }
         __syncthreads();
         if (tid == 0) publish_done(done + item);
@@ -2511,11 +2774,12 @@ cudaError_t factor_impl(const DevNet& net, const DevFactor& F, const DevWork& W,
                     count_launches(1);
                 }
                 if (nupd > 0) {
-                    const int4* work = ls.d_upd + ls.h_upd_ptr[slot];
                     if constexpr (sizeof(T) == 4)
-                        k_big_update32<<<nupd, kThreads, 0, st>>>(F, W, sv, lx, work, p);
+                        k_big_step32<<<nupd, kThreads, 0, st>>>(F, W, sv, lx, ls.d_step + ls.h_upd_ptr[slot], p,
+                                                                ls.d_pot_cnt);
                     else
-                        k_big_update64<<<nupd, kUpdTile64 * kUpdTile64, 0, st>>>(F, W, sv, lx, work, p);
+                        k_big_update64<<<nupd, kUpdTile64 * kUpdTile64, 0, st>>>(F, W, sv, lx,
+                                                                                 ls.d_upd + ls.h_upd_ptr[slot], p);
                     count_launches(1);
                 }
             }

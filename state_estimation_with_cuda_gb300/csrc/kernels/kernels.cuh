@@ -287,6 +287,16 @@ struct AsmChild {
     int32_t c, j0, j1, ilo, ihi, pad0, pad1, pad2;
 };
 
+// One work item (CTA) of an FP32 tiled front's step p (k_big_step32), with what
+// it needs of its front.  pair >= 0: chunk a (of b) of the next panel, pair =
+// the (front, step) counter of its diagonal tile's readers; pair < 0: the
+// trailing update of tile (a, b).
+struct __align__(16) StepItem {
+    int32_t s, a, b, pair;
+    int32_t f, c0, nc, pad;
+    int64_t lx_off, su_off;
+};
+
 // One work item of the FP32 tiled fronts' dataflow factorisation (one
 // persistent launch per synchronous level).  kind 0: the panel solve of
 // chunk a (of b chunks) of step p, aux = the (front, step) pair of the
@@ -319,8 +329,9 @@ struct LevelSchedule {
     const int4* d_pot = nullptr;            // (big front, chunk, chunks, step pair)
     int32_t* d_pot_cnt = nullptr;           // [n_pot_pairs] CTAs of a (front, step) done reading its diagonal tile
     int32_t n_pot_pairs = 0;
-    const int32_t* h_upd_ptr = nullptr;     // [n_slots+1] offsets into d_upd
-    const int4* d_upd = nullptr;            // (big front, row tile, column tile)
+    const int32_t* h_upd_ptr = nullptr;     // [n_slots+1] offsets into d_upd (FP64), d_step (FP32)
+    const int4* d_upd = nullptr;            // FP64: (big front, row tile, column tile)
+    const StepItem* d_step = nullptr;       // FP32: next panel chunks and update tiles of a step
     // FP32 tiled fronts as dataflow items, one persistent launch per level
     // (n_tt = 0: the per-step panel and update launches above)
     const int32_t* h_tt_ptr = nullptr;      // [n_levels+1] offsets into d_tt
