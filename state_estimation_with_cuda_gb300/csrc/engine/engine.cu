@@ -445,26 +445,28 @@ void Engine::build_schedule(bool targets_ready) {
         int64_t total = 0;
         for (int32_t s = 0; s < ns; ++s)
             if (!big[s] && flow_phase_[s] != 3) {
-                asm_slot_[s] = slots++;
+                asm_slot_[s] = slots;
+                slots += asm_warps(mixed_, flow_phase_[s] != 1);
                 for (int32_t ci = P.sn_child_ptr[s]; ci < P.sn_child_ptr[s + 1]; ++ci) {
                     const int32_t c = P.sn_child[ci];
                     total += P.sn_f[c] - (P.sn_c0[c + 1] - P.sn_c0[c]);
                 }
             }
-        asm_ptr_.reserve(static_cast<size_t>(kAsmWarps) * slots + 1);
+        asm_ptr_.reserve(static_cast<size_t>(slots) + 1);
         asm_ent_.reserve(total);
-        std::vector<int2> list[kAsmWarps];
+        std::vector<int2> list[asm_warps(true, true)];
         for (int32_t s = 0; s < ns; ++s) {
             if (big[s] || flow_phase_[s] == 3) continue;
+            const int32_t nw = asm_warps(mixed_, flow_phase_[s] != 1);
             for (auto& l : list) l.clear();
             for (int32_t ci = P.sn_child_ptr[s]; ci < P.sn_child_ptr[s + 1]; ++ci) {
                 const int32_t c = P.sn_child[ci];
                 const int32_t m = P.sn_f[c] - (P.sn_c0[c + 1] - P.sn_c0[c]);
                 const int32_t* rel = P.sn_relmap.data() + P.sn_su_off[c];
-                for (int32_t j = 0; j < m; ++j) list[rel[j] % kAsmWarps].push_back(make_int2(ci, j | rel[j] << 16));
+                for (int32_t j = 0; j < m; ++j) list[rel[j] % nw].push_back(make_int2(ci, j | rel[j] << 16));
             }
-            for (const auto& l : list) {
-                asm_ent_.insert(asm_ent_.end(), l.begin(), l.end());
+            for (int32_t w = 0; w < nw; ++w) {
+                asm_ent_.insert(asm_ent_.end(), list[w].begin(), list[w].end());
                 asm_ptr_.push_back(static_cast<int32_t>(asm_ent_.size()));
             }
         }
@@ -577,7 +579,8 @@ void Engine::build_schedule(bool targets_ready) {
                         const int32_t ilo = static_cast<int32_t>(std::lower_bound(rel, rel + m, R0) - rel);
                         const int32_t ihi = static_cast<int32_t>(std::lower_bound(rel + ilo, rel + m, R1) - rel);
                         if (j0 < j1 && std::max(j0, ilo) < ihi)
-                            sch_asm_child_.push_back(AsmChild{c, j0, j1, ilo, ihi, 0, 0, 0});
+                            sch_asm_child_.push_back(AsmChild{j0, j1, ilo, ihi, lay_u_off_[c], P.sn_su_off[c], lay_u_ld_[c],
+                                                              lay_u_big_[c], 0, 0});
                     }
                     it.ch_hi = static_cast<int32_t>(sch_asm_child_.size());
                     sch_asm_.push_back(it);

@@ -134,8 +134,7 @@ __device__ __forceinline__ const T* update_of(const DevFactor& F, const T* lx, c
 }
 
 // Extend-add of every child of a single-CTA front with no barrier between
-// children: warp w owns the front's columns t with t % kAsmWarps == w and
-// walks its list of the children's columns (DevFactor::asm_ent, in child
+// children: warp w owns the front's columns t = w (mod warps) and walks its list of the children's columns (DevFactor::asm_ent, in child
 // order), so no two warps touch the same entry and each entry's additions keep
 // the children's order.  Bound: load latency.  The 32 list entries and child
 // records of a round are fetched a lane each; columns go eight at a time, 32
@@ -156,8 +155,8 @@ __device__ __forceinline__ void extend_add_children(const DevFactor& F, const So
     constexpr unsigned kAll = 0xffffffffu;
     constexpr int kB = 8;  // columns per step
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int e1 = F.asm_ptr[R.asm_slot * kAsmWarps + warp + 1];
-    for (int eb = F.asm_ptr[R.asm_slot * kAsmWarps + warp]; eb < e1; eb += 32) {
+    const int e1 = F.asm_ptr[R.asm_slot + warp + 1];
+    for (int eb = F.asm_ptr[R.asm_slot + warp]; eb < e1; eb += 32) {
         const int n = min(32, e1 - eb);
         const T* up = nullptr;
         const int* rel = nullptr;
@@ -760,16 +759,13 @@ __device__ __forceinline__ void front_store(const SolveVecs& sv, T* lx, T* ub, c
     const int ldf = front_ld<T>(f);
     const int tid = threadIdx.x, nth = blockDim.x, lane = tid & 31, warp = tid >> 5;
     for (int r = tid; r < f; r += nth) *rhs_entry<T>(sv, c0, nc, R.su_off, r) = rhs[r * rhs_ld];
+    const int nwarp = nth >> 5, m = f - nc;
     T* L = lx + R.lx_off;
-    for (int x = tid; x < f * nc; x += nth) {
-        const int c = x / f;
-        L[x] = Fm[(x - c * f) + c * ldf];
-    }
-    const int m = f - nc;
+    for (int c = warp; c < nc; c += nwarp)
+        for (int r = (c & ~31) + lane; r < f; r += 32) L[r + c * f] = Fm[r + c * ldf];
     T* U = ub + R.u_off;
-    const int nwarp = nth >> 5;
     for (int j = warp; j < m; j += nwarp)
-        for (int i = lane; i < m; i += 32) U[i + (int64_t)j * m] = Fm[(nc + i) + (nc + j) * ldf];
+        for (int i = (j & ~31) + lane; i < m; i += 32) U[i + j * m] = Fm[(nc + i) + (nc + j) * ldf];
 }
 
 // Assembles and partially factorises front s in shared memory, FP64, with
@@ -1062,8 +1058,14 @@ constexpr int kPanelSmall = kPanelFlowA;
 template <typename T>
 constexpr int kMinBlocksA = sizeof(T) == 4 ? 3 : 2;
 
+// Threads of a front's CTA: the wide FP32 fronts (phase B, synchronous levels)
+// have an SM to themselves, and sixteen warps keep twice the children's loads
+// and update tiles in flight that eight do.
+template <typename T, int KP>
+constexpr int kFrontThreads = 32 * asm_warps(sizeof(T) == 4, KP == kPanel);
+
 template <typename T>
-__global__ void __launch_bounds__(kThreads, 1) k_front_small(DevFactor F, DevWork W, SolveVecs sv, const T* gv, T* lx,
+__global__ void __launch_bounds__(kFrontThreads<T, kPanel>, 1) k_front_small(DevFactor F, DevWork W, SolveVecs sv, const T* gv, T* lx,
                                                              T* ub, const int* fronts) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ FrontSmem<T> sm;
@@ -1134,7 +1136,7 @@ __device__ __forceinline__ int continue_up(const DevFactor& F, const int8_t* pha
 }
 
 template <typename T, int KP, int kMinBlocks>
-__global__ void __launch_bounds__(kThreads, kMinBlocks) k_front_flow(DevFactor F, DevWork W, SolveVecs sv, const T* gv,
+__global__ void __launch_bounds__(kFrontThreads<T, KP>, kMinBlocks) k_front_flow(DevFactor F, DevWork W, SolveVecs sv, const T* gv,
                                                                      T* lx, T* ub, const int* ready, const int* n_ready,
                                                                      int* counter, int* cnt) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -1170,69 +1172,105 @@ __device__ __forceinline__ int lower_bound_i32(const int* a, int lo, int hi, int
 }
 
 // Assembly of a tiled front, one CTA per (tile column tj, block rb of
-// kAsmRows rows from the tile's first column down): zero the block's lower
-// part, write its G entries, then add the update-matrix entries of the
-// children that land in it, child by child (a barrier between children keeps
-// every entry's sum in child order, as in the single-CTA fronts).  The
-// block's target range and its contributing children with their column and
-// row ranges come from the host schedule (AsmItem / AsmChild).
+// kAsmRows rows from the tile's first column down): the block's G entries, then
+// the update-matrix entries of the children that land in it, child by child (a
+// barrier between children keeps every entry's sum in child order, as in the
+// single-CTA fronts).  The block's target range and its contributing children
+// with their column and row ranges come from the host schedule (AsmItem /
+// AsmChild).  Bound: load latency, child after child; the block is summed in
+// shared memory and written once, and the next child's entries (four columns a
+// warp, four rows a lane) are in flight while one is added (20 us a level as
+// read-modify-writes of the front, ASMBIG with this, at 60k buses).
+// Row block 0 also assembles the tile column's right-hand-side entries: it
+// holds the diagonal, so its list has every child with a column here.
 template <typename T>
 __global__ void __launch_bounds__(kThreads) k_big_assemble(DevFactor F, DevWork W, SolveVecs sv, const T* gv, T* lx,
                                                            T* ub, const AsmItem* work, const AsmChild* kids) {
+    static_assert(kThreads == 256 && kTile == 32 && kAsmRows == 128, "four columns a warp, four rows a lane");
+    constexpr int kKids = 32;
+    __shared__ T tile[kTile * kAsmRows];  // [c][r]
+    __shared__ T vv[kTile];
+    __shared__ AsmChild ks[kKids];
     const AsmItem wk = work[blockIdx.x];
     const int s = wk.s, tj = wk.tj, rb = wk.rb;
-    if (front_frozen(F, W, s)) return;  // the whole CTA, before any barrier
-    const int f = F.sn_f[s];
-    T* B = lx + F.sn_lx_off[s];
+    const FrontRec R = F.rec[s];
+    if (front_frozen(W, R)) return;  // the whole CTA, before any barrier
+    const int f = R.f, nc = R.nc;
+    T* B = lx + R.lx_off;
     const int c0 = tj * kTile, c1 = min(c0 + kTile, f);
     const int R0 = c0 + rb * kAsmRows, R1 = min(R0 + kAsmRows, f);
-    const int tid = threadIdx.x, nth = blockDim.x;
-    // Row block 0 also assembles the tile column's right-hand-side entries (b of
-    // its pivots, the children's solve update vectors): it holds the diagonal,
-    // so its list has every child with a column here.
-    __shared__ T vv[kTile];
-    const int p0 = F.sn_c0[s], nc = F.sn_c0[s + 1] - p0;
-    if (rb == 0 && tid < kTile) vv[tid] = c0 + tid < nc ? static_cast<const T*>(sv.rhs)[p0 + c0 + tid] : T(0);
-    for (int x = tid; x < (c1 - c0) * (R1 - R0); x += nth) {
-        const int c = c0 + x / (R1 - R0), r = R0 + x % (R1 - R0);
-        if (r >= c) B[r + (int64_t)c * f] = T(0);
-    }
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    constexpr int nwarp = kThreads / 32;
+    if (rb == 0 && tid < kTile) vv[tid] = c0 + tid < nc ? static_cast<const T*>(sv.rhs)[R.c0 + c0 + tid] : T(0);
+    for (int x = tid; x < kTile * kAsmRows; x += kThreads) tile[x] = T(0);
     __syncthreads();
-    for (int tg = wk.tg_lo + tid; tg < wk.tg_hi; tg += nth) {
+    for (int tg = wk.tg_lo + tid; tg < wk.tg_hi; tg += kThreads) {
         const int l = F.tgt_local[tg];
-        const int r = l % f;
-        if (r >= R0 && r < R1) B[l] = gv[tg];
+        const int c = l / f, r = l - c * f;
+        if (r >= R0 && r < R1) tile[(c - c0) * kAsmRows + r - R0] = gv[tg];
     }
-    __syncthreads();
-    for (int ci = wk.ch_lo; ci < wk.ch_hi; ++ci) {
-        const AsmChild ch = kids[ci];
-        const int c = ch.c;
-        const int* rel = F.sn_relmap + F.sn_su_off[c];
-        const T* U = update_of<T>(F, lx, ub, c);
-        const int uld = F.sn_u_ld[c];
-        const int lane = tid & 31, warp = tid >> 5, nwarp = nth >> 5;
-        if (rb == 0 && warp == nwarp - 1 && ch.j0 + lane < ch.j1)
-            vv[rel[ch.j0 + lane] - c0] += static_cast<const T*>(sv.su)[F.sn_su_off[c] + ch.j0 + lane];
-        for (int j = ch.j0 + warp; j < ch.j1; j += nwarp) {
-            const int64_t pj = (int64_t)rel[j] * f;
-            const T* Uj = U + (int64_t)j * uld;
-            for (int i0 = max(j, ch.ilo) + lane; i0 < ch.ihi; i0 += 128) {
-                T u[4];
-                int r[4];
+    T u[4][4], un[4][4], bv, bn;
+    int ri[4], rn[4], pj[4], pn[4], pb, pbn;
+    auto load = [&](const AsmChild& ch, T (&x)[4][4], int (&r)[4], int (&pc)[4], T& b, int& bt) {
+        const int* rel = F.sn_relmap + ch.su_off;
+        const T* U = (ch.big ? lx : ub) + ch.u_off;
 #pragma unroll
-                for (int t = 0; t < 4; ++t) {
-                    const int i = i0 + 32 * t;
-                    u[t] = (i < ch.ihi) ? Uj[i] : T(0);
-                    r[t] = (i < ch.ihi) ? rel[i] : 0;
-                }
+        for (int t = 0; t < 4; ++t) {
+            const int i = ch.ilo + lane + 32 * t;
+            r[t] = i < ch.ihi ? rel[i] - R0 : -1;
+        }
 #pragma unroll
-                for (int t = 0; t < 4; ++t)
-                    if (i0 + 32 * t < ch.ihi) B[r[t] + pj] += u[t];
+        for (int a = 0; a < 4; ++a) {
+            const int j = ch.j0 + warp + nwarp * a;
+            pc[a] = j < ch.j1 ? rel[j] - c0 : -1;
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {
+                const int i = ch.ilo + lane + 32 * t;
+                x[a][t] = (j < ch.j1 && i >= j && i < ch.ihi) ? U[(int64_t)j * ch.ld + i] : T(0);
             }
         }
+        bt = -1;
+        b = T(0);
+        if (rb == 0 && warp == nwarp - 1 && ch.j0 + lane < ch.j1) {
+            bt = rel[ch.j0 + lane] - c0;
+            b = static_cast<const T*>(sv.su)[ch.su_off + ch.j0 + lane];
+        }
+    };
+    for (int cb = wk.ch_lo; cb < wk.ch_hi; cb += kKids) {
+        const int n = min(kKids, wk.ch_hi - cb);
+        constexpr int kW16 = sizeof(AsmChild) / 16;
+        static_assert(kKids * kW16 <= kThreads, "one 16-byte word per thread");
+        if (tid < n * kW16) reinterpret_cast<int4*>(ks)[tid] = reinterpret_cast<const int4*>(kids + cb)[tid];
         __syncthreads();
+        load(ks[0], u, ri, pj, bv, pb);
+        for (int q = 0; q < n; ++q) {
+            if (q + 1 < n) load(ks[q + 1], un, rn, pn, bn, pbn);
+            const AsmChild& ch = ks[q];
+#pragma unroll
+            for (int a = 0; a < 4; ++a) {
+                const int j = ch.j0 + warp + nwarp * a;
+#pragma unroll
+                for (int t = 0; t < 4; ++t)
+                    if (pj[a] >= 0 && ri[t] >= 0 && ch.ilo + lane + 32 * t >= j) tile[pj[a] * kAsmRows + ri[t]] += u[a][t];
+            }
+            if (pb >= 0) vv[pb] += bv;
+            __syncthreads();
+#pragma unroll
+            for (int a = 0; a < 4; ++a) {
+                pj[a] = pn[a];
+                ri[a] = rn[a];
+#pragma unroll
+                for (int t = 0; t < 4; ++t) u[a][t] = un[a][t];
+            }
+            bv = bn;
+            pb = pbn;
+        }
     }
-    if (rb == 0 && tid < c1 - c0) *rhs_entry<T>(sv, p0, nc, F.sn_su_off[s], c0 + tid) = vv[tid];
+    __syncthreads();
+    for (int c = warp; c < c1 - c0; c += nwarp)
+        for (int r = lane; r < R1 - R0; r += 32)
+            if (R0 + r >= c0 + c) B[R0 + r + (int64_t)(c0 + c) * f] = tile[c * kAsmRows + r];
+    if (rb == 0 && tid < c1 - c0) *rhs_entry<T>(sv, R.c0, nc, R.su_off, c0 + tid) = vv[tid];
 }
 
 // FP64 panel step p of the tiled fronts: the diagonal block's factorisation
@@ -2725,7 +2763,7 @@ cudaError_t factor_impl(const DevNet& net, const DevFactor& F, const DevWork& W,
         }
         if (ls.flow_b_n > 0) {
             const int mf = ls.flow_b_maxf;
-            k_front_flow<T, kPanel, 1><<<ls.flow_b_grid, kThreads, front_smem<T>(mf), st>>>(
+            k_front_flow<T, kPanel, 1><<<ls.flow_b_grid, kFrontThreads<T, kPanel>, front_smem<T>(mf), st>>>(
                 F, W, sv, gv, lx, ub, ls.d_flow_b, ls.d_ready_n + 1, counters + 1, W.flow);
             count_launches(1);
         }
@@ -2743,7 +2781,7 @@ cudaError_t factor_impl(const DevNet& net, const DevFactor& F, const DevWork& W,
         const int ns = ls.h_small_ptr[l + 1] - ls.h_small_ptr[l];
         if (ns > 0) {
             const int mf = ls.h_small_maxf[l];
-            k_front_small<T><<<ns, kThreads, front_smem<T>(mf), st>>>(F, W, sv, gv, lx, ub,
+            k_front_small<T><<<ns, kFrontThreads<T, kPanel>, front_smem<T>(mf), st>>>(F, W, sv, gv, lx, ub,
                                                                       ls.d_small + ls.h_small_ptr[l]);
             count_launches(1);
         }
@@ -2861,13 +2899,13 @@ FlowGrids flow_grids_impl(int32_t maxf_a, int32_t maxf_b, int32_t solve_maxf, in
     int dev = 0, sms = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return g;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return g;
-    auto resident = [&](const void* fn, size_t smem) {
+    auto resident = [&](const void* fn, size_t smem, int threads = kThreads) {
         int per_sm = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kThreads, smem) != cudaSuccess) return 0;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, smem) != cudaSuccess) return 0;
         return per_sm * sms;
     };
     g.a = resident((const void*)k_front_flow<T, kPanelSmall, kMinBlocksA<T>>, front_smem<T>(maxf_a));
-    g.b = resident((const void*)k_front_flow<T, kPanel, 1>, front_smem<T>(maxf_b));
+    g.b = resident((const void*)k_front_flow<T, kPanel, 1>, front_smem<T>(maxf_b), kFrontThreads<T, kPanel>);
     if (solve_maxf <= 16384) g.solve = resident((const void*)k_fwd_flow<T, T>, solve_smem<T>(solve_maxf));
     g.w = resident((const void*)k_front_warp<T>, sizeof(WarpTile<T>) * kWarpsPerCta);
     g.wsolve = resident((const void*)k_fwd_warp<T, T>, 0);

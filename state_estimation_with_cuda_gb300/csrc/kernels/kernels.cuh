@@ -94,7 +94,7 @@ struct __align__(16) FrontRec {
     int64_t su_off;
     int32_t up_n;  // children of the parent in this front's dataflow phase (0: the parent is not in it)
     int32_t grid;
-    int32_t asm_slot;  // single-CTA fronts: its lists in asm_ptr
+    int32_t asm_slot;  // single-CTA fronts: its first list in asm_ptr
     int32_t pw;        // columns per panel of the factorisation
     int64_t rows_off;  // rows below the pivots in sn_rows
 };
@@ -103,7 +103,8 @@ struct __align__(16) ChildRec {
     int64_t u_off, su_off;
     int32_t m, ld, big, pad;  // update matrix: m x m, leading dimension, in the factor array (big) or u
 };
-constexpr int kAsmWarps = 8;  // warps of a single-CTA front's assembly
+// Warps of a single-CTA front's CTA (wide: phase B and the synchronous levels).
+__host__ __device__ constexpr int asm_warps(bool fp32, bool wide) { return fp32 && wide ? 16 : 8; }
 
 // Factorisation plan (device).
 struct DevFactor {
@@ -141,10 +142,10 @@ struct DevFactor {
     const int8_t* sn_pw;
     const FrontRec* rec;         // [n_super]
     const ChildRec* child_rec;   // [children], as sn_child
-    // Assembly of the single-CTA fronts: per front (FrontRec::asm_slot) and warp
-    // w, the children's columns whose front column t has t % kAsmWarps == w, in
-    // child order: (child position, child column | t << 16)
-    const int32_t* asm_ptr;      // [kAsmWarps * slots + 1]
+    // Assembly of the single-CTA fronts: per front (from FrontRec::asm_slot) and
+    // warp w, the children's columns whose front column t = w (mod the CTA's
+    // warps), in child order: (child position, child column | t << 16)
+    const int32_t* asm_ptr;      // [lists + 1]
     const int2* asm_ent;
 };
 
@@ -282,9 +283,12 @@ struct AsmItem {
 };
 // One child's part of an assembly block: its update-matrix columns [j0, j1)
 // that land in the tile column and rows [ilo, ihi) that land in the row
-// block (positions in the child's relative map).
-struct AsmChild {
-    int32_t c, j0, j1, ilo, ihi, pad0, pad1, pad2;
+// block (positions in the child's relative map, which starts at su_off), and
+// its update matrix (in the factor array when big, else in u).
+struct __align__(16) AsmChild {
+    int32_t j0, j1, ilo, ihi;
+    int64_t u_off, su_off;
+    int32_t ld, big, pad0, pad1;
 };
 
 // One work item (CTA) of an FP32 tiled front's step p (k_big_step32), with what
