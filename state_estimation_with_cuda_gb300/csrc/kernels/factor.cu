@@ -303,85 +303,142 @@ __device__ __forceinline__ void store4<double>(double* p, const double (&v)[4]) 
 template <typename T>
 constexpr bool kInvDiag = sizeof(T) == 4;
 
-// FP32 diagonal blocks in one warp's registers.  warp_potrf_bcast eliminates the
-// first kb columns of the rows the warp holds: lane i owns row i in a[]
-// (entries j <= i; zeros elsewhere); the remaining columns receive the Schur
-// complement update.  Per pivot k the pivot comes by shuffle, lanes below
-// scale their entry by 1 / L_kk, and every entry a_ij, k < j <= i, gets
-// a_ij -= l_ik l_jk, the column l_jk broadcast through the 16-byte-aligned
-// shared buffer col[] (four entries per load).  Entries
-// above the diagonal are left unmasked: a lane reads col[j] only for j > k,
-// written by lane j, whose value there is an entry of L, and the entries
-// above the diagonal are never written out.  Fully unrolled and branch-free
-// (a branch per column, even one always taken, keeps the next step's loads
-// from overlapping the pivot chain).  On return a[] is row i of L and
-// *inv_out = 1 / L_ii; returns true if a pivot was not positive and finite
-// (then replaced by 1).  warp_trinv_v4 forms L^-1 one column per lane
-// (L^-1 e_j by right-looking substitution, its rows read four at a time) and
-// writes rows i >= j to dst[i + j * ld].
-template <int KP>
-__device__ __forceinline__ bool warp_potrf_bcast(float (&a)[KP], int kb, int lane, float* inv_out, float* col) {
-    static_assert(KP % 4 == 0, "whole float4 groups");
+// FP32 diagonal blocks, one warp, kb <= 32 columns in blocks of eight.  An
+// outer step takes the updates of the columns before it (each lane's row against
+// the block's eight, read as two broadcast vectors) and then works the eight in
+// registers; every entry gets the operations of the plain right-looking order in
+// the same order.  As straight code for 32 columns they were some 600
+// instructions each and held 32 entries a lane (128 registers for the wide
+// fronts' kernel, 99 now); rolled over blocks of eight they take about the same
+// time on a whole block (6.5k, 3.1k and 4.0k cycles) and less on the narrow
+// panels that most fronts have: phase A 300 -> 284 us and phase B 157 -> 132 us
+// a call at 200k buses (mixed).
+//
+// Cholesky: lane i owns row i; get(j) is its entry of column j <= i (else
+// anything finite).  L goes to lt[c * ld + r] (16-byte aligned rows, ld > kb),
+// which may be where get reads.  *inv_out = 1 / L_ii of the lane's row; returns
+// true if a pivot was not positive and finite (then replaced by 1).
+constexpr int kBlk = 8;
+template <typename Get>
+__device__ __forceinline__ bool warp_potrf(int kb, int lane, float* lt, int ld, float* inv_out, Get&& get) {
     bool bad = false;
     float my_inv = 0.f;
+#pragma unroll 1
+    for (int b0 = 0; b0 < kb; b0 += kBlk) {
+        float a[kBlk];
 #pragma unroll
-    for (int k = 0; k < KP; ++k) {
-        if (k < kb) {
-            float d = __shfl_sync(0xffffffffu, a[k], k);
-            const bool ok = pivot_ok(d);
-            bad |= !ok;
-            d = ok ? d : 1.f;
-            float sq, inv;
-            pivot_value(d, &sq, &inv);
-            const float lk = (lane == k) ? sq : (lane > k ? a[k] * inv : a[k]);
-            a[k] = lk;
-            my_inv = (lane == k) ? inv : my_inv;
-            if (k + 1 < KP) {
-                col[lane] = lk;
-                __syncwarp();
+        for (int q = 0; q < kBlk; ++q) a[q] = (lane < kb && b0 + q <= lane) ? get(b0 + q) : 0.f;
+#pragma unroll 2
+        for (int k = 0; k < b0; ++k) {
+            const float lk = lt[k * ld + lane];
+            float w[kBlk];
+            *reinterpret_cast<float4*>(w) = *reinterpret_cast<const float4*>(lt + k * ld + b0);
+            *reinterpret_cast<float4*>(w + 4) = *reinterpret_cast<const float4*>(lt + k * ld + b0 + 4);
 #pragma unroll
-                for (int g = (k + 1) / 4; g < KP / 4; ++g) {
-                    const float4 v = reinterpret_cast<const float4*>(col)[g];
-                    const float w[4] = {v.x, v.y, v.z, v.w};
+            for (int q = 0; q < kBlk; ++q) a[q] = a[q] - lk * w[q];
+        }
+        float d = __shfl_sync(0xffffffffu, a[0], b0);
 #pragma unroll
-                    for (int q = 0; q < 4; ++q)
-                        if (4 * g + q > k) a[4 * g + q] = a[4 * g + q] - lk * w[q];
+        for (int q = 0; q < kBlk; ++q) {
+            const int k = b0 + q;
+            if (k < kb) {
+                const bool ok = pivot_ok(d);
+                bad |= !ok;
+                d = ok ? d : 1.f;
+                float sq, inv;
+                pivot_value(d, &sq, &inv);
+                const float lk = (lane == k) ? sq : (lane > k ? a[q] * inv : a[q]);
+                my_inv = (lane == k) ? inv : my_inv;
+                if (q + 1 < kBlk) {
+                    // the next pivot first: lane k + 1 has its own l to update it
+                    d = __shfl_sync(0xffffffffu, a[q + 1] - lk * lk, (k + 1) & 31);
                 }
-                __syncwarp();
+                if (lane < ld) lt[k * ld + lane] = lk;
+                if (q + 1 < kBlk) {
+                    __syncwarp();
+                    float w[kBlk];
+                    if (q < 3) *reinterpret_cast<float4*>(w) = *reinterpret_cast<const float4*>(lt + k * ld + b0);
+                    *reinterpret_cast<float4*>(w + 4) = *reinterpret_cast<const float4*>(lt + k * ld + b0 + 4);
+#pragma unroll
+                    for (int t = q + 1; t < kBlk; ++t) a[t] = a[t] - lk * w[t];
+                }
             }
         }
+        __syncwarp();
     }
     *inv_out = my_inv;
     return bad;
 }
 
-// lt rows 16-byte aligned (LTLD % 4 == 0): each row of L is read four
-// entries per broadcast load.
-template <int KP, int LTLD>
-__device__ __forceinline__ void warp_trinv_v4(const float (*lt)[LTLD], const float* rinv, int kb, int lane, float* dst,
-                                              int ld) {
-    static_assert(KP % 4 == 0 && LTLD % 4 == 0, "whole, aligned float4 groups");
-    float x[KP];
+// L^-1, one column per lane (L^-1 e_j by right-looking substitution, lane j):
+// rows i >= j to dst[i + j * dld].  rinv: the reciprocal diagonal.
+__device__ __forceinline__ void load_row8(const float* p, float (&w)[kBlk]) {
+    *reinterpret_cast<float4*>(w) = *reinterpret_cast<const float4*>(p);
+    *reinterpret_cast<float4*>(w + 4) = *reinterpret_cast<const float4*>(p + 4);
+}
+__device__ __forceinline__ void warp_trinv(const float* __restrict__ lt, int ld, const float* __restrict__ rinv, int kb,
+                                           int lane, float* __restrict__ dst, int dld) {
+    float* const mine = dst + lane * dld;
+#pragma unroll 1
+    for (int b0 = 0; b0 < kb; b0 += kBlk) {
+        float x[kBlk], ri[kBlk], w[kBlk][kBlk];
 #pragma unroll
-    for (int i = 0; i < KP; ++i) x[i] = (i == lane) ? 1.f : 0.f;
-#pragma unroll
-    for (int c = 0; c < KP; ++c) {
-        if (c < kb) {
-            x[c] *= rinv[c];
-#pragma unroll
-            for (int g = (c + 1) / 4; g < KP / 4; ++g) {
-                const float4 v = reinterpret_cast<const float4*>(lt[c])[g];
-                const float w[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-                for (int q = 0; q < 4; ++q)
-                    if (4 * g + q > c) x[4 * g + q] -= x[c] * w[q];
-            }
+        for (int q = 0; q < kBlk; ++q) {
+            x[q] = (b0 + q == lane) ? 1.f : 0.f;
+            ri[q] = b0 + q < kb ? rinv[b0 + q] : 0.f;
         }
-    }
-    if (lane < kb) {
+#pragma unroll 4
+        for (int c = 0; c < b0; ++c) {
+            const float xc = (lane < kb && c >= lane) ? mine[c] : 0.f;
+            float v[kBlk];
+            load_row8(lt + c * ld + b0, v);
 #pragma unroll
-        for (int i = 0; i < KP; ++i)
-            if (i >= lane && i < kb) dst[i + lane * ld] = x[i];
+            for (int q = 0; q < kBlk; ++q) x[q] -= xc * v[q];
+        }
+#pragma unroll
+        for (int q = 0; q + 1 < kBlk; ++q) load_row8(lt + min(b0 + q, kb - 1) * ld + b0, w[q]);
+#pragma unroll
+        for (int q = 0; q < kBlk; ++q) {
+            x[q] *= ri[q];
+#pragma unroll
+            for (int t = q + 1; t < kBlk; ++t) x[t] -= x[q] * w[q][t];
+        }
+#pragma unroll
+        for (int q = 0; q < kBlk; ++q)
+            if (b0 + q < kb && b0 + q >= lane) mine[b0 + q] = x[q];
+    }
+}
+
+// One row of X = A L^-T by substitution, in place: entry c at row[c * rld].
+__device__ __forceinline__ void row_trsm(const float* __restrict__ lt, int ld, const float* __restrict__ rinv, int kb,
+                                         float* __restrict__ row, int rld) {
+#pragma unroll 1
+    for (int b0 = 0; b0 < kb; b0 += kBlk) {
+        float x[kBlk], ri[kBlk];
+#pragma unroll
+        for (int q = 0; q < kBlk; ++q) {
+            x[q] = b0 + q < kb ? row[(b0 + q) * rld] : 0.f;
+            ri[q] = b0 + q < kb ? rinv[b0 + q] : 0.f;
+        }
+#pragma unroll 4
+        for (int c = 0; c < b0; ++c) {
+            const float xc = row[c * rld];
+            float v[kBlk];
+            load_row8(lt + c * ld + b0, v);
+#pragma unroll
+            for (int q = 0; q < kBlk; ++q) x[q] -= xc * v[q];
+        }
+#pragma unroll
+        for (int q = 0; q < kBlk; ++q) {
+            x[q] *= ri[q];
+            float v[kBlk];
+            if (q + 1 < kBlk) load_row8(lt + min(b0 + q, kb - 1) * ld + b0, v);
+#pragma unroll
+            for (int t = q + 1; t < kBlk; ++t) x[t] -= x[q] * v[t];
+        }
+#pragma unroll
+        for (int q = 0; q < kBlk; ++q)
+            if (b0 + q < kb) row[(b0 + q) * rld] = x[q];
     }
 }
 
@@ -698,19 +755,20 @@ __device__ __forceinline__ void hand_over(int k) {
 __device__ __forceinline__ void take_over(int k) { asm volatile("bar.sync %0, 64;" ::"r"(1 + (k & 7)) : "memory"); }
 
 // Shared-memory scratch of one front besides the front itself.
-template <typename T>
+template <typename T, int KP>
 struct FrontSmem;
-template <>
-struct FrontSmem<float> {
-    __align__(16) float lt[kPanel][kPanel + 4];  // lt[c][r] = L11[r][c] of the current panel (16-byte aligned rows)
-    __align__(16) float col[kPanel];             // pivot column broadcast of warp_potrf_bcast
-    float rinv[kPanel];                          // 1 / L11[c][c]
-    float v[kSmallFrontMax32];                   // right-hand side of the front's rows
+template <int KP>
+struct FrontSmem<float, KP> {
+    static constexpr int kLd = KP + 4;
+    __align__(16) float lt[KP * kLd];  // lt[c * kLd + r] = L11[r][c] of the current panel
+    float li[KP * (KP + 1)];        // L11^-1, column c at li + c * (KP + 1)
+    float rinv[KP];                 // 1 / L11[c][c]
+    float v[kSmallFrontMax32];      // right-hand side of the front's rows
 };
-template <>
-struct FrontSmem<double> {
-    double ms[kPanel][kPanel];  // column k of the current panel's block, unscaled, over its pivot
-    double dk[kPanel];          // pivots, then 1 / sqrt
+template <int KP>
+struct FrontSmem<double, KP> {
+    double ms[KP][kPanel];      // column k of the current panel's block, unscaled, over its pivot
+    double dk[KP];              // pivots, then 1 / sqrt
     int ready, ready_x;         // columns published: first 32 rows, rows below
 };
 
@@ -782,7 +840,7 @@ __device__ __forceinline__ void front_store(const SolveVecs& sv, T* lx, T* ub, c
 // update: phase B 337 -> 202 us, phase A 261 -> 159, synchronous levels 82 -> 50.
 template <int KP>
 __device__ void front_factor(const DevFactor& F, const DevWork& W, const SolveVecs& sv, const double* gv, double* lx,
-                             double* ub, const FrontRec& R, int s, double* Fm, FrontSmem<double>& sm) {
+                             double* ub, const FrontRec& R, int s, double* Fm, FrontSmem<double, KP>& sm) {
     static_assert(KP <= kPanel && kThreads == 256, "columns over eight warps");
     constexpr int kW = kThreads / 32, kQ = KP / kW;
     constexpr int kG = ((KP == kPanel ? kSmallFrontMax : kFlowSmallFMax) + 1 + 31) / 32;  // row groups of 32
@@ -917,7 +975,7 @@ __device__ void front_factor(const DevFactor& F, const DevWork& W, const SolveVe
 // FP32, with panels of KP <= kPanel columns.
 template <int KP>
 __device__ void front_factor(const DevFactor& F, const DevWork& W, const SolveVecs& sv, const float* gv, float* lx,
-                             float* ub, const FrontRec& R, int s, float* Fm, FrontSmem<float>& sm) {
+                             float* ub, const FrontRec& R, int s, float* Fm, FrontSmem<float, KP>& sm) {
     using T = float;
     static_assert(KP <= kPanel && KP <= 32, "panel wider than a warp");
     const int f = R.f, c0 = R.c0, nc = R.nc;
@@ -937,62 +995,41 @@ __device__ void front_factor(const DevFactor& F, const DevWork& W, const SolveVe
 #pragma unroll 1
     for (int k0 = 0; k0 < nc; k0 += KP) {
         const int kb = min(KP, nc - k0);
-        // (1) diagonal block, one warp, in registers.  The loop over the
-        // block's columns stays rolled (compact code for a single warp); the
-        // current column is picked out of the row registers by selects.
+        // (1) diagonal block, one warp
         if (warp == 0) {
-            T a[KP];
-            const int i = k0 + lane;
-#pragma unroll
-            for (int j = 0; j < KP; ++j) a[j] = (lane < kb && j <= lane) ? Fm[i + (k0 + j) * ldf] : T(0);
-            T my_inv;
-            const bool bad = warp_potrf_bcast<KP>(a, kb, lane, &my_inv, sm.col);
+            constexpr int kLd = FrontSmem<float, KP>::kLd;
+            float* P = Fm + k0 + k0 * ldf;
+            float my_inv;
+            const bool bad = warp_potrf(kb, lane, sm.lt, kLd, &my_inv, [&](int j) { return P[lane + j * ldf]; });
             if (lane < kb) {
                 sm.rinv[lane] = my_inv;
                 rdg[k0 + lane] = my_inv;
             }
             if (bad && lane == 0) atomicOr(singular_flags(F, W, s), FLAG_SINGULAR);
-#pragma unroll
-            for (int j = 0; j < KP; ++j)
-                if (lane < kb && j <= lane) {
-                    Fm[i + (k0 + j) * ldf] = a[j];
-                    sm.lt[j][lane] = a[j];
-                }
         } else if (k0 > 0) {
             rhs_below(k0 - KP, KP, 32, nth - 32);  // the other warps meanwhile: the previous panel's y
         }
         __syncthreads();
-        // (2) warp 0 writes the inverse of the diagonal block into its slot;
+        // (2) warp 0 inverts the diagonal block, which then goes into its slot;
         // the other threads: rows below the block, x = a L11^-T, one row per
         // thread (f - q0 < kThreads - 32)
         const int q0 = k0 + kb;
         if (warp == 0) {
-            warp_trinv_v4<KP, kPanel + 4>(sm.lt, sm.rinv, kb, lane, Fm + k0 + k0 * ldf, ldf);
+            constexpr int kLd = FrontSmem<float, KP>::kLd;
+            warp_trinv(sm.lt, kLd, sm.rinv, kb, lane, sm.li, KP + 1);
+            __syncwarp();
+            for (int j = 0; j < kb; ++j)
+                if (lane >= j && lane < kb) Fm[k0 + lane + (k0 + j) * ldf] = sm.li[lane + j * (KP + 1)];
         } else {
             const int r = q0 + tid - 32;
-            if (r < f) {
-                T x[KP];
-#pragma unroll
-                for (int c = 0; c < KP; ++c) x[c] = (c < kb) ? Fm[r + (k0 + c) * ldf] : T(0);
-#pragma unroll
-                for (int c = 0; c < KP; ++c) {
-                    if (c < kb) {
-                        x[c] *= sm.rinv[c];
-#pragma unroll
-                        for (int c2 = c + 1; c2 < KP; ++c2) x[c2] -= x[c] * sm.lt[c][c2];
-                    }
-                }
-#pragma unroll
-                for (int c = 0; c < KP; ++c)
-                    if (c < kb) Fm[r + (k0 + c) * ldf] = x[c];
-            }
+            if (r < f) row_trsm(sm.lt, FrontSmem<float, KP>::kLd, sm.rinv, kb, Fm + r + k0 * ldf, ldf);
         }
         __syncthreads();
         // y = L11^-1 v of the panel's rows, a lane per row (as in the forward sweep)
         if (warp == 0) {
             float y = 0.f;
             if (lane < kb)
-                for (int j = 0; j <= lane; ++j) y += Fm[k0 + lane + (k0 + j) * ldf] * sm.v[k0 + j];
+                for (int j = 0; j <= lane; ++j) y += sm.li[lane + j * (KP + 1)] * sm.v[k0 + j];
             __syncwarp();
             if (lane < kb) sm.v[k0 + lane] = y;
         }
@@ -1068,7 +1105,7 @@ template <typename T>
 __global__ void __launch_bounds__(kFrontThreads<T, kPanel>, 1) k_front_small(DevFactor F, DevWork W, SolveVecs sv, const T* gv, T* lx,
                                                              T* ub, const int* fronts) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ FrontSmem<T> sm;
+    __shared__ FrontSmem<T, kPanel> sm;
     const int s = fronts[blockIdx.x];
     const FrontRec R = F.rec[s];
     if (front_frozen(W, R)) return;
@@ -1140,7 +1177,7 @@ __global__ void __launch_bounds__(kFrontThreads<T, KP>, kMinBlocks) k_front_flow
                                                                      T* lx, T* ub, const int* ready, const int* n_ready,
                                                                      int* counter, int* cnt) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ FrontSmem<T> sm;
+    __shared__ FrontSmem<T, KP> sm;
     __shared__ int slot;
     const int nr = *n_ready;
     for (;;) {
@@ -1293,7 +1330,7 @@ __global__ void __launch_bounds__(kThreads) k_big_assemble(DevFactor F, DevWork 
 // step in about 37k cycles (18 us), where one warp's factorisation of the block
 // and a launch of one-warp row solves took 47 + 22 us; the linear solve of a
 // 30k-bus grid went from 5.04 to 3.08 ms with this and k_big_update64.
-__global__ void __launch_bounds__(kPanelThreads64) k_big_panel64(DevFactor F, DevWork W, SolveVecs sv, double* lx,
+__global__ void __launch_bounds__(kPanelThreads64, 2) k_big_panel64(DevFactor F, DevWork W, SolveVecs sv, double* lx,
                                                                  const int4* work, int p, int* step_cnt) {
     static_assert(kPanelThreads64 == 256 && kPanelRows64 == 16 && kTile == 32, "thread tiling below");
     constexpr int kW = kPanelThreads64 / 32, kQ = kTile / kW;  // columns per warp
@@ -1442,8 +1479,7 @@ __device__ __forceinline__ void big_panel32_item(const DevFactor& F, const DevWo
     constexpr int ld = kTile + 4;          // 16-byte aligned rows
     constexpr int lt_ld = kTile + 4;       // 16-byte aligned rows
     constexpr int as_ld = kPanelRows + 4;  // 16-byte aligned rows
-    __shared__ __align__(16) float D[kTile * ld];  // D[i + j * ld] = L_dd[i][j]
-    __shared__ __align__(16) float colbuf[kTile];
+    __shared__ __align__(16) float D[kTile * ld];  // D[i + j * ld]: the block, then L_dd
     __shared__ float rdiag[kTile];
     __shared__ __align__(16) float Lt[kTile * lt_ld];  // Lt[k][c] = L_dd^-1[c][k]
     __shared__ __align__(16) float As[kTile * as_ld];  // As[k][r] = A[r0 + r][k], then X
@@ -1491,19 +1527,13 @@ __device__ __forceinline__ void big_panel32_item(const DevFactor& F, const DevWo
     if (tid == 0) last = !pre && (atomicAdd(step_cnt + pair, 1) == nchunk - 1);  // this CTA's tile reads are done
     if (tid < 32 && !pre) {
         const int i = tid;
-        float a[kTile];
-#pragma unroll
-        for (int j = 0; j < kTile; ++j) a[j] = (i < pb && j <= i) ? D[i + j * ld] : 0.f;
         float inv;
-        const bool bad = warp_potrf_bcast<kTile>(a, pb, i, &inv, colbuf);
+        const bool bad = warp_potrf(pb, i, D, ld, &inv, [&](int j) { return D[i + j * ld]; });
         if (bad && i == 0 && chunk == 0) atomicOr(singular_flags(F, W, s), FLAG_SINGULAR);
-#pragma unroll
-        for (int j = 0; j < kTile; ++j)
-            if (i < pb && j <= i) D[i + j * ld] = a[j];
         if (i < pb) rdiag[i] = inv;
         if (chunk == 0 && i < pb) reinterpret_cast<float*>(W.rdiag)[F.sn_c0[s] + p0 + i] = inv;
         __syncwarp();
-        warp_trinv_v4<kTile, ld>(reinterpret_cast<const float (*)[ld]>(D), rdiag, pb, i, Lt, lt_ld);
+        warp_trinv(D, ld, rdiag, pb, i, Lt, lt_ld);
     }
     __syncthreads();
     if (chunk == 0 && tid < 32) {
@@ -1638,26 +1668,20 @@ __device__ __forceinline__ void big_update_item(const DevFactor& F, const DevWor
         __shared__ __align__(16) float D[kTile * dld];
         __shared__ float rdiag[kTile];
         __shared__ float Lt[kTile * lt_ld];
-        __shared__ __align__(16) float colbuf[kTile];
         __syncthreads();  // every update of this tile is written
         const int pb2 = min(kTile, nc - q0);
         if (threadIdx.x < 32) {
             const int i = threadIdx.x;
-            float a[kTile];
-#pragma unroll
-            for (int j = 0; j < kTile; ++j)
-                a[j] = (i < pb2 && j <= i) ? ld_entry<kL2>(B + (q0 + i) + (int64_t)(q0 + j) * f) : 0.f;
             float inv;
-            const bool bad = warp_potrf_bcast<kTile>(a, pb2, i, &inv, colbuf);
+            const bool bad = warp_potrf(pb2, i, D, dld, &inv,
+                                        [&](int j) { return ld_entry<kL2>(B + (q0 + i) + (int64_t)(q0 + j) * f); });
             if (bad && i == 0) atomicOr(singular_flags(F, W, s), FLAG_SINGULAR);
-#pragma unroll
-            for (int j = 0; j < kTile; ++j) D[i + j * dld] = (i < pb2 && j <= i) ? a[j] : 0.f;
             if (i < pb2) {
                 rdiag[i] = inv;
                 reinterpret_cast<float*>(W.rdiag)[F.sn_c0[s] + q0 + i] = inv;
             }
             __syncwarp();
-            warp_trinv_v4<kTile, dld>(reinterpret_cast<const float (*)[dld]>(D), rdiag, pb2, i, Lt, lt_ld);
+            warp_trinv(D, dld, rdiag, pb2, i, Lt, lt_ld);
             __syncwarp();
             for (int c = 0; c < pb2; ++c)
                 if (i >= c && i < pb2) B[(q0 + i) + (int64_t)(q0 + c) * f] = Lt[c * lt_ld + i];
@@ -1682,7 +1706,7 @@ struct StepPanelSmem {
     float lt[kTile * kStepLd];    // [k][c] = L_dd^-1[c][k]
     float xc[kTile * kStepRows];  // [k][r]: panel p, the chunk's rows
     float as[kTile * kStepRows];  // [j][r]: the chunk, then X
-    float col[kTile], rdiag[kTile], v[kTile];
+    float rdiag[kTile], v[kTile];
     int last;
 };
 struct StepTileSmem {
@@ -1756,21 +1780,14 @@ __device__ __forceinline__ void step_panel(const DevFactor& F, const DevWork& W,
     __syncthreads();
     if (warp == 0) {
         const int i = lane;
-        float a[kTile];
-#pragma unroll
-        for (int j = 0; j < kTile; ++j) a[j] = (i < pb && j <= i) ? sm.d[i + j * kStepLd] : 0.f;
+        for (int j = 0; j < kTile; ++j) sm.lt[j * kStepLd + i] = 0.f;
         float inv;
-        const bool bad = warp_potrf_bcast<kTile>(a, pb, i, &inv, sm.col);
+        const bool bad = warp_potrf(pb, i, sm.d, kStepLd, &inv, [&](int j) { return sm.d[i + j * kStepLd]; });
         if (bad && i == 0 && chunk == 0) atomicOr(singular_flags(F, W, it.s), FLAG_SINGULAR);
-#pragma unroll
-        for (int j = 0; j < kTile; ++j) {
-            sm.d[i + j * kStepLd] = (i < pb && j <= i) ? a[j] : 0.f;
-            sm.lt[j * kStepLd + i] = 0.f;
-        }
         if (i < pb) sm.rdiag[i] = inv;
         if (chunk == 0 && i < pb) reinterpret_cast<float*>(W.rdiag)[it.c0 + q0 + i] = inv;
         __syncwarp();
-        warp_trinv_v4<kTile, kStepLd>(reinterpret_cast<const float (*)[kStepLd]>(sm.d), sm.rdiag, pb, i, sm.lt, kStepLd);
+        warp_trinv(sm.d, kStepLd, sm.rdiag, pb, i, sm.lt, kStepLd);
     } else {
         // the chunk's update, 4 x 4 entries a turn
         for (int t = tid - 32; t < kThreads; t += kThreads - 32) {
