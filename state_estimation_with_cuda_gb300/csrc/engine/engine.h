@@ -327,6 +327,8 @@ private:
     void* h_batch_out_ = nullptr;     // pinned: flags, iters, mismatch, objective, running
     size_t h_batch_cap_ = 0;
     SolveRequest stream_rq_{};
+    std::vector<uint8_t> staged_;  // grids whose staged telemetry copy may still be running
+    int32_t batch_reads_ = 0;      // grid states read since the last batch solve
     std::vector<uint8_t> in_flight_;
     std::vector<int32_t> stream_iters_;
     int32_t analyze_batch();

@@ -114,6 +114,8 @@ __device__ __forceinline__ void pivot_value(float d, float* sq, float* inv) {
     *sq = d * y;
     *inv = y;
 }
+__device__ __noinline__ double slow_sqrt(double d) { return sqrt(d); }
+__device__ __noinline__ double slow_recip(double d) { return 1.0 / d; }
 __device__ __forceinline__ void pivot_value(double d, double* sq, double* inv) {
     if (in_fp32_range(d)) {
         const double y = widen_fp32(rsqrtf(leading_fp32(d)));
@@ -122,15 +124,9 @@ __device__ __forceinline__ void pivot_value(double d, double* sq, double* inv) {
         *sq = d * z;
         *inv = z;
     } else {
-        *sq = sqrt(d);
-        *inv = 1.0 / *sq;
+        *sq = slow_sqrt(d);
+        *inv = slow_recip(*sq);
     }
-}
-
-// Extend-add child c's update matrix (lower triangle) into a front buffer.
-template <typename T>
-__device__ __forceinline__ const T* update_of(const DevFactor& F, const T* lx, const T* ub, int c) {
-    return (F.sn_u_big[c] ? lx : ub) + F.sn_u_off[c];
 }
 
 // Extend-add of every child of a single-CTA front with no barrier between
@@ -271,29 +267,11 @@ __device__ __forceinline__ void extend_add_children(const DevFactor& F, const So
 constexpr int kPanel = 32;  // widest panel of the in-shared-memory factorisation
 static_assert(kThreads - 32 >= kSmallFrontMax32, "one thread per front row besides warp 0");
 
-template <typename T>
-__device__ __forceinline__ void load4(const T* p, T (&v)[4]);
-template <>
-__device__ __forceinline__ void load4<float>(const float* p, float (&v)[4]) {
-    const float4 q = *reinterpret_cast<const float4*>(p);
-    v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
+__device__ __forceinline__ void load4(const float* p, float (&v)[4]) {
+    *reinterpret_cast<float4*>(v) = *reinterpret_cast<const float4*>(p);
 }
-template <>
-__device__ __forceinline__ void load4<double>(const double* p, double (&v)[4]) {
-    const double2 q0 = reinterpret_cast<const double2*>(p)[0];
-    const double2 q1 = reinterpret_cast<const double2*>(p)[1];
-    v[0] = q0.x; v[1] = q0.y; v[2] = q1.x; v[3] = q1.y;
-}
-template <typename T>
-__device__ __forceinline__ void store4(T* p, const T (&v)[4]);
-template <>
-__device__ __forceinline__ void store4<float>(float* p, const float (&v)[4]) {
-    *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
-}
-template <>
-__device__ __forceinline__ void store4<double>(double* p, const double (&v)[4]) {
-    reinterpret_cast<double2*>(p)[0] = make_double2(v[0], v[1]);
-    reinterpret_cast<double2*>(p)[1] = make_double2(v[2], v[3]);
+__device__ __forceinline__ void store4(float* p, const float (&v)[4]) {
+    *reinterpret_cast<float4*>(p) = *reinterpret_cast<const float4*>(v);
 }
 
 // FP32 factors store L11^-1 in each diagonal block's slot, so that the solves
@@ -719,7 +697,7 @@ __device__ __forceinline__ double pivot_recip(double& d, bool& bad) {
         bad = true;
         d = 1.0;
     }
-    return 1.0 / d;
+    return slow_recip(d);
 }
 
 // Column counters of an elimination within one CTA: a column's owner raises
@@ -1059,8 +1037,8 @@ __device__ void front_factor(const DevFactor& F, const DevWork& W, const SolveVe
                 for (int c = 0; c < kb; ++c) {
                     const T* col = Fm + (k0 + c) * ldf;
                     T av[4], bv[4];
-                    load4<T>(col + i0, av);
-                    load4<T>(col + j0, bv);
+                    load4(col + i0, av);
+                    load4(col + j0, bv);
 #pragma unroll
                     for (int u = 0; u < 4; ++u)
 #pragma unroll
@@ -1072,11 +1050,11 @@ __device__ void front_factor(const DevFactor& F, const DevWork& W, const SolveVe
                     if (j < q0 || j >= f) continue;
                     T* dst = Fm + i0 + j * ldf;
                     T cur[4];
-                    load4<T>(dst, cur);
+                    load4(dst, cur);
 #pragma unroll
                     for (int u = 0; u < 4; ++u)
                         if (i0 + u >= j && i0 + u < f) cur[u] -= acc[u][v];
-                    store4<T>(dst, cur);
+                    store4(dst, cur);
                 }
             }
         }
@@ -1200,14 +1178,6 @@ __global__ void __launch_bounds__(kFrontThreads<T, KP>, kMinBlocks) k_front_flow
 // Big fronts, in place (L panel and update matrix share the f x f region at
 // sn_lx_off with ld = f).  Work lists hold int4 (front, a, b, 0).
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ int lower_bound_i32(const int* a, int lo, int hi, int key) {
-    while (lo < hi) {
-        const int mid = (lo + hi) >> 1;
-        if (a[mid] < key) lo = mid + 1; else hi = mid;
-    }
-    return lo;
-}
-
 // Assembly of a tiled front, one CTA per (tile column tj, block rb of
 // kAsmRows rows from the tile's first column down): the block's G entries, then
 // the update-matrix entries of the children that land in it, child by child (a
@@ -1800,8 +1770,8 @@ __device__ __forceinline__ void step_panel(const DevFactor& F, const DevWork& W,
 #pragma unroll 8
             for (int k = 0; k < kTile; ++k) {
                 float av[4], bv[4];
-                load4<float>(&sm.xc[k * kStepRows + 4 * rg], av);
-                load4<float>(&sm.xd[k * kStepLd + 4 * cg], bv);
+                load4(&sm.xc[k * kStepRows + 4 * rg], av);
+                load4(&sm.xd[k * kStepLd + 4 * cg], bv);
 #pragma unroll
                 for (int u = 0; u < 4; ++u)
 #pragma unroll
@@ -1810,10 +1780,10 @@ __device__ __forceinline__ void step_panel(const DevFactor& F, const DevWork& W,
 #pragma unroll
             for (int v = 0; v < 4; ++v) {
                 float cur[4];
-                load4<float>(&sm.as[(4 * cg + v) * kStepRows + 4 * rg], cur);
+                load4(&sm.as[(4 * cg + v) * kStepRows + 4 * rg], cur);
 #pragma unroll
                 for (int u = 0; u < 4; ++u) cur[u] = cur[u] - acc[u][v];
-                store4<float>(&sm.as[(4 * cg + v) * kStepRows + 4 * rg], cur);
+                store4(&sm.as[(4 * cg + v) * kStepRows + 4 * rg], cur);
             }
         }
         if (chunk == 0 && warp == 1) {
@@ -1849,8 +1819,8 @@ __device__ __forceinline__ void step_panel(const DevFactor& F, const DevWork& W,
 #pragma unroll 8
         for (int k = 0; k < kTile; ++k) {
             float av[4], lv[4];
-            load4<float>(&sm.as[k * kStepRows + 4 * rg], av);
-            load4<float>(&sm.lt[k * kStepLd + 4 * cg], lv);
+            load4(&sm.as[k * kStepRows + 4 * rg], av);
+            load4(&sm.lt[k * kStepLd + 4 * cg], lv);
             if (k >= pb) {
 #pragma unroll
                 for (int u = 0; u < 4; ++u) av[u] = 0.f;
