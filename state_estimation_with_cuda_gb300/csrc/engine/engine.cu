@@ -1343,12 +1343,16 @@ void Engine::collect_stage_times() {
     ev_used_ = 0;
 }
 
-int32_t Engine::enqueue_iteration(const SolveParams& sp, bool refactor, int64_t* per_stage, bool host_copies) {
-    cudaError_t e = cudaMemsetAsync(&work_.status->flags, 0, sizeof(uint32_t), st_);
-    if (e == cudaSuccess && batch_mode()) e = cudaMemsetAsync(batch_.running, 0, sizeof(int32_t), st_);
-    auto update = [&](const double* step) {
-        return batch_mode() ? launch_batch_update(net_, fac_, work_, batch_, sp, step, st_)
-                            : launch_update(net_, fac_, work_, sp, step, st_);
+int32_t Engine::enqueue_iteration(const SolveParams& sp, bool refactor, int64_t* per_stage,
+                                  const cudaGraphConditionalHandle* loop) {
+    cudaError_t e = cudaSuccess;
+    // the host reads the status after each step, except in a device-run loop
+    DevStatus* host = loop ? nullptr : h_status_;
+    auto update = [&](const auto* step) {
+        if (!batch_mode()) return launch_update(net_, fac_, work_, sp, step, host, st_);
+        const size_t G = static_cast<size_t>(batch_.n_grids);
+        int32_t* h_running = reinterpret_cast<int32_t*>(static_cast<char*>(h_batch_out_) + G * 24);
+        return launch_batch_update(net_, fac_, work_, batch_, sp, step, loop, host, h_running, st_);
     };
     auto stage = [&](int32_t st, auto&& fn) {
         if (e != cudaSuccess) return;
@@ -1360,18 +1364,17 @@ int32_t Engine::enqueue_iteration(const SolveParams& sp, bool refactor, int64_t*
     };
     if (sched_.compact) stage(ST_OTHER, [&] { return launch_ready_compact(fac_, work_, sched_, st_); });
     stage(ST_EVALUATE, [&] { return launch_evaluate(net_, work_, sp, st_); });
-    // a refactorisation takes the right-hand side along (launch_factor)
-    stage(ST_RHS, [&] { return launch_rhs(net_, fac_, work_, st_); });
+    // a refactorisation computes the right-hand side and takes it along (launch_factor)
+    if (!refactor) stage(ST_RHS, [&] { return launch_rhs(net_, fac_, work_, true, st_); });
     if (!mixed_) {
-        if (refactor) stage(ST_FACTOR, [&] { return launch_factor(net_, fac_, work_, sched_, st_); });
+        if (refactor) stage(ST_FACTOR, [&] { return launch_factor(net_, fac_, work_, sched_, true, st_); });
         stage(ST_SOLVE, [&] { return launch_solve(fac_, work_, sched_, !refactor, st_); });
         stage(ST_UPDATE, [&] { return update(work_.sol); });
     } else {
-        stage(ST_SOLVE, [&] { return launch_to_fp32(fac_, work_, st_); });
-        if (refactor) stage(ST_FACTOR, [&] { return launch_factor32(net_, fac_, work_, sched_, st_); });
+        if (refactor) stage(ST_FACTOR, [&] { return launch_factor32(net_, fac_, work_, sched_, true, st_); });
         stage(ST_SOLVE, [&] {
             cudaError_t ee = launch_solve32(fac_, work_, sched_, !refactor, st_);
-            if (ee == cudaSuccess) ee = launch_refine_begin(fac_, work_, st_);
+            if (ee == cudaSuccess && cfg.refine_steps > 0) ee = launch_refine_begin(fac_, work_, st_);
             for (int32_t k = 0; k < cfg.refine_steps && ee == cudaSuccess; ++k) {
                 ee = launch_refine_residual(net_, fac_, work_, st_);
                 if (ee == cudaSuccess) ee = launch_solve32(fac_, work_, sched_, true, st_);
@@ -1379,14 +1382,7 @@ int32_t Engine::enqueue_iteration(const SolveParams& sp, bool refactor, int64_t*
             }
             return ee;
         });
-        stage(ST_UPDATE, [&] { return update(work_.dx); });
-    }
-    if (e == cudaSuccess && host_copies)
-        e = cudaMemcpyAsync(h_status_, work_.status, sizeof(DevStatus), cudaMemcpyDeviceToHost, st_);
-    if (e == cudaSuccess && host_copies && batch_mode()) {
-        const int32_t G = batch_.n_grids;
-        int32_t* h_running = reinterpret_cast<int32_t*>(static_cast<char*>(h_batch_out_) + static_cast<size_t>(G) * 24);
-        e = cudaMemcpyAsync(h_running, batch_.running, sizeof(int32_t), cudaMemcpyDeviceToHost, st_);
+        stage(ST_UPDATE, [&] { return cfg.refine_steps > 0 ? update(work_.dx) : update(work_.sol32); });
     }
     if (e != cudaSuccess) {
         set_cuda_error(e, "iteration");
@@ -1438,11 +1434,8 @@ int32_t Engine::run_device_loop(const SolveParams& sp, int32_t max_iter, int32_t
             cudaGraph_t body = np.conditional.phGraph_out[0];
             e = cudaStreamBeginCaptureToGraph(st_, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
             if (e == cudaSuccess) {
-                rc = enqueue_iteration(sp, true, g.launches, false);
-                cudaError_t ek = rc == 0 ? launch_gn_loop_next(h, batch_, work_, st_) : cudaSuccess;
-                g.launches[ST_OTHER] += 1;
+                rc = enqueue_iteration(sp, true, g.launches, &h);
                 e = cudaStreamEndCapture(st_, &body);
-                if (e == cudaSuccess) e = ek;
             }
         }
         g.total = t_kernel_launches - before;
@@ -1771,7 +1764,7 @@ int32_t Engine::evaluate_at(const double* v, const double* th, int32_t exact) {
     sp.vmax = cfg.voltage_max_pu;
     if (e == cudaSuccess) e = launch_evaluate(net_, work_, sp, st_);
     if (e == cudaSuccess) e = launch_objective(net_, work_, cfg.bad_data_threshold, st_);
-    if (e == cudaSuccess) e = launch_rhs(net_, fac_, work_, st_);
+    if (e == cudaSuccess) e = launch_rhs(net_, fac_, work_, false, st_);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st_);
     if (e != cudaSuccess) return set_cuda_error(e, "evaluate");
     stale_ = DL_ALL;
@@ -1820,7 +1813,7 @@ int32_t Engine::factor_and_solve(const double* rhs_orig, double* x_orig) {
     for (int32_t p = 0; p < P.n_state; ++p) b[p] = rhs_orig[P.state_of_ps[p]];
     cudaError_t e = cudaMemsetAsync(&work_.status->flags, 0, sizeof(uint32_t), st_);
     if (e == cudaSuccess) e = cudaMemcpyAsync(work_.rhs, b.data(), sizeof(double) * P.n_state, cudaMemcpyHostToDevice, st_);
-    if (e == cudaSuccess) e = launch_factor(net_, fac_, work_, sched_, st_);
+    if (e == cudaSuccess) e = launch_factor(net_, fac_, work_, sched_, false, st_);
     if (e == cudaSuccess) e = launch_solve(fac_, work_, sched_, false, st_);
     std::vector<double> x(P.n_state);
     if (e == cudaSuccess) e = cudaMemcpyAsync(x.data(), work_.sol, sizeof(double) * P.n_state, cudaMemcpyDeviceToHost, st_);

@@ -362,9 +362,10 @@ private:
     // body is one step (with refactorisation) and the loop-control kernel.
     IterGraph loop_graph_;
     void drop_graphs();
-    // host_copies: end the step with the status and running-count copies the
-    // host loop reads (left out of the device loop's body).
-    int32_t enqueue_iteration(const SolveParams& sp, bool refactor, int64_t* per_stage, bool host_copies = true);
+    // loop: the while node of a device-run loop whose body the step is; without
+    // it the step leaves its status (and running count) where the host reads them.
+    int32_t enqueue_iteration(const SolveParams& sp, bool refactor, int64_t* per_stage,
+                              const cudaGraphConditionalHandle* loop = nullptr);
     // Runs up to max_iter steps of a batch solve on the device; `steps` gets
     // the number run.  -1: the graph path is off (use the host loop).
     int32_t run_device_loop(const SolveParams& sp, int32_t max_iter, int32_t& steps);

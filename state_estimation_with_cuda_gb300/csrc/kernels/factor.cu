@@ -56,12 +56,51 @@ __device__ __forceinline__ ACC gain_entry(const DevFactor& F, const HV* hval, co
     return acc;
 }
 
+// a11: entry t of b = H^T (w r) in permuted state order (gather).
+__device__ __forceinline__ void rhs_value(const DevFactor& F, const DevWork& W, const int32_t* h_row, int t) {
+    if (F.ps_grid && (W.grid_flags[F.ps_grid[t]] & FLAG_FROZEN)) return;
+    double acc = 0.0;
+    for (int x = F.rhs_ptr[t]; x < F.rhs_ptr[t + 1]; ++x) {
+        const int h = F.rhs_h[x];
+        acc += W.hval[h] * W.wr[h_row[h]];
+    }
+    W.rhs[t] = acc;
+    if (W.rhs32) W.rhs32[t] = static_cast<float>(acc);
+}
+
+__global__ void k_rhs(DevFactor F, DevWork W, const int32_t* h_row, int begin) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (begin && t == 0) W.status->flags = 0u;
+    if (t < F.n_state) rhs_value(F, W, h_row, t);
+}
+
+// Counters that a factorisation starts from zero.
+struct ZeroLists {
+    int* p[3];
+    int n[3];
+};
+
 // All gain entries of the factorisation at once: fully parallel, so the
 // dependent gathers are hidden by occupancy instead of sitting on the
-// elimination tree's critical path.
+// elimination tree's critical path.  The first rhs_blocks CTAs compute the
+// right-hand side of a Gauss-Newton step meanwhile (it has the longest chain
+// of gathers per thread and needs few threads), and all clear the counters:
+// with this and the step's end in one kernel (k_update) a step has seven nodes
+// fewer, which took 25 us of 727 at 10k buses (FP32) and 65 of the 573 us of a
+// whole estimate at 14 buses (FP64).
 template <typename T, typename HV, typename ACC = double>
-__global__ void k_gain_values(DevFactor F, DevWork W, const HV* hval, const HV* hw, T* gv, int n_tgt) {
-    for (int tg = blockIdx.x * blockDim.x + threadIdx.x; tg < n_tgt; tg += gridDim.x * blockDim.x) {
+__global__ void k_gain_values(DevFactor F, DevWork W, const HV* hval, const HV* hw, T* gv, int n_tgt,
+                              const int32_t* h_row, int rhs_blocks, ZeroLists Z) {
+    const int me = blockIdx.x * blockDim.x + threadIdx.x, all = gridDim.x * blockDim.x;
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+        for (int i = me; i < Z.n[k]; i += all) Z.p[k][i] = 0;
+    if (blockIdx.x < rhs_blocks) {
+        if (me == 0) W.status->flags = 0u;
+        if (me < F.n_state) rhs_value(F, W, h_row, me);
+        return;
+    }
+    for (int tg = me - rhs_blocks * blockDim.x; tg < n_tgt; tg += (gridDim.x - rhs_blocks) * blockDim.x) {
         if (F.tgt_grid && (W.grid_flags[F.tgt_grid[tg]] & FLAG_FROZEN)) continue;
         gv[tg] = static_cast<T>(gain_entry<HV, ACC>(F, hval, hw, tg));
     }
@@ -1187,7 +1226,7 @@ __global__ void __launch_bounds__(kFrontThreads<T, KP>, kMinBlocks) k_front_flow
 // AsmChild).  Bound: load latency, child after child; the block is summed in
 // shared memory and written once, and the next child's entries (four columns a
 // warp, four rows a lane) are in flight while one is added (20 us a level as
-// read-modify-writes of the front, ASMBIG with this, at 60k buses).
+// read-modify-writes of the front, 18.6 us with this, FP64 at 60k buses).
 // Row block 0 also assembles the tile column's right-hand-side entries: it
 // holds the diagonal, so its list has every child with a column here.
 template <typename T>
@@ -2720,20 +2759,19 @@ cudaError_t prepare_impl() {
 
 template <typename T, typename HV>
 cudaError_t factor_impl(const DevNet& net, const DevFactor& F, const DevWork& W, const LevelSchedule& ls, const HV* hval,
-                        const HV* hw,
-                        T* lx, T* ub, SolveVecs sv, cudaStream_t st) {
+                        const HV* hw, T* lx, T* ub, SolveVecs sv, bool begin, cudaStream_t st) {
     T* gv = reinterpret_cast<T*>(W.gvals);
-    if (ls.n_tgt > 0) {
-        if (sizeof(T) == 4 && ls.gain_acc32)
-            k_gain_values<T, HV, float><<<grid_for(ls.n_tgt, 256), 256, 0, st>>>(F, W, hval, hw, gv, ls.n_tgt);
-        else
-            k_gain_values<T, HV, double><<<grid_for(ls.n_tgt, 256), 256, 0, st>>>(F, W, hval, hw, gv, ls.n_tgt);
-        count_launches(1);
-    }
+    const bool tile_flow = sizeof(T) == 4 && ls.n_tt > 0;
     {
         // the flags and counters of the factorisation and of the backward sweep after it
-        cudaError_t e = cudaMemsetAsync(W.flow, 0, sizeof(int) * (3 * (size_t)F.n_super + 16), st);
-        if (e != cudaSuccess) return e;
+        const ZeroLists Z{{W.flow, ls.d_pot_cnt, ls.d_tt_done},
+                          {3 * F.n_super + 16, ls.n_pot_pairs, tile_flow ? ls.n_tt + ls.n_levels : 0}};
+        const int nr = begin ? (F.n_state + kThreads - 1) / kThreads : 0, nb = nr + grid_for(ls.n_tgt, kThreads);
+        if (sizeof(T) == 4 && ls.gain_acc32)
+            k_gain_values<T, HV, float><<<nb, kThreads, 0, st>>>(F, W, hval, hw, gv, ls.n_tgt, net.h_row, nr, Z);
+        else
+            k_gain_values<T, HV, double><<<nb, kThreads, 0, st>>>(F, W, hval, hw, gv, ls.n_tgt, net.h_row, nr, Z);
+        count_launches(1);
     }
     if (ls.flow_a_n + ls.flow_b_n + ls.flow_w_n > 0) {
         int* counters = W.flow + F.n_super;
@@ -2754,15 +2792,6 @@ cudaError_t factor_impl(const DevNet& net, const DevFactor& F, const DevWork& W,
                 F, W, sv, gv, lx, ub, ls.d_flow_b, ls.d_ready_n + 1, counters + 1, W.flow);
             count_launches(1);
         }
-    }
-    if (ls.n_pot_pairs > 0) {
-        cudaError_t e = cudaMemsetAsync(ls.d_pot_cnt, 0, sizeof(int) * (size_t)ls.n_pot_pairs, st);
-        if (e != cudaSuccess) return e;
-    }
-    const bool tile_flow = sizeof(T) == 4 && ls.n_tt > 0;
-    if (tile_flow) {
-        cudaError_t e = cudaMemsetAsync(ls.d_tt_done, 0, sizeof(int) * (size_t)(ls.n_tt + ls.n_levels), st);
-        if (e != cudaSuccess) return e;
     }
     for (int l = 0; l < ls.n_levels; ++l) {
         const int ns = ls.h_small_ptr[l + 1] - ls.h_small_ptr[l];
@@ -2940,9 +2969,15 @@ SolveVecs vecs32(const DevWork& W) { return SolveVecs{W.rhs32, W.sol32, W.su32};
 SolveVecs vecs64(const DevWork& W) { return SolveVecs{W.rhs, W.sol, W.su}; }
 }  // namespace
 
+cudaError_t launch_rhs(const DevNet& net, const DevFactor& F, const DevWork& W, bool begin, cudaStream_t st) {
+    k_rhs<<<(F.n_state + kThreads - 1) / kThreads, kThreads, 0, st>>>(F, W, net.h_row, begin ? 1 : 0);
+    count_launches(1);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_factor32(const DevNet& net, const DevFactor& F, const DevWork& W, const LevelSchedule& ls,
-                            cudaStream_t st) {
-    return factor_impl<float, float>(net, F, W, ls, W.hval32, W.hw32, W.lx32, W.u32, vecs32(W), st);
+                            bool begin, cudaStream_t st) {
+    return factor_impl<float, float>(net, F, W, ls, W.hval32, W.hw32, W.lx32, W.u32, vecs32(W), begin, st);
 }
 
 cudaError_t launch_solve32(const DevFactor& F, const DevWork& W, const LevelSchedule& ls, bool forward,
@@ -2950,9 +2985,9 @@ cudaError_t launch_solve32(const DevFactor& F, const DevWork& W, const LevelSche
     return solve_impl<float>(F, W, ls, W.lx32, reinterpret_cast<const float*>(W.rdiag), vecs32(W), forward, st);
 }
 
-cudaError_t launch_factor(const DevNet& net, const DevFactor& F, const DevWork& W, const LevelSchedule& ls,
+cudaError_t launch_factor(const DevNet& net, const DevFactor& F, const DevWork& W, const LevelSchedule& ls, bool begin,
                           cudaStream_t st) {
-    return factor_impl<double, double>(net, F, W, ls, W.hval, W.hw, W.lx, W.u, vecs64(W), st);
+    return factor_impl<double, double>(net, F, W, ls, W.hval, W.hw, W.lx, W.u, vecs64(W), begin, st);
 }
 
 cudaError_t launch_solve(const DevFactor& F, const DevWork& W, const LevelSchedule& ls, bool forward,
@@ -3066,7 +3101,7 @@ cudaError_t launch_factor_solve_noalloc(const DevNet& net, const DevFactor& F, c
         k_state_to_ps<<<grid_for(n, 256), 256, 0, st>>>(net, F, d_rhs, W2.rhs);
         count_launches(1);
     }
-    e = launch_factor(net, F, W2, ls, st);
+    e = launch_factor(net, F, W2, ls, false, st);
     if (e == cudaSuccess) e = launch_solve(F, W2, ls, false, st);
     if (e != cudaSuccess) return e;
     if (n > 0) {

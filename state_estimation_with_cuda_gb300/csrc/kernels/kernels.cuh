@@ -27,7 +27,7 @@ struct DevStatus {
     int32_t largest_idx;
     uint32_t flags;
     int32_t bad_count;     // rows with |r|/sigma > threshold (bad-data pass)
-    int32_t pad;
+    uint32_t blocks_done;  // CTAs of the running state update that are through; zero between updates
 };
 
 // Static network data (device).
@@ -252,15 +252,13 @@ cudaError_t launch_admittance_and_ybus(const DevNet& net, cudaStream_t st);
 
 // One evaluation pass: h(x), r, H values, weights, objective partials.
 cudaError_t launch_evaluate(const DevNet& net, const DevWork& w, const SolveParams& sp, cudaStream_t st);
-// RHS b = H^T (w r), permuted.
-cudaError_t launch_rhs(const DevNet& net, const DevFactor& f, const DevWork& w, cudaStream_t st);
-// State update x += step (permuted step vector) + convergence / validity,
-// then status finalisation.
+// State update x += step (permuted step vector) + convergence / validity, then
+// status finalisation; the final status also goes to `host` (pinned host
+// memory) when given.  step: FP64, or the FP32 solution of a mixed step.
+template <typename V>
 cudaError_t launch_update(const DevNet& net, const DevFactor& f, const DevWork& w, const SolveParams& sp,
-                          const double* step, cudaStream_t st);
+                          const V* step, DevStatus* host, cudaStream_t st);
 // Mixed-precision refinement pieces (the solves run in FP32):
-//   rhs32 = (float) rhs
-cudaError_t launch_to_fp32(const DevFactor& f, const DevWork& w, cudaStream_t st);
 //   b0 = rhs (kept), dx = sol32
 cudaError_t launch_refine_begin(const DevFactor& f, const DevWork& w, cudaStream_t st);
 //   rhs32 = b0 - H^T W H dx  (FP64 accumulation over the FP32 H)
@@ -404,8 +402,12 @@ cudaError_t launch_ready_compact(const DevFactor& f, const DevWork& w, const Lev
 // Batch control: begin (flags, flat starts), per-grid update + convergence,
 // per-grid objective at the final state.
 cudaError_t launch_batch_begin(const DevNet& net, const DevWork& w, const DevBatch& b, cudaStream_t st);
+// loop: the while node of a device-run Gauss-Newton loop, or null.  host,
+// host_running (pinned host memory): the step's status and running count, or null.
+template <typename V>
 cudaError_t launch_batch_update(const DevNet& net, const DevFactor& f, const DevWork& w, const DevBatch& b,
-                                const SolveParams& sp, const double* step, cudaStream_t st);
+                                const SolveParams& sp, const V* step, const cudaGraphConditionalHandle* loop,
+                                DevStatus* host, int32_t* host_running, cudaStream_t st);
 // Objective of every grid that is not inactive and whose flags hold `need`.
 cudaError_t launch_batch_objective(const DevNet& net, const DevWork& w, const DevBatch& b, uint32_t need,
                                    cudaStream_t st);
@@ -425,12 +427,11 @@ cudaError_t launch_islands(const DevNet& net, int32_t* parent, int32_t* out, int
 // others as they are; retire the grids with retire[g] = 1 (frozen, inactive).
 cudaError_t launch_batch_activate(const DevNet& net, const DevWork& w, const DevBatch& b, cudaStream_t st);
 cudaError_t launch_batch_retire(const DevBatch& b, cudaStream_t st);
-// Device Gauss-Newton loop of a batch solve: the host captures one step and
-// launch_gn_loop_next into the body of a conditional while node; the node
-// repeats the body while grids are running, no wait has timed out and fewer
-// than `limit` steps have run (launch_gn_loop_init, before each launch).
+// Device Gauss-Newton loop of a batch solve: the host captures one step into
+// the body of a conditional while node, which the step's update
+// (launch_batch_update) repeats while grids are running, no wait has timed out
+// and fewer than `limit` steps have run (launch_gn_loop_init, before each launch).
 cudaError_t launch_gn_loop_init(const DevBatch& b, int32_t limit, cudaStream_t st);
-cudaError_t launch_gn_loop_next(cudaGraphConditionalHandle h, const DevBatch& b, const DevWork& w, cudaStream_t st);
 
 // Largest front the high-occupancy dataflow phase may hold (its kernel keeps
 // 16-column panels and a register budget for several CTAs per SM).
@@ -488,17 +489,22 @@ constexpr int kUpdTile64 = 16;
 // Sets the kernel attributes (dynamic shared memory limits) on the current
 // device; call before launching or capturing the factorisation.
 cudaError_t prepare_factor_kernels();
+// Right-hand side b = H^T (w r), permuted, in rhs (and rounded in rhs32, when
+// there is one).  begin: first part of a step, which clears the status flags.
+cudaError_t launch_rhs(const DevNet& net, const DevFactor& f, const DevWork& w, bool begin, cudaStream_t st);
 // The factorisation carries the right-hand side (DevWork::rhs, FP32: rhs32)
 // along and leaves y = L^-1 b in sol (sol32); launch_solve with forward =
 // false then runs the backward sweep.  With forward = true it solves for a new
-// right-hand side with the factor at hand.
-cudaError_t launch_factor(const DevNet& net, const DevFactor& f, const DevWork& w, const LevelSchedule& ls,
+// right-hand side with the factor at hand.  begin: the factorisation of a
+// Gauss-Newton step, which first does what launch_rhs with begin does, in the
+// launch that computes the gain values.
+cudaError_t launch_factor(const DevNet& net, const DevFactor& f, const DevWork& w, const LevelSchedule& ls, bool begin,
                           cudaStream_t st);
 cudaError_t launch_solve(const DevFactor& f, const DevWork& w, const LevelSchedule& ls, bool forward,
                          cudaStream_t st);
 // FP32 gain / factor and mixed solves (FP32 L, FP64 vectors).
 cudaError_t launch_factor32(const DevNet& net, const DevFactor& f, const DevWork& w, const LevelSchedule& ls,
-                            cudaStream_t st);
+                            bool begin, cudaStream_t st);
 cudaError_t launch_solve32(const DevFactor& f, const DevWork& w, const LevelSchedule& ls, bool forward,
                            cudaStream_t st);
 

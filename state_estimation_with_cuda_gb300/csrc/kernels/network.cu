@@ -667,27 +667,8 @@ __global__ void k_huber_objective(DevWork w, int nblk) {
     if (threadIdx.x == 0) w.status->huber_objective = acc;
 }
 
-// a11: b = H^T (w r) in permuted state order, one thread per state (gather).
-__global__ void k_rhs(DevNet net, DevFactor f, DevWork w) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= f.n_state) return;
-    if (f.ps_grid && (w.grid_flags[f.ps_grid[t]] & FLAG_FROZEN)) return;
-    double acc = 0.0;
-    for (int x = f.rhs_ptr[t]; x < f.rhs_ptr[t + 1]; ++x) {
-        const int hidx = f.rhs_h[x];
-        acc += w.hval[hidx] * w.wr[net.h_row[hidx]];
-    }
-    w.rhs[t] = acc;
-}
-
 // Mixed-precision refinement of one Gauss-Newton step (FP32 factor M ~ G):
 //   dx0 = M^-1 b;  repeat: rho = b - H^T W (H dx) in FP64, dx += M^-1 rho.
-__global__ void k_to_fp32(DevFactor f, DevWork w) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= f.n_state) return;
-    w.rhs32[t] = static_cast<float>(w.rhs[t]);
-}
-
 __global__ void k_refine_begin(DevFactor f, DevWork w) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= f.n_state) return;
@@ -804,52 +785,76 @@ __global__ void k_objective(DevNet net, DevWork w, int nblk, int nblk_eval) {
     }
 }
 
-// a13: x += dx (slack angle fixed), V clamped, block maxima of |dx|.
-__global__ void __launch_bounds__(kBlock) k_update(DevNet net, DevFactor f, DevWork w, SolveParams sp,
-                                                   const double* step) {
-    __shared__ double sh[32];
-    __shared__ int bad;
-    if (threadIdx.x == 0) bad = 0;
+// Counts the CTA in and tells whether it is the grid's last: what the others
+// wrote before is then visible to all of its threads.  The counter wraps back
+// to zero.
+__device__ __forceinline__ bool last_block(uint32_t* done) {
+    __shared__ bool last;
+    __syncthreads();  // the CTA's writes are made
+    if (threadIdx.x == 0) {
+        __threadfence();
+        last = atomicInc(done, gridDim.x - 1) == gridDim.x - 1;
+        __threadfence();
+    }
     __syncthreads();
+    return last;
+}
+
+// One bus's step: x += dx (slack angle fixed), V clamped.  Returns |dx|, 0 for
+// a NaN; bad is set when the step is not finite.
+template <typename V>
+__device__ __forceinline__ double update_bus(const DevFactor& f, const DevWork& w, const SolveParams& sp,
+                                             const V* step, int i, int& bad) {
+    const int pt = f.bus_ps_theta[i];
+    const double dv = static_cast<double>(step[f.bus_ps_v[i]]);
+    double dt = 0.0;
+    if (pt >= 0) {
+        dt = static_cast<double>(step[pt]);
+        w.th[i] += dt;
+    }
+    double vn = w.v[i] + dv;
+    vn = fmax(vn, sp.vmin);
+    vn = fmin(vn, sp.vmax);
+    w.v[i] = vn;
+    if (!isfinite(dt) || !isfinite(dv)) bad = 1;
+    const double m = fmax(fabs(dt), fabs(dv));
+    return m != m ? 0.0 : m;
+}
+
+// a13: x += dx, block maxima of |dx|; the last CTA takes the maximum over them
+// and writes the step's status, on the device and in host memory (a second
+// kernel and a copy node before; figures at k_gain_values).
+//
+// A step with a non-finite entry (FLAG_NONFINITE) is never converged and
+// reports a NaN max |dx|: the reference's max reduction turns NaN once a NaN
+// step fills its blocks (kernels.cu:557-574,752-782), so "max |dx| < tol"
+// fails and checkValidityKernel's flag decides: DIVERGED
+// (wls_solver.cu:493-517, 343-352).
+template <typename V>
+__global__ void __launch_bounds__(kBlock) k_update(DevNet net, DevFactor f, DevWork w, SolveParams sp,
+                                                   const V* step, DevStatus* host) {
+    __shared__ double sh[32];
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     double mx = 0.0;
-    if (i < net.n_bus) {
-        const int pt = f.bus_ps_theta[i];
-        const double dv = step[f.bus_ps_v[i]];
-        double dt = 0.0;
-        if (pt >= 0) {
-            dt = step[pt];
-            w.th[i] += dt;
-        }
-        double vn = w.v[i] + dv;
-        vn = fmax(vn, sp.vmin);
-        vn = fmin(vn, sp.vmax);
-        w.v[i] = vn;
-        if (!isfinite(dt) || !isfinite(dv)) bad = 1;
-        mx = fmax(fabs(dt), fabs(dv));
-        if (mx != mx) mx = 0.0;
-    }
+    int bad = 0;
+    if (i < net.n_bus) mx = update_bus(f, w, sp, step, i, bad);
+    bad = __syncthreads_or(bad);
     const double m = block_max(mx, sh);
     if (threadIdx.x == 0) {
         w.part[blockIdx.x] = m;
         if (bad) atomicOr(&w.status->flags, FLAG_NONFINITE);
     }
-}
-
-// A step with a non-finite entry (FLAG_NONFINITE from k_update) is never
-// converged and reports a NaN max |dx|: the reference's max reduction turns
-// NaN once a NaN step fills its blocks (kernels.cu:557-574,752-782), so
-// "max |dx| < tol" fails and checkValidityKernel's flag decides: DIVERGED
-// (wls_solver.cu:493-517, 343-352).
-__global__ void k_update_finalize(DevWork w, int nblk, double tol) {
-    __shared__ double sh[32];
-    double m = 0.0;
-    for (int b = threadIdx.x; b < nblk; b += blockDim.x) m = fmax(m, w.part[b]);
-    m = block_max(m, sh);
+    if (!last_block(&w.status->blocks_done)) return;
+    mx = 0.0;
+    for (int b = threadIdx.x; b < gridDim.x; b += blockDim.x) mx = fmax(mx, __ldcg(w.part + b));
+    mx = block_max(mx, sh);
     if (threadIdx.x == 0) {
-        const bool bad = (w.status->flags & FLAG_NONFINITE) != 0;
-        w.status->max_mismatch = bad ? __longlong_as_double(0x7ff8000000000000LL) : m;
-        if (!bad && m < tol) atomicOr(&w.status->flags, FLAG_CONVERGED);
+        uint32_t fl = atomicOr(&w.status->flags, 0u);
+        const bool nonfinite = (fl & FLAG_NONFINITE) != 0;
+        if (!nonfinite && mx < sp.tol) fl |= FLAG_CONVERGED;
+        w.status->flags = fl;
+        w.status->max_mismatch = nonfinite ? __longlong_as_double(0x7ff8000000000000LL) : mx;
+        if (host) *host = *w.status;
     }
 }
 
@@ -978,65 +983,72 @@ __global__ void k_batch_retire(DevBatch b) {
 // factorisation flagged a non-positive pivot stops as singular without
 // applying the step; otherwise it stops when max |dx| < tol (converged) or
 // dx is not finite (diverged).
-__global__ void __launch_bounds__(kBlock) k_batch_update_part(DevFactor f, DevWork w, DevBatch b, SolveParams sp,
-                                                              const double* step) {
+//
+// The last CTA does the second part, and inside a device-run loop it also
+// takes the decision of the host loop of Engine::batch_solve for the graph's
+// while node (in_loop): the step's flags and the running count are final then.
+template <typename V>
+__global__ void __launch_bounds__(kBlock) k_batch_update(DevFactor f, DevWork w, DevBatch b, SolveParams sp,
+                                                         const V* step, cudaGraphConditionalHandle h, int in_loop,
+                                                         DevStatus* host, int32_t* host_running) {
     __shared__ double sh[32];
-    const int2 it = b.bus_items[blockIdx.x];
-    const int g = it.x;
-    const uint32_t fl = b.flags[g];
-    if (fl & (FLAG_FROZEN | FLAG_SINGULAR)) return;  // the whole CTA
-    const int end = min(it.y + kBatchChunk, b.bus_off[g + 1]);
-    double mx = 0.0;
-    int bad = 0;
-    for (int i = it.y + threadIdx.x; i < end; i += blockDim.x) {
-        const int pt = f.bus_ps_theta[i];
-        const double dv = step[f.bus_ps_v[i]];
-        double dt = 0.0;
-        if (pt >= 0) {
-            dt = step[pt];
-            w.th[i] += dt;
+    if (blockIdx.x < b.n_bus_items) {
+        const int2 it = b.bus_items[blockIdx.x];
+        if (!(b.flags[it.x] & (FLAG_FROZEN | FLAG_SINGULAR))) {  // the whole CTA
+            const int end = min(it.y + kBatchChunk, b.bus_off[it.x + 1]);
+            double mx = 0.0;
+            int bad = 0;
+            for (int i = it.y + threadIdx.x; i < end; i += blockDim.x)
+                mx = fmax(mx, update_bus(f, w, sp, step, i, bad));
+            bad = __syncthreads_or(bad);
+            const double m = block_max(mx, sh);
+            if (threadIdx.x == 0) {
+                b.part[blockIdx.x] = m;
+                b.part_bad[blockIdx.x] = bad;
+            }
         }
-        double vn = w.v[i] + dv;
-        vn = fmax(vn, sp.vmin);
-        vn = fmin(vn, sp.vmax);
-        w.v[i] = vn;
-        if (!isfinite(dt) || !isfinite(dv)) bad = 1;
-        double m = fmax(fabs(dt), fabs(dv));
-        if (m != m) m = 0.0;
-        mx = fmax(mx, m);
     }
-    bad = __syncthreads_or(bad);
-    const double m = block_max(mx, sh);
+    if (!last_block(&w.status->blocks_done)) return;
+    int running = 0;
+    for (int g0 = 0; g0 < b.n_grids; g0 += blockDim.x) {
+        const int g = g0 + threadIdx.x;
+        bool runs = false;
+        const uint32_t fl = g < b.n_grids ? b.flags[g] : FLAG_FROZEN;
+        if (!(fl & FLAG_FROZEN)) {
+            b.iters[g] += 1;
+            if (fl & FLAG_SINGULAR) {
+                b.flags[g] = fl | FLAG_FROZEN;
+            } else {
+                double m = 0.0;
+                int bad = 0;
+                for (int k = b.bus_item_ptr[g]; k < b.bus_item_ptr[g + 1]; ++k) {
+                    m = fmax(m, __ldcg(b.part + k));
+                    bad |= __ldcg(b.part_bad + k);
+                }
+                b.mismatch[g] = bad ? __longlong_as_double(0x7ff8000000000000LL) : m;
+                if (bad)
+                    b.flags[g] = fl | FLAG_NONFINITE | FLAG_FROZEN;
+                else if (m < sp.tol)
+                    b.flags[g] = fl | FLAG_CONVERGED | FLAG_FROZEN;
+                else
+                    runs = true;
+            }
+        }
+        running += __syncthreads_count(runs);
+    }
     if (threadIdx.x == 0) {
-        b.part[blockIdx.x] = m;
-        b.part_bad[blockIdx.x] = bad;
-    }
-}
-
-__global__ void k_batch_update_fin(DevBatch b, double tol) {
-    const int g = blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= b.n_grids) return;
-    const uint32_t fl = b.flags[g];
-    if (fl & FLAG_FROZEN) return;
-    if (fl & FLAG_SINGULAR) {
-        b.flags[g] = fl | FLAG_FROZEN;
-        b.iters[g] += 1;
-        return;
-    }
-    double m = 0.0;
-    int bad = 0;
-    for (int k = b.bus_item_ptr[g]; k < b.bus_item_ptr[g + 1]; ++k) {
-        m = fmax(m, b.part[k]);
-        bad |= b.part_bad[k];
-    }
-    b.mismatch[g] = bad ? __longlong_as_double(0x7ff8000000000000LL) : m;
-    b.iters[g] += 1;
-    if (bad) {
-        b.flags[g] = fl | FLAG_NONFINITE | FLAG_FROZEN;
-    } else if (m < tol) {
-        b.flags[g] = fl | FLAG_CONVERGED | FLAG_FROZEN;
-    } else {
-        atomicAdd(b.running, 1);
+        *b.running = running;
+        if (host) {
+            *host = *w.status;
+            *host_running = running;
+        }
+        if (in_loop) {
+            const int32_t steps = b.loop[0] + 1;
+            b.loop[0] = steps;
+            const bool timed_out = (w.status->flags & FLAG_TIMEOUT) != 0u;
+            if (timed_out) b.loop[2] = 1;
+            cudaGraphSetConditional(h, (!timed_out && running > 0 && steps < b.loop[1]) ? 1u : 0u);
+        }
     }
 }
 
@@ -1076,16 +1088,6 @@ __global__ void k_gn_loop_init(DevBatch b, int32_t limit) {
     b.loop[2] = 0;
 }
 
-// One thread, after the step's last kernel: the step's flags and the running
-// count are final.  Same decision as the host loop of Engine::batch_solve.
-__global__ void k_gn_loop_next(cudaGraphConditionalHandle h, DevBatch b, const DevStatus* st) {
-    const int32_t steps = b.loop[0] + 1;
-    b.loop[0] = steps;
-    const bool timed_out = (st->flags & FLAG_TIMEOUT) != 0u;
-    if (timed_out) b.loop[2] = 1;
-    cudaGraphSetConditional(h, (!timed_out && *b.running > 0 && steps < b.loop[1]) ? 1u : 0u);
-}
-
 inline int nblocks(int n) { return (n + kBlock - 1) / kBlock; }
 
 }  // namespace
@@ -1097,17 +1099,23 @@ cudaError_t launch_batch_begin(const DevNet& net, const DevWork& w, const DevBat
     return cudaGetLastError();
 }
 
+template <typename V>
 cudaError_t launch_batch_update(const DevNet& net, const DevFactor& f, const DevWork& w, const DevBatch& b,
-                                const SolveParams& sp, const double* step, cudaStream_t st) {
+                                const SolveParams& sp, const V* step, const cudaGraphConditionalHandle* loop,
+                                DevStatus* host, int32_t* host_running, cudaStream_t st) {
     if (b.n_grids <= 0) return cudaSuccess;
-    if (b.n_bus_items > 0) {
-        k_batch_update_part<<<b.n_bus_items, kBlock, 0, st>>>(f, w, b, sp, step);
-        count_launches(1);
-    }
-    k_batch_update_fin<<<nblocks(b.n_grids), kBlock, 0, st>>>(b, sp.tol);
+    k_batch_update<<<std::max(b.n_bus_items, 1), kBlock, 0, st>>>(f, w, b, sp, step,
+                                                                  loop ? *loop : cudaGraphConditionalHandle{},
+                                                                  loop ? 1 : 0, host, host_running);
     count_launches(1);
     return cudaGetLastError();
 }
+template cudaError_t launch_batch_update(const DevNet&, const DevFactor&, const DevWork&, const DevBatch&,
+                                         const SolveParams&, const float*, const cudaGraphConditionalHandle*,
+                                         DevStatus*, int32_t*, cudaStream_t);
+template cudaError_t launch_batch_update(const DevNet&, const DevFactor&, const DevWork&, const DevBatch&,
+                                         const SolveParams&, const double*, const cudaGraphConditionalHandle*,
+                                         DevStatus*, int32_t*, cudaStream_t);
 
 cudaError_t launch_islands(const DevNet& net, int32_t* parent, int32_t* out, int32_t max_rounds, cudaStream_t st) {
     const int nb = nblocks(std::max(net.n_bus, 1));
@@ -1155,12 +1163,6 @@ cudaError_t launch_batch_retire(const DevBatch& b, cudaStream_t st) {
 
 cudaError_t launch_gn_loop_init(const DevBatch& b, int32_t limit, cudaStream_t st) {
     k_gn_loop_init<<<1, 1, 0, st>>>(b, limit);
-    count_launches(1);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_gn_loop_next(cudaGraphConditionalHandle h, const DevBatch& b, const DevWork& w, cudaStream_t st) {
-    k_gn_loop_next<<<1, 1, 0, st>>>(h, b, w.status);
     count_launches(1);
     return cudaGetLastError();
 }
@@ -1224,26 +1226,17 @@ cudaError_t launch_objective(const DevNet& net, const DevWork& w, double bad_thr
     return cudaGetLastError();
 }
 
-cudaError_t launch_rhs(const DevNet& net, const DevFactor& f, const DevWork& w, cudaStream_t st) {
-    k_rhs<<<nblocks(f.n_state), kBlock, 0, st>>>(net, f, w);
-    count_launches(1);
-    return cudaGetLastError();
-}
-
+template <typename V>
 cudaError_t launch_update(const DevNet& net, const DevFactor& f, const DevWork& w, const SolveParams& sp,
-                          const double* step, cudaStream_t st) {
-    const int nb = nblocks(net.n_bus);
-    k_update<<<nb, kBlock, 0, st>>>(net, f, w, sp, step);
-    k_update_finalize<<<1, 1024, 0, st>>>(w, nb, sp.tol);
-    count_launches(2);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_to_fp32(const DevFactor& f, const DevWork& w, cudaStream_t st) {
-    k_to_fp32<<<nblocks(f.n_state), kBlock, 0, st>>>(f, w);
+                          const V* step, DevStatus* host, cudaStream_t st) {
+    k_update<<<nblocks(net.n_bus), kBlock, 0, st>>>(net, f, w, sp, step, host);
     count_launches(1);
     return cudaGetLastError();
 }
+template cudaError_t launch_update(const DevNet&, const DevFactor&, const DevWork&, const SolveParams&, const float*,
+                                   DevStatus*, cudaStream_t);
+template cudaError_t launch_update(const DevNet&, const DevFactor&, const DevWork&, const SolveParams&, const double*,
+                                   DevStatus*, cudaStream_t);
 
 cudaError_t launch_refine_begin(const DevFactor& f, const DevWork& w, cudaStream_t st) {
     k_refine_begin<<<nblocks(f.n_state), kBlock, 0, st>>>(f, w);
