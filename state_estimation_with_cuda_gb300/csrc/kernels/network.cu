@@ -2,6 +2,7 @@
 // measurement evaluation (h(x), residual, weights, Jacobian values), the
 // gain right-hand side, state update / convergence and the result pass.
 #include "kernels.cuh"
+#include "round32.h"
 
 #include <cfloat>
 
@@ -95,64 +96,78 @@ __global__ void k_ybus(DevNet net) {
     net.y_b[e0] = db;
 }
 
+// A flow row's value and derivatives by the row's own end (o) and the other (x).
 struct FlowTerms {
     double val;
-    double d[4];  // theta_i, V_i, theta_j, V_j
+    double dto, dvo, dvx;  // theta_o (theta_x has the opposite sign), V_o, V_x
 };
 
-// a4 + a8 flow rows: value of P/Q at one end and its derivatives, given
-// s, c = sin, cos of theta_i - theta_j - shift.
-__device__ FlowTerms flow_terms_sc(const DevNet& net, const double* v, int k, bool is_q, bool to_end, bool exact,
-                                   double s, double c) {
-    const int i = net.br_from[k], j = net.br_to[k];
-    const double Vi = v[i], Vj = v[j];
-    const double g = net.br_g[k], b = net.br_b[k];
-    // 1 / a and 1 / a^2 of the tap a (clamped as the reference clamps it),
-    // computed once per branch: the rows multiply instead of dividing
-    const double inv = net.br_itap[k], ia2 = net.br_itap2[k];
-    const double on = net.br_closed[k] ? 1.0 : 0.0;
-    const double vv = Vi * Vj * inv;
-    FlowTerms f;
-    if (!is_q && !to_end) {
-        f.val = Vi * Vi * ia2 * g - vv * (g * c + b * s);
-        f.d[0] = vv * (g * s - b * c);
-        f.d[1] = 2.0 * Vi * ia2 * g - Vj * inv * (g * c + b * s);
-        f.d[2] = -f.d[0];
-        f.d[3] = -Vi * inv * (g * c + b * s);
-    } else if (is_q && !to_end) {
-        const double bsf = net.br_bsf[k];
-        f.val = -(Vi * Vi * ia2) * (b + bsf) - vv * (g * s - b * c);
-        f.d[0] = -vv * (g * c + b * s);
-        f.d[1] = (exact ? -2.0 * Vi * (b + bsf) * ia2 : -2.0 * Vi * b * ia2) - Vj * inv * (g * s - b * c);
-        f.d[2] = -f.d[0];
-        f.d[3] = -Vi * inv * (g * s - b * c);
-    } else if (!is_q && to_end) {
-        f.val = Vj * Vj * g - vv * (g * c - b * s);
-        // exact: dP_t/dtheta_i = (ViVj/a)(g s + b c); the reference flips the sign.
-        f.d[0] = exact ? vv * (g * s + b * c) : vv * (-g * s - b * c);
-        f.d[1] = -Vj * inv * (g * c - b * s);
-        f.d[2] = -f.d[0];
-        f.d[3] = 2.0 * Vj * g - Vi * inv * (g * c - b * s);
-    } else {
-        const double bst = net.br_bst[k];
-        f.val = -Vj * Vj * (b + bst) + vv * (g * s + b * c);
-        f.d[0] = vv * (g * c - b * s);
-        f.d[1] = Vj * inv * (g * s + b * c);
-        f.d[2] = -f.d[0];
-        f.d[3] = (exact ? -2.0 * Vj * (b + bst) : -2.0 * Vj * b) + Vi * inv * (g * s + b * c);
-    }
-    f.val *= on;
-    if (exact) {
-        for (int x = 0; x < 4; ++x) f.d[x] *= on;
-    }
-    return f;
+// What the P and Q flow at one end of branch k share (a4 + a8 flow rows).
+// With s the sine of the angle from that end, both rows are
+//   h = V_o (V_o q + V_x inv A),  dh/dtheta_o = -V_o V_x inv B  (signs below)
+// with (A, B) = (g c + b s, g s - b c) for P and (g s - b c, -(g c + b s)) for
+// Q, q the end's own admittance (over the tap squared at the from end).
+//
+// An FP64 instruction holds its pipe for 64 cycles a warp whatever lanes it
+// has, and the evaluation is bound by that pipe.  The form shares factors
+// between value and derivatives, and one sequence serves the four kinds of
+// flow row (bit selects instead of branches; as four branches of the printed
+// formulas a warp of mixed rows ran about 90 FP64 instructions, now about 22).
+// Injections are written the same way (InjSums), and the H entries are rounded
+// to FP32 on the integer pipe (round32.h).  The evaluation of 512 grids (pairs)
+// went from 311 to 229 us, of 200k buses from 153 to 120, of 20k (rows) from 39
+// to 31; against extended precision the rows' values lose a fifth of their error.
+struct FlowEnd {
+    double Vo, Vx, x1, x2;  // x1 = inv (g c + b s), x2 = inv (g s - b c)
+    double w;               // 1 / a^2 at the from end, 1 at the to end
+};
+
+__device__ __forceinline__ double flip(double v, bool neg) {  // the sign bit, off the FP64 pipe
+    return __hiloint2double(__double2hiint(v) ^ (neg ? static_cast<int>(0x80000000) : 0), __double2loint(v));
+}
+// v == 0, off the FP64 pipe
+__device__ __forceinline__ bool is_zero(double v) { return ((__double2hiint(v) & 0x7fffffff) | __double2loint(v)) == 0; }
+
+// s, c: sin, cos of theta_i - theta_j - shift.  1 / a and 1 / a^2 of the tap a
+// (clamped as the reference clamps it) are computed once per branch.
+__device__ __forceinline__ FlowEnd flow_end(const DevNet& net, const double* v, int k, bool to_end, double s, double c) {
+    const double Vi = v[net.br_from[k]], Vj = v[net.br_to[k]];
+    const double g = net.br_g[k], b = net.br_b[k], inv = net.br_itap[k], ia2 = net.br_itap2[k];
+    s = flip(s, to_end);
+    FlowEnd E;
+    E.Vo = to_end ? Vj : Vi;
+    E.Vx = to_end ? Vi : Vj;
+    E.x1 = inv * (g * c + b * s);
+    E.x2 = inv * (g * s - b * c);
+    E.w = to_end ? 1.0 : ia2;
+    return E;
 }
 
-__device__ FlowTerms flow_terms(const DevNet& net, const double* v, const double* th, int k, bool is_q,
-                                bool to_end, bool exact) {
-    double s, c;
-    sincos(th[net.br_from[k]] - th[net.br_to[k]] - net.br_shift[k], &s, &c);
-    return flow_terms_sc(net, v, k, is_q, to_end, exact, s, c);
+__device__ __forceinline__ FlowTerms flow_row(const DevNet& net, const FlowEnd& E, int k, bool is_q, bool to_end,
+                                              bool exact) {
+    const double g = net.br_g[k], b = net.br_b[k];
+    const double q0 = is_q ? -(b + (to_end ? net.br_bst[k] : net.br_bsf[k])) : g;
+    const double A = is_q ? E.x2 : E.x1, B = is_q ? flip(E.x1, true) : E.x2;
+    const double q = E.w * q0, u = E.Vx * A;
+    const double r = fma(E.Vo, q, -u);
+    FlowTerms f;
+    f.val = E.Vo * r;
+    f.dvo = fma(E.Vo, q, r);
+    // the reference leaves the charging out of dQ/dV
+    if (is_q && !exact) f.dvo = fma(-2.0 * E.Vo, E.w * b, -u);
+    f.dvx = flip(E.Vo * A, true);
+    f.dto = E.Vo * (E.Vx * B);
+    // the reference flips the sign of dP/dtheta at the to end
+    if (!exact && to_end && !is_q) f.dto = flip(f.dto, true);
+    if (!net.br_closed[k]) {
+        f.val *= 0.0;
+        if (exact) {
+            f.dto *= 0.0;
+            f.dvo *= 0.0;
+            f.dvx *= 0.0;
+        }
+    }
+    return f;
 }
 
 // sin and cos of theta_i - theta_j from the buses' (cos, sin): four FMAs in
@@ -167,20 +182,13 @@ __device__ __forceinline__ void angle_diff(const double2 a, const double2 b, dou
 __device__ __forceinline__ void branch_angle(const DevNet& net, const double2* cs, int k, double* s, double* c) {
     angle_diff(cs[net.br_from[k]], cs[net.br_to[k]], s, c);
     const double phi = net.br_shift[k];
-    if (phi != 0.0) {
+    if (!is_zero(phi)) {
         double sp, cp;
         sincos(phi, &sp, &cp);
         const double c2 = *c * cp + *s * sp;
         *s = *s * cp - *c * sp;
         *c = c2;
     }
-}
-
-__device__ __forceinline__ FlowTerms flow_terms_cs(const DevNet& net, const double* v, const double2* cs, int k,
-                                                   bool is_q, bool to_end, bool exact) {
-    double s, c;
-    branch_angle(net, cs, k, &s, &c);
-    return flow_terms_sc(net, v, k, is_q, to_end, exact, s, c);
 }
 
 // cos and sin of every bus angle of the grids being evaluated.
@@ -196,57 +204,69 @@ __global__ void k_bus_trig(DevNet net, DevWork w, SolveParams sp) {
     w.bus_cs[i] = make_double2(c, s);
 }
 
-__device__ __forceinline__ void put_flow(double* hrow, int fpos, const double d[4]) {
+// Adds a flow row's derivatives to its (zeroed) H row; fpos: positions of
+// theta_i, V_i, theta_j, V_j, i the from bus (0xFF: none).  The four are
+// distinct columns, so they are stored, unless the branch ends where it starts.
+__device__ __forceinline__ void put_flow(double* hrow, int fpos, bool to_end, const FlowTerms& f) {
+    const double dtx = flip(f.dto, true);
+    const double d[4] = {to_end ? dtx : f.dto, to_end ? f.dvx : f.dvo, to_end ? f.dto : dtx, to_end ? f.dvo : f.dvx};
+    const bool loop = ((fpos >> 8) & 0xFF) == ((fpos >> 24) & 0xFF);
+#pragma unroll
     for (int x = 0; x < 4; ++x) {
         const int p = (fpos >> (8 * x)) & 0xFF;
-        if (p != 0xFF) hrow[p] += d[x];
+        if (p == 0xFF) continue;
+        if (loop)
+            hrow[p] += d[x];
+        else
+            hrow[p] = d[x];
     }
 }
 
-// a3/a6/a7/a8/a9 fused: one thread per measurement row.
-// P and Q flow at one end of branch k from the same angle difference: the
-// two rows' values and derivatives with the expressions of flow_terms_sc.
-__device__ __forceinline__ void flow_terms_pq(const DevNet& net, const double* v, int k, bool to_end, bool exact,
-                                              double s, double c, FlowTerms& P, FlowTerms& Q) {
-    const int i = net.br_from[k], j = net.br_to[k];
-    const double Vi = v[i], Vj = v[j];
-    const double g = net.br_g[k], b = net.br_b[k];
-    const double inv = net.br_itap[k], ia2 = net.br_itap2[k];
+// Current magnitude |S| / V at one end of branch k.
+__device__ __forceinline__ FlowTerms current_row(const DevNet& net, const DevWork& w, int k, bool to_end, bool exact) {
+    double s, c;
+    branch_angle(net, w.bus_cs, k, &s, &c);
+    const FlowEnd E = flow_end(net, w.v, k, to_end, s, c);
+    const FlowTerms P = flow_row(net, E, k, false, to_end, exact), Q = flow_row(net, E, k, true, to_end, exact);
     const double on = net.br_closed[k] ? 1.0 : 0.0;
-    const double vv = Vi * Vj * inv;
-    if (!to_end) {
-        P.val = Vi * Vi * ia2 * g - vv * (g * c + b * s);
-        P.d[0] = vv * (g * s - b * c);
-        P.d[1] = 2.0 * Vi * ia2 * g - Vj * inv * (g * c + b * s);
-        P.d[2] = -P.d[0];
-        P.d[3] = -Vi * inv * (g * c + b * s);
-        const double bsf = net.br_bsf[k];
-        Q.val = -(Vi * Vi * ia2) * (b + bsf) - vv * (g * s - b * c);
-        Q.d[0] = -vv * (g * c + b * s);
-        Q.d[1] = (exact ? -2.0 * Vi * (b + bsf) * ia2 : -2.0 * Vi * b * ia2) - Vj * inv * (g * s - b * c);
-        Q.d[2] = -Q.d[0];
-        Q.d[3] = -Vi * inv * (g * s - b * c);
+    const double vs = fmax(E.Vo, kEps);
+    const double S = sqrt(P.val * P.val + Q.val * Q.val);
+    FlowTerms f;
+    f.val = S / vs * on;
+    if (!exact) {  // the reference reuses the P-flow derivatives
+        f.dto = P.dto;
+        f.dvo = P.dvo;
+        f.dvx = P.dvx;
     } else {
-        P.val = Vj * Vj * g - vv * (g * c - b * s);
-        P.d[0] = exact ? vv * (g * s + b * c) : vv * (-g * s - b * c);
-        P.d[1] = -Vj * inv * (g * c - b * s);
-        P.d[2] = -P.d[0];
-        P.d[3] = 2.0 * Vj * g - Vi * inv * (g * c - b * s);
-        const double bst = net.br_bst[k];
-        Q.val = -Vj * Vj * (b + bst) + vv * (g * s + b * c);
-        Q.d[0] = vv * (g * c - b * s);
-        Q.d[1] = Vj * inv * (g * s + b * c);
-        Q.d[2] = -Q.d[0];
-        Q.d[3] = (exact ? -2.0 * Vj * (b + bst) : -2.0 * Vj * b) + Vi * inv * (g * s + b * c);
+        auto d = [&](double p, double q) { return (S > 0.0) ? (P.val * p + Q.val * q) / (S * vs) * on : 0.0; };
+        f.dto = d(P.dto, Q.dto);
+        f.dvo = d(P.dvo, Q.dvo);
+        f.dvx = d(P.dvx, Q.dvx);
+        if (E.Vo > kEps) f.dvo -= S / (vs * vs) * on;
     }
-    P.val *= on;
-    Q.val *= on;
-    if (exact) {
-        for (int x = 0; x < 4; ++x) {
-            P.d[x] *= on;
-            Q.d[x] *= on;
-        }
-    }
+    return f;
+}
+
+// Row sums of an injection at bus i over its neighbours: a = sum V_j A_j,
+// b = sum V_j B_j with (A, B) as for a flow (G, B the Ybus entry), c, d the
+// diagonal's (G, B) for P and (-B, G) for Q.  Then h = V_i (V_i c + a),
+// dh/dV_i = 2 V_i c + a, dh/dtheta_i = -V_i b (the reference adds V_i^2 d).
+struct InjSums {
+    double a, b, c, d;
+};
+__device__ __forceinline__ double inj_value(const InjSums& S, double Vi, bool exact, double* dv, double* dt) {
+    const double r = fma(Vi, S.c, S.a);
+    *dv = fma(Vi, S.c, r);
+    *dt = flip(Vi * S.b, true);
+    if (!exact) *dt += Vi * Vi * S.d;
+    return Vi * r;
+}
+
+// float(v) off the FP64 pipe where the result is a normal number.
+__device__ __forceinline__ float to_f32(double v) {
+    const uint32_t hi = static_cast<uint32_t>(__double2hiint(v)), lo = static_cast<uint32_t>(__double2loint(v));
+    if (round32_takes(hi)) return __uint_as_float(round32_bits(hi, lo));
+    return static_cast<float>(v);
 }
 
 // H entries of a warp's rows (a contiguous range of the CSR values) staged
@@ -356,96 +376,73 @@ __global__ void __launch_bounds__(kBlock) k_evaluate_pairs(DevNet net, DevWork w
             double* hq = qq >= 0 ? row_of(qq) : nullptr;
             const double Vi = w.v[loc];
             const double2 cs_i = w.bus_cs[loc];
-            double hvp = 0.0, dVip = 0.0, dTip = 0.0, hvq = 0.0, dViq = 0.0, dTiq = 0.0;
+            InjSums P{}, Q{};
             const int e0 = net.y_ptr[loc], e1 = net.y_ptr[loc + 1];
             for (int e = e0; e < e1; ++e) {
-                const int j = net.y_col[e];
-                const double G = net.y_g[e], B = net.y_b[e];
+                const int j = __ldg(net.y_col + e);
+                const double G = __ldg(net.y_g + e), B = __ldg(net.y_b + e);
                 if (j == loc) {
-                    hvp += Vi * Vi * G;
-                    dVip += 2.0 * Vi * G;
-                    if (!exact) dTip += Vi * Vi * B;
-                    hvq -= Vi * Vi * B;
-                    dViq -= 2.0 * Vi * B;
-                    if (!exact) dTiq += Vi * Vi * G;
-                } else {
-                    const double Vj = w.v[j];
-                    double sn, cn;
-                    angle_diff(cs_i, w.bus_cs[j], &sn, &cn);
-                    const double gcbs = G * cn + B * sn, gsbc = G * sn - B * cn;
-                    const int pt = net.y_hpos_t[e], pv = net.y_hpos_v[e];
-                    if (hp) {
-                        hvp += Vi * Vj * gcbs;
-                        dVip += Vj * gcbs;
-                        dTip -= Vi * Vj * gsbc;
-                        if (pt >= 0) hp[pt] += Vi * Vj * gsbc;
-                        hp[pv] += Vi * gcbs;
-                    }
-                    if (hq) {
-                        hvq += Vi * Vj * gsbc;
-                        dViq += Vj * gsbc;
-                        dTiq += Vi * Vj * gcbs;
-                        if (pt >= 0) hq[pt] += -Vi * Vj * gcbs;
-                        hq[pv] += Vi * gsbc;
-                    }
+                    P.c += G;
+                    P.d += B;
+                    continue;
+                }
+                const double Vj = __ldg(w.v + j);
+                const int pt = __ldg(net.y_hpos_t + e), pv = __ldg(net.y_hpos_v + e);
+                double sn, cn;
+                angle_diff(cs_i, __ldg(w.bus_cs + j), &sn, &cn);
+                const double gc = G * cn + B * sn, gs = G * sn - B * cn;
+                const double vg = Vj * gc, vs = Vj * gs;
+                P.a += vg;
+                P.b += vs;
+                if (hp) {
+                    if (pt >= 0) hp[pt] += Vi * vs;
+                    hp[pv] += Vi * gc;
+                }
+                if (hq) {
+                    if (pt >= 0) hq[pt] -= Vi * vg;
+                    hq[pv] += Vi * gs;
                 }
             }
+            Q.a = P.b;
+            Q.b = flip(P.a, true);
+            Q.c = flip(P.d, true);
+            Q.d = P.c;
             const int pt = net.y_hpos_t[e0], pv = net.y_hpos_v[e0];
+            double dv, dt;
             if (hp) {
-                if (pt >= 0) hp[pt] += dTip;
-                hp[pv] += dVip;
-                finish(qp, kind, hvp, hp);
+                const double hv = inj_value(P, Vi, exact, &dv, &dt);
+                if (pt >= 0) hp[pt] += dt;
+                hp[pv] += dv;
+                finish(qp, kind, hv, hp);
             }
             if (hq) {
-                if (pt >= 0) hq[pt] += dTiq;
-                hq[pv] += dViq;
-                finish(qq, kind, hvq, hq);
+                const double hv = inj_value(Q, Vi, exact, &dv, &dt);
+                if (pt >= 0) hq[pt] += dt;
+                hq[pv] += dv;
+                finish(qq, kind, hv, hq);
             }
         } else if (kind == 3) {  // P/Q flow; with its twin at the same end when qb >= 0
             const bool to_end = net.m_end[qa] != 0;
-            if (qb < 0) {
-                double* hrow = row_of(qa);
-                const FlowTerms f = flow_terms_cs(net, w.v, w.bus_cs, loc, ty == 5, to_end, exact);
-                put_flow(hrow, net.m_fpos[qa], f.d);
-                finish(qa, kind, f.val, hrow);
-            } else {
-                const bool a_is_q = ty == 5;
-                const int qp = a_is_q ? qb : qa, qq = a_is_q ? qa : qb;
-                double sn, cn;
-                branch_angle(net, w.bus_cs, loc, &sn, &cn);
-                FlowTerms fp, fq;
-                flow_terms_pq(net, w.v, loc, to_end, exact, sn, cn, fp, fq);
-                double* hp = row_of(qp);
-                put_flow(hp, net.m_fpos[qp], fp.d);
-                finish(qp, kind, fp.val, hp);
-                double* hq = row_of(qq);
-                put_flow(hq, net.m_fpos[qq], fq.d);
-                finish(qq, kind, fq.val, hq);
+            const bool a_is_q = ty == 5;
+            double sn, cn;
+            branch_angle(net, w.bus_cs, loc, &sn, &cn);
+            const FlowEnd E = flow_end(net, w.v, loc, to_end, sn, cn);
+            double* ha = row_of(qa);
+            const FlowTerms fa = flow_row(net, E, loc, a_is_q, to_end, exact);
+            put_flow(ha, net.m_fpos[qa], to_end, fa);
+            finish(qa, kind, fa.val, ha);
+            if (qb >= 0) {
+                double* hb = row_of(qb);
+                const FlowTerms fb = flow_row(net, E, loc, !a_is_q, to_end, exact);
+                put_flow(hb, net.m_fpos[qb], to_end, fb);
+                finish(qb, kind, fb.val, hb);
             }
         } else if (kind == 4) {  // current magnitude
             double* hrow = row_of(qa);
             const bool to_end = net.m_end[qa] != 0;
-            const FlowTerms fp = flow_terms_cs(net, w.v, w.bus_cs, loc, false, to_end, exact);
-            const int ib = to_end ? net.br_to[loc] : net.br_from[loc];
-            const double ve = w.v[ib];
-            const double vs = fmax(ve, kEps);
-            const double on = net.br_closed[loc] ? 1.0 : 0.0;
-            double d[4];
-            double hv;
-            if (!exact) {  // the reference reuses the P-flow derivatives
-                const FlowTerms fq = flow_terms_cs(net, w.v, w.bus_cs, loc, true, to_end, exact);
-                hv = sqrt(fp.val * fp.val + fq.val * fq.val) / vs * on;
-                for (int x = 0; x < 4; ++x) d[x] = fp.d[x];
-            } else {
-                const FlowTerms fq = flow_terms_cs(net, w.v, w.bus_cs, loc, true, to_end, exact);
-                const double S = sqrt(fp.val * fp.val + fq.val * fq.val);
-                hv = S / vs * on;
-                for (int x = 0; x < 4; ++x)
-                    d[x] = (S > 0.0) ? (fp.val * fp.d[x] + fq.val * fq.d[x]) / (S * vs) * on : 0.0;
-                if (ve > kEps) d[to_end ? 3 : 1] -= S / (vs * vs) * on;
-            }
-            put_flow(hrow, net.m_fpos[qa], d);
-            finish(qa, kind, hv, hrow);
+            const FlowTerms f = current_row(net, w, loc, to_end, exact);
+            put_flow(hrow, net.m_fpos[qa], to_end, f);
+            finish(qa, kind, f.val, hrow);
         } else {
             double* hrow = row_of(qa);
             finish(qa, kind, 0.0, hrow);
@@ -459,8 +456,8 @@ __global__ void __launch_bounds__(kBlock) k_evaluate_pairs(DevNet net, DevWork w
             const double v = hs[warp][x];
             w.hval[hw0 + x] = v;
             if (sp.mixed) {
-                w.hval32[hw0 + x] = static_cast<float>(v);
-                if (w.hw32) w.hw32[hw0 + x] = static_cast<float>(wes[warp][r] * v);
+                w.hval32[hw0 + x] = to_f32(v);
+                if (w.hw32) w.hw32[hw0 + x] = to_f32(wes[warp][r] * v);
             } else if (w.hw) {
                 w.hw[hw0 + x] = wes[warp][r] * v;
             }
@@ -531,75 +528,44 @@ __global__ void __launch_bounds__(kBlock) k_evaluate_rows(DevNet net, DevWork w,
             const bool isq = (ty == 3 || ty == 8);
             const double Vi = w.v[loc];
             const double2 cs_i = w.bus_cs[loc];
-            double dVi = 0.0, dTi = 0.0;
+            InjSums S{};
             const int e0 = net.y_ptr[loc], e1 = net.y_ptr[loc + 1];
             for (int e = e0; e < e1; ++e) {
-                const int j = net.y_col[e];
-                const double G = net.y_g[e], B = net.y_b[e];
+                const int j = __ldg(net.y_col + e);
+                const double G = __ldg(net.y_g + e), B = __ldg(net.y_b + e);
                 if (j == loc) {
-                    if (!isq) {
-                        hv += Vi * Vi * G;
-                        dVi += 2.0 * Vi * G;
-                        if (!exact) dTi += Vi * Vi * B;
-                    } else {
-                        hv -= Vi * Vi * B;
-                        dVi -= 2.0 * Vi * B;
-                        if (!exact) dTi += Vi * Vi * G;
-                    }
-                } else {
-                    const double Vj = w.v[j];
-                    double s, c;
-                    angle_diff(cs_i, w.bus_cs[j], &s, &c);
-                    const double gcbs = G * c + B * s, gsbc = G * s - B * c;
-                    double dTj, dVj;
-                    if (!isq) {
-                        hv += Vi * Vj * gcbs;
-                        dVi += Vj * gcbs;
-                        dTi -= Vi * Vj * gsbc;
-                        dTj = Vi * Vj * gsbc;
-                        dVj = Vi * gcbs;
-                    } else {
-                        hv += Vi * Vj * gsbc;
-                        dVi += Vj * gsbc;
-                        dTi += Vi * Vj * gcbs;
-                        dTj = -Vi * Vj * gcbs;
-                        dVj = Vi * gsbc;
-                    }
-                    const int pt = net.y_hpos_t[e];
-                    if (pt >= 0) hrow[pt] += dTj;
-                    hrow[net.y_hpos_v[e]] += dVj;
+                    S.c += isq ? flip(B, true) : G;
+                    S.d += isq ? G : B;
+                    continue;
                 }
+                const double Vj = __ldg(w.v + j);
+                const int pt = __ldg(net.y_hpos_t + e), pv = __ldg(net.y_hpos_v + e);
+                double sn, cn;
+                angle_diff(cs_i, __ldg(w.bus_cs + j), &sn, &cn);
+                const double gc = G * cn + B * sn, gs = G * sn - B * cn;
+                const double A = isq ? gs : gc, vb = Vj * (isq ? flip(gc, true) : gs);
+                S.a += Vj * A;
+                S.b += vb;
+                if (pt >= 0) hrow[pt] += Vi * vb;
+                hrow[pv] += Vi * A;
             }
+            double dv, dt;
+            hv = inj_value(S, Vi, exact, &dv, &dt);
             const int pt = net.y_hpos_t[e0];
-            if (pt >= 0) hrow[pt] += dTi;
-            hrow[net.y_hpos_v[e0]] += dVi;
+            if (pt >= 0) hrow[pt] += dt;
+            hrow[net.y_hpos_v[e0]] += dv;
         } else if (kind == 3) {  // P/Q flow
             const bool to_end = net.m_end[q] != 0;
-            const FlowTerms f = flow_terms_cs(net, w.v, w.bus_cs, loc, ty == 5, to_end, exact);
+            double sn, cn;
+            branch_angle(net, w.bus_cs, loc, &sn, &cn);
+            const FlowTerms f = flow_row(net, flow_end(net, w.v, loc, to_end, sn, cn), loc, ty == 5, to_end, exact);
             hv = f.val;
-            put_flow(hrow, net.m_fpos[q], f.d);
+            put_flow(hrow, net.m_fpos[q], to_end, f);
         } else if (kind == 4) {  // current magnitude
             const bool to_end = net.m_end[q] != 0;
-            const FlowTerms fp = flow_terms_cs(net, w.v, w.bus_cs, loc, false, to_end, exact);
-            const int ib = to_end ? net.br_to[loc] : net.br_from[loc];
-            const double ve = w.v[ib];
-            const double vs = fmax(ve, kEps);
-            const double on = net.br_closed[loc] ? 1.0 : 0.0;
-            double d[4];
-            if (!exact) {  // the reference reuses the P-flow derivatives
-                hv = 0.0;
-                const FlowTerms fq = flow_terms_cs(net, w.v, w.bus_cs, loc, true, to_end, exact);
-                hv = sqrt(fp.val * fp.val + fq.val * fq.val) / vs * on;
-                for (int x = 0; x < 4; ++x) d[x] = fp.d[x];
-            } else {
-                const FlowTerms fq = flow_terms_cs(net, w.v, w.bus_cs, loc, true, to_end, exact);
-                const double S = sqrt(fp.val * fp.val + fq.val * fq.val);
-                hv = S / vs * on;
-                for (int x = 0; x < 4; ++x)
-                    d[x] = (S > 0.0) ? (fp.val * fp.d[x] + fq.val * fq.d[x]) / (S * vs) * on : 0.0;
-                if (ve > kEps) d[to_end ? 3 : 1] -= S / (vs * vs) * on;
-            }
-            put_flow(hrow, net.m_fpos[q], d);
+            const FlowTerms f = current_row(net, w, loc, to_end, exact);
+            hv = f.val;
+            put_flow(hrow, net.m_fpos[q], to_end, f);
         }
         if (sp.mixed && !staged)
             for (int x = 0; x < nh; ++x) w.hval32[base + x] = static_cast<float>(hrow[x]);
@@ -642,8 +608,8 @@ __global__ void __launch_bounds__(kBlock) k_evaluate_rows(DevNet net, DevWork w,
             const double v = hs[warp][x];
             w.hval[hw0 + x] = v;
             if (sp.mixed) {
-                w.hval32[hw0 + x] = static_cast<float>(v);
-                if (w.hw32) w.hw32[hw0 + x] = static_cast<float>(wes[warp][r] * v);
+                w.hval32[hw0 + x] = to_f32(v);
+                if (w.hw32) w.hw32[hw0 + x] = to_f32(wes[warp][r] * v);
             } else if (w.hw) {
                 w.hw[hw0 + x] = wes[warp][r] * v;
             }
@@ -888,10 +854,13 @@ __global__ void k_injections(DevNet net, DevWork w) {
 __global__ void k_flows(DevNet net, DevWork w) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= net.n_branch) return;
-    w.pf[k] = flow_terms(net, w.v, w.th, k, false, false, true).val;
-    w.qf[k] = flow_terms(net, w.v, w.th, k, true, false, true).val;
-    w.pt[k] = flow_terms(net, w.v, w.th, k, false, true, true).val;
-    w.qt[k] = flow_terms(net, w.v, w.th, k, true, true, true).val;
+    double s, c;
+    sincos(w.th[net.br_from[k]] - w.th[net.br_to[k]] - net.br_shift[k], &s, &c);
+    const FlowEnd F = flow_end(net, w.v, k, false, s, c), T = flow_end(net, w.v, k, true, s, c);
+    w.pf[k] = flow_row(net, F, k, false, false, true).val;
+    w.qf[k] = flow_row(net, F, k, true, false, true).val;
+    w.pt[k] = flow_row(net, T, k, false, true, true).val;
+    w.qt[k] = flow_row(net, T, k, true, true, true).val;
 }
 
 // Batch: one block per grid.  Clears the grid's flags (FROZEN for grids not

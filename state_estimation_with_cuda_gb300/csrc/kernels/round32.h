@@ -1,0 +1,31 @@
+// Rounding of an FP64 value to FP32 on the integer pipe.
+//
+// Any FP64 instruction, a conversion too, holds an SM sub-partition's FP64 pipe
+// for 64 cycles a warp; the dozen integer instructions of this take about as
+// many cycles.
+#pragma once
+#include <cstdint>
+
+#ifdef __CUDACC__
+#define SLE_HD __host__ __device__ __forceinline__
+#else
+#define SLE_HD inline
+#endif
+
+namespace sle_gb300 {
+
+// Can round32_bits take the value with this upper word?  Its FP64 exponent is
+// one of a normal FP32 number (rounding up to infinity included); zeros,
+// FP32 subnormals, infinities and NaN are not.
+SLE_HD bool round32_takes(uint32_t hi) { return ((hi >> 20) & 0x7ffu) - 897u < 254u; }
+
+// Bits of the FP32 value nearest to the FP64 value hi:lo, ties to even: the 23
+// leading mantissa bits behind the exponent's low eight (whose bias differs by
+// 896 = 128 modulo 256), rounded on the 29 bits that go.
+SLE_HD uint32_t round32_bits(uint32_t hi, uint32_t lo) {
+    const uint32_t m = (((hi << 3) | (lo >> 29)) & 0x7fffffffu) ^ 0x40000000u;
+    const uint32_t up = (lo & 0x1fffffffu) + (m & 1u) > 0x10000000u ? 1u : 0u;
+    return (m + up) | (hi & 0x80000000u);
+}
+
+}  // namespace sle_gb300
