@@ -29,6 +29,7 @@ namespace sle_gb300 {
 namespace {
 
 constexpr int kThreads = 256;
+constexpr int kSMs = 152;
 
 struct SolveVecs {
     const void* rhs;  // [n_state] right-hand side, permuted (V)
@@ -120,7 +121,7 @@ __device__ __forceinline__ bool front_frozen(const DevWork& W, const FrontRec& R
 }
 
 // Positive and finite?  FP64 by the bit pattern: an FP64 comparison or
-// conversion occupies the FP64 pipe for 64 cycles, as any FP64 instruction.
+// conversion is an FP64 instruction like any (60 cycles, 19 of the SM's pipe).
 __device__ __forceinline__ bool pivot_ok(float d) { return d > 0.f && isfinite(d); }
 __device__ __forceinline__ bool pivot_ok(double d) {
     const int hi = __double2hiint(d);
@@ -522,7 +523,7 @@ __device__ __forceinline__ int warp_continue_up(const DevFactor& F, const int8_t
 // the operations of the right-looking order in the same order, without its
 // read-modify-write of the tile per pivot (one shared-memory round trip per
 // entry and pivot was three quarters of a front's time).  FP64 packs the
-// trailing triangle into whole warps: an FP64 instruction costs 64 cycles
+// trailing triangle into whole warps: an FP64 instruction costs the same
 // whatever its lanes do.  Measured on a 301-bus grid's chain of six warp fronts:
 // 73 -> 46 us (mixed), on a 30k-bus grid's 172 -> 108 us (FP64).
 template <typename T>
@@ -743,10 +744,10 @@ __device__ __forceinline__ double pivot_recip(double& d, bool& bad) {
 // the counter after writing the column to shared memory, the other warps wait
 // for it (the CTA's warps are all resident, so the owner always runs; the wait
 // is bounded all the same).
-__device__ __forceinline__ void wait_column(int* ready, int k, uint32_t* status) {
+__device__ __forceinline__ int wait_column(int* ready, int k, uint32_t* status) {
     const unsigned at = static_cast<unsigned>(__cvta_generic_to_shared(ready));
+    int v;
     for (int spins = 0;; ++spins) {
-        int v;
         asm volatile("ld.acquire.cta.shared.b32 %0, [%1];" : "=r"(v) : "r"(at) : "memory");
         if (v >= k) break;
         if (spins > (1 << 22)) {
@@ -755,6 +756,7 @@ __device__ __forceinline__ void wait_column(int* ready, int k, uint32_t* status)
         }
     }
     __syncwarp();
+    return v;
 }
 __device__ __forceinline__ void post_column(int* ready, int k) {
     __syncwarp();
@@ -844,8 +846,8 @@ __device__ __forceinline__ void front_store(const SolveVecs& sv, T* lx, T* ub, c
 }
 
 // Assembles and partially factorises front s in shared memory, FP64, with
-// panels of KP columns.  Bound: FP64 issue (a warp instruction takes 64 cycles
-// of its scheduler) and the pivots' chain, as in k_big_panel64, whose scheme
+// panels of KP columns.  Bound: the FP64 pipe (a warp instruction per 19
+// cycles of the SM) and the pivots' chain, as in k_big_panel64, whose elimination
 // the panels use: warp w owns the panel's columns w (mod 8), a lane per row,
 // in registers; a column's unscaled rows are published in its place in Fm and
 // its block's rows over the pivot in ms; the rows past the first 32 follow one
@@ -1324,29 +1326,38 @@ __global__ void __launch_bounds__(kThreads) k_big_assemble(DevFactor F, DevWork 
 // block itself; the CTA that reads the block last writes it back, so no CTA
 // reads an overwritten block and none waits for another).
 //
-// Bound: an FP64 warp instruction takes 64 cycles of its scheduler however
-// many lanes are active, so what counts is FP64 instructions per scheduler and
-// the serial chain of a pivot.  Hence: eight warps, two per scheduler (one
-// waits while the other issues; four warps took 45k cycles, eight 34k), each
-// owning the columns c = warp (mod 8) of the block (a lane per row) and of the
-// chunk (two columns of 16 rows per instruction); the elimination is
-// a_ij -= u_i (u_j / d) with the unscaled column u, so the chain holds a
-// reciprocal (3 FP64 instructions) instead of a square root (10), and the
-// square roots of all pivots are taken together, a lane each, at the end.
-// The owner of column k + 1 updates and publishes that column before its
-// others, and warps wait for columns, not for each other.  The chunk follows
-// one column behind the block, off the chain of the pivots.  Measured: a full
-// step in about 37k cycles (18 us), where one warp's factorisation of the block
-// and a launch of one-warp row solves took 47 + 22 us; the linear solve of a
-// 30k-bus grid went from 5.04 to 3.08 ms with this and k_big_update64.
+// Bound: an FP64 warp instruction has a latency of 60 cycles and an SM finishes
+// one in 19, however many lanes are active.  So what counts is the serial chain
+// of the pivots, the number of FP64 instructions beside it, and that few of them
+// are in flight at a time: with more than three, each one on the chain waits.  The
+// elimination is a_ij -= u_i (u_j / d) with the unscaled column u, so a pivot's
+// chain is one update, a reciprocal (3 instructions; a square root takes 10) and
+// the product u / d; the square roots of all pivots come together at the end.
+// Warp roles:
+//  - one warp runs the chain, alone on its scheduler: it takes column k + 2 as
+//    the others left it (updated by the pivots before k), applies the pivots k
+//    and k + 1 itself and publishes u and u / d, a lane per row;
+//  - four warps bring the columns to that point, each a column from its first
+//    pivot to its last in the order the chain needs them (columns from 16 on in
+//    pairs, 16 rows each);
+//  - two warps solve the chunk, eight rows each, four columns an instruction, so
+//    that they wait for the chain only.
+// Columns reach the chain over named barriers (a flag cost it 170 cycles).  With
+// the columns dealt round eight warps, each in turn on the chain, a pivot took
+// about 1000 cycles and a full step 37k; with this 650 to 700 (alone on the SM the
+// chain takes 600) and 25k.  On average over a 60k-bus grid's steps 18.1 -> 13.5
+// us (47 + 22 us as one warp's factorisation and a launch of one-warp row solves);
+// two warps for the columns or one for the chunk are slower (20 to 33 us against
+// 18 with the launch).  A second CTA of an SM has its chain on another scheduler.
 __global__ void __launch_bounds__(kPanelThreads64, 2) k_big_panel64(DevFactor F, DevWork W, SolveVecs sv, double* lx,
                                                                  const int4* work, int p, int* step_cnt) {
-    static_assert(kPanelThreads64 == 256 && kPanelRows64 == 16 && kTile == 32, "thread tiling below");
-    constexpr int kW = kPanelThreads64 / 32, kQ = kTile / kW;  // columns per warp
-    __shared__ double us[kTile][kTile + kPanelRows64];  // column k: block rows, then chunk rows
-    __shared__ double ms[kTile][kTile];                 // u / d
-    __shared__ double dk[kTile];                        // pivots, then 1 / sqrt
-    __shared__ int ready, ready_x, last;            // columns published: block, chunk
+    static_assert(kPanelThreads64 == 256 && kPanelRows64 == 16 && kTile == 32, "warp roles below");
+    constexpr int kW = kPanelThreads64 / 32;
+    __shared__ double us[kTile][kTile];  // column k as eliminated so far, then final (u)
+    __shared__ double ms[kTile][kTile];  // u / d
+    __shared__ double dk[kTile];         // pivots, then 1 / sqrt
+    __shared__ int ready;                // pivots published
+    __shared__ int last;
     const int4 wk = work[blockIdx.x];
     const int s = wk.x, chunk = wk.y;
     if (front_frozen(F, W, s)) return;  // the whole CTA, before any barrier
@@ -1359,89 +1370,105 @@ __global__ void __launch_bounds__(kPanelThreads64, 2) k_big_panel64(DevFactor F,
     const int r0 = p0 + pb + chunk * kPanelRows64;
     const int nr = min(kPanelRows64, f + 1 - r0);  // row f: the right-hand side
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int xr = lane & (kPanelRows64 - 1), xh = lane >> 4;
-    // entry (r0 + xr, p0 + c) of the chunk: column stride 1 in the right-hand-side row
+    const int role = (w - static_cast<int>(blockIdx.x / kSMs)) & (kW - 1);
+    // chunk: entry (r0 + xr, p0 + c), column stride 1 in the right-hand-side row
+    const int xr = 8 * (role & 1) + (lane & 7), xg = lane >> 3;
+    const bool solves = role == 5 || role == 6, in = solves && xr < nr;
     double* const xb = r0 + xr == f ? static_cast<double*>(sv.sol) + c0 + p0 : B + (r0 + xr) + (int64_t)p0 * f;
     const int64_t xld = r0 + xr == f ? 1 : f;
-    if (threadIdx.x == 0) ready = ready_x = -1;
-    double a[kQ], x[kQ / 2];  // columns w + kW q; chunk columns w + kW (2 h + xh)
+    if (threadIdx.x == 0) ready = -1;
+    double x[kTile / 4];  // columns 4 i + xg
 #pragma unroll
-    for (int q = 0; q < kQ; ++q) {
-        const int c = w + kW * q;
-        a[q] = (c < pb && lane >= c && lane < pb) ? B[(p0 + lane) + (int64_t)(p0 + c) * f] : 0.0;
-    }
+    for (int i = 0; i < kTile / 4; ++i) x[i] = (in && 4 * i + xg < pb) ? xb[(4 * i + xg) * xld] : 0.0;
+    {
+        double a[kTile / kW];
 #pragma unroll
-    for (int h = 0; h < kQ / 2; ++h) {
-        const int c = w + kW * (2 * h + xh);
-        x[h] = (c < pb && xr < nr) ? xb[c * xld] : 0.0;
+        for (int q = 0; q < kTile / kW; ++q) {
+            const int c = w + kW * q;
+            a[q] = (c < pb && lane >= c && lane < pb) ? B[(p0 + lane) + (int64_t)(p0 + c) * f] : 0.0;
+        }
+#pragma unroll
+        for (int q = 0; q < kTile / kW; ++q) us[w + kW * q][lane] = a[q];
     }
     __syncthreads();
     bool bad = false;
     uint32_t* status = &W.status->flags;
-    // column k of this warp's block rows is final: its pivot, u and u / d
-    auto publish = [&](double& aq, int k) {
-        double d = __shfl_sync(0xffffffffu, aq, k);
-        us[k][lane] = aq;
-        ms[k][lane] = aq * pivot_recip(d, bad);
-        if (k + 1 < pb) hand_over(k);
-        if (lane == k) aq = d;
-        if (lane == 0) dk[k] = d;
-        post_column(&ready, k);
-    };
-    if (w == 0) publish(a[0], 0);
-#pragma unroll
-    for (int qq = 0; qq < kQ; ++qq) {
+    int seen = -1;  // pivots known to be published
+    if (role == 0) {
+        double cur = us[0][lane], next = us[1][lane];
 #pragma unroll 1
-        for (int kk = 0; kk < kW; ++kk) {
-            const int k = kW * qq + kk;
+        for (int k = 0; k < pb; ++k) {
+            double d = __shfl_sync(0xffffffffu, cur, k);
+            const double m = cur * pivot_recip(d, bad);
+            us[k][lane] = lane == k ? d : cur;
+            ms[k][lane] = m;
+            if (lane == 0) dk[k] = d;
+            post_column(&ready, k);
+            double after = 0.0;
+            if (k + 2 < pb) {
+                if (k > 0) take_over(k + 2);
+                after = us[k + 2][lane];
+            }
+            const double m1 = __shfl_sync(0xffffffffu, m, k + 1), m2 = __shfl_sync(0xffffffffu, m, k + 2);
+            const double u = cur;
+            cur = fma(-u, m1, next);
+            next = fma(-u, m2, after);
+        }
+    } else if (solves) {
+#pragma unroll
+        for (int k = 0; k < kTile; ++k) {
+            constexpr int kG = kTile / 4;
             if (k >= pb) break;
-            const bool next = w == ((kk + 1) & (kW - 1)) && k + 1 < pb;
-            if (next) take_over(k);
-            else wait_column(&ready, k, status);
-            const double ub = us[k][lane];
-            int done = k;  // block columns up to here are final or updated
-            if (next) {
-                // the owner of column k + 1: q = qq, or qq + 1 past the group's end
-                const double m = ms[k][k + 1];
-                if (kk + 1 < kW) {
-                    a[qq] = fma(-ub, m, a[qq]);
-                    publish(a[qq], k + 1);
-                } else if (qq + 1 < kQ) {
-                    const int qn = qq + 1 < kQ ? qq + 1 : kQ - 1;
-                    a[qn] = fma(-ub, m, a[qn]);
-                    publish(a[qn], k + 1);
-                }
-                done = k + 1;
+            if (seen < k) seen = wait_column(&ready, k, status);
+            const double u = __shfl_sync(0xffffffffu, x[k / 4], 8 * (k & 3) + (lane & 7));
+            if ((k & 3) < 3) {
+                const double xn = fma(-u, ms[k][4 * (k / 4) + xg], x[k / 4]);
+                if (xg > (k & 3)) x[k / 4] = xn;
             }
 #pragma unroll
-            for (int q = qq; q < kQ; ++q) {
-                const int c = w + kW * q;
-                if (c > done && c < pb) a[q] = fma(-ub, ms[k][c], a[q]);
+            for (int i = k / 4 + 1; i < kG; ++i) x[i] = fma(-u, ms[k][4 * i + xg], x[i]);
+        }
+    } else if (role == 4) {
+        // shares the chain's scheduler and stays out of its way; this CTA has read the block
+        if (lane == 0) last = atomicAdd(step_cnt + wk.w, 1) == wk.z - 1;
+    } else {
+        constexpr unsigned kOwner = 0x273173u;
+        // entry (row, c) by the pivots up to k1
+        auto eliminate = [&](double& a, int row, int c, int k, int k1) {
+            while (k <= k1) {
+                if (seen < k) seen = wait_column(&ready, k, status);
+                const int hi = min(k1, max(seen, k));
+#pragma unroll 4
+                for (; k <= hi; ++k) a = fma(-us[k][row], ms[k][c], a);
             }
-            // the chunk's columns behind k - 1 by column k - 1; column k is then final
-            if (k > 0) {
-                wait_column(&ready_x, k - 1, status);
-                const double uc = us[k - 1][kTile + xr];
-#pragma unroll
-                for (int h = qq / 2; h < kQ / 2; ++h) {
-                    const int c = w + kW * (2 * h + xh);
-                    if (w + kW * (2 * h + 1) >= k) {
-                        const double xn = fma(-uc, ms[k - 1][c], x[h]);
-                        if (c >= k) x[h] = xn;
-                    }
-                    if (h == qq / 2 && w == kk) {
-                        if (xh == (qq & 1)) us[k][kTile + xr] = x[h];
-                        post_column(&ready_x, k);
-                    }
-                }
-            } else if (w == 0) {
-                if (xh == 0) us[0][kTile + xr] = x[0];
-                post_column(&ready_x, 0);
+        };
+        // columns 3..15, then the pairs from 16 on; roles 3 and 7, whose scheduler has no
+        // solver, take two of three
+        for (int i = 0; i < 13 + 8; ++i) {
+            if (static_cast<int>((kOwner >> (4 * (i % 6))) & 15u) != role) continue;
+            const int c = i < 13 ? 3 + i : 16 + 2 * (i - 13);
+            if (c >= pb) break;
+            if (c < 16) {
+                double a = us[c][lane];
+                eliminate(a, lane, c, 0, c - 3);
+                us[c][lane] = a;
+                hand_over(c);
+            } else {
+                const int row = 16 + (lane & 15), h = lane >> 4;
+                double a = us[c + h][row];
+                eliminate(a, row, c + h, 0, c - 3);
+                if (h == 0) us[c][row] = a;
+                __syncwarp();
+                hand_over(c);
+                if (c + 1 >= pb) break;
+                eliminate(a, row, c + h, c - 2, c - 2);
+                if (h == 1) us[c + 1][row] = a;
+                __syncwarp();
+                hand_over(c + 1);
             }
         }
     }
-    __syncthreads();  // every pivot is in dk; this CTA's reads of the block are long done
-    if (threadIdx.x == 0) last = atomicAdd(step_cnt + wk.w, 1) == wk.z - 1;
+    __syncthreads();  // every pivot is in dk
     if (bad && lane == 0 && chunk == 0) atomicOr(singular_flags(F, W, s), FLAG_SINGULAR);
     if (w == 0 && lane < pb) {
         double sq, rs;
@@ -1451,15 +1478,15 @@ __global__ void __launch_bounds__(kPanelThreads64, 2) k_big_panel64(DevFactor F,
     }
     __syncthreads();
 #pragma unroll
-    for (int h = 0; h < kQ / 2; ++h) {
-        const int c = w + kW * (2 * h + xh);
-        if (c < pb && xr < nr) xb[c * xld] = x[h] * dk[c];
+    for (int i = 0; i < kTile / 4; ++i) {
+        const int c = 4 * i + xg;
+        if (in && c < pb) xb[c * xld] = x[i] * dk[c];
     }
     if (last) {
 #pragma unroll
-        for (int q = 0; q < kQ; ++q) {
+        for (int q = 0; q < kTile / kW; ++q) {
             const int c = w + kW * q;
-            if (c < pb && lane >= c && lane < pb) B[(p0 + lane) + (int64_t)(p0 + c) * f] = a[q] * dk[c];
+            if (c < pb && lane >= c && lane < pb) B[(p0 + lane) + (int64_t)(p0 + c) * f] = us[c][lane] * dk[c];
         }
     }
 }
@@ -2723,7 +2750,7 @@ __global__ void k_gain_export(DevFactor F, const HV* hval, const HV* hw, int n_t
 
 inline int grid_for(int64_t n, int threads) {
     int64_t g = (n + threads - 1) / threads;
-    if (g > 152 * 16) g = 152 * 16;
+    if (g > kSMs * 16) g = kSMs * 16;
     return (int)(g < 1 ? 1 : g);
 }
 

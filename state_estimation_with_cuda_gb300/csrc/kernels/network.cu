@@ -108,8 +108,8 @@ struct FlowTerms {
 // with (A, B) = (g c + b s, g s - b c) for P and (g s - b c, -(g c + b s)) for
 // Q, q the end's own admittance (over the tap squared at the from end).
 //
-// An FP64 instruction holds its pipe for 64 cycles a warp whatever lanes it
-// has, and the evaluation is bound by that pipe.  The form shares factors
+// An SM finishes one FP64 warp instruction in 19 cycles whatever lanes it has,
+// and the evaluation is bound by that.  The form shares factors
 // between value and derivatives, and one sequence serves the four kinds of
 // flow row (bit selects instead of branches; as four branches of the printed
 // formulas a warp of mixed rows ran about 90 FP64 instructions, now about 22).
