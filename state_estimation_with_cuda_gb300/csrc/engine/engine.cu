@@ -51,6 +51,9 @@ Engine::~Engine() {
     const DeviceScope dev_scope(cfg.device_id);
     release_device();
     if (st_) cudaStreamDestroy(st_);
+    if (sched_.side) cudaStreamDestroy(sched_.side);
+    if (sched_.fork) cudaEventDestroy(sched_.fork);
+    if (sched_.join) cudaEventDestroy(sched_.join);
     if (ev0_) cudaEventDestroy(ev0_);
     if (ev1_) cudaEventDestroy(ev1_);
     if (h_status_) cudaFreeHost(h_status_);
@@ -105,6 +108,10 @@ int32_t Engine::initialize() {
     if ((e = cudaSetDevice(cfg.device_id)) != cudaSuccess) return set_cuda_error(e, "cudaSetDevice");
     if ((e = cudaStreamCreateWithPriority(&st_, cudaStreamNonBlocking, cfg.stream_priority)) != cudaSuccess)
         return set_cuda_error(e, "stream");
+    if ((e = cudaStreamCreateWithPriority(&sched_.side, cudaStreamNonBlocking, cfg.stream_priority)) != cudaSuccess ||
+        (e = cudaEventCreateWithFlags(&sched_.fork, cudaEventDisableTiming)) != cudaSuccess ||
+        (e = cudaEventCreateWithFlags(&sched_.join, cudaEventDisableTiming)) != cudaSuccess)
+        return set_cuda_error(e, "side stream");
     cudaEventCreate(&ev0_);
     cudaEventCreate(&ev1_);
     if ((e = cudaMallocHost(&h_status_, sizeof(DevStatus))) != cudaSuccess) return set_cuda_error(e, "cudaMallocHost");

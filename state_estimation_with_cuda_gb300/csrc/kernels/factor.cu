@@ -2855,18 +2855,33 @@ cudaError_t factor_impl(const DevNet& net, const DevFactor& F, const DevWork& W,
     }
     for (int l = 0; l < ls.n_levels; ++l) {
         const int ns = ls.h_small_ptr[l + 1] - ls.h_small_ptr[l];
+        const int na = ls.h_asm_ptr[l + 1] - ls.h_asm_ptr[l];
+        const int nt = tile_flow ? ls.h_tt_ptr[l + 1] - ls.h_tt_ptr[l] : 0;
+        // The fronts of a level do not depend on each other: its single-CTA ones
+        // run on the side stream beside the tiled ones' steps, which leave most
+        // SMs idle (60k buses FP64 26.1 -> 23.8 ms, 64 grids 13.7 -> 12.3).  Not
+        // beside the tile dataflow kernel, whose CTAs fill the GPU and wait for
+        // one another.
+        const bool beside = ns > 0 && na > 0 && nt == 0;
+        if (beside) {
+            cudaError_t e = cudaEventRecord(ls.fork, st);
+            if (e == cudaSuccess) e = cudaStreamWaitEvent(ls.side, ls.fork, 0);
+            if (e != cudaSuccess) return e;
+        }
         if (ns > 0) {
             const int mf = ls.h_small_maxf[l];
-            k_front_small<T><<<ns, kFrontThreads<T, kPanel>, front_smem<T>(mf), st>>>(F, W, sv, gv, lx, ub,
-                                                                      ls.d_small + ls.h_small_ptr[l]);
+            k_front_small<T><<<ns, kFrontThreads<T, kPanel>, front_smem<T>(mf), beside ? ls.side : st>>>(
+                F, W, sv, gv, lx, ub, ls.d_small + ls.h_small_ptr[l]);
             count_launches(1);
         }
-        const int na = ls.h_asm_ptr[l + 1] - ls.h_asm_ptr[l];
+        if (beside) {
+            cudaError_t e = cudaEventRecord(ls.join, ls.side);
+            if (e != cudaSuccess) return e;
+        }
         if (na > 0) {
             k_big_assemble<T><<<na, kThreads, 0, st>>>(F, W, sv, gv, lx, ub, ls.d_asm + ls.h_asm_ptr[l],
                                                    ls.d_asm_child);
             count_launches(1);
-            const int nt = tile_flow ? ls.h_tt_ptr[l + 1] - ls.h_tt_ptr[l] : 0;
             if constexpr (sizeof(T) == 4) {
                 if (nt > 0) {
                     k_big_flow32<<<std::min(nt, ls.tt_grid), kThreads, 0, st>>>(
@@ -2897,6 +2912,10 @@ cudaError_t factor_impl(const DevNet& net, const DevFactor& F, const DevWork& W,
                     count_launches(1);
                 }
             }
+        }
+        if (beside) {
+            cudaError_t e = cudaStreamWaitEvent(st, ls.join, 0);
+            if (e != cudaSuccess) return e;
         }
     }
     return cudaGetLastError();

@@ -317,6 +317,9 @@ struct __align__(16) TileTask {
 // Work-list entries are int4 (front, a, b, 0).
 struct LevelSchedule {
     int32_t n_levels = 0;
+    // a level's single-CTA fronts run beside its tiled ones (factor_impl)
+    cudaStream_t side = nullptr;
+    cudaEvent_t fork = nullptr, join = nullptr;
     int32_t n_tgt = 0;                      // gain entries (targets)
     int32_t gain_acc32 = 0;                 // mixed pipeline: sum the gain entries in FP32 (else FP64)
     const int32_t* h_small_ptr = nullptr;   // [n_levels+1] offsets into d_small
