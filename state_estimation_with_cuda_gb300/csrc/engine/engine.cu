@@ -394,14 +394,22 @@ void Engine::build_schedule(bool targets_ready) {
         double fl = 0.0;
         for (int64_t c = 0; c < nc; ++c) fl += static_cast<double>(f - c - 1) * (f - c);
         // FP64 work per front is costly on this GPU, so the FP64 pipeline moves
-        // fronts with many flops to the tiled path; in FP32 only size decides
+        // fronts with many flops to the tiled path; in FP32 only size decides.
+        // Both sides of the line (8e4, 1e5, 2e5; phase A up to 128), the speed of a
+        // step against 2e5 with phase A up to 64, five grids a size: 2000 buses
+        // 1.13, 1.14, 1.12; 10k 1.08, 1.06, 1.04; 30k 1.07, 1.06, 1.03; 60k 1.05,
+        // 1.04, 0.99; 100k 1.01, 1.02, 0.96 (single grids a few percent either
+        // way); 64 grids together 1.10, 1.12, 1.11
         const int64_t fmax = mixed_ ? kSmallFrontMax32 : kSmallFrontMax;
         big[s] = (f > fmax || (!mixed_ && fl > cfg.big_front_flops)) ? 1 : 0;
     }
     // Dataflow phases: a front whose subtree holds no big front is factorised
     // by the persistent kernels (phase A if no front of its subtree is wider
     // than cfg.flow_small_f, phase B otherwise); the rest stays level-synchronous.
-    const int32_t want_f = cfg.flow_small_f > 0 ? cfg.flow_small_f : (mixed_ ? 128 : 64);
+    // By default phase A takes all it can hold: two phases are one after the
+    // other (FP64, the line above at 1e5: a step is 1.04 times as fast at 1000
+    // buses as up to 64, 1.14 at 2000, 1.05 at 10k, 1.03 at 60k)
+    const int32_t want_f = cfg.flow_small_f > 0 ? cfg.flow_small_f : kFlowSmallFMax;
     const int32_t flow_small_f = std::max(8, std::min(want_f, kFlowSmallFMax));
     std::vector<char> sub_big(ns, 0);
     std::vector<int32_t> sub_maxf(ns, 0);

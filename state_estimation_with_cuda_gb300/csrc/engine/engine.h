@@ -40,11 +40,11 @@ struct EngineConfig {
     int32_t exact_jacobian = 1;  // 0: the reference's Jacobian formulas
     int32_t gain_policy = 0;     // 0: refactor every iteration; 1: reuse the factor until invalidated
     int32_t ordering = 0;        // symbolic ordering (see SymbolicParams)
-    double big_front_flops = 2.0e5;  // FP64: fronts above this many factor flops use the tiled multi-CTA path
+    double big_front_flops = 1.0e5;  // FP64: fronts above this many factor flops use the tiled multi-CTA path
     int32_t refine_steps = 0;        // mixed precision: extra refinement steps per Gauss-Newton step
     int32_t dataflow = 1;            // persistent dataflow kernels below the big fronts and for the solves
     int32_t flow_small_f = 0;        // widest front of the high-occupancy dataflow phase (<= kFlowSmallFMax;
-                                     // 0: 128 for the mixed pipeline, 64 for FP64)
+                                     // 0: 128)
     int32_t warp_fronts = -1;        // warp phase for fronts whose subtree is at most kWarpFrontMax wide:
                                      // 1 on, 0 off, -1 per grid with at least kWarpPhaseMinFronts of them
     int32_t stream_priority = 0;     // CUDA stream priority of the engine's stream (lower = more urgent)
