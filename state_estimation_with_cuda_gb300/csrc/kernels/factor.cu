@@ -299,12 +299,15 @@ __device__ __forceinline__ void extend_add_children(const DevFactor& F, const So
 #pragma unroll
                 for (int k = 0; k < kB; ++k) cur[k] = ri[k] >= 0 ? dst[to[k]] : T(0);
 #pragma unroll
-                for (int k = 0; k < kB; ++k)
+                for (int k = 0; k < kB; ++k) {
+                    if (k >= z.cnt) break;
                     if (ri[k] >= 0) dst[to[k]] = cur[k] + u[k];
+                }
             } else {
 #pragma unroll
                 for (int k = 0; k < kB; ++k) {
-                    if (lane == z.q0 + k && k < z.cnt) rhs[t * rhs_ld] += bv;  // a batch of one step
+                    if (k >= z.cnt) break;
+                    if (lane == z.q0 + k) rhs[t * rhs_ld] += bv;  // a batch of one step
                     if (ri[k] >= 0) dst[to[k]] += u[k];
                     __syncwarp();
                 }
@@ -636,8 +639,10 @@ __device__ void warp_front_factor(const DevFactor& F, const DevWork& W, const So
                 cur[k] = to[k] >= 0 ? t.a[to[k]] : T(0);
             }
 #pragma unroll
-            for (int k = 0; k < kB; ++k)
+            for (int k = 0; k < kB; ++k) {
+                if (j0 + k >= mm) break;
                 if (to[k] >= 0) t.a[to[k]] = cur[k] + u[k];
+            }
             __syncwarp();
             if (!more) break;
             ch = nch;
@@ -890,6 +895,9 @@ __device__ __forceinline__ void front_store(const SolveVecs& sv, T* lx, T* ub, c
 // so that no lane idles.  Measured on a 30k-bus grid, against one warp's
 // factorisation of the block, a thread per row below it and 4 x 4 tiles in the
 // update: phase B 337 -> 202 us, phase A 261 -> 159, synchronous levels 82 -> 50.
+// An FP64 instruction costs the same with every lane off, so row groups and
+// columns that a panel does not have are left by branches, not by predicates
+// (2003 buses: phase A 137 -> 122 us, synchronous levels 97 -> 64).
 template <int KP>
 __device__ void front_factor(const DevFactor& F, const DevWork& W, const SolveVecs& sv, const double* gv, double* lx,
                              double* ub, const FrontRec& R, int s, double* Fm, FrontSmem<double, KP>& sm) {
@@ -961,25 +969,19 @@ __device__ void front_factor(const DevFactor& F, const DevWork& W, const SolveVe
                     // the rows past the first 32: columns behind k - 1 by column k - 1, then column k is final
                     if (k > 0) {
                         wait_column(&sm.ready_x, k - 1, status);
-                        double u[kG];
 #pragma unroll
-                        for (int g = 1; g < kG; ++g) u[g] = (32 * g + lane < nrow) ? P[32 * g + lane + (k - 1) * ldf] : 0.0;
+                        for (int g = 1; g < kG; ++g) {
+                            if (g >= ng) break;
+                            const double u = (32 * g + lane < nrow) ? P[32 * g + lane + (k - 1) * ldf] : 0.0;
 #pragma unroll
-                        for (int q = qq; q < kQ; ++q) {
-                            const int c = w + kW * q;
-                            if (c >= k && c < kb) {
-                                const double m = sm.ms[k - 1][c];
-#pragma unroll
-                                for (int g = 1; g < kG; ++g)
-                                    if (g < ng) a[q][g] = fma(-u[g], m, a[q][g]);
+                            for (int q = qq; q < kQ; ++q) {
+                                const int c = w + kW * q;
+                                if (c >= kb) break;
+                                if (c >= k) a[q][g] = fma(-u, sm.ms[k - 1][c], a[q][g]);
                             }
-                            if (q == qq && w == kk) {
-#pragma unroll
-                                for (int g = 1; g < kG; ++g)
-                                    if (32 * g + lane < nrow) P[32 * g + lane + k * ldf] = a[q][g];
-                                post_column(&sm.ready_x, k);
-                            }
+                            if (w == kk && 32 * g + lane < nrow) P[32 * g + lane + k * ldf] = a[qq][g];
                         }
+                        if (w == kk) post_column(&sm.ready_x, k);
                     } else if (w == 0) {
                         post_column(&sm.ready_x, 0);  // column 0 is in place
                     }
@@ -998,11 +1000,12 @@ __device__ void front_factor(const DevFactor& F, const DevWork& W, const SolveVe
 #pragma unroll
         for (int q = 0; q < kQ; ++q) {
             const int c = w + kW * q;
-            if (c < kb) {
-                const double rs = sm.dk[c];
+            if (c >= kb) break;
+            const double rs = sm.dk[c];
 #pragma unroll
-                for (int g = 0; g < kG; ++g)
-                    if (g < ng && 32 * g + lane < nrow) P[32 * g + lane + c * ldf] = a[q][g] * rs;
+            for (int g = 0; g < kG; ++g) {
+                if (g >= ng) break;
+                if (32 * g + lane < nrow) P[32 * g + lane + c * ldf] = a[q][g] * rs;
             }
         }
         __syncthreads();
