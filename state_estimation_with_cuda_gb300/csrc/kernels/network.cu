@@ -125,6 +125,14 @@ struct FlowEnd {
 __device__ __forceinline__ double flip(double v, bool neg) {  // the sign bit, off the FP64 pipe
     return __hiloint2double(__double2hiint(v) ^ (neg ? static_cast<int>(0x80000000) : 0), __double2loint(v));
 }
+// A sum that few lanes need.  A call, so that it is behind a branch: an FP64
+// instruction takes its pipe's time with every lane off as well.
+__device__ __noinline__ double add_apart(double a, double b) { return a + b; }
+// v * 0.0: a zero of v's sign, NaN for an infinity or NaN; off the FP64 pipe
+__device__ __forceinline__ double times_zero(double v) {
+    const int hi = __double2hiint(v);
+    return __hiloint2double((hi & 0x7ff00000) == 0x7ff00000 ? 0x7ff80000 : hi & static_cast<int>(0x80000000), 0);
+}
 // v == 0, off the FP64 pipe
 __device__ __forceinline__ bool is_zero(double v) { return ((__double2hiint(v) & 0x7fffffff) | __double2loint(v)) == 0; }
 
@@ -143,8 +151,8 @@ __device__ __forceinline__ FlowEnd flow_end(const DevNet& net, const double* v, 
     return E;
 }
 
-__device__ __forceinline__ FlowTerms flow_row(const DevNet& net, const FlowEnd& E, int k, bool is_q, bool to_end,
-                                              bool exact) {
+template <bool exact>
+__device__ __forceinline__ FlowTerms flow_row(const DevNet& net, const FlowEnd& E, int k, bool is_q, bool to_end) {
     const double g = net.br_g[k], b = net.br_b[k];
     const double q0 = is_q ? -(b + (to_end ? net.br_bst[k] : net.br_bsf[k])) : g;
     const double A = is_q ? E.x2 : E.x1, B = is_q ? flip(E.x1, true) : E.x2;
@@ -153,19 +161,20 @@ __device__ __forceinline__ FlowTerms flow_row(const DevNet& net, const FlowEnd& 
     FlowTerms f;
     f.val = E.Vo * r;
     f.dvo = fma(E.Vo, q, r);
-    // the reference leaves the charging out of dQ/dV
-    if (is_q && !exact) f.dvo = fma(-2.0 * E.Vo, E.w * b, -u);
+    if (!exact) {  // the reference leaves the charging out of dQ/dV
+        const double dq = fma(-2.0 * E.Vo, E.w * b, -u);
+        if (is_q) f.dvo = dq;
+    }
     f.dvx = flip(E.Vo * A, true);
     f.dto = E.Vo * (E.Vx * B);
     // the reference flips the sign of dP/dtheta at the to end
     if (!exact && to_end && !is_q) f.dto = flip(f.dto, true);
-    if (!net.br_closed[k]) {
-        f.val *= 0.0;
-        if (exact) {
-            f.dto *= 0.0;
-            f.dvo *= 0.0;
-            f.dvx *= 0.0;
-        }
+    const bool closed = net.br_closed[k] != 0;
+    f.val = closed ? f.val : times_zero(f.val);
+    if (exact) {
+        f.dto = closed ? f.dto : times_zero(f.dto);
+        f.dvo = closed ? f.dvo : times_zero(f.dvo);
+        f.dvx = closed ? f.dvx : times_zero(f.dvx);
     }
     return f;
 }
@@ -215,19 +224,17 @@ __device__ __forceinline__ void put_flow(double* hrow, int fpos, bool to_end, co
     for (int x = 0; x < 4; ++x) {
         const int p = (fpos >> (8 * x)) & 0xFF;
         if (p == 0xFF) continue;
-        if (loop)
-            hrow[p] += d[x];
-        else
-            hrow[p] = d[x];
+        hrow[p] = loop ? add_apart(hrow[p], d[x]) : d[x];
     }
 }
 
 // Current magnitude |S| / V at one end of branch k.
-__device__ __forceinline__ FlowTerms current_row(const DevNet& net, const DevWork& w, int k, bool to_end, bool exact) {
+template <bool exact>
+__device__ __forceinline__ FlowTerms current_row(const DevNet& net, const DevWork& w, int k, bool to_end) {
     double s, c;
     branch_angle(net, w.bus_cs, k, &s, &c);
     const FlowEnd E = flow_end(net, w.v, k, to_end, s, c);
-    const FlowTerms P = flow_row(net, E, k, false, to_end, exact), Q = flow_row(net, E, k, true, to_end, exact);
+    const FlowTerms P = flow_row<exact>(net, E, k, false, to_end), Q = flow_row<exact>(net, E, k, true, to_end);
     const double on = net.br_closed[k] ? 1.0 : 0.0;
     const double vs = fmax(E.Vo, kEps);
     const double S = sqrt(P.val * P.val + Q.val * Q.val);
@@ -254,7 +261,8 @@ __device__ __forceinline__ FlowTerms current_row(const DevNet& net, const DevWor
 struct InjSums {
     double a, b, c, d;
 };
-__device__ __forceinline__ double inj_value(const InjSums& S, double Vi, bool exact, double* dv, double* dt) {
+template <bool exact>
+__device__ __forceinline__ double inj_value(const InjSums& S, double Vi, double* dv, double* dt) {
     const double r = fma(Vi, S.c, S.a);
     *dv = fma(Vi, S.c, r);
     *dt = flip(Vi * S.b, true);
@@ -280,6 +288,7 @@ constexpr int kEvalSpan = 512;
 // the rows come in order (the usual case); their H entries are then built in
 // shared memory and the warp writes the range out coalesced, skipping rows
 // it does not evaluate.  Otherwise each thread writes its rows in place.
+template <bool exact>
 __global__ void __launch_bounds__(kBlock) k_evaluate_pairs(DevNet net, DevWork w, SolveParams sp) {
     __shared__ double sh[32];
     __shared__ double hs[kBlock / 32][kEvalSpan];
@@ -306,7 +315,6 @@ __global__ void __launch_bounds__(kBlock) k_evaluate_pairs(DevNet net, DevWork w
         const uint32_t gf = w.grid_flags[net.meas_grid[un.x]];
         skip = (gf & sp.skip_flags) || (gf & sp.need_flags) != sp.need_flags;
     }
-    const bool exact = sp.exact_jacobian != 0;
     // the H row of row q: in the warp's staged range or in place (zeroed)
     auto row_of = [&](int q) -> double* {
         const int base = net.h_ptr[q], nh = net.h_ptr[q + 1] - base;
@@ -378,12 +386,14 @@ __global__ void __launch_bounds__(kBlock) k_evaluate_pairs(DevNet net, DevWork w
             const double2 cs_i = w.bus_cs[loc];
             InjSums P{}, Q{};
             const int e0 = net.y_ptr[loc], e1 = net.y_ptr[loc + 1];
-            for (int e = e0; e < e1; ++e) {
+            P.c = __ldg(net.y_g + e0);  // the diagonal comes first
+            P.d = __ldg(net.y_b + e0);
+            for (int e = e0 + 1; e < e1; ++e) {
                 const int j = __ldg(net.y_col + e);
                 const double G = __ldg(net.y_g + e), B = __ldg(net.y_b + e);
-                if (j == loc) {
-                    P.c += G;
-                    P.d += B;
+                if (j == loc) {  // a branch that ends where it starts
+                    P.c = add_apart(P.c, G);
+                    P.d = add_apart(P.d, B);
                     continue;
                 }
                 const double Vj = __ldg(w.v + j);
@@ -410,13 +420,13 @@ __global__ void __launch_bounds__(kBlock) k_evaluate_pairs(DevNet net, DevWork w
             const int pt = net.y_hpos_t[e0], pv = net.y_hpos_v[e0];
             double dv, dt;
             if (hp) {
-                const double hv = inj_value(P, Vi, exact, &dv, &dt);
+                const double hv = inj_value<exact>(P, Vi, &dv, &dt);
                 if (pt >= 0) hp[pt] += dt;
                 hp[pv] += dv;
                 finish(qp, kind, hv, hp);
             }
             if (hq) {
-                const double hv = inj_value(Q, Vi, exact, &dv, &dt);
+                const double hv = inj_value<exact>(Q, Vi, &dv, &dt);
                 if (pt >= 0) hq[pt] += dt;
                 hq[pv] += dv;
                 finish(qq, kind, hv, hq);
@@ -428,19 +438,19 @@ __global__ void __launch_bounds__(kBlock) k_evaluate_pairs(DevNet net, DevWork w
             branch_angle(net, w.bus_cs, loc, &sn, &cn);
             const FlowEnd E = flow_end(net, w.v, loc, to_end, sn, cn);
             double* ha = row_of(qa);
-            const FlowTerms fa = flow_row(net, E, loc, a_is_q, to_end, exact);
+            const FlowTerms fa = flow_row<exact>(net, E, loc, a_is_q, to_end);
             put_flow(ha, net.m_fpos[qa], to_end, fa);
             finish(qa, kind, fa.val, ha);
             if (qb >= 0) {
                 double* hb = row_of(qb);
-                const FlowTerms fb = flow_row(net, E, loc, !a_is_q, to_end, exact);
+                const FlowTerms fb = flow_row<exact>(net, E, loc, !a_is_q, to_end);
                 put_flow(hb, net.m_fpos[qb], to_end, fb);
                 finish(qb, kind, fb.val, hb);
             }
         } else if (kind == 4) {  // current magnitude
             double* hrow = row_of(qa);
             const bool to_end = net.m_end[qa] != 0;
-            const FlowTerms f = current_row(net, w, loc, to_end, exact);
+            const FlowTerms f = current_row<exact>(net, w, loc, to_end);
             put_flow(hrow, net.m_fpos[qa], to_end, f);
             finish(qa, kind, f.val, hrow);
         } else {
@@ -476,6 +486,7 @@ __global__ void __launch_bounds__(kBlock) k_evaluate_pairs(DevNet net, DevWork w
 // evaluations with no paired rows: twice the threads of k_evaluate_pairs,
 // which a small grid needs to fill the GPU).
 
+template <bool exact>
 __global__ void __launch_bounds__(kBlock) k_evaluate_rows(DevNet net, DevWork w, SolveParams sp) {
     __shared__ double sh[32];
     // A warp's rows own the contiguous H range [hw0, hw1).  When it fits,
@@ -508,7 +519,6 @@ __global__ void __launch_bounds__(kBlock) k_evaluate_rows(DevNet net, DevWork w,
         const int kind = net.m_kind[q];
         const int ty = net.m_type[q];
         const int loc = net.m_loc[q];
-        const bool exact = sp.exact_jacobian != 0;
         const int base = net.h_ptr[q];
         const int nh = net.h_ptr[q + 1] - base;
         double* hrow = staged ? &hs[warp][base - hw0] : w.hval + base;
@@ -530,12 +540,17 @@ __global__ void __launch_bounds__(kBlock) k_evaluate_rows(DevNet net, DevWork w,
             const double2 cs_i = w.bus_cs[loc];
             InjSums S{};
             const int e0 = net.y_ptr[loc], e1 = net.y_ptr[loc + 1];
-            for (int e = e0; e < e1; ++e) {
+            {
+                const double G = __ldg(net.y_g + e0), B = __ldg(net.y_b + e0);  // the diagonal comes first
+                S.c = isq ? flip(B, true) : G;
+                S.d = isq ? G : B;
+            }
+            for (int e = e0 + 1; e < e1; ++e) {
                 const int j = __ldg(net.y_col + e);
                 const double G = __ldg(net.y_g + e), B = __ldg(net.y_b + e);
-                if (j == loc) {
-                    S.c += isq ? flip(B, true) : G;
-                    S.d += isq ? G : B;
+                if (j == loc) {  // a branch that ends where it starts
+                    S.c = add_apart(S.c, isq ? flip(B, true) : G);
+                    S.d = add_apart(S.d, isq ? G : B);
                     continue;
                 }
                 const double Vj = __ldg(w.v + j);
@@ -550,7 +565,7 @@ __global__ void __launch_bounds__(kBlock) k_evaluate_rows(DevNet net, DevWork w,
                 hrow[pv] += Vi * A;
             }
             double dv, dt;
-            hv = inj_value(S, Vi, exact, &dv, &dt);
+            hv = inj_value<exact>(S, Vi, &dv, &dt);
             const int pt = net.y_hpos_t[e0];
             if (pt >= 0) hrow[pt] += dt;
             hrow[net.y_hpos_v[e0]] += dv;
@@ -558,12 +573,12 @@ __global__ void __launch_bounds__(kBlock) k_evaluate_rows(DevNet net, DevWork w,
             const bool to_end = net.m_end[q] != 0;
             double sn, cn;
             branch_angle(net, w.bus_cs, loc, &sn, &cn);
-            const FlowTerms f = flow_row(net, flow_end(net, w.v, loc, to_end, sn, cn), loc, ty == 5, to_end, exact);
+            const FlowTerms f = flow_row<exact>(net, flow_end(net, w.v, loc, to_end, sn, cn), loc, ty == 5, to_end);
             hv = f.val;
             put_flow(hrow, net.m_fpos[q], to_end, f);
         } else if (kind == 4) {  // current magnitude
             const bool to_end = net.m_end[q] != 0;
-            const FlowTerms f = current_row(net, w, loc, to_end, exact);
+            const FlowTerms f = current_row<exact>(net, w, loc, to_end);
             hv = f.val;
             put_flow(hrow, net.m_fpos[q], to_end, f);
         }
@@ -857,10 +872,10 @@ __global__ void k_flows(DevNet net, DevWork w) {
     double s, c;
     sincos(w.th[net.br_from[k]] - w.th[net.br_to[k]] - net.br_shift[k], &s, &c);
     const FlowEnd F = flow_end(net, w.v, k, false, s, c), T = flow_end(net, w.v, k, true, s, c);
-    w.pf[k] = flow_row(net, F, k, false, false, true).val;
-    w.qf[k] = flow_row(net, F, k, true, false, true).val;
-    w.pt[k] = flow_row(net, T, k, false, true, true).val;
-    w.qt[k] = flow_row(net, T, k, true, true, true).val;
+    w.pf[k] = flow_row<true>(net, F, k, false, false).val;
+    w.qf[k] = flow_row<true>(net, F, k, true, false).val;
+    w.pt[k] = flow_row<true>(net, T, k, false, true).val;
+    w.qt[k] = flow_row<true>(net, T, k, true, true).val;
 }
 
 // Batch: one block per grid.  Clears the grid's flags (FROZEN for grids not
@@ -1172,10 +1187,11 @@ cudaError_t launch_evaluate(const DevNet& net, const DevWork& w, const SolvePara
     if (net.n_meas <= 0) return cudaSuccess;
     k_bus_trig<<<nblocks(net.n_bus), kBlock, 0, st>>>(net, w, sp);
     // the unit list has as many units as rows when no row is paired
+    const bool exact = sp.exact_jacobian != 0;
     if (net.n_units < net.n_meas)
-        k_evaluate_pairs<<<nblocks(net.n_units), kBlock, 0, st>>>(net, w, sp);
+        (exact ? k_evaluate_pairs<true> : k_evaluate_pairs<false>)<<<nblocks(net.n_units), kBlock, 0, st>>>(net, w, sp);
     else
-        k_evaluate_rows<<<nblocks(net.n_meas), kBlock, 0, st>>>(net, w, sp);
+        (exact ? k_evaluate_rows<true> : k_evaluate_rows<false>)<<<nblocks(net.n_meas), kBlock, 0, st>>>(net, w, sp);
     count_launches(2);
     if (sp.huber_objective) {
         k_huber_objective<<<1, 1024, 0, st>>>(w, nblocks(net.n_units));
