@@ -1568,8 +1568,8 @@ __device__ __forceinline__ void big_panel32_item(const DevFactor& F, const DevWo
     const int nr = max(0, min(kPanelRows, f - r0));  // its rows
     const int tid = threadIdx.x;
     // From the second step on, the previous step's trailing update has already
-    // factored and inverted this diagonal block (look-ahead in k_big_update):
-    // its slot holds L_dd^-1, the pivots are checked and rdiag is written.
+    // factored and inverted this diagonal block: its slot holds L_dd^-1, the
+    // pivots are checked and rdiag is written.
     const bool pre = p > 0;
     {
         // all staging loads in flight before the first shared-memory store:

@@ -104,22 +104,23 @@ struct FlowTerms {
 
 // What the P and Q flow at one end of branch k share (a4 + a8 flow rows).
 // With s the sine of the angle from that end, both rows are
-//   h = V_o (V_o q + V_x inv A),  dh/dtheta_o = -V_o V_x inv B  (signs below)
+//   h = V_o^2 q - V_o V_x inv A,  dh/dtheta_o = V_o V_x inv B
 // with (A, B) = (g c + b s, g s - b c) for P and (g s - b c, -(g c + b s)) for
 // Q, q the end's own admittance (over the tap squared at the from end).
 //
 // An SM finishes one FP64 warp instruction in 19 cycles whatever lanes it has,
-// and the evaluation is bound by that.  The form shares factors
-// between value and derivatives, and one sequence serves the four kinds of
-// flow row (bit selects instead of branches; as four branches of the printed
-// formulas a warp of mixed rows ran about 90 FP64 instructions, now about 22).
-// Injections are written the same way (InjSums), and the H entries are rounded
-// to FP32 on the integer pipe (round32.h).  The evaluation of 512 grids (pairs)
-// went from 311 to 229 us, of 200k buses from 153 to 120, of 20k (rows) from 39
-// to 31; against extended precision the rows' values lose a fifth of their error.
+// and the evaluation is bound by that.  One sequence serves the four kinds of
+// flow row and both kinds of injection (selects on the integer pipe instead of
+// branches, which a warp of mixed rows runs one after the other); sums that few
+// rows need are behind calls, and the H entries are rounded to FP32 on the
+// integer pipe (round32.h).  Products are rounded and fused as in the formulas
+// one by one, so the bits are theirs: the mixed pipeline's estimates of stiff
+// grids move by up to 3e-8 when an ulp of H does.  The evaluation of 512 grids
+// (pairs) went from 311 to 243 us, of 200k buses from 153 to 122, of 20k
+// (rows) from 39 to 33.
 struct FlowEnd {
-    double Vo, Vx, x1, x2;  // x1 = inv (g c + b s), x2 = inv (g s - b c)
-    double w;               // 1 / a^2 at the from end, 1 at the to end
+    double Vo, Vx, gc, gs;  // g c + b s, g s - b c
+    double inv, w;          // 1 / a; 1 / a^2 at the from end, 1 at the to end
 };
 
 __device__ __forceinline__ double flip(double v, bool neg) {  // the sign bit, off the FP64 pipe
@@ -128,6 +129,7 @@ __device__ __forceinline__ double flip(double v, bool neg) {  // the sign bit, o
 // A sum that few lanes need.  A call, so that it is behind a branch: an FP64
 // instruction takes its pipe's time with every lane off as well.
 __device__ __noinline__ double add_apart(double a, double b) { return a + b; }
+__device__ __noinline__ double fma_apart(double a, double b, double c) { return fma(a, b, c); }
 // v * 0.0: a zero of v's sign, NaN for an infinity or NaN; off the FP64 pipe
 __device__ __forceinline__ double times_zero(double v) {
     const int hi = __double2hiint(v);
@@ -145,8 +147,9 @@ __device__ __forceinline__ FlowEnd flow_end(const DevNet& net, const double* v, 
     FlowEnd E;
     E.Vo = to_end ? Vj : Vi;
     E.Vx = to_end ? Vi : Vj;
-    E.x1 = inv * (g * c + b * s);
-    E.x2 = inv * (g * s - b * c);
+    E.gc = g * c + b * s;
+    E.gs = g * s - b * c;
+    E.inv = inv;
     E.w = to_end ? 1.0 : ia2;
     return E;
 }
@@ -155,18 +158,18 @@ template <bool exact>
 __device__ __forceinline__ FlowTerms flow_row(const DevNet& net, const FlowEnd& E, int k, bool is_q, bool to_end) {
     const double g = net.br_g[k], b = net.br_b[k];
     const double q0 = is_q ? -(b + (to_end ? net.br_bst[k] : net.br_bsf[k])) : g;
-    const double A = is_q ? E.x2 : E.x1, B = is_q ? flip(E.x1, true) : E.x2;
-    const double q = E.w * q0, u = E.Vx * A;
-    const double r = fma(E.Vo, q, -u);
+    const double A = is_q ? E.gs : E.gc, B = is_q ? flip(E.gc, true) : E.gs;
+    const double vv = E.Vo * E.Vx * E.inv;
     FlowTerms f;
-    f.val = E.Vo * r;
-    f.dvo = fma(E.Vo, q, r);
-    if (!exact) {  // the reference leaves the charging out of dQ/dV
-        const double dq = fma(-2.0 * E.Vo, E.w * b, -u);
-        if (is_q) f.dvo = dq;
-    }
-    f.dvx = flip(E.Vo * A, true);
-    f.dto = E.Vo * (E.Vx * B);
+    // (which product of a difference is rounded follows the formulas' signs)
+    const bool second = is_q && to_end;
+    const double s2 = E.Vo * E.Vo * E.w;
+    f.val = fma(second ? -vv : s2, second ? A : q0, second ? s2 * q0 : -(vv * A));
+    const double qd = exact || !is_q ? q0 : -b;  // the reference leaves the charging out of dQ/dV
+    const double t1 = 2.0 * E.Vo * (is_q ? qd : E.w), t2 = is_q ? E.w : qd, xi = E.Vx * E.inv;
+    f.dvo = fma(second ? -xi : t1, second ? A : t2, second ? t1 * t2 : -(xi * A));
+    f.dvx = flip(E.Vo * E.inv * A, true);
+    f.dto = vv * B;
     // the reference flips the sign of dP/dtheta at the to end
     if (!exact && to_end && !is_q) f.dto = flip(f.dto, true);
     const bool closed = net.br_closed[k] != 0;
@@ -252,22 +255,6 @@ __device__ __forceinline__ FlowTerms current_row(const DevNet& net, const DevWor
         if (E.Vo > kEps) f.dvo -= S / (vs * vs) * on;
     }
     return f;
-}
-
-// Row sums of an injection at bus i over its neighbours: a = sum V_j A_j,
-// b = sum V_j B_j with (A, B) as for a flow (G, B the Ybus entry), c, d the
-// diagonal's (G, B) for P and (-B, G) for Q.  Then h = V_i (V_i c + a),
-// dh/dV_i = 2 V_i c + a, dh/dtheta_i = -V_i b (the reference adds V_i^2 d).
-struct InjSums {
-    double a, b, c, d;
-};
-template <bool exact>
-__device__ __forceinline__ double inj_value(const InjSums& S, double Vi, double* dv, double* dt) {
-    const double r = fma(Vi, S.c, S.a);
-    *dv = fma(Vi, S.c, r);
-    *dt = flip(Vi * S.b, true);
-    if (!exact) *dt += Vi * Vi * S.d;
-    return Vi * r;
 }
 
 // float(v) off the FP64 pipe where the result is a normal number.
@@ -384,52 +371,63 @@ __global__ void __launch_bounds__(kBlock) k_evaluate_pairs(DevNet net, DevWork w
             double* hq = qq >= 0 ? row_of(qq) : nullptr;
             const double Vi = w.v[loc];
             const double2 cs_i = w.bus_cs[loc];
-            InjSums P{}, Q{};
+            double hvp = 0.0, dVip = 0.0, dTip = 0.0, hvq = 0.0, dViq = 0.0, dTiq = 0.0;
             const int e0 = net.y_ptr[loc], e1 = net.y_ptr[loc + 1];
-            P.c = __ldg(net.y_g + e0);  // the diagonal comes first
-            P.d = __ldg(net.y_b + e0);
-            for (int e = e0 + 1; e < e1; ++e) {
-                const int j = __ldg(net.y_col + e);
-                const double G = __ldg(net.y_g + e), B = __ldg(net.y_b + e);
-                if (j == loc) {  // a branch that ends where it starts
-                    P.c = add_apart(P.c, G);
-                    P.d = add_apart(P.d, B);
-                    continue;
-                }
-                const double Vj = __ldg(w.v + j);
-                const int pt = __ldg(net.y_hpos_t + e), pv = __ldg(net.y_hpos_v + e);
-                double sn, cn;
-                angle_diff(cs_i, __ldg(w.bus_cs + j), &sn, &cn);
-                const double gc = G * cn + B * sn, gs = G * sn - B * cn;
-                const double vg = Vj * gc, vs = Vj * gs;
-                P.a += vg;
-                P.b += vs;
-                if (hp) {
-                    if (pt >= 0) hp[pt] += Vi * vs;
-                    hp[pv] += Vi * gc;
-                }
-                if (hq) {
-                    if (pt >= 0) hq[pt] -= Vi * vg;
-                    hq[pv] += Vi * gs;
+            {
+                const double G = net.y_g[e0], B = net.y_b[e0];  // the diagonal comes first
+                hvp = __dmul_rn(Vi * Vi, G);
+                dVip = __dmul_rn(2.0 * Vi, G);
+                hvq = __dmul_rn(Vi * Vi, -B);
+                dViq = __dmul_rn(2.0 * Vi, -B);
+                if (!exact) {
+                    dTip = __dmul_rn(Vi * Vi, B);
+                    dTiq = hvp;
                 }
             }
-            Q.a = P.b;
-            Q.b = flip(P.a, true);
-            Q.c = flip(P.d, true);
-            Q.d = P.c;
+            for (int e = e0 + 1; e < e1; ++e) {
+                const int j = net.y_col[e];
+                const double G = net.y_g[e], B = net.y_b[e];
+                if (j == loc) {  // a branch that ends where it starts
+                    hvp = fma_apart(Vi * Vi, G, hvp);
+                    dVip = fma_apart(2.0 * Vi, G, dVip);
+                    hvq = fma_apart(Vi * Vi, -B, hvq);
+                    dViq = fma_apart(2.0 * Vi, -B, dViq);
+                    if (!exact) {
+                        dTip = fma_apart(Vi * Vi, B, dTip);
+                        dTiq = fma_apart(Vi * Vi, G, dTiq);
+                    }
+                } else {
+                    const double Vj = w.v[j];
+                    double sn, cn;
+                    angle_diff(cs_i, w.bus_cs[j], &sn, &cn);
+                    const double gcbs = G * cn + B * sn, gsbc = G * sn - B * cn;
+                    const int pt = net.y_hpos_t[e], pv = net.y_hpos_v[e];
+                    if (hp) {
+                        hvp += Vi * Vj * gcbs;
+                        dVip += Vj * gcbs;
+                        dTip -= Vi * Vj * gsbc;
+                        if (pt >= 0) hp[pt] += Vi * Vj * gsbc;
+                        hp[pv] += Vi * gcbs;
+                    }
+                    if (hq) {
+                        hvq += Vi * Vj * gsbc;
+                        dViq += Vj * gsbc;
+                        dTiq += Vi * Vj * gcbs;
+                        if (pt >= 0) hq[pt] += -Vi * Vj * gcbs;
+                        hq[pv] += Vi * gsbc;
+                    }
+                }
+            }
             const int pt = net.y_hpos_t[e0], pv = net.y_hpos_v[e0];
-            double dv, dt;
             if (hp) {
-                const double hv = inj_value<exact>(P, Vi, &dv, &dt);
-                if (pt >= 0) hp[pt] += dt;
-                hp[pv] += dv;
-                finish(qp, kind, hv, hp);
+                if (pt >= 0) hp[pt] += dTip;
+                hp[pv] += dVip;
+                finish(qp, kind, hvp, hp);
             }
             if (hq) {
-                const double hv = inj_value<exact>(Q, Vi, &dv, &dt);
-                if (pt >= 0) hq[pt] += dt;
-                hq[pv] += dv;
-                finish(qq, kind, hv, hq);
+                if (pt >= 0) hq[pt] += dTiq;
+                hq[pv] += dViq;
+                finish(qq, kind, hvq, hq);
             }
         } else if (kind == 3) {  // P/Q flow; with its twin at the same end when qb >= 0
             const bool to_end = net.m_end[qa] != 0;
@@ -538,37 +536,42 @@ __global__ void __launch_bounds__(kBlock) k_evaluate_rows(DevNet net, DevWork w,
             const bool isq = (ty == 3 || ty == 8);
             const double Vi = w.v[loc];
             const double2 cs_i = w.bus_cs[loc];
-            InjSums S{};
+            // One sequence for P and Q: (A, D) = (gcbs, gsbc) or (gsbc, -gcbs)
+            double dVi = 0.0, dTi = 0.0;
             const int e0 = net.y_ptr[loc], e1 = net.y_ptr[loc + 1];
             {
                 const double G = __ldg(net.y_g + e0), B = __ldg(net.y_b + e0);  // the diagonal comes first
-                S.c = isq ? flip(B, true) : G;
-                S.d = isq ? G : B;
+                const double c = isq ? flip(B, true) : G;
+                hv = __dmul_rn(Vi * Vi, c);
+                dVi = __dmul_rn(2.0 * Vi, c);
+                if (!exact) dTi = __dmul_rn(Vi * Vi, isq ? G : B);
             }
             for (int e = e0 + 1; e < e1; ++e) {
                 const int j = __ldg(net.y_col + e);
                 const double G = __ldg(net.y_g + e), B = __ldg(net.y_b + e);
-                if (j == loc) {  // a branch that ends where it starts
-                    S.c = add_apart(S.c, isq ? flip(B, true) : G);
-                    S.d = add_apart(S.d, isq ? G : B);
-                    continue;
-                }
                 const double Vj = __ldg(w.v + j);
                 const int pt = __ldg(net.y_hpos_t + e), pv = __ldg(net.y_hpos_v + e);
-                double sn, cn;
-                angle_diff(cs_i, __ldg(w.bus_cs + j), &sn, &cn);
-                const double gc = G * cn + B * sn, gs = G * sn - B * cn;
-                const double A = isq ? gs : gc, vb = Vj * (isq ? flip(gc, true) : gs);
-                S.a += Vj * A;
-                S.b += vb;
-                if (pt >= 0) hrow[pt] += Vi * vb;
-                hrow[pv] += Vi * A;
+                if (j == loc) {  // a branch that ends where it starts
+                    const double c = isq ? flip(B, true) : G;
+                    hv = fma_apart(Vi * Vi, c, hv);
+                    dVi = fma_apart(2.0 * Vi, c, dVi);
+                    if (!exact) dTi = fma_apart(Vi * Vi, isq ? G : B, dTi);
+                    continue;
+                }
+                double s, c;
+                angle_diff(cs_i, __ldg(w.bus_cs + j), &s, &c);
+                const double gcbs = G * c + B * s, gsbc = G * s - B * c;
+                const double A = isq ? gsbc : gcbs, D = isq ? flip(gcbs, true) : gsbc;
+                const double vv = Vi * Vj, p = __dmul_rn(vv, D);
+                hv = __dadd_rn(hv, __dmul_rn(vv, A));
+                dVi = fma(Vj, A, dVi);
+                dTi = fma(isq ? vv : p, isq ? flip(D, true) : -1.0, dTi);
+                if (pt >= 0) hrow[pt] += p;
+                hrow[pv] += __dmul_rn(Vi, A);
             }
-            double dv, dt;
-            hv = inj_value<exact>(S, Vi, &dv, &dt);
             const int pt = net.y_hpos_t[e0];
-            if (pt >= 0) hrow[pt] += dt;
-            hrow[net.y_hpos_v[e0]] += dv;
+            if (pt >= 0) hrow[pt] += dTi;
+            hrow[net.y_hpos_v[e0]] += dVi;
         } else if (kind == 3) {  // P/Q flow
             const bool to_end = net.m_end[q] != 0;
             double sn, cn;
