@@ -245,7 +245,8 @@ SLE_API SLE_StatusCode SLE_CALL sle_ExBatchUpdateTelemetry(SLE_Handle handle, in
 SLE_API SLE_StatusCode SLE_CALL sle_ExBatchSolve(SLE_Handle handle, int32_t n, const int32_t* grids,
                                                  const uint8_t* flat_start, int32_t max_iterations, double tolerance,
                                                  int32_t robust, double huber_gamma, SLE_ExGridResult* results);
-/* |V| and theta of one grid (its n_bus values each; either may be NULL). */
+/* |V| and theta of one grid (its n_bus values each; either may be NULL).  A
+ * grid added since the last solve reads as its start state. */
 SLE_API SLE_StatusCode SLE_CALL sle_ExBatchGetState(SLE_Handle handle, int32_t grid, SLE_Real* v, SLE_Real* theta);
 /* Breaker edit: open (0) or close (1) branch `branch` of grid `grid`. */
 SLE_API SLE_StatusCode SLE_CALL sle_ExBatchSetBranchStatus(SLE_Handle handle, int32_t grid, int32_t branch,

@@ -1726,7 +1726,10 @@ int32_t Engine::download_results(int32_t what) {
     const DeviceScope dev_scope(cfg.device_id);
     what &= stale_;
     if (!uploaded_ || !what) return 0;
-    const int32_t n = model.n_bus(), m = model.n_meas(), nbr = model.n_branch();
+    // The device arrays are as long as at the last upload; the model may have
+    // grown (grids or elements added) or shrunk since.
+    const int32_t n = std::min(model.n_bus(), net_.n_bus), m = std::min(model.n_meas(), net_.n_meas),
+                  nbr = std::min(model.n_branch(), net_.n_branch);
     cudaError_t e = cudaSuccess;
     auto get = [&](double* dst, const double* src, int32_t cnt) {
         if (cnt > 0 && e == cudaSuccess) e = cudaMemcpyAsync(dst, src, sizeof(double) * cnt, cudaMemcpyDeviceToHost, st_);
@@ -2260,7 +2263,7 @@ int32_t Engine::batch_get_state(int32_t grid, double* v, double* th) {
         return -4;
     }
     const GridSpan& S = grids_[grid];
-    if (!uploaded_) {
+    if (!uploaded_ || S.bus0 + S.nbus > net_.n_bus) {  // not on the device (yet): its start or saved state
         if (v) std::memcpy(v, model.bus_v.data() + S.bus0, sizeof(double) * S.nbus);
         if (th) std::memcpy(th, model.bus_th.data() + S.bus0, sizeof(double) * S.nbus);
         return 0;
@@ -2268,8 +2271,9 @@ int32_t Engine::batch_get_state(int32_t grid, double* v, double* th) {
     // From the second grid read after a solve on, the whole batch's states come
     // in one copy to the host model and the next reads are served from it; one
     // grid read alone costs its own two copies.  Not in stream mode, whose
-    // states change step by step.
-    if (in_flight_.empty()) {
+    // states change step by step, nor once the host model's structure is no
+    // longer the uploaded one.
+    if (in_flight_.empty() && !model.structure_dirty) {
         if ((stale_ & DL_STATE) && ++batch_reads_ >= 2) {
             const int32_t rc = download_results(DL_STATE);
             if (rc) return rc;
