@@ -2501,19 +2501,25 @@ __device__ void front_bwd(const DevFactor& F, const FrontRec& R, const T* lx, co
 }
 
 template <typename T, typename V>
-__global__ void __launch_bounds__(kThreads) k_fwd(DevFactor F, const T* lx, const T* rdiag, SolveVecs sv,
+__global__ void __launch_bounds__(kThreads) k_fwd(DevFactor F, DevWork W, const T* lx, const T* rdiag, SolveVecs sv,
                                                   const int* fronts) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ T D[kTile * (kTile + 1)];
-    front_fwd<T, V>(F, lx, rdiag, sv, fronts[blockIdx.x], reinterpret_cast<V*>(smem_raw), D);
+    const int s = fronts[blockIdx.x];
+    if (front_frozen(F, W, s)) return;
+    front_fwd<T, V>(F, lx, rdiag, sv, s, reinterpret_cast<V*>(smem_raw), D);
 }
 
+// A frozen grid's sol holds its last solution, not y: the factorisation has
+// left its fronts out.
 template <typename T>
-__global__ void __launch_bounds__(kThreads) k_bwd(DevFactor F, const T* lx, const T* rdiag, SolveVecs sv, int maxf,
-                                                  int cap, const int* fronts) {
+__global__ void __launch_bounds__(kThreads) k_bwd(DevFactor F, DevWork W, const T* lx, const T* rdiag, SolveVecs sv,
+                                                  int maxf, int cap, const int* fronts) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     T* x = reinterpret_cast<T*>(smem_raw);
-    front_bwd<T>(F, F.rec[fronts[blockIdx.x]], lx, rdiag, sv, x, x + (maxf + 3) / 4 * 4, cap, [] { __syncthreads(); });
+    const FrontRec R = F.rec[fronts[blockIdx.x]];
+    if (front_frozen(W, R)) return;
+    front_bwd<T>(F, R, lx, rdiag, sv, x, x + (maxf + 3) / 4 * 4, cap, [] { __syncthreads(); });
 }
 
 // Forward sweep by continuation from the leaves (see continue_up).
@@ -2977,7 +2983,7 @@ cudaError_t solve_impl(const DevFactor& F, const DevWork& W, const LevelSchedule
     for (int l = 0; forward && l < ls.n_levels; ++l) {
         const int n = ls.h_all_ptr[l + 1] - ls.h_all_ptr[l];
         if (n > 0) {
-            k_fwd<T, T><<<n, kThreads, solve_smem<T>(ls.h_lvl_maxf[l]), st>>>(F, lx, rdiag, sv,
+            k_fwd<T, T><<<n, kThreads, solve_smem<T>(ls.h_lvl_maxf[l]), st>>>(F, W, lx, rdiag, sv,
                                                                                ls.d_all + ls.h_all_ptr[l]);
             count_launches(1);
         }
@@ -2986,7 +2992,7 @@ cudaError_t solve_impl(const DevFactor& F, const DevWork& W, const LevelSchedule
         const int n = ls.h_all_ptr[l + 1] - ls.h_all_ptr[l];
         if (n > 0) {
             const int mf = ls.h_lvl_maxf[l];
-            k_bwd<T><<<n, kThreads, bwd_smem<T>(mf, kBwdCap), st>>>(F, lx, rdiag, sv, mf, kBwdCap,
+            k_bwd<T><<<n, kThreads, bwd_smem<T>(mf, kBwdCap), st>>>(F, W, lx, rdiag, sv, mf, kBwdCap,
                                                                    ls.d_all + ls.h_all_ptr[l]);
             count_launches(1);
         }
