@@ -2152,6 +2152,7 @@ int32_t Engine::batch_solve(int32_t n, const int32_t* ids, const uint8_t* flat, 
     const SolveParams sp = params(rq);
     stale_ = DL_ALL;  // also when the solve ends in an error
     batch_reads_ = 0;
+    streaming_ = false;
     std::memset(h_batch_in_, 0, 2 * static_cast<size_t>(G));
     for (int32_t i = 0; i < n; ++i) {
         h_batch_in_[ids[i]] = 1;
@@ -2273,7 +2274,7 @@ int32_t Engine::batch_get_state(int32_t grid, double* v, double* th) {
     // grid read alone costs its own two copies.  Not in stream mode, whose
     // states change step by step, nor once the host model's structure is no
     // longer the uploaded one.
-    if (in_flight_.empty() && !model.structure_dirty) {
+    if (!streaming_ && !model.structure_dirty) {
         if ((stale_ & DL_STATE) && ++batch_reads_ >= 2) {
             const int32_t rc = download_results(DL_STATE);
             if (rc) return rc;
@@ -2337,6 +2338,7 @@ int32_t Engine::stream_begin(const SolveRequest& rq) {
     const int32_t G = static_cast<int32_t>(grids_.size());
     in_flight_.assign(G, 0);
     stream_iters_.assign(G, 0);
+    streaming_ = true;
     std::memset(h_batch_in_, 0, 3 * static_cast<size_t>(G));
     // every grid starts out of the batch
     cudaError_t e = cudaMemcpyAsync(const_cast<uint8_t*>(batch_.active), h_batch_in_, 3 * static_cast<size_t>(G),
@@ -2351,6 +2353,7 @@ int32_t Engine::stream_activate(int32_t n, const int32_t* ids, const uint8_t* fl
     const DeviceScope dev_scope(cfg.device_id);
     const int32_t G = static_cast<int32_t>(grids_.size());
     if (n <= 0) return 0;
+    streaming_ = true;
     std::memset(h_batch_in_, 0, 3 * static_cast<size_t>(G));
     for (int32_t i = 0; i < n; ++i) {
         const int32_t g = ids[i];

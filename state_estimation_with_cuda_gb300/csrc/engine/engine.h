@@ -329,6 +329,7 @@ private:
     SolveRequest stream_rq_{};
     std::vector<uint8_t> staged_;  // grids whose staged telemetry copy may still be running
     int32_t batch_reads_ = 0;      // grid states read since the last batch solve
+    bool streaming_ = false;       // stream mode since the last batch solve
     std::vector<uint8_t> in_flight_;
     std::vector<int32_t> stream_iters_;
     int32_t analyze_batch();

@@ -66,3 +66,15 @@ PROBE int32_t probe_solution(Engine* e, int32_t grid, double* out) {
     std::copy(x.begin(), x.end(), out);
     return 0;
 }
+// One grid through stream mode.
+PROBE int32_t probe_stream(Engine* e, int32_t grid, double tol) {
+    int32_t rc = e->stream_begin(request(20, tol));
+    if (rc == 0) rc = e->stream_activate(1, &grid, nullptr);
+    std::vector<int32_t> done;
+    std::vector<Engine::GridResult> res;
+    while (rc == 0 && done.empty()) rc = e->stream_step(done, res);
+    return rc;
+}
+PROBE int32_t probe_state(Engine* e, int32_t grid, double* v, double* th) { return e->batch_get_state(grid, v, th); }
+// Do reads come from the host model (one copy of the whole batch's states)?
+PROBE int32_t probe_reads_shared(Engine* e) { return (e->stale_ & Engine::DL_STATE) == 0; }

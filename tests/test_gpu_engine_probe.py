@@ -51,6 +51,14 @@ class Batch:
         assert self.lib.probe_solution(self.e, i, ptr(x)) == 0
         return x
 
+    def stream(self, i, tol=1e-6):
+        assert self.lib.probe_stream(self.e, i, ctypes.c_double(tol)) == 0
+
+    def state(self, i):
+        v, th = np.empty(self.grids[i].n_bus), np.empty(self.grids[i].n_bus)
+        assert self.lib.probe_state(self.e, i, ptr(v), ptr(th)) == 0
+        return np.concatenate([v, th])
+
     def close(self):
         self.lib.probe_delete(self.e)
 
@@ -71,3 +79,33 @@ def test_solution_of_a_finished_grid_stays(probe, mixed, dataflow):
         assert np.array_equal(b.solution(i), a.solution(0)), i
         a.close()
     b.close()
+
+
+def test_states_come_in_one_copy_again_after_stream_mode(probe):
+    """In stream mode each grid's state is read from the device, before and
+    after it from one copy of the batch's states; the values are those of the
+    grid alone each time."""
+    grids = [SyntheticGrid(n, int(round(1.4 * n)), 0x9700 + n) for n in (30, 71, 150)]
+    b = Batch(probe, grids, True, 1)
+    alone = [Batch(probe, [g], True, 1) for g in grids]
+
+    def check(shared):
+        for i, a in enumerate(alone):
+            assert np.array_equal(b.state(i), a.state(0)), i
+        assert probe.probe_reads_shared(b.e) == shared
+
+    b.solve([1, 1, 1])
+    [a.solve([1]) for a in alone]
+    check(1)
+    for i in (1, 0, 1):
+        b.stream(i, 1e-9)
+        alone[i].stream(0, 1e-9)
+        check(0)
+    b.solve([0, 1, 0])
+    [a.solve([f]) for a, f in zip(alone, (0, 1, 0))]
+    check(1)
+    b.stream(2, 1e-9)
+    alone[2].stream(0, 1e-9)
+    check(0)
+    b.close()
+    [a.close() for a in alone]
