@@ -190,7 +190,10 @@ SLE_API SLE_StatusCode SLE_CALL sle_ExTimer(SLE_Handle handle, int32_t op, doubl
 
 typedef struct SLE_ExStats {
     /* stages: 0 evaluate, 1 factorisation, 2 right-hand side, 3 solves,
-     * 4 state update, 5 final evaluation / other */
+     * 4 state update, 5 final evaluation / other.  A step that refactorises
+     * does its forward substitution in stage 1, and, unless enable_profiling
+     * is set, its right-hand side in that stage's first launch (stage 2 then
+     * counts the call but no launch). */
     int64_t launches[6];
     double ms[6];          /* CUDA-event time per stage (enable_profiling = 1) */
     int64_t calls[6];

@@ -1379,14 +1379,16 @@ int32_t Engine::enqueue_iteration(const SolveParams& sp, bool refactor, int64_t*
     };
     if (sched_.compact) stage(ST_OTHER, [&] { return launch_ready_compact(fac_, work_, sched_, st_); });
     stage(ST_EVALUATE, [&] { return launch_evaluate(net_, work_, sp, st_); });
-    // a refactorisation computes the right-hand side and takes it along (launch_factor)
-    if (!refactor) stage(ST_RHS, [&] { return launch_rhs(net_, fac_, work_, true, st_); });
+    // a refactorisation computes the right-hand side itself and takes it along
+    // (launch_factor); for the stage times it is a launch of its own (same bits)
+    const bool own_rhs = !refactor || cfg.enable_profiling != 0;
+    if (own_rhs) stage(ST_RHS, [&] { return launch_rhs(net_, fac_, work_, true, st_); });
     if (!mixed_) {
-        if (refactor) stage(ST_FACTOR, [&] { return launch_factor(net_, fac_, work_, sched_, true, st_); });
+        if (refactor) stage(ST_FACTOR, [&] { return launch_factor(net_, fac_, work_, sched_, !own_rhs, st_); });
         stage(ST_SOLVE, [&] { return launch_solve(fac_, work_, sched_, !refactor, st_); });
         stage(ST_UPDATE, [&] { return update(work_.sol); });
     } else {
-        if (refactor) stage(ST_FACTOR, [&] { return launch_factor32(net_, fac_, work_, sched_, true, st_); });
+        if (refactor) stage(ST_FACTOR, [&] { return launch_factor32(net_, fac_, work_, sched_, !own_rhs, st_); });
         stage(ST_SOLVE, [&] {
             cudaError_t ee = launch_solve32(fac_, work_, sched_, !refactor, st_);
             if (ee == cudaSuccess && cfg.refine_steps > 0) ee = launch_refine_begin(fac_, work_, st_);
