@@ -188,7 +188,7 @@ __device__ __forceinline__ void pivot_value(float d, float* sq, float* inv) {
     *inv = y;
 }
 __device__ __noinline__ double slow_sqrt(double d) { return sqrt(d); }
-__device__ __noinline__ double slow_recip(double d) { return 1.0 / d; }
+__device__ __noinline__ double slow_div(double a, double b) { return a / b; }
 __device__ __forceinline__ void pivot_value(double d, double* sq, double* inv) {
     if (in_fp32_range(d)) {
         const double y = widen_fp32(rsqrtf(leading_fp32(d)));
@@ -198,7 +198,7 @@ __device__ __forceinline__ void pivot_value(double d, double* sq, double* inv) {
         *inv = z;
     } else {
         *sq = slow_sqrt(d);
-        *inv = slow_recip(*sq);
+        *inv = slow_div(1.0, *sq);
     }
 }
 
@@ -761,21 +761,23 @@ __device__ void warp_front_factor(const DevFactor& F, const DevWork& W, const So
     if (lane < f) *rhs_entry<T>(sv, c0, nc, R.su_off, lane) = vi;
 }
 
-// 1 / d of a pivot, by the same means (y (1 + e + e^2), e = 1 - d y); a d
-// that is not positive and finite is replaced by 1 and reported.
-__device__ __forceinline__ double pivot_recip(double& d, bool& bad) {
+// u / d of an entry u and its column's pivot d: u times the reciprocal by the
+// same means (y (1 + e + e^2), e = 1 - d y).  Outside the FP32 range a division:
+// the reciprocal of a pivot below 2^-1024 is infinite.  A d that is not positive
+// and finite is replaced by 1 and reported.
+__device__ __forceinline__ double over_pivot(double u, double& d, bool& bad) {
     if (in_fp32_range(d)) {
         float yf;
         asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(yf) : "f"(leading_fp32(d)));
         const double y = widen_fp32(yf);
         const double e = fma(-d, y, 1.0);
-        return fma(y, fma(e, e, e), y);
+        return u * fma(y, fma(e, e, e), y);
     }
     if (!pivot_ok(d)) {
         bad = true;
         d = 1.0;
     }
-    return slow_recip(d);
+    return slow_div(u, d);
 }
 
 // Column counters of an elimination within one CTA: a column's owner raises
@@ -930,7 +932,7 @@ __device__ void front_factor(const DevFactor& F, const DevWork& W, const SolveVe
         auto publish = [&](double& aq, int k) {
             double d = __shfl_sync(0xffffffffu, aq, k);
             if (lane < nrow) P[lane + k * ldf] = aq;
-            sm.ms[k][lane] = aq * pivot_recip(d, bad);
+            sm.ms[k][lane] = over_pivot(aq, d, bad);
             if (k + 1 < kb) hand_over(k);
             if (lane == k) aq = d;
             if (lane == 0) sm.dk[k] = d;
@@ -1438,7 +1440,7 @@ __global__ void __launch_bounds__(kPanelThreads64, 2) k_big_panel64(DevFactor F,
 #pragma unroll 1
         for (int k = 0; k < pb; ++k) {
             double d = __shfl_sync(0xffffffffu, cur, k);
-            const double m = cur * pivot_recip(d, bad);
+            const double m = over_pivot(cur, d, bad);
             us[k][lane] = lane == k ? d : cur;
             ms[k][lane] = m;
             if (lane == 0) dk[k] = d;
