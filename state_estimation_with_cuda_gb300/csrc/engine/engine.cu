@@ -365,7 +365,6 @@ void Engine::build_schedule(bool targets_ready) {
     sch_step_ptr_.assign(nl + 1, 0);
     sch_all_ptr_.assign(nl + 1, 0);
     sch_maxf_.assign(nl, 0);
-    sch_maxpanel_.assign(nl, 0);
     sch_small_.clear();
     sch_all_.clear();
     sch_asm_.clear();
@@ -514,8 +513,6 @@ void Engine::build_schedule(bool targets_ready) {
             lvl_of[s] = l;
             sch_all_.push_back(s);
             sch_maxf_[l] = std::max(sch_maxf_[l], P.sn_f[s]);
-            sch_maxpanel_[l] = std::max<int64_t>(sch_maxpanel_[l],
-                                                 static_cast<int64_t>(P.sn_f[s]) * (P.sn_c0[s + 1] - P.sn_c0[s]));
             if (flow_phase_[s] == 1) flow_a_maxf_ = std::max(flow_a_maxf_, P.sn_f[s]);
             if (flow_phase_[s] == 2) flow_b_maxf_ = std::max(flow_b_maxf_, P.sn_f[s]);
         }
@@ -802,15 +799,12 @@ int32_t Engine::upload() {
         fac_.sn_c0 = c.take<int32_t>(ns + 1);
         fac_.sn_f = c.take<int32_t>(ns);
         fac_.sn_parent = c.take<int32_t>(ns);
-        fac_.sn_rows_off = c.take<int64_t>(ns + 1);
         fac_.sn_rows = c.take<int32_t>(P.sn_rows.size());
         fac_.sn_lx_off = c.take<int64_t>(ns + 1);
-        fac_.sn_u_off = c.take<int64_t>(ns + 1);
         fac_.sn_su_off = c.take<int64_t>(ns + 1);
         fac_.sn_child_ptr = c.take<int32_t>(ns + 1);
         fac_.sn_child = c.take<int32_t>(P.sn_child.size());
         fac_.sn_relmap = c.take<int32_t>(P.sn_relmap.size());
-        fac_.sn_tgt_ptr = c.take<int32_t>(ns + 1);
         fac_.tgt_local = c.take<int32_t>(P.tgt_local.size());
         fac_.tgt_pair_ptr = c.take<int64_t>(P.tgt_pair_ptr.size());
         fac_.pair_a = c.take<int32_t>(P.pair_a.size());
@@ -819,8 +813,6 @@ int32_t Engine::upload() {
         fac_.rhs_h = c.take<int32_t>(P.rhs_h.size());
         fac_.bus_ps_theta = c.take<int32_t>(n);
         fac_.bus_ps_v = c.take<int32_t>(n);
-        fac_.sn_u_ld = c.take<int32_t>(ns);
-        fac_.sn_u_big = c.take<uint8_t>(ns);
         fac_.sn_pw = c.take<int8_t>(ns);
         fac_.rec = c.take<FrontRec>(ns);
         fac_.child_rec = c.take<ChildRec>(P.sn_child.size());
@@ -1010,15 +1002,12 @@ int32_t Engine::upload() {
     chk(put(const_cast<int32_t*>(fac_.sn_c0), P.sn_c0, st_));
     chk(put(const_cast<int32_t*>(fac_.sn_f), P.sn_f, st_));
     chk(put(const_cast<int32_t*>(fac_.sn_parent), P.sn_parent, st_));
-    chk(put(const_cast<int64_t*>(fac_.sn_rows_off), P.sn_rows_off, st_));
     chk(put(const_cast<int32_t*>(fac_.sn_rows), P.sn_rows, st_));
     chk(put(const_cast<int64_t*>(fac_.sn_lx_off), lay_lx_off_, st_));
-    chk(put(const_cast<int64_t*>(fac_.sn_u_off), lay_u_off_, st_));
     chk(put(const_cast<int64_t*>(fac_.sn_su_off), P.sn_su_off, st_));
     chk(put(const_cast<int32_t*>(fac_.sn_child_ptr), P.sn_child_ptr, st_));
     chk(put(const_cast<int32_t*>(fac_.sn_child), P.sn_child, st_));
     chk(put(const_cast<int32_t*>(fac_.sn_relmap), P.sn_relmap, st_));
-    chk(put(const_cast<int32_t*>(fac_.sn_tgt_ptr), P.sn_tgt_ptr, st_));
     chk(put(const_cast<int32_t*>(fac_.tgt_local), P.tgt_local, st_));
     chk(put(const_cast<int64_t*>(fac_.tgt_pair_ptr), P.tgt_pair_ptr, st_));
     chk(put(const_cast<int32_t*>(fac_.pair_a), P.pair_a, st_));
@@ -1027,8 +1016,6 @@ int32_t Engine::upload() {
     chk(put(const_cast<int32_t*>(fac_.rhs_h), P.rhs_h, st_));
     chk(put(const_cast<int32_t*>(fac_.bus_ps_theta), P.bus_ps_theta, st_));
     chk(put(const_cast<int32_t*>(fac_.bus_ps_v), P.bus_ps_v, st_));
-    chk(put(const_cast<int32_t*>(fac_.sn_u_ld), lay_u_ld_, st_));
-    chk(put(const_cast<uint8_t*>(fac_.sn_u_big), lay_u_big_, st_));
     chk(put(const_cast<int32_t*>(fac_.asm_ptr), asm_ptr_, st_));
     chk(put(const_cast<int2*>(fac_.asm_ent), asm_ent_, st_));
     std::vector<FrontRec> recs(ns);
@@ -1183,7 +1170,6 @@ int32_t Engine::upload() {
     sched_.h_all_ptr = sch_all_ptr_.data();
     sched_.d_all = d_all_;
     sched_.h_lvl_maxf = sch_maxf_.data();
-    sched_.h_lvl_maxpanel = sch_maxpanel_.data();
     {
         const int32_t ms = max_solve_front();
         FlowGrids g = flow_grids(mixed_, flow_a_maxf_, flow_b_maxf_, ms, down_maxf_);

@@ -281,7 +281,6 @@ private:
     // FP32 tiled fronts as dataflow items (TileTask), per level
     std::vector<TileTask> sch_tt_;
     std::vector<int32_t> sch_tt_ptr_;
-    std::vector<int64_t> sch_maxpanel_;
     std::vector<int32_t> sch_flow_a_, sch_flow_b_, sch_down_, sch_down_top_, sch_up_, sch_flow_w_, sch_down_w_, phase_nchild_, nchild_;
     std::vector<char> flow_phase_;
     int32_t sync_by_depth_ = 0;

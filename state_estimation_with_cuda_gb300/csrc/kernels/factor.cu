@@ -1206,16 +1206,15 @@ __device__ __forceinline__ int claim(int* counter, int* slot) {
     return *slot;
 }
 
-// After front s is complete (all threads past a barrier): thread 0 counts s
-// into its parent's completed children; the CTA that completes the last child
-// of a parent handled by the same sweep (phase[p] == ph, or every front when
-// phase is null) continues with that parent.  Returns the next front or -1.
-__device__ __forceinline__ int continue_up(const DevFactor& F, const int8_t* phase, int ph, const int32_t* nchild,
-                                           int* cnt, int s, int* slot) {
+// Forward sweep, after front s is complete (all threads past a barrier): thread 0
+// counts s into its parent's completed children; the CTA that completes the
+// last child of a parent continues with that parent.  Returns the next front
+// or -1.
+__device__ __forceinline__ int continue_up(const DevFactor& F, const int32_t* nchild, int* cnt, int s, int* slot) {
     if (threadIdx.x == 0) {
         int nxt = -1;
         const int p = F.sn_parent[s];
-        if (p >= 0 && (phase == nullptr || phase[p] == ph)) {
+        if (p >= 0) {
             __threadfence();
             if (atomicAdd(cnt + p, 1) + 1 == nchild[p]) {
                 __threadfence();
@@ -2540,7 +2539,7 @@ __global__ void __launch_bounds__(kThreads) k_fwd_flow(DevFactor F, DevWork W, c
         while (s >= 0) {
             if (!front_frozen(F, W, s)) front_fwd<T, V>(F, lx, rdiag, sv, s, reinterpret_cast<V*>(smem_raw), D);
             __syncthreads();
-            s = continue_up(F, nullptr, 0, nchild, cnt, s, &slot);
+            s = continue_up(F, nchild, cnt, s, &slot);
         }
     }
 }

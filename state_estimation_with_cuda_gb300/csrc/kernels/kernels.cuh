@@ -101,7 +101,10 @@ struct __align__(16) FrontRec {
 // A child as its parent's assembly reads it.
 struct __align__(16) ChildRec {
     int64_t u_off, su_off;
-    int32_t m, ld, big, pad;  // update matrix: m x m, leading dimension, in the factor array (big) or u
+    // update matrix, m x m with leading dimension ld: a block of its own in u
+    // (single-CTA fronts, ld = m) or, big, in place in its front's f x f region
+    // of the factor array (tiled fronts, ld = f)
+    int32_t m, ld, big, pad;
 };
 // Warps of a single-CTA front's CTA (wide: phase B and the synchronous levels).
 __host__ __device__ constexpr int asm_warps(bool fp32, bool wide) { return fp32 && wide ? 16 : 8; }
@@ -112,15 +115,12 @@ struct DevFactor {
     const int32_t* sn_c0;
     const int32_t* sn_f;
     const int32_t* sn_parent;
-    const int64_t* sn_rows_off;
     const int32_t* sn_rows;
     const int64_t* sn_lx_off;
-    const int64_t* sn_u_off;
     const int64_t* sn_su_off;
     const int32_t* sn_child_ptr;
     const int32_t* sn_child;
     const int32_t* sn_relmap;
-    const int32_t* sn_tgt_ptr;
     const int32_t* tgt_local;
     const int64_t* tgt_pair_ptr;
     const int32_t* pair_a;
@@ -129,11 +129,6 @@ struct DevFactor {
     const int32_t* rhs_h;
     const int32_t* bus_ps_theta;
     const int32_t* bus_ps_v;
-    // update-matrix leading dimension and location: small fronts keep a
-    // compact (f-nc)^2 block in the update array; big fronts keep it in place
-    // inside their f x f region of the factor array (sn_u_big = 1, ld = f)
-    const int32_t* sn_u_ld;
-    const uint8_t* sn_u_big;
     const int32_t* sn_grid;  // batch: grid of each front (nullptr for one grid)
     const int32_t* tgt_grid; // batch: grid of each gain target
     const int32_t* ps_grid;  // batch: grid of each permuted state
@@ -346,7 +341,6 @@ struct LevelSchedule {
     const int32_t* h_all_ptr = nullptr;     // [n_levels+1] offsets into d_all
     const int32_t* d_all = nullptr;         // every front, per level (solves)
     const int32_t* h_lvl_maxf = nullptr;    // [n_levels] largest front per level
-    const int64_t* h_lvl_maxpanel = nullptr;  // [n_levels] largest f * nc per level
     // dataflow phases of the factorisation (fronts below every big front):
     // A = fronts whose whole subtree has f <= flow_small_f, B = the rest.  A
     // CTA claims an initially ready front of its phase (no children in the
