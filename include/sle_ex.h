@@ -60,7 +60,7 @@ SLE_API SLE_StatusCode SLE_CALL sle_ExLoadNetwork(SLE_Handle handle, int32_t n_b
  *                           factorised and solved one per warp: 1 on, 0 off,
  *                           -1 (default) for each grid that has such fronts
  *                           (re-uploads)
- *   "spin_limit"            polls (about 64 ns each) after which a dataflow
+ *   "spin_limit"            polls (about 0.5 us each) after which a dataflow
  *                           wait of the solves gives up; the call then fails
  *                           with SLE_ERROR_CUDA_FAILURE and the message
  *                           "factorisation dataflow wait timed out" instead
@@ -86,9 +86,9 @@ SLE_API SLE_StatusCode SLE_CALL sle_ExLoadNetwork(SLE_Handle handle, int32_t n_b
  *                           of each synchronous level in one persistent
  *                           dataflow launch (panel chunks and update tiles
  *                           as items that wait, bounded, for their inputs);
- *                           0 (default): a panel launch and an update launch
- *                           per 32-column step.  Same arithmetic, same bits
- *                           (re-uploads)
+ *                           0 (default): one launch per 32-column step, its
+ *                           update and the next panel.  Same arithmetic, same
+ *                           bits (re-uploads)
  *   "device_loop"           batch solves: 1 (default) runs the Gauss-Newton
  *                           loop on the device, as a CUDA graph whose
  *                           conditional while node repeats one step while

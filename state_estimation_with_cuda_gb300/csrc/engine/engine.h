@@ -43,7 +43,7 @@ struct EngineConfig {
     double big_front_flops = 1.0e5;  // FP64: fronts above this many factor flops use the tiled multi-CTA path
     int32_t refine_steps = 0;        // mixed precision: extra refinement steps per Gauss-Newton step
     int32_t dataflow = 1;            // persistent dataflow kernels below the big fronts and for the solves
-    int32_t flow_small_f = 0;        // widest front of the high-occupancy dataflow phase (<= kFlowSmallFMax;
+    int32_t flow_small_f = 0;        // widest front of dataflow phase A (<= kFlowSmallFMax;
                                      // 0: 128)
     int32_t warp_fronts = -1;        // warp phase for fronts whose subtree is at most kWarpFrontMax wide:
                                      // 1 on, 0 off, -1 per grid with at least kWarpPhaseMinFronts of them
@@ -54,8 +54,8 @@ struct EngineConfig {
                                      // than this fraction in an iteration (0: the reference's test only)
     int32_t hold_front = -1;         // test hook: front whose backward-sweep completion is withheld
     int32_t eval_pair_rows = 1 << 18;  // evaluation: a P row and its Q twin share one thread from this many rows
-    int32_t tile_flow = 0;           // FP32 tiled fronts: 1 = one dataflow launch per level; 0 = a panel and
-                                     // an update launch per step (faster on the measured grids)
+    int32_t tile_flow = 0;           // FP32 tiled fronts: 1 = one dataflow launch per level; 0 = one launch
+                                     // per step (faster on the measured grids)
     int32_t device_loop = 1;         // batch solves: Gauss-Newton loop in a conditional graph node (needs
                                      // use_cuda_graphs and no profiling); 0: one host round trip per step
 };
@@ -306,7 +306,7 @@ private:
     int8_t* d_phase_ = nullptr;
     int32_t* d_phase_nchild_ = nullptr;
     int32_t* d_nchild_ = nullptr;
-    int32_t* d_ready_n_ = nullptr;               // [4] claim-list lengths
+    int32_t* d_ready_n_ = nullptr;               // [kReadyLists] claim-list lengths
     int32_t* d_pot_cnt_ = nullptr;               // tiled fronts: per (front, step) tile readers
     TileTask* d_tt_ = nullptr;
     int32_t* d_tt_done_ = nullptr;
@@ -322,7 +322,7 @@ private:
     std::vector<GridSpan> grids_;
     std::vector<Plan> grid_plans_;
     DevBatch batch_{};
-    uint8_t* h_batch_in_ = nullptr;   // pinned [2 * G]: active, flat
+    uint8_t* h_batch_in_ = nullptr;   // pinned [3 * G]: active, flat, retire
     void* h_batch_out_ = nullptr;     // pinned: flags, iters, mismatch, objective, running
     size_t h_batch_cap_ = 0;
     SolveRequest stream_rq_{};
@@ -359,7 +359,7 @@ private:
     };
     IterGraph graphs_[2];
     // Batch solve's whole Gauss-Newton loop: a conditional while node whose
-    // body is one step (with refactorisation) and the loop-control kernel.
+    // body is one step (with refactorisation), whose update sets the condition.
     IterGraph loop_graph_;
     void drop_graphs();
     // loop: the while node of a device-run loop whose body the step is; without

@@ -13,10 +13,12 @@
 // Small fronts (little work) are one CTA each with the whole front in shared
 // memory.  Big fronts live in place in an f x f region (L panel = first nc
 // columns, update matrix = trailing block, both column-major with ld = f) and
-// are processed for a whole level at once by tile work lists: an assembly
-// kernel (one CTA per 32-column tile column, so every entry has one writer), a
-// panel kernel (each CTA factors the 32 x 32 diagonal tile and solves a chunk
-// of rows against it) and a trailing-update kernel (one CTA per tile).
+// are processed for a whole level at once by work lists: an assembly kernel
+// (one CTA per 32-column tile column and block of rows, so every entry has one
+// writer), then per 32-column step a panel (each CTA factors the diagonal block
+// and solves a chunk of rows against it) and the trailing update (one CTA per
+// tile): FP64 in two launches a step, FP32 in one that does a step's update and
+// the next step's panel, after a panel launch for the first.
 // The factor type T is double for the FP64 pipeline and float for the
 // mixed-precision one; the mixed pipeline forms the gain entries' sums in
 // float (gain_acc32, the default) or in double.
@@ -332,11 +334,11 @@ __device__ __forceinline__ void extend_add_children(const DevFactor& F, const So
 // (front_ld), so four consecutive rows of a column are one or two aligned
 // vector loads.  The FP32 partial factorisation runs over panels (FP64: see
 // front_factor):
-//   (1) warp 0 factors the diagonal block in registers (lane i holds row i,
-//       columns broadcast by shuffles) and leaves L11^T and 1/diag in shared
-//       memory;
-//   (2) every thread solves one row of the panel below the block,
-//       x = a L11^-T, by forward substitution in registers;
+//   (1) warp 0 factors the diagonal block (warp_potrf) and leaves L11^T and
+//       1/diag in shared memory;
+//   (2) warp 0 inverts the block (warp_trinv) while every other thread solves
+//       one row of the panel below it, x = a L11^-T, by forward substitution
+//       (row_trsm);
 //   (3) the trailing lower triangle is updated by 4x4 register tiles,
 //       A22 -= X X^T, two vector loads and sixteen FMAs per panel column.
 // ---------------------------------------------------------------------------
@@ -1145,9 +1147,13 @@ __device__ void front_factor(const DevFactor& F, const DevWork& W, const SolveVe
     front_store<T>(sv, lx, ub, R, Fm, sm.v, 1);
 }
 
-// Panel widths: fronts of the high-occupancy dataflow phase (f <= 64) use
-// 16-column panels and a register budget for several CTAs per SM; the rest
-// use 32-column panels and the full register file (one CTA per SM anyway).
+// Panel widths: fronts of dataflow phase A (f <= kFlowSmallFMax) use 16-column
+// panels and a register budget for several CTAs per SM; the rest use 32-column
+// panels and the full register file (one CTA per SM anyway).  A launch's CTAs
+// take the shared memory of its widest front (FP64, 128 rows: 135 KB, one CTA
+// per SM), so the budget pays where a phase's fronts are narrow: 64 grids of 30
+// to 5000 buses FP64 8.49 ms a pass with it, 8.87 without; single grids of 2000
+// to 60k buses the same either way.
 constexpr int kPanelSmall = kPanelFlowA;
 template <typename T>
 constexpr int kMinBlocksA = sizeof(T) == 4 ? 3 : 2;
@@ -1254,7 +1260,7 @@ __global__ void __launch_bounds__(kFrontThreads<T, KP>, kMinBlocks) k_front_flow
 
 // ---------------------------------------------------------------------------
 // Big fronts, in place (L panel and update matrix share the f x f region at
-// sn_lx_off with ld = f).  Work lists hold int4 (front, a, b, 0).
+// sn_lx_off with ld = f).  Work lists: LevelSchedule.
 // ---------------------------------------------------------------------------
 // Assembly of a tiled front, one CTA per (tile column tj, block rb of
 // kAsmRows rows from the tile's first column down): the block's G entries, then
@@ -1541,10 +1547,9 @@ __device__ __forceinline__ T ld_entry(const T* p) {
 }
 
 // FP32 panel step p of the tiled fronts.  The rows below the diagonal block
-// are cut into chunks of kPanelRows, one CTA each.  Every CTA
-// factors the 32 x 32 diagonal block itself (warp 0, in registers) and
-// inverts it while the other warps stage the chunk's rows of the panel; then
-// it solves the chunk as X = A L_dd^-T = A (L_dd^-1)^T, a register-tiled
+// are cut into chunks of kPanelRows, one CTA each.  Every CTA stages the block
+// and its chunk, factors the 32 x 32 diagonal block itself and inverts it (warp
+// 0), and solves the chunk as X = A L_dd^-T = A (L_dd^-1)^T, a register-tiled
 // product with 4 x 4 outputs per thread.  The CTA that reads the diagonal
 // tile last (a counter per front and step) writes L_dd^-1 into it for the
 // solves: no CTA reads an overwritten tile, and none waits for another.
@@ -1773,8 +1778,10 @@ __device__ __forceinline__ void big_update_item(const DevFactor& F, const DevWor
 // block is updated and factored by every chunk's CTA, and the one that has read
 // it last (a counter per front and step) writes L_dd^-1 into its slot.  The
 // other tiles are plain updates.  Bound: the chain of load latency, the block's
-// 32 pivots and its inverse.  Measured at 200k buses: 10.2 us a step, where the
-// update and the next panel as two launches took 11.0 + 5.1 us and two gaps.
+// 32 pivots and its inverse.  Measured at 200k buses: 9.9 us a step, where the
+// update (with the next diagonal block's factorisation in it) and the next panel
+// as two launches took 11.3 + 4.7 us and two gaps.  (64 registers and 24 bytes of
+// spills a thread.)
 constexpr int kStepLd = kTile + 4, kStepRows = kPanelRows + 4;  // 16-byte aligned rows
 struct StepPanelSmem {
     float xd[kTile * kStepLd];    // [k][r]: panel p, rows of the next diagonal block
@@ -2388,8 +2395,10 @@ constexpr size_t bwd_smem(int maxf, int cap) {
     return sizeof(T) * ((size_t)(maxf + 3) / 4 * 4 + 2 * ((size_t)kStageD + cap));
 }
 // Stage capacities.  The narrow fronts' launch wants many CTAs per SM (their
-// blocks hold a few hundred entries); the wide fronts' one, few and long, takes
-// what shared memory holds, up to a whole 32-column block.
+// blocks hold a few hundred entries; the line is flat: with 1024 or 4096 whole
+// passes at 10k, 60k and 200k buses and of batches take the same within 0.5 %, or
+// within the spread of runs, 1.3 % for 512 grids); the wide fronts' one, few and
+// long, takes what shared memory holds, up to a whole 32-column block.
 constexpr int kBwdCap = 2048;
 constexpr size_t kBwdSmemMax = 200 * 1024;
 template <typename T>
@@ -2575,11 +2584,10 @@ __global__ void __launch_bounds__(kThreads) k_bwd_flow(DevFactor F, DevWork W, c
 // Warp fronts: a front whose whole subtree is at most kWarpFrontMax wide is
 // handled by one warp (eight fronts per CTA, no block barriers).  Factor: the
 // front is assembled in the warp's tile in shared memory (original entries,
-// then the children's update matrices in child order), loaded row per lane
-// into registers and partially factorised there (the first nc pivots, which
-// also leave the Schur complement in the trailing columns), then L (FP32:
-// with L11^-1 in its diagonal block) and the update matrix are written out.
-// Solves: the forward and backward steps of the same fronts, a lane per row.
+// then the children's update matrices in child order) and partially factorised
+// there, left-looking (warp_front_factor); L (FP32: with L11^-1 in its diagonal
+// block) and the update matrix are written out.  Solves: the forward steps of
+// the same fronts, a lane per row, and the backward ones, a lane per column.
 // A warp continues with the parent when it completes the parent's last child
 // in the same phase, as the CTA sweeps do.
 // ---------------------------------------------------------------------------
