@@ -175,17 +175,23 @@ def load_peaks():
         return 6800.0, "fallback"
 
 
-def profile_traffic(kernel):
-    """DRAM bytes per launch from a committed ncu summary, if one exists."""
+def profile_line(kernel, key):
+    """The line `key: value` of a committed ncu summary, if there is one."""
     path = os.path.join(REPO, "profiles", "%s.md" % kernel)
     try:
         with open(path) as fh:
             for line in fh:
-                if line.strip().startswith("traffic_bytes_per_launch:"):
-                    return float(line.split(":", 1)[1])
+                if line.strip().startswith(key + ":"):
+                    return line.split(":", 1)[1].strip()
     except OSError:
         pass
     return None
+
+
+def profile_traffic(kernel):
+    """DRAM bytes per launch from a committed ncu summary, if one exists."""
+    v = profile_line(kernel, "traffic_bytes_per_launch")
+    return None if v is None else float(v)
 
 
 def stage_bytes(info, g, vb=8):
@@ -321,6 +327,7 @@ def roofline(leg, g, mixed):
         kernel = "union_" + kernel
     return {"bound": "hbm", "kernel": kernel, "achieved": round(achieved, 2), "peak": peak, "peak_kind": peak_kind,
             "unit": "GB/s", "frac": round(achieved / peak, 5), "traffic": profile_traffic(kernel),
+            "traffic_note": profile_line(kernel, "traffic_note"),
             "algorithmic_bytes_per_call": int(sb[dom])}
 
 
@@ -547,7 +554,7 @@ def run_batch512():
                                              "iterations_mean": round(float(np.mean(its)), 3),
                                              "iterations_max": int(max(its))}
     out["config"] = ("512 grids, log-uniform 30..5000 buses (%d buses, %d rows); hot start after a 1%% re-noise; "
-                     "size buckets %s (one batch each, solved concurrently), phase-A width %s (mixed; FP64 64); "
+                     "size buckets %s (one batch each, solved concurrently), phase-A width %s (mixed; FP64 the default); "
                      "wall clock including the telemetry copies"
                      % (sum(g.n_bus for g in grids), sum(g.n_meas for g in grids), list(bounds) or "[all]",
                         width or 64))
@@ -854,7 +861,8 @@ def run_gb300(args, world, rank, local):
             "clocks": sm["clk"],
         }
         if union:
-            out["roofline"] = {k: union[k] for k in ("bound", "kernel", "achieved", "peak", "unit", "frac", "traffic")}
+            out["roofline"] = {k: union[k] for k in ("bound", "kernel", "achieved", "peak", "unit", "frac", "traffic",
+                                                     "traffic_note")}
             out["roofline"]["workload"] = "one loaded Gauss-Newton pass of the 512-grid batch (factorisation stage)"
     return out, stream, (lo, hi)
 
